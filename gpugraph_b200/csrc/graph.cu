@@ -98,8 +98,14 @@ int ensure_multi(mg_graph *g) {
     cudaError_t e = cudaMemcpy(off.data(), g->csr.csc_offsets, (V + 1) * 4, cudaMemcpyDeviceToHost);
     if ((st = cuda_status(e, "in-list lengths")) != MG_OK) return st;
     std::vector<int32_t> heavy;
-    for (size_t v = 0; v < V; ++v)
+    size_t hub = 0;
+    for (size_t v = 0; v < V; ++v) {
       if (off[v + 1] - off[v] > kMsHeavyList) heavy.push_back((int32_t)v);
+      if (off[v + 1] - off[v] > off[hub + 1] - off[hub]) hub = v;
+    }
+    const double mean = std::max(1.0, (double)g->edges / (double)V);
+    g->mss_hub = (double)(off[hub + 1] - off[hub]) > kMssSkew * mean ? (int32_t)hub : -1;
+    if ((st = device_alloc(g, (void **)&g->mss_offs, 67 * 4)) != MG_OK) return st;
     std::stable_sort(heavy.begin(), heavy.end(),
                      [&](int32_t x, int32_t y) { return off[x + 1] - off[x] > off[y + 1] - off[y]; });
     if ((st = device_alloc(g, (void **)&g->ms_heavy, std::max<size_t>(heavy.size(), 1) * 4)) != MG_OK) return st;

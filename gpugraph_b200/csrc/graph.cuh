@@ -33,6 +33,9 @@ constexpr uint32_t kMsStackLevels = 16;
 // In-lists longer than this are pulled by a warp of their own in a batched BFS
 // pull level (a 32-vertex group holding one would carry most of a warp's work).
 constexpr int32_t kMsHeavyList = 512;
+// A batched SSSP keeps edge bounds (multi.cu) where the longest in-list is this
+// many times the mean.
+constexpr double kMssSkew = 64.0;
 
 struct DevCsr {
   int32_t *row_offsets = nullptr;
@@ -104,6 +107,8 @@ struct mg_graph {
   uint32_t *multi_stk_bm = nullptr;     // [kMsStackLevels][V/32] valid entries of push-made stack levels
   int32_t *ms_heavy = nullptr;          // vertices with more than kMsHeavyList in-edges, longest first
   int32_t ms_nheavy = -1;               // their number (-1: not built yet)
+  int32_t *mss_offs = nullptr;          // batched SSSP: offsets of the edge bounds (multi.cu)
+  int32_t mss_hub = -1;                 // the vertex they are measured at, -1: the graph is not skewed
   int32_t *multi_stage = nullptr;       // [64][V] transposed results on their way to host memory
   size_t multi_bytes = 0;
   // PageRank plan (built on first mg_pagerank): heavy in-lists split into

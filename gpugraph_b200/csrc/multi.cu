@@ -28,12 +28,12 @@
 // BFS levels switch between push (the GAS engine's load-balanced expand with
 // an OR-into-mask Program, next frontier as a vertex queue) and pull (every
 // vertex still missing sources ORs its in-neighbours' frontier masks, stopping
-// as soon as every missing source is found). SSSP relaxes warp-per-edge:
-// lane l owns sources l and l+32, so one edge reads the two 256-byte distance
-// rows with coalesced loads and atomicMin's only improved entries.
+// as soon as every missing source is found). SSSP levels relax the edges of the
+// improved vertices in vertex order (k_mss_scan, k_mss_bounds, k_mss_expand).
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 #include <cstring>
 #include <type_traits>
 #include <vector>
@@ -48,11 +48,18 @@ namespace mg {
 typedef unsigned long long u64;
 constexpr int kMVTS = 4;
 constexpr int kMVT = 8;
-// Batched SSSP relaxes four edges per warp step (each 512 bytes of distance
-// rows), so its expand tiles are the smallest the workspace allows (1024
-// items): more CTAs share a level's edges.
+// A batched SSSP edge costs up to 512 bytes of distance rows, so its expand
+// tiles are the smallest the workspace allows (1024 items): more CTAs share a
+// level's edges.
 constexpr int kMSVT = 4;
-constexpr int kMssSparse = 24; // active sources per edge up to which a lane relaxes a whole edge alone
+// Edges whose row loads a warp has in flight (R-MAT 20, 37 sources: 4.9 ms with
+// 8, 5.1 with 16, 5.1 with 4 and the tails' rows held in registers).
+constexpr int kMssEdges = 8;
+// Active sources per edge up to which a lane relaxes a whole edge alone: below,
+// the row accesses of a warp-wide edge carry mostly inactive entries, above, the
+// lane's scalar loads touch a sector per source (R-MAT 20, 37 sources / road
+// 1200, 64 sources: 5.1 / 26.2 ms at 4, 4.9 / 23.8 at 12, 5.5 / 24.5 at 24).
+constexpr int kMssSparse = 12;
 
 // Push step of the batched BFS as a GAS Program: expand_edge emits the
 // sources that reach the neighbour for the first time, contract ORs them into
@@ -118,6 +125,7 @@ struct MultiArgs {
   uint32_t *bm0, *bm1;
   unsigned long long *status;
   Ctl *ctl;
+  int32_t *mss_offs;  // batched SSSP: the edge bounds' offsets (MssBounds)
   u64 all;  // mask of the sources in use
 };
 
@@ -151,6 +159,11 @@ struct SrcList {
   float alpha, beta;
 };
 
+// The mask bit of source s in a batched SSSP, and back: the two sources of a
+// row pair are the two bits of one lane (k_mss_expand).
+MG_DEVINL int mss_bit(int s) { return (s >> 1) + 32 * (s & 1); }
+MG_DEVINL int mss_source(int bit) { return 2 * (bit & 31) + (bit >> 5); }
+
 // Level-0 state of a batched run (one CTA of 64 threads).
 // bfs: 0 = SSSP (int32 rows), 1 = BFS with int32 depth rows, 2 = BFS with the
 // level stack and uint16 rows.
@@ -158,7 +171,7 @@ __global__ void k_ms_init(MultiArgs a, SrcList L, int bfs) {
   const int t = threadIdx.x;
   if (t < L.nsrc) {
     const int v = L.src[t];
-    atomicOr(&a.F0[v], 1ull << t);
+    atomicOr(&a.F0[v], 1ull << (bfs ? t : mss_bit(t)));
     if (bfs) atomicOr(&a.visit[v], 1ull << t);
     if (bfs == 0) a.out[(int64_t)v * 64 + t] = 0;
     else if (bfs == 1) depth_rows<int32_t>(a)[(int64_t)v * 64 + t] = 0;
@@ -173,6 +186,12 @@ __global__ void k_ms_init(MultiArgs a, SrcList L, int bfs) {
       stk_level(a, 0)[v] = m;
       atomicOr(&a.stk_bm[v >> 5], 1u << (v & 31));
     }
+  }
+  if (!bfs) {
+    if (t < L.ndistinct) atomicOr(&a.bm0[L.distinct[t] >> 5], 1u << (L.distinct[t] & 31));
+    a.mss_offs[t] = 0;
+    if (t < 2) a.mss_offs[64 + t] = 0;
+    if (t == 2) a.mss_offs[66] = L.nsrc;
   }
   if (t == 0 && bfs) {
     a.ctl->srcmask[0] = a.all;
@@ -1071,31 +1090,188 @@ __global__ void k_ms_mask_stats(const u64 *visit, u64 all, const int32_t *ro, in
 }
 
 // ------------------------------------------------------------ batched SSSP --
-struct mssp_scan {
-  typedef int DataType;
-  typedef int MiscType;
-  typedef int GatherType;
-  typedef int VertexId;
-  typedef int SizeT;
-  struct VertexType {
-    int nodes;
-  };
-  struct EdgeType {
-    int nodes;
-  };
-  struct expand_vertex {
-    __device__ bool operator()(const int, const char, VertexType &, EdgeType &) { return true; }
-  };
-};
-
-// Clears the previous level's masks (they were read by the previous expand).
-__global__ void __launch_bounds__(kNT) k_mss_clear(MultiArgs a) {
+// Start of a level: the frontier's vertices (the bits the previous expand set)
+// in vertex order into the queue, with the exclusive prefix of their degrees and
+// the merge-path tile partitions of k_mss_expand (as k_frontier_scan makes them
+// from a queue); the bitmap words are cleared on the way. In vertex order the
+// rows a level touches follow each other in memory, so on a grid the four
+// edges that meet at a vertex find its row in L2 (the distance rows are larger
+// than it) and no expand warp reserves queue space. A warp takes kMsScanWords
+// words, a lane a vertex of the current word, twice: totals first, then, with
+// the prefixes of the earlier tiles (two look-backs, the vertices by warp 0 and
+// the degrees by warp 1), the entries. With it a batched SSSP took 4.5 instead
+// of 4.9 ms at R-MAT 20 (37 sources) and 19.2 instead of 23.8 ms on the
+// 1200x1200 road grid (64 sources).
+constexpr int kMsScanWords = 16;
+template <int VT>
+__global__ void __launch_bounds__(kNT) k_mss_scan(MultiArgs a, uint32_t *scan, int32_t *part,
+                                                  unsigned long long *status2) {
+  constexpr uint32_t NV = kNT * VT, W = kMsScanWords;
+  __shared__ uint32_t s_cnt[kNW], s_deg[kNW];
+  __shared__ uint32_t s_tile;
+  __shared__ int s_fail;
   Ctl *ctl = a.ctl;
   if (!ctl->active) return;
-  const uint32_t L = ctl->level, pn = ctl->prev_size;
+  const uint32_t L = ctl->level, epoch = ctl->epoch;
+  const unsigned long long spin_limit = ctl->spin_limit;
+  uint32_t *bm = (L & 1) ? a.bm1 : a.bm0;
+  int32_t *Q = cur_Q(a, L);
+  const int32_t *ro = a.g.row_offsets;
+  const uint32_t V = (uint32_t)a.g.V, words = (V + 31) / 32;
+  const uint32_t ntiles = (words + W * kNW - 1) / (W * kNW);
+  const int lane = lane_id(), warp = warp_id();
+  unsigned long long my_bytes = 0;
+  if (threadIdx.x == 0) s_fail = 0;
+  for (;;) {
+    const uint32_t tile = next_tile(&ctl->tile_ctr[0], &s_tile);
+    if (tile >= ntiles || s_fail) break;
+    const uint32_t w0 = (tile * kNW + warp) * W;
+    const uint32_t mine = lane < (int)W && w0 + lane < words ? bm[w0 + lane] : 0u;
+    if (mine) bm[w0 + lane] = 0u;
+    uint32_t deg = 0, d[W];  // the lane's vertex of every word, all loads in flight
+#pragma unroll
+    for (uint32_t q = 0; q < W; ++q) {
+      const uint32_t x = __shfl_sync(0xffffffffu, mine, q);
+      const uint32_t v = (w0 + q) * 32 + lane;
+      d[q] = (x >> lane) & 1u ? (uint32_t)(ro[v + 1] - ro[v]) : 0u;
+    }
+#pragma unroll
+    for (uint32_t q = 0; q < W; ++q) deg += d[q];
+    const uint32_t cw = warp_sum((uint32_t)__popc(mine));
+    deg = warp_sum(deg);
+    if (lane == 0) {
+      s_cnt[warp] = cw;
+      s_deg[warp] = deg;
+    }
+    __syncthreads();
+    if (warp < 2) {
+      uint32_t *p = warp == 0 ? s_cnt : s_deg;
+      const uint32_t x = lane < kNW ? p[lane] : 0u;
+      const uint32_t inc = warp_inclusive_sum(x);
+      const uint32_t tot = __shfl_sync(0xffffffffu, inc, kNW - 1);
+      bool failed = false;
+      const uint32_t pre = lookback(warp == 0 ? a.status : status2, tile, tot, epoch + warp, spin_limit, &failed);
+      if (lane < kNW) p[lane] = pre + inc - x;
+      if (lane == 0 && failed) {
+        s_fail = 1;
+        raise_error(ctl, MG_ERR_TIMEOUT);
+      }
+      if (lane == 0 && !failed && tile == ntiles - 1) {
+        if (warp == 0) ctl->frontier_size = pre + tot;
+        else ctl->edge_total = pre + tot;
+      }
+    }
+    __syncthreads();
+    if (s_fail) break;
+    uint32_t pos = s_cnt[warp], run = s_deg[warp];
+    if (tile == ntiles - 1 && warp == kNW - 1 && lane == 0)
+      ctl->exp_tiles = (uint32_t)(((unsigned long long)(pos + cw) + (run + deg) + NV - 1) / NV);
+#pragma unroll
+    for (uint32_t q = 0; q < W; ++q) {
+      const uint32_t x = __shfl_sync(0xffffffffu, mine, q);
+      if (!x) continue;
+      const uint32_t v = (w0 + q) * 32 + lane;
+      const uint32_t inc = warp_inclusive_sum(d[q]);
+      if ((x >> lane) & 1u) {
+        const uint32_t i = pos + __popc(x & lanemask_lt()), base = run + inc - d[q];
+        Q[i] = (int32_t)v;
+        scan[i] = base;
+        const unsigned long long first = (unsigned long long)i + base;
+        const uint32_t t0 = (uint32_t)((first + NV - 1) / NV), t1 = (uint32_t)((first + d[q]) / NV);
+        for (uint32_t t = t0; t <= t1; ++t) part[t] = (int32_t)i;
+        my_bytes += 16;  // two row offsets, queue and scan entries
+      }
+      pos += __popc(x);
+      run += __shfl_sync(0xffffffffu, inc, 31);
+    }
+  }
+  add_bytes(ctl, KID_SCAN, my_bytes);
+}
+
+// Edge bounds of a batched SSSP on a skewed graph. With any constants c_s per
+// source, an edge (u,v) of weight w can improve no source when
+//     lo[u] + w >= hi[v],   lo[u] = min over u's active sources of d_s(u) - c_s,
+//                           hi[v] = max over all sources of d_s(v) - c_s,
+// so the expand drops it on one 4-byte load instead of reading two 256-byte
+// rows. c_s = d_s(hub), the distance of the vertex with the longest in-list:
+// the sources of a power-law graph reach its core with about the same profile,
+// so the spread of d_s - c_s is a few weights (in a simulation at R-MAT 15 with
+// 37 sources 64 % of all expansions are dropped, 1.3 kept edges per improving
+// one). On a grid the distances have no common profile and nothing would be
+// dropped, so the bounds are kept only where the longest in-list is
+// kMssSkew times the mean. A stored hi stays valid while distances fall; it is redone
+// for the queued vertices (the improved ones) each level and for every vertex
+// when a c_s changed (3-4 times a run). At R-MAT 20 with 37 sources the bytes of
+// the expand fell from 21 to 6.8 GB and the run from 6.2 to 5.1 ms.
+struct MssBounds {
+  int32_t *lo, *hi;   // [V]; lo is set for the queued vertices
+  // c_s of every source, then [64] = 1 once all of them reached the hub,
+  // [65] = 1: redo every hi, [66] = number of sources
+  int32_t *offs;
+  int32_t hub;  // < 0: no bounds on this graph
+};
+
+// Clears the previous level's masks (they were read by the previous expand) and
+// brings the bounds up to date. A warp takes four rows at
+// a time, lane l the entries 2l and 2l+1; bound by the row reads (256 bytes per
+// vertex: 50 us for every row of R-MAT 20).
+__global__ void __launch_bounds__(kNT) k_mss_bounds(MultiArgs a, MssBounds m) {
+  Ctl *ctl = a.ctl;
+  if (!ctl->active) return;
+  const uint32_t L = ctl->level, pn = ctl->prev_size, n = ctl->frontier_size;
   u64 *Fp = nxt_F(a, L);
-  const int32_t *Qp = nxt_Q(a, L);
+  const int32_t *Qp = nxt_Q(a, L), *Q = cur_Q(a, L);
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < pn; i += gridDim.x * blockDim.x) Fp[Qp[i]] = 0;
+  if (m.hub < 0 || !m.offs[64]) return;
+  const bool full = m.offs[65] != 0;
+  const int lane = lane_id();
+  const int nsrc = m.offs[66];
+  const bool k0 = 2 * lane < nsrc, k1 = 2 * lane + 1 < nsrc;
+  const int c0 = m.offs[2 * lane], c1 = m.offs[2 * lane + 1];
+  const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
+  const u64 *Fc = cur_F(a, L);
+  constexpr int R = 4;
+  unsigned long long my_bytes = 0;
+  if (full) {
+    const uint32_t V = (uint32_t)a.g.V;
+    for (uint32_t vb = gw * R; vb < V; vb += nw * R) {
+      int2 d[R];
+#pragma unroll
+      for (int q = 0; q < R; ++q)
+        d[q] = vb + q < V ? *reinterpret_cast<const int2 *>(a.out + (int64_t)(vb + q) * 64 + 2 * lane) : make_int2(0, 0);
+#pragma unroll
+      for (int q = 0; q < R; ++q) {
+        const int x = __reduce_max_sync(0xffffffffu, max(k0 ? d[q].x - c0 : INT_MIN, k1 ? d[q].y - c1 : INT_MIN));
+        if (lane == 0 && vb + q < V) m.hi[vb + q] = x;
+      }
+      my_bytes += 8 * R;  // its share of R rows
+    }
+  }
+  for (uint32_t ib = gw * R; ib < n; ib += nw * R) {
+    int v[R];
+    int2 d[R];
+    u64 am[R];
+#pragma unroll
+    for (int q = 0; q < R; ++q) v[q] = ib + q < n ? Q[ib + q] : -1;
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+      am[q] = v[q] >= 0 ? Fc[v[q]] : 0ull;
+      d[q] = v[q] >= 0 ? *reinterpret_cast<const int2 *>(a.out + (int64_t)v[q] * 64 + 2 * lane) : make_int2(0, 0);
+    }
+#pragma unroll
+    for (int q = 0; q < R; ++q) {
+      const int x0 = d[q].x - c0, x1 = d[q].y - c1;
+      const int lo = __reduce_min_sync(0xffffffffu, min((am[q] >> lane) & 1ull ? x0 : INT_MAX,
+                                                        (am[q] >> (lane + 32)) & 1ull ? x1 : INT_MAX));
+      const int hi = __reduce_max_sync(0xffffffffu, max(k0 ? x0 : INT_MIN, k1 ? x1 : INT_MIN));
+      if (lane == 0 && v[q] >= 0) {
+        m.lo[v[q]] = lo;
+        m.hi[v[q]] = hi;
+      }
+    }
+    my_bytes += 8 * R;
+  }
+  add_bytes(ctl, KID_MS_APPLY, my_bytes);
 }
 
 // Lowers a distance entry to c (a fire-and-forget reduction: nothing waits for
@@ -1109,15 +1285,36 @@ MG_DEVINL void relax_min(int32_t *p, int32_t c, u64 &imp, int t) {
   imp |= 1ull << t;
 }
 
+// One level's relaxations. The warps of a CTA first test their items of the
+// tile against the edge bounds (columns, weights and the heads' bounds of four
+// items per lane in flight), packing the edges that may improve something into
+// shared memory; then each warp relaxes its own kept edges 32 at a time. If
+// every edge of a batch carries at most kMssSparse active sources, each lane
+// relaxes its own edge source by source (scalar loads from the two 256-byte
+// rows); otherwise the whole warp takes the edges kMssEdges at a time, lane l
+// owning sources 2l and 2l+1: a row is one coalesced load (of the pairs with an
+// active source; relaxing the other source of a pair as well is harmless) and
+// the improved-source mask the two ballots, which is why source s is bit
+// s/2 + 32 (s%2) of an SSSP mask.
+//
+// Bound by the latency of the random row reads (the rows are larger than L2):
+// what counts is edges in flight per SM, 32 warps of 8 here; fewer registers
+// and more warps, or more edges and fewer warps, were slower (48 registers and
+// 5 CTAs per SM: 5.8 ms at R-MAT 20; 3 CTAs: 5.2 ms, against 4.3). Before, with
+// a 32-byte row piece per lane, 8 scattered reductions per step and a queue
+// reservation per 4 edges: 7.8 ms a run, now 4.5.
 template <int VT>
-__global__ void __launch_bounds__(kNT) k_mss_expand(MultiArgs a, const uint32_t *scan, const int32_t *part) {
+__global__ void __launch_bounds__(kNT, 4) k_mss_expand(MultiArgs a, MssBounds mb, const uint32_t *scan,
+                                                       const int32_t *part) {
   constexpr int NV = kNT * VT;
   constexpr int PER_WARP = NV / kNW;
   __shared__ int32_t s_v[NV + 1];
   __shared__ int32_t s_base[NV + 1];
   __shared__ int32_t s_rs[NV + 1];
   __shared__ int32_t s_own[NV];
-  __shared__ int32_t s_q[NV];  // per warp: its queued vertices of the current tile
+  __shared__ int32_t s_lo[NV + 1];  // per block: its tail's lower bound
+  __shared__ u64 s_am[NV + 1];      // per block: its tail's active sources
+  __shared__ int4 s_e[NV];          // per warp: its kept edges (block, head, weight, lanes with an active source)
   __shared__ uint32_t s_tile;
   __shared__ int s_fail;
   Ctl *ctl = a.ctl;
@@ -1125,21 +1322,37 @@ __global__ void __launch_bounds__(kNT) k_mss_expand(MultiArgs a, const uint32_t 
   const uint32_t L = ctl->level, n = ctl->frontier_size, total = ctl->edge_total, ntiles = ctl->exp_tiles;
   const unsigned long long items = (unsigned long long)n + total;
   const int32_t *Q = cur_Q(a, L);
-  int32_t *Qn = nxt_Q(a, L);
   const u64 *Fc = cur_F(a, L);
   u64 *Fn = nxt_F(a, L);
-  uint32_t *dedup = (L & 1) ? a.bm0 : a.bm1;
+  uint32_t *next_bm = (L & 1) ? a.bm0 : a.bm1;
   const int32_t *ro = a.g.row_offsets, *col = a.g.col, *wgt = a.g.wgt;
-  const int32_t V = a.g.V;
+  bool any = false;
+  const bool bounds = mb.hub >= 0 && mb.offs[64] != 0;
   const int lane = lane_id(), warp = warp_id();
+  const uint32_t lbit = 1u << lane;
   unsigned long long my_bytes = 0;
-  if (threadIdx.x == 0) s_fail = 0;
+  // the tile after the current one is reserved ahead (the ticket's round trip
+  // is hidden behind the tile's work; a CTA leaves one ticket unused)
+  uint32_t ticket = 0;
+  if (threadIdx.x == 0) {
+    s_fail = 0;
+    ticket = atomicAdd(&ctl->tile_ctr[1], 1u);
+  }
   for (;;) {
-    const uint32_t tile = next_tile(&ctl->tile_ctr[1], &s_tile);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      s_tile = ticket;
+      if (ticket < ntiles) ticket = atomicAdd(&ctl->tile_ctr[1], 1u);
+    }
+    __syncthreads();
+    const uint32_t tile = s_tile;
     if (tile >= ntiles || s_fail) break;
     int cnt;
     if (!decode_tile<VT>(tile, ntiles, n, items, part, scan, Q, ro, s_v, s_base, s_rs, s_own, &cnt,
-                         [](int, int) {})) {
+                         [&](int j, int v) {
+                           s_am[j] = Fc[v];
+                           if (bounds) s_lo[j] = mb.lo[v];
+                         })) {
       if (threadIdx.x == 0) {
         raise_error(ctl, MG_ERR_OVERFLOW);
         s_fail = 1;
@@ -1147,137 +1360,148 @@ __global__ void __launch_bounds__(kNT) k_mss_expand(MultiArgs a, const uint32_t 
       __syncthreads();
       break;
     }
-    // The warp takes its items 32 at a time; lane i loads item k+i's edge (tail,
-    // head, weight, tail's source mask), the next batch while the current one
-    // is relaxed. If every edge of the batch carries at most kMssSparse active
-    // sources, each lane relaxes its own edge source by source (scalar loads
-    // from the two 256-byte rows); otherwise the batch goes four edges per
-    // step, the 8 lanes of group g owning sources 8*sub .. 8*sub+7 of edge
-    // 4q+g, read with two 16-byte loads from each row.
     const int k0 = warp * PER_WARP;
     const int k1 = min(cnt, k0 + PER_WARP);
-    const int grp = lane >> 3, sub = lane & 7;
-    auto fetch = [&](int k, int &u, int &v, int &w, u64 &am) {
-      u = -1;
-      if (k >= k1) return;
-      const int j = s_own[k];
-      const int el = k - s_base[j] - 1;
-      if (el < 0) return;
-      const int eid = s_rs[j] + el;
-      if ((unsigned)eid >= (unsigned)a.g.E) {
-        raise_error(ctl, MG_ERR_OVERFLOW);
-        return;
+    int4 *we = s_e + k0;
+    int kept = 0;  // warp-uniform
+    {
+      constexpr int R = PER_WARP / 32;
+      int j[R], v[R], w[R], hi[R];
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const int k = k0 + 32 * r + lane;
+        v[r] = -1;
+        if (k < k1) {
+          j[r] = s_own[k];
+          const int el = k - s_base[j[r]] - 1;
+          if (el >= 0) {
+            const int eid = s_rs[j[r]] + el;
+            if ((unsigned)eid < (unsigned)a.g.E) {
+              v[r] = __ldcs(col + eid);
+              w[r] = __ldcs(wgt + eid);
+            } else {
+              raise_error(ctl, MG_ERR_OVERFLOW);
+            }
+          }
+        }
       }
-      u = s_v[j];
-      v = __ldcs(col + eid);
-      w = __ldcs(wgt + eid);
-      am = Fc[u];
-    };
-    // next-level mask and dedup bit of the vertices that improved; the ones
-    // that won the dedup bit are staged in the warp's part of s_q (an item
-    // queues at most one vertex, so PER_WARP slots suffice) and reserved in the
-    // queue once per warp and tile (a reservation per step was a same-address
-    // atomic for every 32 or 4 edges)
-    int32_t *wq = s_q + warp * PER_WARP;
-    int qn = 0;  // warp-uniform
-    auto enqueue = [&](bool has, int v, u64 mask) {
-      bool enq = false;
-      if (has) {
-        my_bytes += 8 + 4ull * (unsigned long long)__popcll(mask);
-        atomicOr(&Fn[v], mask);
-        const uint32_t bit = 1u << (v & 31);
-        enq = !(ld_volatile(&dedup[v >> 5]) & bit) && !(atomicOr(&dedup[v >> 5], bit) & bit);
+#pragma unroll
+      for (int r = 0; r < R; ++r) hi[r] = bounds && v[r] >= 0 ? __ldg(mb.hi + v[r]) : 0;
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        u64 am = 0;
+        if (v[r] >= 0) {
+          am = s_am[j[r]];
+          // (a sum past the int range wraps to a kept edge, as without bounds)
+          if (bounds && (int)((uint32_t)s_lo[j[r]] + (uint32_t)w[r]) >= hi[r]) am = 0;
+          my_bytes += (bounds ? 12 : 8) + 8ull * (unsigned long long)__popcll(am);
+        }
+        const uint32_t kb = __ballot_sync(0xffffffffu, am != 0ull);
+        if (am)
+          we[kept + __popc(kb & lanemask_lt())] =
+              make_int4(j[r], v[r], w[r], (int)((uint32_t)am | (uint32_t)(am >> 32)));
+        kept += __popc(kb);
       }
-      const uint32_t eb = __ballot_sync(0xffffffffu, enq);
-      if (enq) {
-        const int pos = qn + __popc(eb & lanemask_lt());
-        if (pos < PER_WARP) wq[pos] = v;
-        else raise_error(ctl, MG_ERR_OVERFLOW);
+    }
+    __syncwarp();
+    for (int b0 = 0; b0 < kept; b0 += 32) {
+      const int nb = min(32, kept - b0);
+      int4 be = make_int4(0, 0, 0, 0);
+      u64 bam = 0, imp = 0;
+      if (lane < nb) {
+        be = we[b0 + lane];
+        bam = s_am[be.x];
       }
-      qn = min(qn + __popc(eb), PER_WARP);
-    };
-    int nu = -1, nv = 0, nw = 0;
-    u64 nam = 0;
-    fetch(k0 + lane, nu, nv, nw, nam);
-    for (int kb = k0; kb < k1; kb += 32) {
-      const int bu = nu, bv = nv, bw = nw;
-      const u64 bam = nam;
-      fetch(kb + 32 + lane, nu, nv, nw, nam);
-      if (bu >= 0) my_bytes += 16 + 8ull * (unsigned long long)__popcll(bam);
-      if (__all_sync(0xffffffffu, bu < 0 || __popcll(bam) <= kMssSparse)) {
-        u64 imp = 0;
-        if (bu >= 0) {
-          const int32_t *du = a.out + (int64_t)bu * 64;
-          int32_t *dv = a.out + (int64_t)bv * 64;
+      if (__all_sync(0xffffffffu, __popcll(bam) <= kMssSparse)) {
+        if (bam) {
+          const int32_t *du = a.out + (int64_t)s_v[be.x] * 64;
+          int32_t *dv = a.out + (int64_t)be.y * 64;
           // four active sources per step, their row entries loaded together
           for (u64 m = bam; m;) {
-            int t[4], du4[4], dv4[4];
+            int t[4], s[4], du4[4], dv4[4];
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
               t[q] = m ? __ffsll((long long)m) - 1 : -1;
+              s[q] = mss_source(t[q]);
               m &= m - 1;
             }
 #pragma unroll
             for (int q = 0; q < 4; ++q)
               if (t[q] >= 0) {
-                du4[q] = __ldcg(du + t[q]);
-                dv4[q] = __ldcg(dv + t[q]);
+                du4[q] = __ldcg(du + s[q]);
+                dv4[q] = __ldcg(dv + s[q]);
               }
 #pragma unroll
             for (int q = 0; q < 4; ++q)
-              if (t[q] >= 0 && du4[q] + bw < dv4[q]) relax_min(dv + t[q], du4[q] + bw, imp, t[q]);
+              if (t[q] >= 0 && du4[q] + be.z < dv4[q]) relax_min(dv + s[q], du4[q] + be.z, imp, t[q]);
           }
         }
-        enqueue(imp != 0, bv, imp);
-        continue;
-      }
+      } else {
 #pragma unroll 1
-      for (int q = 0; q < 8; ++q) {
-        const int src = 4 * q + grp;
-        const int u = __shfl_sync(0xffffffffu, bu, src), v = __shfl_sync(0xffffffffu, bv, src);
-        const int w = __shfl_sync(0xffffffffu, bw, src);
-        const u64 am = __shfl_sync(0xffffffffu, bam, src);
-        uint32_t imp = 0;
-        const uint32_t bits = u >= 0 ? (uint32_t)(am >> (8 * sub)) & 0xffu : 0u;
-        if (bits) {
-          const int4 *pu = reinterpret_cast<const int4 *>(a.out + (int64_t)u * 64 + 8 * sub);
-          int32_t *dvp = a.out + (int64_t)v * 64 + 8 * sub;
-          const int4 *pv = reinterpret_cast<const int4 *>(dvp);
-          const int4 u0 = __ldcg(pu), u1 = __ldcg(pu + 1), v0 = __ldcg(pv), v1 = __ldcg(pv + 1);
-          const int du[8] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
-          const int dv[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+        for (int j0 = 0; j0 < nb; j0 += kMssEdges) {
+          // the heads' rows of all kMssEdges edges in flight; the tails' rows come
+          // through L1 as they are needed (the edges of a tail are neighbours in
+          // the batch; an entry lowered meanwhile is marked and relaxed again next
+          // level), so an edge in flight holds two registers
+          int2 h[kMssEdges];
 #pragma unroll
-          for (int t = 0; t < 8; ++t) {
-            if (((bits >> t) & 1u) && du[t] + w < dv[t]) {
-              atomicMin(&dvp[t], du[t] + w);  // result unused: a reduction (see relax_min)
-              imp |= 1u << t;
+          for (int q = 0; q < kMssEdges; ++q) {
+            h[q] = make_int2(INT_MIN, INT_MIN);  // a pair that is not loaded is never improved
+            const int4 e = we[b0 + j0 + q];
+            if (j0 + q < nb && ((uint32_t)e.w & lbit))
+              h[q] = __ldcg(reinterpret_cast<const int2 *>(a.out + (int64_t)e.y * 64 + 2 * lane));
+          }
+#pragma unroll
+          for (int q = 0; q < kMssEdges; ++q) {
+            const int4 e = we[b0 + j0 + q];
+            bool p0 = false, p1 = false;
+            if (h[q].x != INT_MIN) {
+              const int2 t = *reinterpret_cast<const int2 *>(a.out + (int64_t)s_v[e.x] * 64 + 2 * lane);
+              const int c0 = t.x + e.z, c1 = t.y + e.z;
+              int32_t *hp = a.out + (int64_t)e.y * 64 + 2 * lane;
+              p0 = c0 < h[q].x;
+              p1 = c1 < h[q].y;
+              if (p0) atomicMin(hp, c0);  // result unused: a reduction (see relax_min)
+              if (p1) atomicMin(hp + 1, c1);
             }
+            const uint32_t m0 = __ballot_sync(0xffffffffu, p0), m1 = __ballot_sync(0xffffffffu, p1);
+            if (lane == j0 + q) imp = ((u64)m1 << 32) | m0;
           }
         }
-        // improved sources of the group's edge: OR of the 8 lanes' byte masks
-        u64 mask = (u64)imp << (8 * sub);
-        mask |= __shfl_xor_sync(0xffffffffu, mask, 1);
-        mask |= __shfl_xor_sync(0xffffffffu, mask, 2);
-        mask |= __shfl_xor_sync(0xffffffffu, mask, 4);
-        enqueue(sub == 0 && mask != 0, v, mask);
       }
-    }
-    __syncwarp();
-    if (qn) {
-      uint32_t base = 0;
-      if (lane == 0) base = atomicAdd(&ctl->next_size, (uint32_t)qn);
-      base = __shfl_sync(0xffffffffu, base, 0);
-      for (int i = lane; i < qn; i += 32) {
-        if (base + (uint32_t)i < (uint32_t)V) Qn[base + i] = wq[i];
-        else raise_error(ctl, MG_ERR_OVERFLOW);
+      // next-level mask and frontier bit of the heads that improved
+      if (imp) {
+        my_bytes += 8 + 4ull * (unsigned long long)__popcll(imp);
+        atomicOr(&Fn[be.y], imp);
+        const uint32_t bit = 1u << (be.y & 31);
+        if (!(ld_volatile(&next_bm[be.y >> 5]) & bit)) atomicOr(&next_bm[be.y >> 5], bit);
+        any = true;
       }
     }
   }
+  if (any) ctl->next_size = 1;  // the next scan counts them
   add_bytes(ctl, KID_MSS_EXPAND, my_bytes);
 }
 
-__global__ void k_mss_level_end(Ctl *ctl, cudaGraphConditionalHandle h, int use_handle) {
-  if (threadIdx.x != 0) return;
+// One CTA of 64 threads: thread s also looks after source s's bound offset.
+__global__ void k_mss_level_end(MultiArgs a, MssBounds m, cudaGraphConditionalHandle h, int use_handle) {
+  Ctl *ctl = a.ctl;
+  const int t = threadIdx.x;
+  if (ctl->active && m.hub >= 0) {
+    const int c = t < m.offs[66] ? a.out[(int64_t)m.hub * 64 + t] : 0;
+    const int reached = __syncthreads_and(c < programs::sssp::INIT_VALUE);
+    const int changed = __syncthreads_or(c != m.offs[t]);
+    const int was = m.offs[64];
+    __syncthreads();
+    if (reached) {
+      m.offs[t] = c;
+      if (t == 0) {
+        m.offs[65] = (!was || changed) ? 1 : 0;
+        m.offs[64] = 1;
+      }
+    }
+  }
+  if (t != 0) return;
   if (ctl->active) {
     ctl->prev_size = ctl->frontier_size;
     ctl->level += 1;
@@ -1312,6 +1536,7 @@ static MultiArgs multi_args(mg_graph *g) {
   a.bm1 = g->ws.bm[1];
   a.status = g->ws.status;
   a.ctl = g->ws.ctl;
+  a.mss_offs = g->mss_offs;
   a.all = 0;
   return a;
 }
@@ -1523,21 +1748,6 @@ int mg_sssp_multi(mg_graph *g, const int32_t *srcs, int32_t nsrc, int32_t *dists
   if (st != MG_OK) return st;
   MultiArgs a = multi_args(g);
   a.all = (nsrc == 64) ? ~0ull : ((1ull << nsrc) - 1);
-  GasArgs<mssp_scan> ga;
-  ga.g = g->csr;
-  ga.queue0 = g->ws.queue[0];
-  ga.queue1 = g->ws.queue[1];
-  ga.scan = g->ws.scan + 0;
-  ga.part = g->ws.part;
-  ga.status = g->ws.status;
-  ga.bm0 = g->ws.bm[0];
-  ga.bm1 = g->ws.bm[1];
-  ga.changed = g->ws.changed;
-  ga.gather_tmp = g->ws.gather_tmp;
-  ga.gather_res = g->ws.gather_tmp;
-  ga.ctl = g->ws.ctl;
-  ga.expand_in = 0;
-  ga.gather_dir = NO_GATHER_EDGES;
   const uint32_t max_iter = (uint32_t)std::min<int64_t>(o->iter_num > 0 ? o->iter_num : 0, g->nodes + 2);
   k_ctl_init<<<1, 32, 0, s>>>(g->ws.ctl, (uint32_t)list.ndistinct, max_iter, (unsigned long long)o->spin_limit,
                               MODE_QUEUE, ctl_flags(o));
@@ -1547,11 +1757,18 @@ int mg_sssp_multi(mg_graph *g, const int32_t *srcs, int32_t nsrc, int32_t *dists
   const int grid = persistent_grid(g, o, 4);
   uint32_t *scan = g->ws.scan;
   int32_t *part = g->ws.part;
+  // the scan's second look-back: it has at most V/4096 + 1 tiles, fewer than half the words
+  unsigned long long *status2 = g->ws.status + g->ws.status_cap / 2;
+  MssBounds mb;
+  mb.lo = g->ws.vbuf[0];
+  mb.hi = g->ws.vbuf[1];
+  mb.offs = g->mss_offs;
+  mb.hub = g->mss_hub;
   LevelBody body = [=](cudaStream_t ss, cudaGraphConditionalHandle h, int use_h) {
-    MG_LAUNCH(KID_MS_APPLY, ss, k_mss_clear<<<grid, kNT, 0, ss>>>(a));
-    MG_LAUNCH(KID_SCAN, ss, (k_frontier_scan<mssp_scan, kMVTS, kMSVT><<<grid, kNT, 0, ss>>>(ga)));
-    MG_LAUNCH(KID_MSS_EXPAND, ss, k_mss_expand<kMSVT><<<grid, kNT, 0, ss>>>(a, scan, part));
-    MG_LAUNCH(KID_OTHER, ss, k_mss_level_end<<<1, 32, 0, ss>>>(a.ctl, h, use_h));
+    MG_LAUNCH(KID_SCAN, ss, k_mss_scan<kMSVT><<<grid, kNT, 0, ss>>>(a, scan, part, status2));
+    MG_LAUNCH(KID_MS_APPLY, ss, k_mss_bounds<<<grid, kNT, 0, ss>>>(a, mb));
+    MG_LAUNCH(KID_MSS_EXPAND, ss, k_mss_expand<kMSVT><<<grid, kNT, 0, ss>>>(a, mb, scan, part));
+    MG_LAUNCH(KID_OTHER, ss, k_mss_level_end<<<1, 64, 0, ss>>>(a, mb, h, use_h));
   };
   LoopResult res;
   const auto epi = transpose_epilogue(g, nsrc, dists, false, false);
