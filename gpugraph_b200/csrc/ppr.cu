@@ -476,7 +476,9 @@ static int ppr_solve(mg_graph *g, int dir, const float *w, const float *rhs, flo
     MG_LAUNCH(KID_OTHER, ss, k_ppr_level_end<<<1, 32, 0, ss>>>(a.ctl, tol, h, use_h));
   };
   char key[160];
-  snprintf(key, sizeof(key), "%s/%d/%d/%.9g/%.17g/%.17g", name, grid, nvec, (double)alpha, o->damping, tol);
+  // (ppr_cap_nvec: a wider solve replaced the buffers the cached graph's arguments point to)
+  snprintf(key, sizeof(key), "%s/%d/%d/%d/%.9g/%.17g/%.17g", name, grid, nvec, g->ppr_cap_nvec, (double)alpha,
+           o->damping, tol);
   int st = run_level_loop(g, s, key, 3, body, o->use_cuda_graph != 0, res);
   if (st != MG_OK) return st;
   finish_run(g, res->ctl.level);

@@ -38,3 +38,52 @@ def test_sssp_multi_edge_bounds(kind, nsrc):
         out, _ = g.sssp_multi(srcs, **mode)
         for k, s in enumerate(srcs):
             assert np.array_equal(out[k], oracle.sssp(hg.row_offsets, hg.column_indices, hg.edge_values, s)), k
+
+
+D = 0.85
+
+
+def _ppr_case(nvec, seed=7, scale=9):
+    hg = HostGraph.rmat(scale, 16, seed=seed, symmetrize=False)
+    rng = np.random.default_rng(seed)
+    src = np.repeat(np.arange(hg.nodes), np.diff(hg.row_offsets))
+    w = rng.lognormal(0.0, 1.0, size=hg.edges)
+    w = w / np.bincount(src, weights=w, minlength=hg.nodes)[src]
+    t = np.zeros((hg.nodes, nvec))
+    for c in range(nvec):
+        t[rng.choice(hg.nodes, size=20, replace=False), c] = 0.05
+    return hg, src, w, t, rng.standard_normal((hg.nodes, nvec))
+
+
+def _ppr_dense(torch, hg, src, w, t, c):
+    w64, t64 = torch.tensor(w, requires_grad=True), torch.tensor(t, requires_grad=True)
+    p = torch.zeros((hg.nodes, hg.nodes), dtype=torch.float64).index_put(
+        (torch.as_tensor(src), torch.as_tensor(hg.column_indices.astype(np.int64))), w64, accumulate=True)
+    r = torch.linalg.solve(torch.eye(hg.nodes, dtype=torch.float64) - D * p.T, (1 - D) * t64)
+    (r * torch.tensor(c)).sum().backward()
+    return r.detach(), w64.grad, t64.grad
+
+
+def _ppr_check(torch, g, hg, src, w, t, c):
+    from gpugraph_b200.ppr import ppr
+
+    ref_r, ref_w, ref_t = _ppr_dense(torch, hg, src, w, t, c)
+    wt = torch.tensor(w, dtype=torch.float32, device="cuda", requires_grad=True)
+    tt = torch.tensor(t, dtype=torch.float32, device="cuda", requires_grad=True)
+    r = ppr(g, wt, tt)
+    (r * torch.tensor(c, dtype=torch.float32, device="cuda")).sum().backward()
+    # the solve stops at an L1 change of 1e-7 of its right-hand side, d/(1-d) = 5.7 times that is left;
+    # sums of FP32 products of this size add about 1e-6: the bounds of the other PPR tests
+    assert (r.detach().double().cpu() - ref_r).abs().sum(0).max() < 2e-5
+    assert (wt.grad.double().cpu() - ref_w).norm() / ref_w.norm() < 1e-4
+    assert (tt.grad.double().cpu() - ref_t).norm() / ref_t.norm() < 1e-4
+
+
+def test_ppr_width_grows_and_shrinks_on_one_graph():
+    # the workspace is replaced when the rows get wider; a narrower solve after that must use the new one
+    torch = pytest.importorskip("torch")
+    hg, *_ = _ppr_case(4)
+    g = Graph(hg, directed=True)
+    for nvec in (4, 32, 4, 7, 64, 32, 1):
+        _, src, w, t, c = _ppr_case(nvec)
+        _ppr_check(torch, g, hg, src, w, t, c)
