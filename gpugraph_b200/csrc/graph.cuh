@@ -128,7 +128,7 @@ struct mg_graph {
   struct PprPlan {
     int32_t *cv = nullptr, *cb = nullptr, *ce = nullptr, *cslot = nullptr;
     int32_t *mv = nullptr, *mfirst = nullptr;  // split vertices and their first slot
-    int32_t nchunks = 0, nmulti = 0, nslots = 0;
+    int32_t nchunks = 0, nfull = 0, nmulti = 0, nslots = 0;  // nfull: chunks with edges, first in the plan
   } ppr_plan[2];
   float *ppr_x[2] = {nullptr, nullptr}, *ppr_partial = nullptr;
   float *ppr_rhs = nullptr, *ppr_w = nullptr;  // stable copies of the solve's inputs

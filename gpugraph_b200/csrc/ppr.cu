@@ -12,13 +12,16 @@
 // the L1 norm of their right-hand side (T or G; for teleport columns that are
 // distributions that is tolerance * nvec), or after iter_num iterations.
 //
-// Layout and work split: a warp owns one chunk of one vertex's adjacency and
-// lane c owns columns c and c+32, so every edge costs one coalesced read of a
-// 128-byte row (nvec = 32) plus a broadcast index/weight load; eight edges
-// (four for nvec > 32) are in flight per step. The forward solve reads the
-// weights gathered into CSC order once per solve. In-lists longer than
-// kPprChunk are cut into chunks whose partial rows are added in chunk order by
-// a fix-up pass (deterministic).
+// Layout and work split: the solve's rows are padded to nv = nvec rounded up to
+// a multiple of 4, so every row is 16-byte aligned. A group of G lanes (nv/4
+// rounded up to a power of two) owns one chunk of one vertex's adjacency and
+// lane l of the group columns 4l..4l+3: an edge costs one coalesced row read,
+// and a warp works on 32/G chunks at once. The chunks are taken in descending
+// order of length (vertex order within a length), so the groups of a warp run
+// the same number of steps. Adjacencies longer than kPprChunk are cut into
+// chunks whose partial rows are added in chunk order by a fix-up pass
+// (deterministic). The forward solve reads the weights gathered into CSC order
+// once per solve.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -36,13 +39,13 @@ constexpr int kPprChunk = 256;
 constexpr int kPprMaxVec = 64;
 
 struct PprArgs {
-  const int32_t *off, *idx, *eid;  // adjacency of the solve (CSC forward, CSR adjoint); eid may be null
-  const float *w;                  // weights per CSR edge
-  const float *rhs;                // T (forward) or G (adjoint), [V][nvec]
+  const int32_t *idx;              // adjacency of the solve (CSC forward, CSR adjoint)
+  const float *w;                  // weights in the order of idx
+  const float *rhs;                // T (forward) or G (adjoint), [V][nv]
   float alpha, d;                  // X' = alpha*rhs + d*sum(...)
   float *x0, *x1, *partial;
   const int32_t *cv, *cb, *ce, *cslot, *mv, *mfirst;
-  int32_t nchunks, nmulti, nvec, V;
+  int32_t nchunks, nfull, nmulti, nv, V;  // nfull: chunks that have edges (they come first)
   Ctl *ctl;
 };
 
@@ -53,8 +56,8 @@ MG_DEVINL void ppr_finalize_row(const PprArgs &a, int v, const float (&acc)[NC],
 #pragma unroll
   for (int q = 0; q < NC; ++q) {
     const int c = lane + 32 * q;
-    if (c < a.nvec) {
-      const int64_t o = (int64_t)v * a.nvec + c;
+    if (c < a.nv) {
+      const int64_t o = (int64_t)v * a.nv + c;
       const float xn = fmaf(a.d, acc[q], a.alpha * a.rhs[o]);
       res += (double)fabsf(xn - xold[o]);
       xnew[o] = xn;
@@ -62,74 +65,35 @@ MG_DEVINL void ppr_finalize_row(const PprArgs &a, int v, const float (&acc)[NC],
   }
 }
 
-template <int NC>
-__global__ void __launch_bounds__(kNT) k_ppr_iter(PprArgs a) {
-  Ctl *ctl = a.ctl;
-  if (!ctl->active) return;
-  const uint32_t L = ctl->level;
-  const float *xold = (L & 1) ? a.x1 : a.x0;
-  float *xnew = (L & 1) ? a.x0 : a.x1;
-  const int lane = lane_id();
-  double res = 0.0;
-  unsigned long long my_bytes = 0;
-  const uint32_t nwarps = gridDim.x * kNW;
-  for (uint32_t c = blockIdx.x * kNW + warp_id(); c < (uint32_t)a.nchunks; c += nwarps) {
-    const int v = a.cv[c], b = a.cb[c], e = a.ce[c], slot = a.cslot[c];
-    float acc[NC];
+// The edges [k, k + kPprStep) of a group's chunk, held by its G lanes: lane l
+// has edge k + l (and k + l + G, ... when G < kPprStep). Past the end: u = -1.
+constexpr int kPprStep = 8;
+template <int G>
+struct PprStep {
+  static constexpr int N = G < kPprStep ? kPprStep / G : 1;
+  int u[N];
+  float w[N];
+  MG_DEVINL void load(const int32_t *idx, const float *wgt, int k, int e, int gl) {
 #pragma unroll
-    for (int q = 0; q < NC; ++q) acc[q] = 0.f;
-    // EPS edges per step, all their loads in flight (predicated at the end of
-    // the chunk): index and weight, then the EPS gathered rows
-    constexpr int EPS = NC == 1 ? 8 : 4;
-    for (int k = b; k < e; k += EPS) {
-      int u[EPS];
-      float wt[EPS];
-#pragma unroll
-      for (int j = 0; j < EPS; ++j) {
-        const bool in = k + j < e;
-        u[j] = in ? a.idx[k + j] : -1;
-        wt[j] = in ? a.w[a.eid ? a.eid[k + j] : k + j] : 0.f;
-      }
-      float row[EPS][NC];
-#pragma unroll
-      for (int j = 0; j < EPS; ++j)
-#pragma unroll
-        for (int q = 0; q < NC; ++q) {
-          const int col = lane + 32 * q;
-          row[j][q] = (u[j] >= 0 && col < a.nvec) ? __ldg(&xold[(int64_t)u[j] * a.nvec + col]) : 0.f;
-        }
-#pragma unroll
-      for (int j = 0; j < EPS; ++j)
-#pragma unroll
-        for (int q = 0; q < NC; ++q) acc[q] = fmaf(wt[j], row[j][q], acc[q]);
-    }
-    if (lane == 0) my_bytes += (unsigned long long)(e - b) * (8ull + 4ull * a.nvec);
-    if (slot < 0) {
-      ppr_finalize_row<NC>(a, v, acc, xold, xnew, res);
-      if (lane == 0) my_bytes += 12ull * a.nvec;
-    } else {
-#pragma unroll
-      for (int q = 0; q < NC; ++q) {
-        const int col = lane + 32 * q;
-        if (col < a.nvec) a.partial[(int64_t)slot * a.nvec + col] = acc[q];
-      }
+    for (int i = 0; i < N; ++i) {
+      const int p = k + (gl & (kPprStep - 1)) + i * G;
+      const bool in = p < e;
+      u[i] = in ? __ldcs(idx + p) : -1;
+      w[i] = in && wgt ? __ldcs(wgt + p) : 0.f;
     }
   }
-  add_bytes(ctl, KID_PPR, my_bytes);
-  res = cta_sum_f64(res);
-  if (threadIdx.x == 0 && res != 0.0) atomicAdd(&ctl->acc[1], res);
-}
+  MG_DEVINL int edge(int j) const { return __shfl_sync(0xffffffffu, u[j / G < N ? j / G : 0], j % G, G); }
+  MG_DEVINL float weight(int j) const { return __shfl_sync(0xffffffffu, w[j / G < N ? j / G : 0], j % G, G); }
+};
 
-// Vector variant for nvec % 4 == 0 (rows 16-byte aligned): a group of G lanes
-// owns one chunk and lane l of the group columns 4l..4l+3, one 16-byte load
-// per gathered row, so a warp works on 32/G chunks at once (4 for nvec <= 32,
-// 2 for nvec <= 64): that many chunks' index, weight and row loads are in
-// flight per step instead of one. Per column the edges are added in the same
-// order as in k_ppr_iter, so both give the same ranks.
+// One iteration over the chunks. A step's kPprStep row loads are in flight
+// together, its indices and weights were loaded one step ahead (one coalesced
+// load per group each, passed on by shuffles). Vertices without edges keep
+// alpha*rhs: both iterates hold it after the first two iterations, and from
+// then on their chunks are not visited.
 template <int G>
-__global__ void __launch_bounds__(kNT, 4) k_ppr_iter_v(PprArgs a) {
+__global__ void __launch_bounds__(kNT, 4) k_ppr_iter(PprArgs a) {
   constexpr int PER = 32 / G;
-  constexpr int EPS = 8;
   Ctl *ctl = a.ctl;
   if (!ctl->active) return;
   const uint32_t L = ctl->level;
@@ -138,39 +102,45 @@ __global__ void __launch_bounds__(kNT, 4) k_ppr_iter_v(PprArgs a) {
   const int lane = lane_id();
   const int gl = lane & (G - 1);
   const int col = gl * 4;
-  const bool cok = col < a.nvec;
+  const bool cok = col < a.nv;
   double res = 0.0;
   unsigned long long my_bytes = 0;
+  const uint32_t n = (uint32_t)(L < 2 ? a.nchunks : a.nfull);
   const uint32_t nslots = gridDim.x * kNW * PER;
-  for (uint32_t c = (blockIdx.x * kNW + warp_id()) * PER + lane / G; c < (uint32_t)a.nchunks; c += nslots) {
-    const int v = a.cv[c], b = a.cb[c], e = a.ce[c], slot = a.cslot[c];
+  for (uint32_t c0 = (blockIdx.x * kNW + warp_id()) * PER; c0 < n; c0 += nslots) {
+    const uint32_t c = c0 + lane / G;
+    const bool has = c < n;
+    const int v = has ? a.cv[c] : 0, b = has ? a.cb[c] : 0, e = has ? a.ce[c] : 0;
+    const int slot = has ? a.cslot[c] : 0;
+    const int steps = (__reduce_max_sync(0xffffffffu, e - b) + kPprStep - 1) / kPprStep;
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int k = b; k < e; k += EPS) {
-      int u[EPS];
-      float wt[EPS];
+    PprStep<G> cur;
+    cur.load(a.idx, a.w, b, e, gl);
+    for (int s = 0; s < steps; ++s) {
+      PprStep<G> nxt;
+      nxt.load(a.idx, a.w, b + (s + 1) * kPprStep, e, gl);
+      float4 row[kPprStep];
 #pragma unroll
-      for (int j = 0; j < EPS; ++j) {
-        const bool in = k + j < e;
-        u[j] = in ? a.idx[k + j] : -1;
-        wt[j] = in ? a.w[a.eid ? a.eid[k + j] : k + j] : 0.f;
+      for (int j = 0; j < kPprStep; ++j) {
+        const int u = cur.edge(j);
+        row[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (u >= 0 && cok) row[j] = __ldg(reinterpret_cast<const float4 *>(xold + (int64_t)u * a.nv + col));
       }
-      float4 row[EPS];
 #pragma unroll
-      for (int j = 0; j < EPS; ++j)
-        row[j] = (u[j] >= 0 && cok) ? __ldg(reinterpret_cast<const float4 *>(xold + (int64_t)u[j] * a.nvec + col))
-                                    : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-      for (int j = 0; j < EPS; ++j) {
-        acc.x = fmaf(wt[j], row[j].x, acc.x);
-        acc.y = fmaf(wt[j], row[j].y, acc.y);
-        acc.z = fmaf(wt[j], row[j].z, acc.z);
-        acc.w = fmaf(wt[j], row[j].w, acc.w);
+      for (int j = 0; j < kPprStep; ++j) {
+        const float wt = cur.weight(j);
+        acc.x = fmaf(wt, row[j].x, acc.x);
+        acc.y = fmaf(wt, row[j].y, acc.y);
+        acc.z = fmaf(wt, row[j].z, acc.z);
+        acc.w = fmaf(wt, row[j].w, acc.w);
       }
+      cur = nxt;
     }
-    if (gl == 0) my_bytes += (unsigned long long)(e - b) * (8ull + 4ull * a.nvec);
+    if (!has) continue;
+    if (gl == 0) my_bytes += (unsigned long long)(e - b) * (8ull + 4ull * a.nv);
     if (slot < 0) {
       if (cok) {
-        const int64_t o = (int64_t)v * a.nvec + col;
+        const int64_t o = (int64_t)v * a.nv + col;
         const float4 r = *reinterpret_cast<const float4 *>(a.rhs + o);
         const float4 xo = *reinterpret_cast<const float4 *>(xold + o);
         float4 xn;
@@ -182,9 +152,9 @@ __global__ void __launch_bounds__(kNT, 4) k_ppr_iter_v(PprArgs a) {
                (double)fabsf(xn.w - xo.w);
         *reinterpret_cast<float4 *>(xnew + o) = xn;
       }
-      if (gl == 0) my_bytes += 12ull * a.nvec;
+      if (gl == 0) my_bytes += 12ull * a.nv;
     } else if (cok) {
-      *reinterpret_cast<float4 *>(a.partial + (int64_t)slot * a.nvec + col) = acc;
+      *reinterpret_cast<float4 *>(a.partial + (int64_t)slot * a.nv + col) = acc;
     }
   }
   add_bytes(ctl, KID_PPR, my_bytes);
@@ -219,7 +189,7 @@ __global__ void __launch_bounds__(kNT) k_ppr_fixup(PprArgs a) {
 #pragma unroll
         for (int q = 0; q < NC; ++q) {
           const int col = lane + 32 * q;
-          t[j][q] = col < a.nvec ? a.partial[(int64_t)(s + j) * a.nvec + col] : 0.f;
+          t[j][q] = col < a.nv ? a.partial[(int64_t)(s + j) * a.nv + col] : 0.f;
         }
 #pragma unroll
       for (int j = 0; j < 8; ++j)
@@ -230,7 +200,7 @@ __global__ void __launch_bounds__(kNT) k_ppr_fixup(PprArgs a) {
 #pragma unroll
       for (int q = 0; q < NC; ++q) {
         const int col = lane + 32 * q;
-        if (col < a.nvec) acc[q] += a.partial[(int64_t)s * a.nvec + col];
+        if (col < a.nv) acc[q] += a.partial[(int64_t)s * a.nv + col];
       }
     ppr_finalize_row<NC>(a, v, acc, xold, xnew, res);
   }
@@ -252,57 +222,56 @@ __global__ void k_ppr_level_end(Ctl *ctl, double tol, cudaGraphConditionalHandle
   if (use_handle) cudaGraphSetConditional(h, ctl->active);
 }
 
-// dL/dw(u,v) = d <lambda[v,:], R[u,:]>: warp per out-edge chunk of the CSR
-// chunk plan (a row, or at most kPprChunk edges of a long row, so a hub's row
-// is spread over many warps), R[u,:] held in registers, EPS out-edges per step
-// with all their row gathers in flight before the warp reductions.
-template <int NC>
-__global__ void __launch_bounds__(kNT) k_ppr_edge_grad(const int32_t *cv, const int32_t *cb, const int32_t *ce,
-                                                       int32_t nchunks, const int32_t *col, int32_t nvec,
-                                                       const float *lam, const float *R, float d, float *grad_w,
-                                                       Ctl *ctl) {
-  constexpr int EPS = NC == 1 ? 8 : 4;
+// dL/dw(u,v) = d <lambda[v,:], R[u,:]>: a group of G lanes per out-edge chunk of
+// the CSR chunk plan (a row, or at most kPprChunk edges of a long row), laid out
+// as in k_ppr_iter: R[u,:] held in registers, kPprStep lambda rows in flight,
+// the dot products reduced within the group. R has the caller's row stride nvec.
+template <int G>
+__global__ void __launch_bounds__(kNT, 4) k_ppr_edge_grad(const int32_t *cv, const int32_t *cb, const int32_t *ce,
+                                                          int32_t n, const int32_t *idx, int32_t nvec, int32_t nv,
+                                                          const float *lam, const float *R, float d, float *grad_w,
+                                                          Ctl *ctl) {
+  constexpr int PER = 32 / G;
   const int lane = lane_id();
-  const uint32_t nwarps = gridDim.x * kNW;
+  const int gl = lane & (G - 1);
+  const int col = gl * 4;
+  const uint32_t nslots = gridDim.x * kNW * PER;
   unsigned long long my_bytes = 0;
-  for (uint32_t c = blockIdx.x * kNW + warp_id(); c < (uint32_t)nchunks; c += nwarps) {
-    const int u = cv[c], b = cb[c], e = ce[c];
-    if (b == e) continue;
-    float ru[NC];
+  for (uint32_t c0 = (blockIdx.x * kNW + warp_id()) * PER; c0 < (uint32_t)n; c0 += nslots) {
+    const uint32_t c = c0 + lane / G;
+    const bool has = c < (uint32_t)n;
+    const int u = has ? cv[c] : 0, b = has ? cb[c] : 0, e = has ? ce[c] : 0;
+    float ru[4];
 #pragma unroll
-    for (int q = 0; q < NC; ++q) {
-      const int cc = lane + 32 * q;
-      ru[q] = (cc < nvec) ? R[(int64_t)u * nvec + cc] : 0.f;
-    }
-    for (int k = b; k < e; k += EPS) {
-      int v[EPS];
+    for (int q = 0; q < 4; ++q) ru[q] = has && col + q < nvec ? R[(int64_t)u * nvec + col + q] : 0.f;
+    const int steps = (__reduce_max_sync(0xffffffffu, e - b) + kPprStep - 1) / kPprStep;
+    PprStep<G> cur;
+    cur.load(idx, nullptr, b, e, gl);
+    for (int s = 0; s < steps; ++s) {
+      const int k = b + s * kPprStep;
+      PprStep<G> nxt;
+      nxt.load(idx, nullptr, k + kPprStep, e, gl);
+      float dot[kPprStep];
+      float4 row[kPprStep];
 #pragma unroll
-      for (int j = 0; j < EPS; ++j) v[j] = (k + j < e) ? col[k + j] : -1;
-      float dot[EPS];
-#pragma unroll
-      for (int j = 0; j < EPS; ++j) {
-        dot[j] = 0.f;
-        if (v[j] >= 0) {
-#pragma unroll
-          for (int q = 0; q < NC; ++q) {
-            const int cc = lane + 32 * q;
-            if (cc < nvec) dot[j] = fmaf(__ldg(&lam[(int64_t)v[j] * nvec + cc]), ru[q], dot[j]);
-          }
-        }
+      for (int j = 0; j < kPprStep; ++j) {
+        const int v = cur.edge(j);
+        row[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (v >= 0 && col < nv) row[j] = __ldg(reinterpret_cast<const float4 *>(lam + (int64_t)v * nv + col));
       }
 #pragma unroll
-      for (int j = 0; j < EPS; ++j) {
+      for (int j = 0; j < kPprStep; ++j) {
+        dot[j] = fmaf(row[j].w, ru[3], fmaf(row[j].z, ru[2], fmaf(row[j].y, ru[1], row[j].x * ru[0])));
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) dot[j] += __shfl_xor_sync(0xffffffffu, dot[j], o);
+        for (int o = G / 2; o > 0; o >>= 1) dot[j] += __shfl_xor_sync(0xffffffffu, dot[j], o);
       }
-      // lane j writes edge k + j
-      float mine = dot[0];
+      // lane l of the group writes edge k + l (and k + l + G, ...)
 #pragma unroll
-      for (int j = 1; j < EPS; ++j)
-        if (lane == j) mine = dot[j];
-      if (lane < EPS && k + lane < e) grad_w[k + lane] = d * mine;
+      for (int j = 0; j < kPprStep; ++j)
+        if (gl == j % G && k + j < e) grad_w[k + j] = d * dot[j];
+      cur = nxt;
     }
-    if (lane == 0) my_bytes += 4ull * nvec + (unsigned long long)(e - b) * (8ull + 4ull * nvec);
+    if (has && gl == 0) my_bytes += 4ull * nvec + (unsigned long long)(e - b) * (8ull + 4ull * nv);
   }
   add_bytes(ctl, KID_PPR, my_bytes);
 }
@@ -316,9 +285,14 @@ __global__ void k_ppr_rhs_norm(const float *rhs, int64_t n, Ctl *ctl) {
   if (threadIdx.x == 0 && sum != 0.0) atomicAdd(&ctl->acc[2], sum);
 }
 
-__global__ void k_scale_copy(const float *src, float *dst, float s, int64_t n) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    dst[i] = s * src[i];
+// dst[i][0..nd) = s * src[i][0..ns) for V rows, columns past ns zero: to and
+// from the padded rows of a solve.
+__global__ void k_rows_f32(const float *src, int32_t ns, float *dst, int32_t nd, float s, int64_t V) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < V * nd; i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t r = ns == nd ? 0 : i / nd;
+    const int32_t c = ns == nd ? 0 : (int32_t)(i - r * nd);
+    dst[i] = ns == nd ? s * src[i] : c < ns ? s * src[r * ns + c] : 0.f;
+  }
 }
 
 __global__ void k_copy_f32(const float *src, float *dst, int64_t n) {
@@ -331,32 +305,43 @@ __global__ void k_gather_f32(const int32_t *idx, const float *src, float *dst, i
     dst[i] = src[idx[i]];
 }
 
-// Chunk plan for the solve over `off` (host copy of the offsets).
+// Chunk plan for the solve over `off` (host copy of the offsets): the chunks in
+// descending order of length, by a counting sort over the lengths (stable, so a
+// length's chunks stay in vertex order and read neighbouring indices). Partial
+// slots and split vertices stay in vertex order.
 static int build_plan(mg_graph *g, const std::vector<int32_t> &off, mg_graph::PprPlan *p, cudaStream_t s) {
   const int64_t V = g->nodes;
-  std::vector<int32_t> cv, cb, ce, cs, mv, mf;
+  std::vector<int64_t> at(kPprChunk + 2, 0);  // at[kPprChunk - len + 1]: chunks of a length, then their first place
+  for (int64_t v = 0; v < V; ++v) {
+    const int32_t len = off[v + 1] - off[v];
+    if (len > kPprChunk) at[1] += len / kPprChunk;
+    if (len <= kPprChunk || len % kPprChunk) at[kPprChunk - (len <= kPprChunk ? len : len % kPprChunk) + 1] += 1;
+  }
+  const int64_t n_empty = at[kPprChunk + 1];
+  for (int i = 1; i < kPprChunk + 2; ++i) at[i] += at[i - 1];
+  const size_t n = (size_t)at[kPprChunk + 1];
+  std::vector<int32_t> cv(n), cb(n), ce(n), cs(n), mv, mf;
   int32_t slots = 0;
+  auto put = [&](int64_t v, int32_t b, int32_t e, int32_t slot) {
+    const int64_t i = at[kPprChunk - (e - b)]++;
+    cv[i] = (int32_t)v;
+    cb[i] = b;
+    ce[i] = e;
+    cs[i] = slot;
+  };
   for (int64_t v = 0; v < V; ++v) {
     const int32_t b = off[v], e = off[v + 1];
     if (e - b <= kPprChunk) {
-      cv.push_back((int32_t)v);
-      cb.push_back(b);
-      ce.push_back(e);
-      cs.push_back(-1);
+      put(v, b, e, -1);
     } else {
       mv.push_back((int32_t)v);
       mf.push_back(slots);
-      for (int32_t x = b; x < e; x += kPprChunk) {
-        cv.push_back((int32_t)v);
-        cb.push_back(x);
-        ce.push_back(std::min(e, x + kPprChunk));
-        cs.push_back(slots++);
-      }
+      for (int32_t x = b; x < e; x += std::min(kPprChunk, e - x)) put(v, x, x + std::min(kPprChunk, e - x), slots++);
     }
   }
   mf.push_back(slots);
   int st;
-  const size_t nc = std::max<size_t>(cv.size(), 1), nm = std::max<size_t>(mv.size(), 1);
+  const size_t nc = std::max<size_t>(n, 1), nm = std::max<size_t>(mv.size(), 1);
   if ((st = device_alloc(g, (void **)&p->cv, nc * 4)) != MG_OK ||
       (st = device_alloc(g, (void **)&p->cb, nc * 4)) != MG_OK ||
       (st = device_alloc(g, (void **)&p->ce, nc * 4)) != MG_OK ||
@@ -376,12 +361,22 @@ static int build_plan(mg_graph *g, const std::vector<int32_t> &off, mg_graph::Pp
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) return cuda_status(e, "ppr plan upload");
   p->nchunks = (int32_t)cv.size();
+  p->nfull = (int32_t)(cv.size() - (size_t)n_empty);
   p->nmulti = (int32_t)mv.size();
   p->nslots = slots;
   return MG_OK;
 }
 
-static int ppr_prepare(mg_graph *g, int32_t nvec, cudaStream_t s) {
+// Row stride of a solve's matrices.
+static int32_t ppr_stride(int32_t nvec) { return (nvec + 3) & ~3; }
+// Lanes per chunk: a power of two of 4-column lanes that covers a row.
+static int ppr_group(int32_t nv) {
+  int gsz = 1;
+  while (gsz * 4 < nv) gsz *= 2;
+  return gsz;
+}
+
+static int ppr_prepare(mg_graph *g, int32_t nv, cudaStream_t s) {
   int st;
   if (!g->ppr_plan[0].cv) {
     const int64_t V = g->nodes;
@@ -393,15 +388,15 @@ static int ppr_prepare(mg_graph *g, int32_t nvec, cudaStream_t s) {
     if ((st = build_plan(g, co, &g->ppr_plan[0], s)) != MG_OK) return st;
     if ((st = build_plan(g, ro, &g->ppr_plan[1], s)) != MG_OK) return st;
   }
-  if (g->ppr_cap_nvec < nvec) {
+  if (g->ppr_cap_nvec < nv) {
     const size_t V = (size_t)g->nodes;
     const int32_t slots = std::max(std::max(g->ppr_plan[0].nslots, g->ppr_plan[1].nslots), 1);
-    if ((st = device_alloc(g, (void **)&g->ppr_x[0], V * nvec * 4)) != MG_OK ||
-        (st = device_alloc(g, (void **)&g->ppr_x[1], V * nvec * 4)) != MG_OK ||
-        (st = device_alloc(g, (void **)&g->ppr_rhs, V * nvec * 4)) != MG_OK ||
-        (st = device_alloc(g, (void **)&g->ppr_partial, (size_t)slots * nvec * 4)) != MG_OK)
+    if ((st = device_alloc(g, (void **)&g->ppr_x[0], V * nv * 4)) != MG_OK ||
+        (st = device_alloc(g, (void **)&g->ppr_x[1], V * nv * 4)) != MG_OK ||
+        (st = device_alloc(g, (void **)&g->ppr_rhs, V * nv * 4)) != MG_OK ||
+        (st = device_alloc(g, (void **)&g->ppr_partial, (size_t)slots * nv * 4)) != MG_OK)
       return st;
-    g->ppr_cap_nvec = nvec;
+    g->ppr_cap_nvec = nv;
   }
   if (!g->ppr_w && (st = device_alloc(g, (void **)&g->ppr_w, (size_t)g->edges * 4 + 64)) != MG_OK) return st;
   return MG_OK;
@@ -422,8 +417,9 @@ static int ppr_solve(mg_graph *g, int dir, const float *w, const float *rhs, flo
   const mg_graph::PprPlan &p = g->ppr_plan[dir];
   // The level loop is captured once and replayed: its kernels read the inputs
   // from the graph's own buffers, so callers may pass different pointers.
-  const int64_t n = (int64_t)g->nodes * nvec;
-  k_copy_f32<<<g->num_sms * 4, 256, 0, s>>>(rhs, g->ppr_rhs, n);
+  const int32_t nv = ppr_stride(nvec);
+  const int64_t n = (int64_t)g->nodes * nv;
+  k_rows_f32<<<g->num_sms * 8, 256, 0, s>>>(rhs, nvec, g->ppr_rhs, nv, 1.0f, g->nodes);
   // the weights in the order the solve reads its adjacency (CSC order for the
   // forward pull, so no edge-id indirection per edge and iteration)
   if (dir == 0) k_gather_f32<<<g->num_sms * 4, 256, 0, s>>>(g->csr.csc_eid, w, g->ppr_w, g->edges);
@@ -432,9 +428,7 @@ static int ppr_solve(mg_graph *g, int dir, const float *w, const float *rhs, flo
   w = g->ppr_w;
   rhs = g->ppr_rhs;
   PprArgs a;
-  a.off = dir == 0 ? g->csr.csc_offsets : g->csr.row_offsets;
   a.idx = dir == 0 ? g->csr.csc_rows : g->csr.col;
-  a.eid = nullptr;
   a.w = w;
   a.rhs = rhs;
   a.alpha = alpha;
@@ -449,8 +443,9 @@ static int ppr_solve(mg_graph *g, int dir, const float *w, const float *rhs, flo
   a.mv = p.mv;
   a.mfirst = p.mfirst;
   a.nchunks = p.nchunks;
+  a.nfull = p.nfull;
   a.nmulti = p.nmulti;
-  a.nvec = nvec;
+  a.nv = nv;
   a.V = g->csr.V;
   a.ctl = g->ws.ctl;
   // start from the right-hand side
@@ -461,24 +456,22 @@ static int ppr_solve(mg_graph *g, int dir, const float *w, const float *rhs, flo
   count_launch(3);
   const int grid = persistent_grid(g, o, 4);
   const double tol = o->tolerance;
-  const bool two = nvec > 32;
-  const bool vec = nvec % 4 == 0;  // 16-byte rows: the vector variant
   LevelBody body = [=](cudaStream_t ss, cudaGraphConditionalHandle h, int use_h) {
-    if (two) {
-      if (vec) MG_LAUNCH(KID_PPR, ss, k_ppr_iter_v<16><<<grid, kNT, 0, ss>>>(a));
-      else MG_LAUNCH(KID_PPR, ss, k_ppr_iter<2><<<grid, kNT, 0, ss>>>(a));
-      MG_LAUNCH(KID_PPR, ss, k_ppr_fixup<2><<<grid, kNT, 0, ss>>>(a));
-    } else {
-      if (vec) MG_LAUNCH(KID_PPR, ss, k_ppr_iter_v<8><<<grid, kNT, 0, ss>>>(a));
-      else MG_LAUNCH(KID_PPR, ss, k_ppr_iter<1><<<grid, kNT, 0, ss>>>(a));
-      MG_LAUNCH(KID_PPR, ss, k_ppr_fixup<1><<<grid, kNT, 0, ss>>>(a));
+    switch (ppr_group(nv)) {
+      case 1: MG_LAUNCH(KID_PPR, ss, k_ppr_iter<1><<<grid, kNT, 0, ss>>>(a)); break;
+      case 2: MG_LAUNCH(KID_PPR, ss, k_ppr_iter<2><<<grid, kNT, 0, ss>>>(a)); break;
+      case 4: MG_LAUNCH(KID_PPR, ss, k_ppr_iter<4><<<grid, kNT, 0, ss>>>(a)); break;
+      case 8: MG_LAUNCH(KID_PPR, ss, k_ppr_iter<8><<<grid, kNT, 0, ss>>>(a)); break;
+      default: MG_LAUNCH(KID_PPR, ss, k_ppr_iter<16><<<grid, kNT, 0, ss>>>(a));
     }
+    if (nv > 32) MG_LAUNCH(KID_PPR, ss, k_ppr_fixup<2><<<grid, kNT, 0, ss>>>(a));
+    else MG_LAUNCH(KID_PPR, ss, k_ppr_fixup<1><<<grid, kNT, 0, ss>>>(a));
     MG_LAUNCH(KID_OTHER, ss, k_ppr_level_end<<<1, 32, 0, ss>>>(a.ctl, tol, h, use_h));
   };
   char key[160];
   // (ppr_cap_nvec: a wider solve replaced the buffers the cached graph's arguments point to)
-  snprintf(key, sizeof(key), "%s/%d/%d/%d/%.9g/%.17g/%.17g", name, grid, nvec, g->ppr_cap_nvec, (double)alpha,
-           o->damping, tol);
+  snprintf(key, sizeof(key), "%s/%d/%d/%d/%.9g/%.17g/%.17g", name, grid, nv, g->ppr_cap_nvec, (double)alpha, o->damping,
+           tol);
   int st = run_level_loop(g, s, key, 3, body, o->use_cuda_graph != 0, res);
   if (st != MG_OK) return st;
   finish_run(g, res->ctl.level);
@@ -529,14 +522,18 @@ int mg_ppr_forward(mg_graph *g, const float *edge_weights, const float *teleport
   if (!(o->damping >= 0.0 && o->damping < 1.0)) return set_error(MG_ERR_ARG, "damping must be in [0, 1)");
   cudaStream_t s = run_stream(g, o);
   int st = prepare_run(g, s);
-  if (st != MG_OK || (st = ppr_prepare(g, nvec, s)) != MG_OK) return st;
+  if (st != MG_OK || (st = ppr_prepare(g, ppr_stride(nvec), s)) != MG_OK) return st;
   float *x = nullptr;
   LoopResult res;
   if ((st = ppr_solve(g, 0, edge_weights, teleport, (float)(1.0 - o->damping), nvec, o, s, "ppr_fwd", &x, &res)) !=
       MG_OK)
     return st;
   ppr_stats(stats, res, o->tolerance, g);
-  return copy_out(s, ranks, x, (size_t)g->nodes * nvec * 4, true);
+  const int32_t nv = ppr_stride(nvec);
+  if (nv == nvec) return copy_out(s, ranks, x, (size_t)g->nodes * nvec * 4, true);
+  k_rows_f32<<<g->num_sms * 8, 256, 0, s>>>(x, nv, ranks, nvec, 1.0f, g->nodes);
+  count_launch();
+  return cuda_status(cudaStreamSynchronize(s), "ppr forward");
 }
 
 int mg_ppr_backward(mg_graph *g, const float *edge_weights, const float *ranks, const float *grad_ranks, int32_t nvec,
@@ -555,24 +552,30 @@ int mg_ppr_backward(mg_graph *g, const float *edge_weights, const float *ranks, 
   if (!(o->damping >= 0.0 && o->damping < 1.0)) return set_error(MG_ERR_ARG, "damping must be in [0, 1)");
   cudaStream_t s = run_stream(g, o);
   int st = prepare_run(g, s);
-  if (st != MG_OK || (st = ppr_prepare(g, nvec, s)) != MG_OK) return st;
+  if (st != MG_OK || (st = ppr_prepare(g, ppr_stride(nvec), s)) != MG_OK) return st;
   float *lam = nullptr;
   LoopResult res;
   if ((st = ppr_solve(g, 1, edge_weights, grad_ranks, 1.0f, nvec, o, s, "ppr_adj", &lam, &res)) != MG_OK) return st;
   const int grid = persistent_grid(g, o, 4);
   if (grad_edge_weights) {
     const mg_graph::PprPlan &pl = g->ppr_plan[1];  // chunks of the out-edge rows
-    if (nvec > 32)
-      k_ppr_edge_grad<2><<<grid, kNT, 0, s>>>(pl.cv, pl.cb, pl.ce, pl.nchunks, g->csr.col, nvec, lam, ranks,
-                                              (float)o->damping, grad_edge_weights, g->ws.ctl);
-    else
-      k_ppr_edge_grad<1><<<grid, kNT, 0, s>>>(pl.cv, pl.cb, pl.ce, pl.nchunks, g->csr.col, nvec, lam, ranks,
-                                              (float)o->damping, grad_edge_weights, g->ws.ctl);
+    const int32_t nv = ppr_stride(nvec);
+    auto launch = [&](auto kernel) {
+      kernel<<<grid, kNT, 0, s>>>(pl.cv, pl.cb, pl.ce, pl.nfull, g->csr.col, nvec, nv, lam, ranks, (float)o->damping,
+                                  grad_edge_weights, g->ws.ctl);
+    };
+    switch (ppr_group(nv)) {
+      case 1: launch(k_ppr_edge_grad<1>); break;
+      case 2: launch(k_ppr_edge_grad<2>); break;
+      case 4: launch(k_ppr_edge_grad<4>); break;
+      case 8: launch(k_ppr_edge_grad<8>); break;
+      default: launch(k_ppr_edge_grad<16>);
+    }
     count_launch();
   }
   if (grad_teleport) {
-    k_scale_copy<<<g->num_sms * 4, 256, 0, s>>>(lam, grad_teleport, (float)(1.0 - o->damping),
-                                                (int64_t)g->nodes * nvec);
+    k_rows_f32<<<g->num_sms * 8, 256, 0, s>>>(lam, ppr_stride(nvec), grad_teleport, nvec, (float)(1.0 - o->damping),
+                                              g->nodes);
     count_launch();
   }
   ppr_stats(stats, res, o->tolerance, g);

@@ -79,6 +79,14 @@ def _ppr_check(torch, g, hg, src, w, t, c):
     assert (tt.grad.double().cpu() - ref_t).norm() / ref_t.norm() < 1e-4
 
 
+@pytest.mark.parametrize("nvec", [1, 3, 4, 5, 8, 9, 16, 17, 32, 33, 61, 64])
+def test_ppr_every_row_width(nvec):
+    # 1, 2, 4, 8 and 16 lanes per list, with and without padding columns
+    torch = pytest.importorskip("torch")
+    hg, src, w, t, c = _ppr_case(nvec)
+    _ppr_check(torch, Graph(hg, directed=True), hg, src, w, t, c)
+
+
 def test_ppr_width_grows_and_shrinks_on_one_graph():
     # the workspace is replaced when the rows get wider; a narrower solve after that must use the new one
     torch = pytest.importorskip("torch")
@@ -87,3 +95,23 @@ def test_ppr_width_grows_and_shrinks_on_one_graph():
     for nvec in (4, 32, 4, 7, 64, 32, 1):
         _, src, w, t, c = _ppr_case(nvec)
         _ppr_check(torch, g, hg, src, w, t, c)
+
+
+@pytest.mark.parametrize("length", [0, 1, 7, 8, 9, 255, 256, 257, 513])
+def test_ppr_list_lengths(length):
+    # one vertex with `length` in-edges and out-edges: the steps of 8, the chunks of 256 and what is left over
+    torch = pytest.importorskip("torch")
+    n = 600
+    edges = {(v, 0) for v in range(1, length + 1)} | {(0, v) for v in range(20, length + 20)}
+    edges |= {(v, v % 19 + 1) for v in range(1, 40)}
+    src, dst = np.array(sorted(edges)).T
+    ro = np.concatenate([[0], np.cumsum(np.bincount(src, minlength=n))]).astype(np.int32)
+    hg = HostGraph(ro, dst.astype(np.int32), None, directed=True)
+    rng = np.random.default_rng(length)
+    w = rng.uniform(0.1, 1.0, size=hg.edges)
+    w = w / np.bincount(src, weights=w, minlength=n)[src]
+    t = np.zeros((n, 12))
+    for c in range(12):
+        t[rng.choice(n, 30, replace=False), c] = 1 / 30
+    t[0] += 0.1
+    _ppr_check(torch, Graph(hg, directed=True), hg, src, w, t, rng.standard_normal((n, 12)))
