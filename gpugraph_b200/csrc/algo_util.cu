@@ -12,6 +12,15 @@ int copy_out(cudaStream_t s, void *dst, const void *src, size_t bytes, bool dst_
   return cuda_status(e, "result copy");
 }
 
+bool on_device(const mg_graph *g, const void *p) {
+  cudaPointerAttributes at;
+  if (!p || cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return at.type == cudaMemoryTypeDevice && at.device == g->device;
+}
+
 __global__ void k_reach_stats(const int32_t *vals, int32_t unreached, int nsrc, int stride, const int32_t *ro, int32_t V,
                               unsigned long long *out) {
   unsigned long long cnt = 0, edg = 0;

@@ -16,6 +16,9 @@ namespace mg {
 // and waits for it.
 int copy_out(cudaStream_t s, void *dst, const void *src, size_t bytes, bool dst_on_device);
 
+// True for memory of the graph's own GPU, which a kernel may use as its working array.
+bool on_device(const mg_graph *g, const void *p);
+
 // vertices_reached / edges_traversed: vertices whose value differs from
 // `unreached`, and the sum of their out-degrees (MapGraph "visited edges").
 // vals is [V] or, with stride_src > 1, [V][stride_src] interleaved values of

@@ -18,6 +18,7 @@
 #include "gas/driver.cuh"
 #include "gas/engine.cuh"
 #include "gas/programs.cuh"
+#include "grid_loop.cuh"
 
 namespace mg {
 
@@ -467,6 +468,47 @@ __global__ void k_bfs_start(Ctl *ctl, int32_t *queue0, int32_t root, int32_t *la
   }
 }
 
+int bfs_loop_run(mg_graph *g, cudaStream_t s, const std::vector<int32_t> &roots, uint32_t max_iter,
+                 const mg_options *o, int32_t *labels);  // bfs_loop.cu
+
+// The whole BFS in one launch: the depths go straight to the caller's device
+// buffer, the statistics come with the result block.
+static int bfs_one_launch(mg_graph *g, cudaStream_t s, const std::vector<int32_t> &roots, uint32_t max_iter,
+                          int32_t *depths, mg_stats *stats, const mg_options *o, int32_t *preds) {
+  if (!depths) return set_error(MG_ERR_ARG, "output pointer is NULL");
+  const bool dev = o->outputs_on_device != 0;
+  const cudaMemcpyKind kind = dev ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
+  const size_t bytes = (size_t)g->nodes * 4;
+  const bool direct = dev && on_device(g, depths);
+  int32_t *labels = direct ? depths : g->ws.vbuf[0];
+  int st = bfs_loop_run(g, s, roots, max_iter, o, labels);
+  if (st != MG_OK) return st;
+  cudaError_t e = cudaSuccess;
+  if (preds) {
+    k_bfs_pred<<<g->num_sms * 8, kNT, 0, s>>>(g->csr.csc_offsets, g->csr.csc_rows, labels, g->ws.vbuf[1],
+                                              (int)g->nodes);
+    count_launch();
+    if ((st = launch_check("bfs predecessors")) != MG_OK) return st;
+    e = cudaMemcpyAsync(preds, g->ws.vbuf[1], bytes, kind, s);
+  }
+  if (e == cudaSuccess && !direct) e = cudaMemcpyAsync(depths, labels, bytes, kind, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  if ((st = cuda_status(e, "bfs")) != MG_OK || (st = loop_end(g, s, "bfs")) != MG_OK) return st;
+  if (stats) {
+    const LoopOut &r = *g->loop_out;
+    float ms = 0.f;
+    cudaEventElapsedTime(&ms, g->ev0, g->ev1);
+    stats->iterations = (int32_t)r.level;
+    stats->push_iterations = (int32_t)r.push_levels;
+    stats->pull_iterations = (int32_t)r.pull_levels;
+    stats->converged = r.frontier_size == 0 ? 1 : 0;
+    stats->device_ms = ms;
+    stats->vertices_reached = (int64_t)r.visited_count;
+    stats->edges_traversed = want_stats(o) ? (int64_t)r.visited_edges : 0;
+  }
+  return MG_OK;
+}
+
 // Shared by mg_bfs, mg_bfs_roots and mg_bfs_batch.
 // `preds` (optional): predecessors by the pred_extract rule (k_bfs_pred).
 int bfs_run(mg_graph *g, const std::vector<int32_t> &roots, int32_t *depths, mg_stats *stats, const mg_options *o,
@@ -482,6 +524,14 @@ int bfs_run(mg_graph *g, const std::vector<int32_t> &roots, int32_t *depths, mg_
   cudaStream_t s = run_stream(g, o);
   int st = ensure_workspace(g);
   if (st != MG_OK) return st;
+  // Every level of a traversal settles at least one vertex, so V + 2 levels bound
+  // the device loop even if a Program never empties its frontier.
+  const uint32_t max_iter = (uint32_t)std::min<int64_t>(o->iter_num > 0 ? o->iter_num : 0, g->nodes + 2);
+  // Default: one launch. The level-by-level loop below serves the host-driven
+  // runs (use_cuda_graph = 0, profiling), the ordered frontier and callers that
+  // shorten the waits (a grid barrier waits for the slowest CTA of a level).
+  if (o->use_cuda_graph && !o->ordered_frontier && !prof_on() && o->spin_limit >= kSpinLimitDefault)
+    return bfs_one_launch(g, s, roots, max_iter, depths, stats, o, preds);
   if ((st = prepare_run(g, s)) != MG_OK) return st;
   Workspace &w = g->ws;
   GasArgs<BfsP> a;
@@ -507,9 +557,6 @@ int bfs_run(mg_graph *g, const std::vector<int32_t> &roots, int32_t *depths, mg_
   a.gather_dir = NO_GATHER_EDGES;
   const int V = (int)g->nodes;
   const uint32_t nsrc = (uint32_t)roots.size();
-  // Every level of a traversal settles at least one vertex, so V + 2 levels bound
-  // the device loop even if a Program never empties its frontier.
-  const uint32_t max_iter = (uint32_t)std::min<int64_t>(o->iter_num > 0 ? o->iter_num : 0, g->nodes + 2);
   // one root goes to the start kernel by value; several are copied to the queue
   const int queue0_ready = nsrc > 1 ? 1 : 0;
   if (queue0_ready) {

@@ -10,6 +10,7 @@
 #include <vector>
 
 #include "graph.cuh"
+#include "grid_loop.cuh"
 #include "host_util.h"
 
 namespace mg {
@@ -70,9 +71,13 @@ int ensure_workspace(mg_graph *g) {
   MG_ALLOC(w.vbuf[0], V * 4);
   MG_ALLOC(w.vbuf[1], V * 4);
   MG_ALLOC(w.ctl, sizeof(Ctl));
+  g->loop_cap = V + E / kRange + 64;
+  MG_ALLOC(g->loop_queue, 2 * g->loop_cap * sizeof(int2));
+  MG_ALLOC(g->loop_ctl, sizeof(LoopCtl));
 #undef MG_ALLOC
   cudaError_t e = cudaMemsetAsync(w.status, 0, w.status_cap * 8, g->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(w.ctl, 0, sizeof(Ctl), g->stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(g->loop_ctl, 0, sizeof(LoopCtl), g->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(w.bm[0], 0, w.words * 4, g->stream);
   if (e == cudaSuccess) e = cudaMemsetAsync(w.bm[1], 0, w.words * 4, g->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
@@ -169,7 +174,9 @@ int create_common(const int32_t *row_offsets, const int32_t *col, const void *va
   cudaError_t e = cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaEventCreate(&g->ev0);
   if (e == cudaSuccess) e = cudaEventCreate(&g->ev1);
-  if (e == cudaSuccess) e = cudaMallocHost((void **)&g->host_ctl, sizeof(Ctl));
+  // the loops' result block shares the pinned allocation
+  if (e == cudaSuccess) e = cudaMallocHost((void **)&g->host_ctl, sizeof(Ctl) + sizeof(LoopOut));
+  if (e == cudaSuccess) g->loop_out = reinterpret_cast<LoopOut *>(g->host_ctl + 1);
   if ((st = cuda_status(e, "stream/event setup")) != MG_OK) {
     mg_graph_destroy(g);
     return st;

@@ -73,6 +73,8 @@ struct Workspace {
 }  // namespace mg
 
 namespace mg {
+struct LoopCtl;
+struct LoopOut;
 // An instantiated level loop (CUDA graph with a WHILE node), cached per graph
 // and per loop body so repeated runs only pay cudaGraphLaunch.
 struct LoopCache {
@@ -133,6 +135,14 @@ struct mg_graph {
   float *ppr_x[2] = {nullptr, nullptr}, *ppr_partial = nullptr;
   float *ppr_rhs = nullptr, *ppr_w = nullptr;  // stable copies of the solve's inputs
   int32_t ppr_cap_nvec = 0;
+  // One-launch loops (grid_loop.cuh): control words, the barrier count the next
+  // run starts from, the result block (behind host_ctl), and room for two queues
+  // of loop_cap edge ranges (a range per found vertex and kRange edges).
+  mg::LoopCtl *loop_ctl = nullptr;
+  mg::LoopOut *loop_out = nullptr;
+  uint32_t loop_base = 0;
+  int2 *loop_queue = nullptr;
+  size_t loop_cap = 0;
   size_t device_bytes = 0;
   uint64_t epochs_used = 0;  // look-back epochs consumed since the status words were cleared
   std::vector<void *> allocations;

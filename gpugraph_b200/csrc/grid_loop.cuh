@@ -1,0 +1,90 @@
+// Whole traversals in one cooperative launch: a grid barrier with a bounded
+// wait, the per-level totals that travel with it, and the result block the host
+// reads. Used where a level's work is short beside the launches of a
+// level-by-level loop (12-25 us a level on a B200, against 5-6 us here).
+//
+// The launch is cooperative (cudaLaunchCooperativeKernel), so every CTA is
+// resident and a barrier only waits for CTAs that run. A wait still ends after
+// mg_options.spin_limit polls: the run then stops with MG_ERR_TIMEOUT.
+#pragma once
+#include <cuda_runtime.h>
+
+#include "common.cuh"
+#include "graph.cuh"
+
+namespace mg {
+
+constexpr int kLoopNT = 1024;  // one CTA per SM: the fewest arrivals a barrier can have
+constexpr int kRange = 256;    // edges per entry of a queue of edge ranges
+
+// Device state of a loop. `arrived` grows for the life of the graph (a run
+// starts from the value the host passes in); the totals rotate over three
+// slots, so slot L+1 can be cleared while level L runs.
+struct LoopCtl {
+  unsigned long long count[3];  // vertices found in a level
+  unsigned long long edges[3];  // sum of their out-degrees
+  uint32_t items[3];            // items appended to the next queue
+  uint32_t arrived;
+  int32_t error;
+};
+
+// What the host reads after the launch (pinned memory, written by the kernel).
+struct LoopOut {
+  uint32_t level, push_levels, pull_levels, frontier_size;
+  unsigned long long visited_count, visited_edges;
+  uint32_t barriers;
+  int32_t error;
+};
+
+struct LoopShared {
+  unsigned long long my_count, my_edges;  // this CTA's totals of the level
+  unsigned long long count, edges;        // the grid's, after the level's barrier
+  uint32_t items;
+  int fail;
+};
+
+struct GridLoop {
+  LoopCtl *c;
+  uint32_t base;       // value of c->arrived when the run began
+  unsigned long long spin_limit;
+  LoopOut *out;
+};
+
+// End of a level: adds this CTA's totals (my_count and my_edges, summed by its
+// threads since the last call; cleared here) to slot `slot`, waits for the whole
+// grid and leaves the grid's totals in sh. `n` counts the barriers of the run. False when the wait ran out.
+// Data written before the barrier by any CTA is visible after it to ordinary
+// loads.
+MG_DEVINL bool grid_level_end(const GridLoop &g, LoopShared *sh, uint32_t slot, uint32_t &n) {
+  __syncthreads();
+  ++n;
+  if (threadIdx.x == 0) {
+    if (sh->my_count) atomicAdd(&g.c->count[slot], sh->my_count);
+    if (sh->my_edges) atomicAdd(&g.c->edges[slot], sh->my_edges);
+    sh->my_count = sh->my_edges = 0;
+    __threadfence();
+    atomicAdd(&g.c->arrived, 1u);
+    const uint32_t target = g.base + n * gridDim.x;
+    unsigned long long spins = 0;
+    while ((int32_t)(ld_acquire(&g.c->arrived) - target) < 0) {
+      if (++spins >= g.spin_limit) {
+        sh->fail = 1;
+        break;
+      }
+    }
+    __threadfence();
+    sh->count = *(volatile unsigned long long *)&g.c->count[slot];
+    sh->edges = *(volatile unsigned long long *)&g.c->edges[slot];
+    sh->items = *(volatile uint32_t *)&g.c->items[slot];
+  }
+  __syncthreads();
+  return !sh->fail;
+}
+
+// The GridLoop of a run about to be launched.
+GridLoop loop_begin(mg_graph *g, const mg_options *o);
+// After the stream was synchronised: accounts for the barriers the run used and
+// returns its status.
+int loop_end(mg_graph *g, cudaStream_t s, const char *what);
+
+}  // namespace mg

@@ -124,7 +124,7 @@ void mg_options_init(mg_options *o) {
   o->threshold = 0;
   o->damping = 0.85;
   o->tolerance = 1e-6;
-  o->spin_limit = (int64_t)1 << 22;
+  o->spin_limit = mg::kSpinLimitDefault;
   o->tile_items = 0;
   o->ctas_per_sm = 0;
   o->compute_stats = 1;

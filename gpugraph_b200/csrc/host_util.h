@@ -11,6 +11,8 @@
 
 namespace mg {
 
+constexpr int64_t kSpinLimitDefault = (int64_t)1 << 22;  // mg_options.spin_limit
+
 // Records msg as this thread's last error and returns status unchanged, so a
 // failing path can be written `return set_error(MG_ERR_ARG, "...")`.
 int set_error(int status, const std::string &msg);

@@ -12,10 +12,82 @@ pytestmark = pytest.mark.gpu
 DIRS = [_lib.MG_DIR_AUTO, _lib.MG_DIR_PUSH, _lib.MG_DIR_PULL]
 
 
+def star(n, arms=1):
+    """Vertex 0 joined to every other one (its adjacency spans many queue entries), plus `arms` paths of 3."""
+    edges = [(0, v) for v in range(1, n)]
+    for a in range(arms):
+        b = n + 3 * a
+        edges += [(a + 1, b), (b, b + 1), (b + 1, b + 2)]
+    m = n + 3 * arms
+    src, dst = np.array(edges).T
+    src, dst = np.concatenate([src, dst]), np.concatenate([dst, src])
+    order = np.lexsort((dst, src))
+    ro = np.concatenate([[0], np.cumsum(np.bincount(src, minlength=m))]).astype(np.int32)
+    return HostGraph(ro, dst[order].astype(np.int32), None)
+
+
 def padded(hg, k):
     """hg with k isolated vertices appended."""
     ro = np.concatenate([hg.row_offsets, np.full(k, hg.row_offsets[-1], np.int32)])
     return HostGraph(ro, hg.column_indices, hg.edge_values, hg.directed)
+
+
+# one vertex; a word of vertices and one more; a hub of 255, 256, 257 and 5000 edges (entries hold 256);
+# many levels; a dense graph; a vertex count that is no multiple of 32 or 4
+GRAPHS = {
+    "one": lambda: HostGraph(np.array([0, 0], np.int32), np.zeros(0, np.int32)),
+    "star33": lambda: star(33),
+    "star256": lambda: star(256, 2),
+    "star257": lambda: star(257, 2),
+    "star258": lambda: star(258, 2),
+    "star5001": lambda: star(5001, 40),
+    "road": lambda: HostGraph.road_grid(90, 0.02, 0.0, seed=3),
+    "rmat": lambda: HostGraph.rmat(13, 16, seed=9),
+    "rmat_odd": lambda: padded(HostGraph.rmat(12, 8, seed=5), 3),
+    "directed": lambda: HostGraph.rmat(12, 8, seed=6, symmetrize=False),
+}
+
+
+@pytest.mark.parametrize("name", list(GRAPHS))
+def test_bfs_one_launch_equals_level_loop(name):
+    hg = GRAPHS[name]()
+    g = Graph(hg, directed=name == "directed")
+    deg = hg.out_degree()
+    for s in sorted({0, hg.nodes - 1, int(np.argmax(deg))}):
+        ref = oracle.bfs(hg.row_offsets, hg.column_indices, s)
+        reached = ref >= 0
+        for d in DIRS:
+            for mode in ({}, dict(use_cuda_graph=0), dict(ordered_frontier=1), dict(alpha=1e9, beta=0.5)):
+                out, st = g.bfs(s, direction=d, **mode)
+                assert np.array_equal(out, ref), (s, d, mode)
+                assert st["vertices_reached"] == int(reached.sum())
+                assert st["edges_traversed"] == int(deg[reached].sum())
+                assert st["iterations"] == int(ref.max()) + 1 and st["converged"] == 1
+                assert st["push_iterations"] + st["pull_iterations"] == st["iterations"]
+        for cap in (0, 1, 2):
+            a, sa = g.bfs(s, iter_num=cap)
+            b, sb = g.bfs(s, iter_num=cap, use_cuda_graph=0)
+            assert np.array_equal(a, b) and sa["iterations"] == sb["iterations"]
+            assert sa["converged"] == sb["converged"] and sa["vertices_reached"] == sb["vertices_reached"]
+
+
+def test_bfs_one_launch_roots_and_interleaved_runs():
+    # several roots (more than a warp), other algorithms between runs, and runs on another stream
+    torch = pytest.importorskip("torch")
+    hg = HostGraph.rmat(13, 8, seed=31).with_weights(1, 9, seed=1)
+    g = Graph(hg)
+    rng = np.random.default_rng(0)
+    side = torch.cuda.Stream()
+    for k in (2, 31, 32, 33, 700):
+        roots = rng.choice(hg.nodes, k, replace=False).astype(np.int32)
+        ref = np.stack([oracle.bfs(hg.row_offsets, hg.column_indices, r) for r in roots[:40]])
+        out, _ = g.bfs_roots(roots[:40])
+        best = np.where(ref >= 0, ref, 1 << 30).min(0)
+        assert np.array_equal(out, np.where(best < 1 << 30, best, -1)), k
+        g.cc()
+        a, _ = g.bfs(int(roots[0]), stream=side.cuda_stream)
+        assert np.array_equal(a, ref[0])
+        g.sssp(int(roots[0]))
 
 
 @pytest.mark.parametrize("nsrc", [1, 2, 33, 64])
