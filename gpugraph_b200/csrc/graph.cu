@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstring>
 #include <vector>
 
@@ -208,6 +209,23 @@ int create_common(const int32_t *row_offsets, const int32_t *col, const void *va
       return st;
     }
     e = E ? cudaMemcpy(c.wgt, vals, E * 4, cudaMemcpyHostToDevice) : cudaSuccess;
+    const int32_t *w = static_cast<const int32_t *>(vals);
+    std::atomic<int32_t> lo(INT32_MAX), hi(INT32_MIN);
+    host_parallel_for(edges, [&](int64_t b, int64_t end, unsigned) {
+      int32_t l = INT32_MAX, h = INT32_MIN;
+      for (int64_t j = b; j < end; ++j) {
+        l = std::min(l, w[j]);
+        h = std::max(h, w[j]);
+      }
+      for (int32_t x = lo.load(); l < x && !lo.compare_exchange_weak(x, l);) {
+      }
+      for (int32_t x = hi.load(); h > x && !hi.compare_exchange_weak(x, h);) {
+      }
+    });
+    if (E) {
+      g->weight_min = lo.load();
+      g->weight_max = hi.load();
+    }
     if ((st = cuda_status(e, "edge value upload")) != MG_OK) {
       mg_graph_destroy(g);
       return st;

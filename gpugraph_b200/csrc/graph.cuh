@@ -143,6 +143,7 @@ struct mg_graph {
   uint32_t loop_base = 0;
   int2 *loop_queue = nullptr;
   size_t loop_cap = 0;
+  int32_t weight_min = 0, weight_max = 0;  // range of csr.wgt as int32
   size_t device_bytes = 0;
   uint64_t epochs_used = 0;  // look-back epochs consumed since the status words were cleared
   std::vector<void *> allocations;

@@ -24,6 +24,7 @@ struct LoopCtl {
   unsigned long long count[3];  // vertices found in a level
   unsigned long long edges[3];  // sum of their out-degrees
   uint32_t items[3];            // items appended to the next queue
+  int32_t low[3];               // SSSP: smallest pending distance
   uint32_t arrived;
   int32_t error;
 };
@@ -40,6 +41,7 @@ struct LoopShared {
   unsigned long long my_count, my_edges;  // this CTA's totals of the level
   unsigned long long count, edges;        // the grid's, after the level's barrier
   uint32_t items;
+  int32_t low;
   int fail;
 };
 
@@ -76,6 +78,7 @@ MG_DEVINL bool grid_level_end(const GridLoop &g, LoopShared *sh, uint32_t slot, 
     sh->count = *(volatile unsigned long long *)&g.c->count[slot];
     sh->edges = *(volatile unsigned long long *)&g.c->edges[slot];
     sh->items = *(volatile uint32_t *)&g.c->items[slot];
+    sh->low = *(volatile int32_t *)&g.c->low[slot];
   }
   __syncthreads();
   return !sh->fail;

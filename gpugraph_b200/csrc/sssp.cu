@@ -20,6 +20,7 @@
 
 #include "algo_util.cuh"
 #include "gas/run_gas.cuh"
+#include "grid_loop.cuh"
 
 namespace mg {
 
@@ -162,11 +163,46 @@ __global__ void k_sssp_seed(int32_t *dist, int32_t *queue0, int32_t src) {
 
 }  // namespace
 
+int sssp_loop_run(mg_graph *g, cudaStream_t s, int32_t src, const mg_options *o, int32_t *dist);  // sssp_loop.cu
+
+static int sssp_one_launch(mg_graph *g, cudaStream_t s, int32_t src, int32_t *dists, mg_stats *stats,
+                           const mg_options *o) {
+  const bool dev = o->outputs_on_device != 0, direct = dev && on_device(g, dists);
+  int32_t *dist = direct ? dists : g->ws.vbuf[0];
+  int st = sssp_loop_run(g, s, src, o, dist);
+  if (st != MG_OK) return st;
+  cudaError_t e = cudaSuccess;
+  if (!direct)
+    e = cudaMemcpyAsync(dists, dist, (size_t)g->nodes * 4, dev ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  if ((st = cuda_status(e, "sssp")) != MG_OK || (st = loop_end(g, s, "sssp")) != MG_OK) return st;
+  if (stats) {
+    float ms = 0.f;
+    cudaEventElapsedTime(&ms, g->ev0, g->ev1);
+    stats->iterations = stats->push_iterations = (int32_t)g->loop_out->level;
+    stats->pull_iterations = 0;
+    stats->converged = g->loop_out->frontier_size == 0 ? 1 : 0;
+    stats->device_ms = ms;
+    stats->vertices_reached = 0;
+    stats->edges_traversed = 0;
+    if (want_stats(o) && (st = reach_stats(g, s, dist, sssp_relax::INIT_VALUE, 1, 1, &stats->vertices_reached,
+                                           &stats->edges_traversed)) != MG_OK)
+      return st;
+  }
+  return MG_OK;
+}
+
 // Fused single-source SSSP (called by mg_sssp).
 int sssp_fused(mg_graph *g, int32_t src, int32_t *dists, mg_stats *stats, const mg_options *o) {
   cudaStream_t s = run_stream(g, o);
   int st = prepare_run(g, s);
   if (st != MG_OK) return st;
+  // Default: one launch. The level loop below serves the host-driven runs
+  // (use_cuda_graph = 0, profiling), the ordered frontier, a limit on the levels
+  // (a window is not a level), callers that shorten the waits, and negative weights.
+  if (o->use_cuda_graph && !o->ordered_frontier && !prof_on() && o->spin_limit >= kSpinLimitDefault &&
+      (int64_t)o->iter_num >= g->nodes + 2 && g->weight_min >= 0)
+    return sssp_one_launch(g, s, src, dists, stats, o);
   using P = sssp_relax;
   GasArgs<P> a = base_args<P>(g);
   a.vl.dist = g->ws.vbuf[0];

@@ -1,0 +1,213 @@
+// Single-source SSSP in one cooperative launch (grid_loop.cuh), by distance
+// windows. The vertices whose distance was lowered and not yet relaxed are the
+// bits of a pending bitmap. A step selects those below the window's end (the
+// smallest pending distance plus `delta`), turns them into edge ranges, and
+// relaxes the ranges: an improving candidate lowers the head's distance and
+// sets its pending bit, both without waiting for a result. With non-negative
+// weights the smallest pending distance is final, so every step settles a
+// vertex and V steps suffice; the fixpoint is the one of the level-by-level
+// loop (sssp.cu), the unique shortest distances.
+//
+// Why windows: on a power-law graph relaxing every pending vertex per level
+// expands 3.0 times the edges (R-MAT 17, weights 1..64, simulated), a window of
+// a few weights 1.3 to 1.9 times. It takes two to four times as many steps,
+// which only pays with steps as cheap as here (two grid barriers and no scan;
+// the level loop lost by it: 4.7 against 3.3 ms at R-MAT 22). R-MAT 21: 1.8 ms a
+// run level by level, 1.3 here.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <climits>
+
+#include "algo_util.cuh"
+#include "gas/driver.cuh"
+#include "gas/programs.cuh"
+#include "grid_loop.cuh"
+
+namespace mg {
+
+constexpr int kSpU = 8;        // edges per lane in flight (R-MAT 21: 1.30 ms a run, 1.38 with 4)
+constexpr int kSpWords = 4;    // pending words per warp and step of the selection
+// Window: this many times the largest weight over the mean degree (with uniform
+// weights a vertex has about that many edges inside it). R-MAT 21, weights
+// 1..64: 1.39 ms a run at 2, 1.38 at 4, 1.44 at 8, 1.52 at 32 (no window in effect).
+constexpr double kSsspWindow = 4.0;
+
+struct SsspLoopArgs {
+  DevCsr g;
+  int32_t *dist;
+  uint32_t *pending;
+  int4 *q;       // (first edge, length, distance of the tail, unused)
+  uint32_t cap;  // entries of q
+  int32_t src, delta;
+  uint32_t max_iter;
+  GridLoop loop;
+};
+
+__global__ void __launch_bounds__(kLoopNT, 1) k_sssp_loop(SsspLoopArgs a) {
+  constexpr int32_t INF = programs::sssp::INIT_VALUE;
+  __shared__ LoopShared sh;
+  __shared__ int s_min;
+  const int lane = lane_id();
+  const uint32_t V = (uint32_t)a.g.V, words = (V + 31) / 32;
+  const uint32_t tid = blockIdx.x * kLoopNT + threadIdx.x, nt = gridDim.x * kLoopNT;
+  const uint32_t nw = nt / 32, gw = warp_id() * gridDim.x + blockIdx.x;
+  const int32_t *ro = a.g.row_offsets, *col = a.g.col, *wgt = a.g.wgt;
+  LoopCtl *c = a.loop.c;
+  if (threadIdx.x == 0) {
+    sh.my_count = sh.my_edges = 0;
+    sh.fail = 0;
+    s_min = INT_MAX;
+  }
+  __syncthreads();
+  for (uint32_t i = tid; i < V; i += nt) a.dist[i] = i == (uint32_t)a.src ? 0 : INF;
+  for (uint32_t i = tid; i < words; i += nt) a.pending[i] = i == (uint32_t)a.src >> 5 ? 1u << (a.src & 31) : 0u;
+  if (blockIdx.x == 0 && threadIdx.x < 3) {
+    c->count[threadIdx.x] = c->edges[threadIdx.x] = 0;
+    c->items[threadIdx.x] = 0;
+    c->low[threadIdx.x] = INT_MAX;
+    if (threadIdx.x == 0) c->error = 0;
+  }
+  uint32_t nbar = 0, step = 0;
+  bool ok = grid_level_end(a.loop, &sh, 2, nbar);
+  int low = 0;  // smallest pending distance
+  while (ok && low != INT_MAX && step < a.max_iter) {
+    const uint32_t slot = step % 3;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      c->items[(step + 1) % 3] = 0;
+      c->low[(step + 1) % 3] = INT_MAX;
+    }
+    const int end = (int)min((long long)INT_MAX - 1, (long long)low + a.delta);
+    int rest = INT_MAX;  // smallest pending distance past the window
+    // selection: kSpWords words per warp step, a lane a vertex of each
+    for (uint32_t w0 = gw * kSpWords; w0 < words; w0 += nw * kSpWords) {
+      const uint32_t mine = lane < kSpWords && w0 + lane < words ? __ldcg(&a.pending[w0 + lane]) : 0u;
+      if (!__any_sync(0xffffffffu, mine != 0u)) continue;
+      int d[kSpWords], b[kSpWords], n[kSpWords];
+      bool sel[kSpWords];
+      uint32_t x[kSpWords];
+#pragma unroll
+      for (int k = 0; k < kSpWords; ++k) {
+        x[k] = __shfl_sync(0xffffffffu, mine, k);
+        const uint32_t v = (w0 + k) * 32 + lane;
+        sel[k] = (x[k] >> lane) & 1u;
+        d[k] = sel[k] ? __ldcg(&a.dist[v]) : INT_MAX;
+        b[k] = sel[k] ? ro[v] : 0;
+        n[k] = sel[k] ? ro[v + 1] : 0;
+      }
+      uint32_t need = 0;
+#pragma unroll
+      for (int k = 0; k < kSpWords; ++k) {
+        if (sel[k] && d[k] >= end) {
+          rest = min(rest, d[k]);
+          sel[k] = false;
+        }
+        n[k] = sel[k] ? n[k] - b[k] : 0;
+        const uint32_t bal = __ballot_sync(0xffffffffu, sel[k]);
+        if (lane == 0 && bal) a.pending[w0 + k] = x[k] & ~bal;
+        need += (uint32_t)(n[k] + kRange - 1) / kRange;
+      }
+      if (!__any_sync(0xffffffffu, need != 0u)) continue;
+      const uint32_t inc = warp_inclusive_sum(need);
+      uint32_t at = 0;
+      if (lane == 31) at = atomicAdd(&c->items[slot], inc);
+      at = __shfl_sync(0xffffffffu, at, 31) + inc - need;
+      if (at + need > a.cap) {
+        atomicCAS(&c->error, 0, (int)MG_ERR_OVERFLOW);
+      } else {
+#pragma unroll
+        for (int k = 0; k < kSpWords; ++k)
+          for (int i = 0; i < n[k]; i += kRange)
+            a.q[at++] = make_int4(b[k] + i, min(kRange, n[k] - i), d[k], 0);
+      }
+    }
+    rest = __reduce_min_sync(0xffffffffu, rest);
+    if (lane == 0 && rest != INT_MAX) atomicMin(&s_min, rest);
+    if (!(ok = grid_level_end(a.loop, &sh, slot, nbar))) break;
+    // relaxation of the selected ranges
+    const uint32_t n = sh.items;
+    // ranges are dealt one by one over the warps (a hub's full ranges are
+    // neighbours in the queue: in blocks of 32 they would land on a few warps)
+    const uint32_t per = min(32u, (n + nw - 1) / nw);
+    int best = INT_MAX;  // smallest distance written
+    for (uint32_t base = gw; base < n; base += nw * per) {
+      int4 r = make_int4(0, 0, 0, 0);
+      if (lane < (int)per && base + lane * nw < n) r = __ldcg(&a.q[base + lane * nw]);
+      const int inc = warp_inclusive_sum(r.y);
+      const int total = __shfl_sync(0xffffffffu, inc, 31);
+      const int off = r.x - (inc - r.y);
+      for (int t = 0; t < total; t += 32 * kSpU) {
+        int u[kSpU], cand[kSpU], dv[kSpU];
+#pragma unroll
+        for (int k = 0; k < kSpU; ++k) {
+          const int p = t + 32 * k + lane;
+          int own = 0;  // the first range that ends past p
+          if (per > 1) {
+#pragma unroll
+            for (int s = 16; s > 0; s >>= 1)
+              if (__shfl_sync(0xffffffffu, inc, own + s - 1) <= p) own += s;
+            own = min(own, 31);
+          }
+          const int e = __shfl_sync(0xffffffffu, off, own) + p;
+          const int du = __shfl_sync(0xffffffffu, r.z, own);
+          const bool in = p < total && (unsigned)e < (unsigned)a.g.E;
+          u[k] = in ? __ldcs(col + e) : -1;
+          cand[k] = in ? du + __ldcs(wgt + e) : 0;
+        }
+#pragma unroll
+        for (int k = 0; k < kSpU; ++k) dv[k] = (unsigned)u[k] < V ? __ldcg(&a.dist[u[k]]) : INT_MIN;
+#pragma unroll
+        for (int k = 0; k < kSpU; ++k)
+          if (cand[k] < dv[k]) {
+            atomicMin(&a.dist[u[k]], cand[k]);
+            atomicOr(&a.pending[u[k] >> 5], 1u << (u[k] & 31));
+            best = min(best, cand[k]);
+          }
+      }
+    }
+    best = __reduce_min_sync(0xffffffffu, best);
+    if (lane == 0 && best != INT_MAX) atomicMin(&s_min, best);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      if (s_min != INT_MAX) atomicMin(&c->low[slot], s_min);
+      s_min = INT_MAX;
+    }
+    if (!(ok = grid_level_end(a.loop, &sh, slot, nbar))) break;
+    low = sh.low;
+    ++step;
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    LoopOut *o = a.loop.out;
+    o->level = o->push_levels = step;
+    o->pull_levels = 0;
+    o->frontier_size = low != INT_MAX ? 1u : 0u;
+    o->visited_count = o->visited_edges = 0;
+    o->barriers = nbar;
+    o->error = ok ? *(volatile int32_t *)&c->error : (int32_t)MG_ERR_TIMEOUT;
+  }
+}
+
+// Runs an SSSP on stream s in one launch, distances to `dist` (device).
+int sssp_loop_run(mg_graph *g, cudaStream_t s, int32_t src, const mg_options *o, int32_t *dist) {
+  SsspLoopArgs a;
+  a.g = g->csr;
+  a.dist = dist;
+  a.pending = g->ws.visited;
+  // the room of the two BFS queues: a step selects every vertex at most once
+  static_assert(sizeof(int4) == 2 * sizeof(int2), "one queue of the same number of entries");
+  a.q = reinterpret_cast<int4 *>(g->loop_queue);
+  a.cap = (uint32_t)g->loop_cap;
+  a.src = src;
+  const double mean = std::max(1.0, (double)g->edges / (double)g->nodes);
+  a.delta = (int32_t)std::min(1e9, std::max(1.0, kSsspWindow * (double)std::max(g->weight_max, 0) / mean));
+  a.max_iter = (uint32_t)(g->nodes + 2);
+  a.loop = loop_begin(g, o);
+  void *args[] = {&a};
+  cudaError_t e = cudaEventRecord(g->ev0, s);
+  if (e == cudaSuccess) e = cudaLaunchCooperativeKernel((const void *)k_sssp_loop, dim3(g->num_sms), dim3(kLoopNT), args, 0, s);
+  if (e == cudaSuccess) e = cudaEventRecord(g->ev1, s);
+  count_launch();
+  return cuda_status(e, "sssp loop launch");
+}
+
+}  // namespace mg

@@ -187,3 +187,18 @@ def test_ppr_list_lengths(length):
         t[rng.choice(n, 30, replace=False), c] = 1 / 30
     t[0] += 0.1
     _ppr_check(torch, Graph(hg, directed=True), hg, src, w, t, rng.standard_normal((n, 12)))
+
+
+@pytest.mark.parametrize("name", list(GRAPHS))
+@pytest.mark.parametrize("lo,hi", [(0, 0), (1, 1), (0, 3), (1, 64), (1, 1000), (50_000, 90_000)])
+def test_sssp_one_launch_equals_level_loop(name, lo, hi):
+    # windows of one weight and of many, zero weights, sums past the unreachable distance (100000000)
+    hg = GRAPHS[name]().with_weights(lo, hi, seed=2)
+    g = Graph(hg, directed=name == "directed")
+    for s in sorted({0, hg.nodes - 1, hg.max_degree_vertex()}):
+        ref = oracle.sssp(hg.row_offsets, hg.column_indices, hg.edge_values, s)
+        out, st = g.sssp(s)
+        assert np.array_equal(out, ref) and st["converged"] == 1, s
+        assert st["vertices_reached"] == int((ref < 100000000).sum())
+        host, _ = g.sssp(s, use_cuda_graph=0)
+        assert np.array_equal(host, ref), s
