@@ -34,7 +34,14 @@
 
 namespace mg {
 
-constexpr int kPrBig = 512;     // longer in-lists are summed by the chunk pass
+// Longer in-lists are summed by the chunk pass. It needs no segmented scan, and
+// the groups that are left are of like size: at R-MAT 22 (4.2 M vertices, 65 M
+// edges) the busiest warp has 1.15 times the mean work of the round-robin deal,
+// against 2.7 times with a limit of 512, and a solve takes 3.81 ms against 5.51
+// (limit 256: 4.04, 64: 3.82; chunks of 512 edges: 3.88). Keeping the 45,056
+// most-gathered contributions in shared memory, one CTA per SM, was slower
+// (4.09): the gathers were not the bound, the balance was.
+constexpr int kPrBig = 128;
 constexpr int kPrChunk = 1024;  // edges per chunk of a long in-list
 constexpr int kPrGroup = 32;    // vertices per warp group (one per lane)
 constexpr int kPrSub = 4;       // 32-edge sub-chunks whose loads are in flight together
@@ -463,14 +470,14 @@ extern "C" int mg_pagerank(mg_graph *g, float *ranks, mg_stats *stats, const mg_
   const double tol = o->tolerance;
   LevelBody body = [=](cudaStream_t ss, cudaGraphConditionalHandle h, int use_h) {
     MG_LAUNCH(KID_PR_PULL, ss, k_pr_iter<<<grid, kNT, 0, ss>>>(a));
-    MG_LAUNCH(KID_GATHER, ss, k_pr_fixup<<<fix_grid, kNT, 0, ss>>>(a));
+    if (a.nheavy) MG_LAUNCH(KID_GATHER, ss, k_pr_fixup<<<fix_grid, kNT, 0, ss>>>(a));
     MG_LAUNCH(KID_OTHER, ss, k_pr_level_end<<<1, 32, 0, ss>>>(a.ctl, d, inv_n, tol, h, use_h));
   };
   LoopResult res;
   // the body's kernel arguments carry d and tol: key the cached graph on them
   char key[96];
   snprintf(key, sizeof(key), "pagerank/%d/%.17g/%.17g", grid, d, tol);
-  if ((st = run_level_loop(g, s, key, 3, body, o->use_cuda_graph != 0, &res)) != MG_OK) return st;
+  if ((st = run_level_loop(g, s, key, a.nheavy ? 3 : 2, body, o->use_cuda_graph != 0, &res)) != MG_OK) return st;
   finish_run(g, res.ctl.level);
   if (res.ctl.error) return set_error(res.ctl.error, std::string("pagerank: device reported ") +
                                                          mg_status_string(res.ctl.error));
