@@ -117,7 +117,7 @@ struct mg_graph {
   // fixed-size chunks whose partial sums are combined in chunk order.
   int32_t *pr_chunk_v = nullptr, *pr_chunk_b = nullptr, *pr_chunk_e = nullptr;
   int32_t *pr_heavy_v = nullptr, *pr_heavy_first = nullptr;
-  int32_t pr_nchunks = 0, pr_nheavy = 0;
+  int32_t pr_nchunks = 0, pr_nheavy = 0, pr_max_list = 0;
   int64_t pr_ndangling = 0;
   float *pr_rank[2] = {nullptr, nullptr}, *pr_contrib[2] = {nullptr, nullptr}, *pr_partial = nullptr;
   // The in-lists the PageRank kernels read: on a skewed degree distribution a

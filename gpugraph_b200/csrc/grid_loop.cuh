@@ -25,6 +25,7 @@ struct LoopCtl {
   unsigned long long edges[3];  // sum of their out-degrees
   uint32_t items[3];            // items appended to the next queue
   int32_t low[3];               // SSSP: smallest pending distance
+  double residual[3], dangling[3];  // PageRank: L1 change and dangling mass
   uint32_t arrived;
   int32_t error;
 };
@@ -33,6 +34,7 @@ struct LoopCtl {
 struct LoopOut {
   uint32_t level, push_levels, pull_levels, frontier_size;
   unsigned long long visited_count, visited_edges;
+  double residual;
   uint32_t barriers;
   int32_t error;
 };
@@ -42,6 +44,7 @@ struct LoopShared {
   unsigned long long count, edges;        // the grid's, after the level's barrier
   uint32_t items;
   int32_t low;
+  double residual, dangling;
   int fail;
 };
 
@@ -79,6 +82,8 @@ MG_DEVINL bool grid_level_end(const GridLoop &g, LoopShared *sh, uint32_t slot, 
     sh->edges = *(volatile unsigned long long *)&g.c->edges[slot];
     sh->items = *(volatile uint32_t *)&g.c->items[slot];
     sh->low = *(volatile int32_t *)&g.c->low[slot];
+    sh->residual = *(volatile double *)&g.c->residual[slot];
+    sh->dangling = *(volatile double *)&g.c->dangling[slot];
   }
   __syncthreads();
   return !sh->fail;

@@ -31,6 +31,7 @@
 #include "algo_util.cuh"
 #include "gas/driver.cuh"
 #include "gas/engine.cuh"
+#include "grid_loop.cuh"
 
 namespace mg {
 
@@ -46,6 +47,11 @@ constexpr int kPrChunk = 1024;  // edges per chunk of a long in-list
 constexpr int kPrGroup = 32;    // vertices per warp group (one per lane)
 constexpr int kPrSub = 4;       // 32-edge sub-chunks whose loads are in flight together
 constexpr int kPrSerial = 8;    // a group whose lists are all this short is summed lane by lane
+constexpr int kPrThreadList = 16;  // a one-launch solve gives a vertex a thread when no in-list is longer
+// Vertices + edges up to which a solve is one launch (directed R-MAT, 16 edges a
+// vertex, one launch / level loop: scale 16 462 / 559 us, 19 564 / 614, 20 998 /
+// 1063, 21 1942 / 1921; 2000x2000 road grid 1960 / 2205).
+constexpr int64_t kPrLoopWork = 1 << 25;
 constexpr double kPrSkew = 64.0;  // renumber by out-degree when the largest is this many times the mean
 
 struct PrArgs {
@@ -123,22 +129,16 @@ MG_DEVINL void pr_segment(float x, int ck, int b, int e, bool mine, uint32_t le,
 // offsets while it sweeps the current one. No shared memory, no block
 // barriers. (Staging the 33 offsets of a group with a bulk copy on an
 // mbarrier measured slower than the two coalesced loads per lane.)
-__global__ void __launch_bounds__(kNT, 6) k_pr_iter(PrArgs a) {
-  Ctl *ctl = a.ctl;
-  if (!ctl->active) return;
-  const uint32_t L = ctl->level;
-  const float base = (float)ctl->dangling;
+MG_DEVINL void pr_sweep(const PrArgs &a, uint32_t L, float base, uint32_t gw, uint32_t nwarps, float &rs, float &rc,
+                        float &ds, float &dc, unsigned long long &my_bytes) {
   const float *cold = (L & 1) ? a.c1 : a.c0;
   const float *rold = (L & 1) ? a.r1 : a.r0;
   float *rnew = (L & 1) ? a.r0 : a.r1;
   float *cnew = (L & 1) ? a.c0 : a.c1;
-  float rs = 0.f, rc = 0.f, ds = 0.f, dc = 0.f;
-  unsigned long long my_bytes = 0;
-  const int lane = lane_id(), w = warp_id();
+  const int lane = lane_id();
   const uint32_t le = 0xffffffffu >> (31 - lane);  // lanes [0, lane]
   const uint32_t ngroups = ((uint32_t)a.V + kPrGroup - 1) / kPrGroup;
-  const uint32_t nwarps = gridDim.x * kNW;
-  uint32_t grp = blockIdx.x * kNW + w;
+  uint32_t grp = gw;
   // offsets of the next group, loaded one group ahead (lanes past the last
   // vertex load nothing)
   int nb = 0, ne = 0;
@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(kNT, 6) k_pr_iter(PrArgs a) {
 #pragma unroll
       for (int k = 0; k < kPrSerial; ++k) u[k] = b + k < e ? __ldcs(a.crow + b + k) : -1;
 #pragma unroll
-      for (int k = 0; k < kPrSerial; ++k) x[k] = u[k] >= 0 ? __ldg(&cold[u[k]]) : 0.f;
+      for (int k = 0; k < kPrSerial; ++k) x[k] = u[k] >= 0 ? cold[u[k]] : 0.f;
 #pragma unroll
       for (int k = 0; k < kPrSerial; ++k) acc += x[k];
     } else {
@@ -189,7 +189,7 @@ __global__ void __launch_bounds__(kNT, 6) k_pr_iter(PrArgs a) {
           u[k] = i < seg_e ? __ldcs(a.crow + i) : -1;
         }
 #pragma unroll
-        for (int k = 0; k < kPrSub; ++k) x[k] = u[k] >= 0 ? __ldg(&cold[u[k]]) : 0.f;
+        for (int k = 0; k < kPrSub; ++k) x[k] = u[k] >= 0 ? cold[u[k]] : 0.f;
 #pragma unroll
         for (int k = 0; k < kPrSub; ++k)
           if (c + 32 * k < seg_e) pr_segment(x[k], c + 32 * k, b, e, mine, le, acc);
@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(kNT, 6) k_pr_iter(PrArgs a) {
   // heavy chunks: warp per chunk, round-robin over the grid's warps (a chunk is
   // at most kPrChunk edges, and a shared atomic work counter would serialise
   // tens of thousands of warps on one address)
-  for (uint32_t c = blockIdx.x * kNW + w; c < (uint32_t)a.nchunks; c += nwarps) {
+  for (uint32_t c = gw; c < (uint32_t)a.nchunks; c += nwarps) {
     const int cb = a.chunk_b[c], ce = a.chunk_e[c];
     float acc = 0.f;
     int k = cb + lane;
@@ -218,11 +218,11 @@ __global__ void __launch_bounds__(kNT, 6) k_pr_iter(PrArgs a) {
 #pragma unroll
       for (int j = 0; j < 8; ++j) u[j] = __ldcs(a.crow + k + 32 * j);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) x[j] = __ldg(&cold[u[j]]);
+      for (int j = 0; j < 8; ++j) x[j] = cold[u[j]];
 #pragma unroll
       for (int j = 0; j < 8; ++j) acc += x[j];
     }
-    for (; k < ce; k += 32) acc += __ldg(&cold[__ldcs(a.crow + k)]);
+    for (; k < ce; k += 32) acc += cold[__ldcs(a.crow + k)];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
     if (lane == 0) {
@@ -230,30 +230,162 @@ __global__ void __launch_bounds__(kNT, 6) k_pr_iter(PrArgs a) {
       my_bytes += 4 + 8ull * (unsigned long long)(ce - cb);
     }
   }
-  add_bytes(ctl, KID_PR_PULL, my_bytes);
-  pr_flush(ctl, rs, rc, ds, dc);
 }
 
 // Heavy vertices: chunk partials added in chunk order.
-__global__ void __launch_bounds__(kNT) k_pr_fixup(PrArgs a) {
-  Ctl *ctl = a.ctl;
-  if (!ctl->active) return;
-  const uint32_t L = ctl->level;
-  const float base = (float)ctl->dangling;
+MG_DEVINL void pr_fix(const PrArgs &a, uint32_t L, float base, uint32_t tid, uint32_t nt, float &rs, float &rc,
+                      float &ds, float &dc, unsigned long long &my_bytes) {
   const float *rold = (L & 1) ? a.r1 : a.r0;
   float *rnew = (L & 1) ? a.r0 : a.r1;
   float *cnew = (L & 1) ? a.c0 : a.c1;
-  float rs = 0.f, rc = 0.f, ds = 0.f, dc = 0.f;
-  unsigned long long my_bytes = 0;
-  for (int h = blockIdx.x * blockDim.x + threadIdx.x; h < a.nheavy; h += gridDim.x * blockDim.x) {
+  for (uint32_t h = tid; h < (uint32_t)a.nheavy; h += nt) {
     const int v = a.heavy_v[h];
     float s = 0.f;
     for (int c = a.heavy_first[h]; c < a.heavy_first[h + 1]; ++c) s += a.partial[c];
     pr_finalize(a, v, s, base, rold, rnew, cnew, rs, rc, ds, dc);
     my_bytes += 28 + 4ull * (unsigned long long)(a.heavy_first[h + 1] - a.heavy_first[h]);
   }
+}
+
+__global__ void __launch_bounds__(kNT, 6) k_pr_iter(PrArgs a) {
+  Ctl *ctl = a.ctl;
+  if (!ctl->active) return;
+  float rs = 0.f, rc = 0.f, ds = 0.f, dc = 0.f;
+  unsigned long long my_bytes = 0;
+  pr_sweep(a, ctl->level, (float)ctl->dangling, blockIdx.x * kNW + warp_id(), gridDim.x * kNW, rs, rc, ds, dc,
+           my_bytes);
   add_bytes(ctl, KID_PR_PULL, my_bytes);
   pr_flush(ctl, rs, rc, ds, dc);
+}
+
+__global__ void __launch_bounds__(kNT) k_pr_fixup(PrArgs a) {
+  Ctl *ctl = a.ctl;
+  if (!ctl->active) return;
+  float rs = 0.f, rc = 0.f, ds = 0.f, dc = 0.f;
+  unsigned long long my_bytes = 0;
+  pr_fix(a, ctl->level, (float)ctl->dangling, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x, rs, rc,
+         ds, dc, my_bytes);
+  add_bytes(ctl, KID_PR_PULL, my_bytes);
+  pr_flush(ctl, rs, rc, ds, dc);
+}
+
+// The sweep for graphs whose in-lists are all short (a grid): a thread sums a
+// vertex's list in CSC order, kPrVerts vertices at a time with all their index
+// loads, then all their gathers in flight; a list's entries past kPrSerial one
+// by one. The 1200x1200 road grid: 946 us a solve in the level loop, 728 with
+// the warp sweep in one launch, 565 with this one (three vertices at a time: 679,
+// registers spill).
+constexpr int kPrVerts = 2;
+MG_DEVINL void pr_thread_sweep(const PrArgs &a, uint32_t L, float base, uint32_t tid, uint32_t nt, float &rs,
+                               float &rc, float &ds, float &dc) {
+  const float *cold = (L & 1) ? a.c1 : a.c0;
+  const float *rold = (L & 1) ? a.r1 : a.r0;
+  float *rnew = (L & 1) ? a.r0 : a.r1;
+  float *cnew = (L & 1) ? a.c0 : a.c1;
+  for (uint32_t v0 = tid; v0 < (uint32_t)a.V; v0 += nt * kPrVerts) {
+    int b[kPrVerts], e[kPrVerts], u[kPrVerts][kPrSerial];
+    float r_old[kPrVerts], iv[kPrVerts], x[kPrVerts][kPrSerial];
+#pragma unroll
+    for (int q = 0; q < kPrVerts; ++q) {
+      const uint32_t v = v0 + q * nt;
+      const bool in = v < (uint32_t)a.V;
+      b[q] = in ? a.coff[v] : 0;
+      e[q] = in ? a.coff[v + 1] : 0;
+      r_old[q] = in ? rold[v] : 0.f;
+      iv[q] = in ? a.inv[v] : 0.f;
+    }
+#pragma unroll
+    for (int q = 0; q < kPrVerts; ++q)
+#pragma unroll
+      for (int k = 0; k < kPrSerial; ++k) u[q][k] = b[q] + k < e[q] ? a.crow[b[q] + k] : -1;
+#pragma unroll
+    for (int q = 0; q < kPrVerts; ++q)
+#pragma unroll
+      for (int k = 0; k < kPrSerial; ++k) x[q][k] = u[q][k] >= 0 ? cold[u[q][k]] : 0.f;
+#pragma unroll
+    for (int q = 0; q < kPrVerts; ++q) {
+      const uint32_t v = v0 + q * nt;
+      if (v >= (uint32_t)a.V) continue;
+      float acc = 0.f;
+#pragma unroll
+      for (int k = 0; k < kPrSerial; ++k) acc += x[q][k];
+      for (int k = b[q] + kPrSerial; k < e[q]; ++k) acc += cold[a.crow[k]];
+      pr_store(a.damping, (int)v, acc, base, r_old[q], iv[q], rnew, cnew, rs, rc, ds, dc);
+    }
+  }
+}
+
+// The whole solve in one cooperative launch (grid_loop.cuh): one barrier per
+// iteration, two where in-lists are cut into chunks, and the ranks to `out` in
+// the caller's numbering at the end. For graphs whose iteration is short beside
+// the launches of the level loop.
+struct PrLoopArgs {
+  PrArgs a;
+  float *out;
+  const int32_t *new_of;  // null: not renumbered
+  double damping, inv_n, tol, base0;
+  uint32_t max_iter;
+  int by_thread;  // lists are short: a thread per vertex
+  GridLoop loop;
+};
+
+__global__ void __launch_bounds__(kLoopNT, 1) k_pr_loop(PrLoopArgs p) {
+  __shared__ LoopShared sh;
+  const PrArgs &a = p.a;
+  const uint32_t tid = blockIdx.x * kLoopNT + threadIdx.x, nt = gridDim.x * kLoopNT;
+  const uint32_t nw = nt / 32, gw = warp_id() * gridDim.x + blockIdx.x;
+  LoopCtl *c = p.loop.c;
+  if (threadIdx.x == 0) {
+    sh.my_count = sh.my_edges = 0;
+    sh.fail = 0;
+  }
+  __syncthreads();
+  for (uint32_t v = tid; v < (uint32_t)a.V; v += nt) {
+    a.r0[v] = (float)p.inv_n;
+    a.c0[v] = (float)p.inv_n * a.inv[v];
+  }
+  if (blockIdx.x == 0 && threadIdx.x < 3) {
+    c->count[threadIdx.x] = c->edges[threadIdx.x] = 0;
+    c->residual[threadIdx.x] = c->dangling[threadIdx.x] = 0.0;
+    if (threadIdx.x == 0) c->error = 0;
+  }
+  uint32_t nbar = 0, L = 0;
+  bool ok = grid_level_end(p.loop, &sh, 2, nbar);
+  double base = p.base0, res = 0.0;
+  bool more = p.max_iter > 0;
+  unsigned long long my_bytes = 0;
+  while (ok && more) {
+    const uint32_t slot = L % 3;
+    // slot of the next iteration: last read before the previous one
+    if (blockIdx.x == 0 && threadIdx.x == 0) c->residual[(L + 1) % 3] = c->dangling[(L + 1) % 3] = 0.0;
+    float rs = 0.f, rc = 0.f, ds = 0.f, dc = 0.f;
+    if (p.by_thread) pr_thread_sweep(a, L, (float)base, tid, nt, rs, rc, ds, dc);
+    else pr_sweep(a, L, (float)base, gw, nw, rs, rc, ds, dc, my_bytes);
+    if (a.nheavy) {
+      if (!(ok = grid_level_end(p.loop, &sh, slot, nbar))) break;
+      pr_fix(a, L, (float)base, tid, nt, rs, rc, ds, dc, my_bytes);
+    }
+    const double r = cta_sum_f64((double)rs - (double)rc), d = cta_sum_f64((double)ds - (double)dc);
+    if (threadIdx.x == 0) {
+      if (r != 0.0) atomicAdd(&c->residual[slot], r);
+      if (d != 0.0) atomicAdd(&c->dangling[slot], d);
+    }
+    if (!(ok = grid_level_end(p.loop, &sh, slot, nbar))) break;
+    res = sh.residual;
+    base = (1.0 - p.damping) * p.inv_n + p.damping * sh.dangling * p.inv_n;
+    ++L;
+    more = res > p.tol && L < p.max_iter;
+  }
+  const float *fin = (L & 1) ? a.r1 : a.r0;
+  if (ok)
+    for (uint32_t v = tid; v < (uint32_t)a.V; v += nt) p.out[v] = fin[p.new_of ? p.new_of[v] : (int)v];
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    LoopOut *o = p.loop.out;
+    o->level = L;
+    o->residual = res;
+    o->barriers = nbar;
+    o->error = ok ? *(volatile int32_t *)&c->error : (int32_t)MG_ERR_TIMEOUT;
+  }
 }
 
 __global__ void k_pr_level_end(Ctl *ctl, double damping, double inv_n, double tol, cudaGraphConditionalHandle h,
@@ -365,6 +497,7 @@ static int pr_plan(mg_graph *g, cudaStream_t s) {
   }
   std::vector<float> inv((size_t)V);
   int64_t ndang = 0;
+  int32_t max_list = 0;
   std::vector<int32_t> cv, cb, ce, hv, hf;
   for (int64_t v = 0; v < V; ++v) {
     const int64_t ov = renumber ? old_of[v] : v;  // v in the numbering the kernels use
@@ -372,6 +505,7 @@ static int pr_plan(mg_graph *g, cudaStream_t s) {
     inv[v] = od > 0 ? 1.0f / (float)od : 0.0f;
     ndang += od == 0;
     const int32_t b = co[v], en = co[v + 1];
+    max_list = std::max(max_list, en - b);
     // the same rule as k_pr_iter: in-lists longer than kPrBig are chunked
     if (en - b > kPrBig) {
       hv.push_back((int32_t)v);
@@ -413,7 +547,49 @@ static int pr_plan(mg_graph *g, cudaStream_t s) {
   g->pr_nchunks = (int32_t)cv.size();
   g->pr_nheavy = (int32_t)hv.size();
   g->pr_ndangling = ndang;
+  g->pr_max_list = max_list;
   (void)ro_n;
+  return MG_OK;
+}
+
+static int pr_one_launch(mg_graph *g, cudaStream_t s, const PrArgs &a, float *ranks, mg_stats *stats,
+                         const mg_options *o, double inv_n, double base0, uint32_t max_iter) {
+  int st;
+  const bool dev = o->outputs_on_device != 0, direct = dev && on_device(g, ranks);
+  PrLoopArgs p;
+  p.a = a;
+  p.out = direct ? ranks : reinterpret_cast<float *>(g->ws.vbuf[0]);
+  p.new_of = g->pr_new_of;
+  p.damping = o->damping;
+  p.inv_n = inv_n;
+  p.tol = o->tolerance;
+  p.base0 = base0;
+  p.max_iter = max_iter;
+  p.by_thread = g->pr_max_list <= kPrThreadList ? 1 : 0;
+  p.loop = loop_begin(g, o);
+  void *args[] = {&p};
+  cudaError_t e = cudaEventRecord(g->ev0, s);
+  if (e == cudaSuccess)
+    e = cudaLaunchCooperativeKernel((const void *)k_pr_loop, dim3(g->num_sms), dim3(kLoopNT), args, 0, s);
+  if (e == cudaSuccess) e = cudaEventRecord(g->ev1, s);
+  count_launch();
+  if (e == cudaSuccess && !direct)
+    e = cudaMemcpyAsync(ranks, p.out, (size_t)g->nodes * 4, dev ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  if ((st = cuda_status(e, "pagerank")) != MG_OK || (st = loop_end(g, s, "pagerank")) != MG_OK) return st;
+  if (stats) {
+    const LoopOut &r = *g->loop_out;
+    float ms = 0.f;
+    cudaEventElapsedTime(&ms, g->ev0, g->ev1);
+    stats->iterations = (int32_t)r.level;
+    stats->push_iterations = 0;
+    stats->pull_iterations = (int32_t)r.level;
+    stats->converged = (r.level > 0 && r.residual <= o->tolerance) ? 1 : 0;
+    stats->device_ms = ms;
+    stats->residual = r.residual;
+    stats->vertices_reached = g->nodes;
+    stats->edges_traversed = g->edges * (int64_t)r.level;
+  }
   return MG_OK;
 }
 
@@ -460,8 +636,12 @@ extern "C" int mg_pagerank(mg_graph *g, float *ranks, mg_stats *stats, const mg_
   a.nheavy = g->pr_nheavy;
   a.damping = (float)d;
   a.ctl = g->ws.ctl;
-  k_pr_init<<<g->num_sms * 4, 256, 0, s>>>(a.inv, a.r0, a.c0, V, (float)inv_n);
   const double base0 = (1.0 - d) * inv_n + d * ((double)g->pr_ndangling * inv_n) * inv_n;
+  // Short iterations: one launch (kPrLoopWork). The level loop serves the rest,
+  // the host-driven runs and callers that shorten the waits.
+  if (o->use_cuda_graph && !prof_on() && o->spin_limit >= kSpinLimitDefault && g->edges + V <= kPrLoopWork)
+    return pr_one_launch(g, s, a, ranks, stats, o, inv_n, base0, max_iter);
+  k_pr_init<<<g->num_sms * 4, 256, 0, s>>>(a.inv, a.r0, a.c0, V, (float)inv_n);
   k_pr_ctl_init<<<1, 32, 0, s>>>(a.ctl, max_iter, (unsigned long long)o->spin_limit, ctl_flags(nullptr), base0);
   count_launch(2);
   if ((st = launch_check("pagerank init")) != MG_OK) return st;

@@ -202,3 +202,40 @@ def test_sssp_one_launch_equals_level_loop(name, lo, hi):
         assert st["vertices_reached"] == int((ref < 100000000).sum())
         host, _ = g.sssp(s, use_cuda_graph=0)
         assert np.array_equal(host, ref), s
+
+
+def _lists(lengths, n):
+    """Directed graph whose vertex i has lengths[i] in-edges from distinct vertices; the rest feed vertex 0 in a ring."""
+    edges = set()
+    for i, k in enumerate(lengths):
+        edges |= {((i + 1 + j) % n, i) for j in range(k)}
+    edges |= {(v, (v + 1) % n) for v in range(len(lengths), n, 2)}
+    src, dst = np.array(sorted(edges)).T
+    ro = np.concatenate([[0], np.cumsum(np.bincount(src, minlength=n))]).astype(np.int32)
+    return HostGraph(ro, dst.astype(np.int32), None, directed=True)
+
+
+def test_pagerank_list_lengths_and_loops():
+    # in-lists around the lane-serial (8), chunk (128, 1024) limits; one launch and level loop
+    hg = _lists([0, 1, 7, 8, 9, 31, 127, 128, 129, 1023, 1024, 1025, 1152, 1153, 3000], 4001)
+    g = Graph(hg, directed=True)
+    t = hg.transpose()
+    for iters in (0, 1, 2, 25):
+        a, sa = g.pagerank(iter_num=iters, tolerance=0.0)
+        b, sb = g.pagerank(iter_num=iters, tolerance=0.0, use_cuda_graph=0)
+        ref, _, _ = oracle.pagerank_fp64(hg.row_offsets, t.row_offsets, t.column_indices, 0.85, 0.0, iters)
+        assert sa["iterations"] == sb["iterations"] == iters
+        assert np.abs(a - ref).sum() < 1e-6 and np.abs(b - ref).sum() < 1e-6  # the FP32 bound of the other tests
+
+
+@pytest.mark.parametrize("scale,ef", [(18, 16), (20, 17)])
+def test_pagerank_renumbered_graph_both_loops(scale, ef):
+    # below and above the size up to which a solve is one launch, each also through the host-driven loop
+    hg = HostGraph.rmat(scale, ef, seed=8, symmetrize=False)
+    g = Graph(hg, directed=True)
+    t = hg.transpose()
+    for mode in ({}, dict(use_cuda_graph=0)):
+        r, st = g.pagerank(tolerance=1e-7, iter_num=60, **mode)
+        ref, _, _ = oracle.pagerank_fp64(hg.row_offsets, t.row_offsets, t.column_indices, 0.85, 0.0,
+                                         int(st["iterations"]))
+        assert np.abs(r - ref).sum() < 1e-6
