@@ -8,22 +8,37 @@
 // gas_algos.cu), whose semantics there are not components.
 //
 // Order of work (the sampling scheme of Sutton et al., "Optimizing Parallel
-// Graph Connectivity Computation via Subgraph Sampling", IPDPS 2018):
-//   1. every vertex links with its first kCcSample neighbours, compressing the
-//      trees after each round;
-//   2. the most frequent root among kCcProbe fixed sample vertices names the
+// Graph Connectivity Computation via Subgraph Sampling", IPDPS 2018, with its
+// first round done without atomics: hanging every vertex under a smaller
+// neighbour, which only its own thread writes, is a valid forest):
+//   1. every vertex starts under its first neighbour if that is smaller, else
+//      as a root;
+//   2. every vertex links with its second neighbour, a root of step 1 with its
+//      first as well; the trees are flattened;
+//   3. the most frequent root among kCcProbe fixed sample vertices names the
 //      large component;
-//   3. every vertex not already under that root links the rest of its edges.
-// An edge skipped in step 3 joins two vertices of the large component, or is
-// linked from its other end, which is not in it; on power-law graphs step 3
+//   4. every vertex not already under that root links the rest of its edges.
+// An edge skipped in step 4 joins two vertices of the large component, or is
+// linked from its other end, which is not in it; on power-law graphs step 4
 // touches a small share of the edges.
+//
+// On a skewed graph (kCcSkew) the links of steps 1 and 2 queue up on a few roots
+// (sampling alone took 340 us at R-MAT 21). There a one-launch BFS from the hub,
+// of at most kCcLevels levels, finds the large component instead: what it
+// reached starts under its smallest id, every other vertex links all its edges
+// as in step 4. Any connected set serves, so the cap on the levels keeps long
+// paths out of the BFS without changing a label. R-MAT 21: 0.68 -> 0.20 ms,
+// R-MAT 22: 1.61 -> 0.31 ms.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <climits>
+#include <vector>
 
 #include "algo_util.cuh"
 #include "gas/driver.cuh"
 #include "gas/engine.cuh"
+#include "grid_loop.cuh"
 
 namespace mg {
 
@@ -61,28 +76,76 @@ MG_DEVINL bool cc_unite(int32_t *parent, int32_t a, int32_t b, unsigned long lon
   return false;
 }
 
+// cc_unite for a whole warp (lanes with `pending` link a and b), one atomic per
+// distinct larger root: the lane with the smallest other root hooks it, the
+// lanes that hold the same larger root go on to join their other root with that
+// one. Neighbouring vertices of a grid hang under the same few roots, and their
+// hooks would queue up on one address (1200x1200 road grid: 335 instead of 430 us).
+MG_DEVINL bool cc_unite_warp(int32_t *parent, int32_t a, int32_t b, bool pending, unsigned long long limit) {
+  const int lane = lane_id();
+  for (unsigned long long it = 0; it < limit; ++it) {
+    if (pending) {
+      a = cc_find(parent, a);
+      b = cc_find(parent, b);
+      pending = a != b;
+    }
+    if (!__any_sync(0xffffffffu, pending)) return true;
+    const int32_t hi = pending ? max(a, b) : -1 - lane, lo = min(a, b);
+    const uint32_t same = __match_any_sync(0xffffffffu, hi);
+    const int32_t least = __reduce_min_sync(same, lo);
+    const uint32_t holders = __match_any_sync(0xffffffffu, ((unsigned long long)(uint32_t)hi << 32) | (uint32_t)lo);
+    if (!pending) continue;
+    if (lo != least) {
+      a = lo;
+      b = least;
+    } else if (lane == __ffs(holders) - 1) {
+      const int32_t old = atomicMin(&parent[hi], lo);
+      pending = old != hi;
+      a = old;
+      b = lo;
+    } else {
+      pending = false;  // the same pair as the lane that hooks it
+    }
+  }
+  return !__any_sync(0xffffffffu, pending);
+}
+
 constexpr int kCcSample = 2;    // neighbours linked per vertex before the large component is picked
 constexpr int kCcProbe = 1024;  // sample vertices voting for the large component (one CTA)
 
-// Step 1, round r: vertex v links with its r-th neighbour.
+// Step 1: parent[v] = min(v, first neighbour).
+__global__ void __launch_bounds__(kNT) k_cc_start(const int32_t *ro, const int32_t *col, int32_t *parent, int32_t V,
+                                                  Ctl *ctl) {
+  unsigned long long my_bytes = 0;
+  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x) {
+    const int b = ro[v], e = ro[v + 1];
+    parent[v] = b < e ? min(v, col[b]) : v;
+    my_bytes += b < e ? 16 : 12;  // two offsets, the neighbour id, the parent
+  }
+  add_bytes(ctl, KID_CC, my_bytes);
+}
+
+// Step 2: vertex v links with its second neighbour, and with its first when
+// step 1 left it a root.
 __global__ void __launch_bounds__(kNT) k_cc_sample(const int32_t *ro, const int32_t *col, int32_t *parent, int32_t V,
-                                                   int r, Ctl *ctl) {
+                                                   Ctl *ctl) {
   const unsigned long long limit = ctl->spin_limit;
   bool ok = true;
   unsigned long long my_bytes = 0;
-  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x) {
-    const int e = ro[v] + r;
-    my_bytes += 8;  // two offsets
-    if (e < ro[v + 1]) {
-      my_bytes += 12;  // the neighbour id, the two parents read by the link
-      if (!cc_unite(parent, v, col[e], limit)) ok = false;
-    }
+  for (int64_t v0 = blockIdx.x * (int64_t)blockDim.x + (threadIdx.x & ~31u); v0 < V;
+       v0 += (int64_t)gridDim.x * blockDim.x) {
+    const int v = (int)v0 + lane_id();
+    const int b = v < V ? ro[v] : 0, e = v < V ? ro[v + 1] : 0;
+    const int u0 = b < e ? col[b] : -1, u1 = b + 1 < e ? col[b + 1] : -1;
+    my_bytes += 8 + (u0 > v ? 12 : b < e ? 4 : 0) + (u1 >= 0 ? 12 : 0);  // offsets; neighbour ids, parents read
+    ok &= cc_unite_warp(parent, v, u0, u0 > v, limit);
+    ok &= cc_unite_warp(parent, v, u1, u1 >= 0, limit);
   }
   if (!ok) raise_error(ctl, MG_ERR_TIMEOUT);
   add_bytes(ctl, KID_CC, my_bytes);
 }
 
-// Step 2: the root held by most of kCcProbe fixed sample vertices (ties: the
+// Step 3: the root held by most of kCcProbe fixed sample vertices (ties: the
 // smaller root); parent[] is flat here. Written to *giant.
 __global__ void __launch_bounds__(kCcProbe) k_cc_giant(const int32_t *parent, int32_t V, int32_t *giant) {
   __shared__ int32_t s_lab[kCcProbe];
@@ -115,11 +178,11 @@ __global__ void __launch_bounds__(kCcProbe) k_cc_giant(const int32_t *parent, in
   }
 }
 
-// Step 3: vertices outside the large component link their remaining edges. A
+// Step 4: vertices outside the large component link their edges from the skip-th on. A
 // warp takes 32 consecutive vertices; lists up to 32 edges are walked by their
 // own lane, longer ones by the whole warp (32 edges per step).
 __global__ void __launch_bounds__(kNT) k_cc_rest(const int32_t *ro, const int32_t *col, int32_t *parent, int32_t V,
-                                                 const int32_t *giant, Ctl *ctl) {
+                                                 const int32_t *giant, int skip, Ctl *ctl) {
   const unsigned long long limit = ctl->spin_limit;
   const int32_t big = *giant;
   const int lane = lane_id();
@@ -133,7 +196,7 @@ __global__ void __launch_bounds__(kNT) k_cc_rest(const int32_t *ro, const int32_
     int b = 0, e = 0;
     if (v < V) {
       my_bytes += 12;  // parent, two offsets
-      b = ro[v] + kCcSample;
+      b = ro[v] + skip;
       e = ro[v + 1];
       work = b < e && __ldcg(&parent[v]) != big;
     }
@@ -159,16 +222,44 @@ __global__ void __launch_bounds__(kNT) k_cc_rest(const int32_t *ro, const int32_
   add_bytes(ctl, KID_CC, my_bytes);
 }
 
-// Final labels: every vertex's root (the smallest id of its component).
-__global__ void __launch_bounds__(kNT) k_cc_flatten(int32_t *parent, int32_t V, Ctl *ctl) {
+// Every vertex's root (in the end the smallest id of its component) to `out`.
+// Between the steps that is `parent` itself: there a path halving that read an
+// older ancestor may still replace a root just written, which only makes the
+// tree less flat; the labels therefore go to an array of their own.
+__global__ void __launch_bounds__(kNT) k_cc_flatten(int32_t *parent, int32_t *out, int32_t V, Ctl *ctl) {
   unsigned long long my_bytes = 0;
   for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x) {
-    const int r = cc_find(parent, v);
-    parent[v] = r;
+    out[v] = cc_find(parent, v);
     my_bytes += 12;  // the vertex's parent, its root's parent, the write
   }
   add_bytes(ctl, KID_CC, my_bytes);
 }
+
+// The smallest vertex a BFS reached, then every vertex's start: under it, or a root.
+__global__ void __launch_bounds__(kNT) k_cc_low(const int32_t *depth, int32_t V, int32_t *low) {
+  int m = INT_MAX;
+  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < V && m == INT_MAX; v += gridDim.x * blockDim.x)
+    if (depth[v] >= 0) m = v;  // a thread's vertices ascend
+  m = __reduce_min_sync(0xffffffffu, m);
+  if (lane_id() == 0 && m < *(volatile int32_t *)low) atomicMin(low, m);
+}
+
+__global__ void __launch_bounds__(kNT) k_cc_seed(const int32_t *depth, int32_t V, const int32_t *low, int32_t *parent,
+                                                 Ctl *ctl) {
+  const int32_t root = *low;
+  unsigned long long my_bytes = 0;
+  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x) {
+    parent[v] = depth[v] >= 0 ? root : v;
+    my_bytes += 8;
+  }
+  add_bytes(ctl, KID_CC, my_bytes);
+}
+
+constexpr double kCcSkew = 8.0;      // longest list over the mean from which the BFS finds the large component
+constexpr uint32_t kCcLevels = 16;
+
+int bfs_loop_run(mg_graph *g, cudaStream_t s, const std::vector<int32_t> &roots, uint32_t max_iter,
+                 const mg_options *o, int32_t *labels);  // bfs_loop.cu
 
 // Union-find CC on a symmetric graph (called by mg_cc).
 int cc_union_find(mg_graph *g, int32_t *labels, mg_stats *stats, const mg_options *o) {
@@ -183,22 +274,39 @@ int cc_union_find(mg_graph *g, int32_t *labels, mg_stats *stats, const mg_option
   if (e != cudaSuccess) return cuda_status(e, "event record");
   int32_t *giant = reinterpret_cast<int32_t *>(g->ws.scan);  // scratch word (the scan buffer is free here)
   const int vgrid = g->num_sms * 8;
-  MG_LAUNCH(KID_CC, s, (k_sequence_i32<<<g->num_sms * 4, 256, 0, s>>>(parent, V)));
+  // the last pass writes the caller's buffer when it is this GPU's memory
+  const bool direct = o->outputs_on_device != 0 && on_device(g, labels);
+  int32_t *out = direct ? labels : g->ws.vbuf[1];
   k_ctl_init<<<1, 32, 0, s>>>(ctl, 1u, 1u, (unsigned long long)o->spin_limit, MODE_QUEUE, ctl_flags(nullptr));
-  for (int r = 0; r < kCcSample; ++r) {
-    MG_LAUNCH(KID_CC, s, (k_cc_sample<<<vgrid, kNT, 0, s>>>(g->csr.row_offsets, g->csr.col, parent, V, r, ctl)));
-    MG_LAUNCH(KID_CC, s, (k_cc_flatten<<<vgrid, kNT, 0, s>>>(parent, V, ctl)));
+  const bool by_bfs = g->hub >= 0 && o->use_cuda_graph && !prof_on() && o->spin_limit >= kSpinLimitDefault &&
+                      (double)g->hub_degree > kCcSkew * std::max(1.0, (double)g->edges / (double)V);
+  if (by_bfs) {
+    int32_t *depth = g->ws.gather_tmp;
+    mg_options bo;
+    mg_options_init(&bo);
+    if ((st = bfs_loop_run(g, s, {g->hub}, kCcLevels, &bo, depth)) != MG_OK) return st;
+    k_fill_i32<<<1, 32, 0, s>>>(giant, INT_MAX, 1);
+    k_cc_low<<<vgrid, kNT, 0, s>>>(depth, V, giant);
+    k_cc_seed<<<vgrid, kNT, 0, s>>>(depth, V, giant, parent, ctl);
+    k_cc_rest<<<vgrid, kNT, 0, s>>>(g->csr.row_offsets, g->csr.col, parent, V, giant, 0, ctl);
+    count_launch(6);
+  } else {
+    MG_LAUNCH(KID_CC, s, (k_cc_start<<<vgrid, kNT, 0, s>>>(g->csr.row_offsets, g->csr.col, parent, V, ctl)));
+    MG_LAUNCH(KID_CC, s, (k_cc_sample<<<vgrid, kNT, 0, s>>>(g->csr.row_offsets, g->csr.col, parent, V, ctl)));
+    MG_LAUNCH(KID_CC, s, (k_cc_flatten<<<vgrid, kNT, 0, s>>>(parent, parent, V, ctl)));
+    MG_LAUNCH(KID_CC, s, (k_cc_giant<<<1, kCcProbe, 0, s>>>(parent, V, giant)));
+    MG_LAUNCH(KID_CC, s, (k_cc_rest<<<vgrid, kNT, 0, s>>>(g->csr.row_offsets, g->csr.col, parent, V, giant, kCcSample,
+                                                          ctl)));
+    count_launch(7);
   }
-  MG_LAUNCH(KID_CC, s, (k_cc_giant<<<1, kCcProbe, 0, s>>>(parent, V, giant)));
-  MG_LAUNCH(KID_CC, s, (k_cc_rest<<<vgrid, kNT, 0, s>>>(g->csr.row_offsets, g->csr.col, parent, V, giant, ctl)));
-  MG_LAUNCH(KID_CC, s, (k_cc_flatten<<<vgrid, kNT, 0, s>>>(parent, V, ctl)));
-  count_launch(5 + 2 * kCcSample);
+  MG_LAUNCH(KID_CC, s, (k_cc_flatten<<<vgrid, kNT, 0, s>>>(parent, out, V, ctl)));
   if ((st = launch_check("cc union-find")) != MG_OK) return st;
   e = cudaEventRecord(g->ev1, s);
   if (e != cudaSuccess) return cuda_status(e, "event record");
   Ctl c;
   if ((st = read_ctl(g, s, &c)) != MG_OK) return st;
   prof_flush(s, c.kbytes);
+  if (by_bfs && (st = loop_end(g, s, "cc")) != MG_OK) return st;
   if (c.error) return set_error(c.error, std::string("cc: device reported ") + mg_status_string(c.error));
   float ms = 0.f;
   cudaEventElapsedTime(&ms, g->ev0, g->ev1);
@@ -213,7 +321,7 @@ int cc_union_find(mg_graph *g, int32_t *labels, mg_stats *stats, const mg_option
     stats->vertices_reached = g->nodes;
     stats->edges_traversed = g->edges;
   }
-  return copy_out(s, labels, parent, (size_t)V * 4, o->outputs_on_device != 0);
+  return direct ? MG_OK : copy_out(s, labels, out, (size_t)V * 4, o->outputs_on_device != 0);
 }
 
 }  // namespace mg

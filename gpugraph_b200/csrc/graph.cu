@@ -104,13 +104,9 @@ int ensure_multi(mg_graph *g) {
     cudaError_t e = cudaMemcpy(off.data(), g->csr.csc_offsets, (V + 1) * 4, cudaMemcpyDeviceToHost);
     if ((st = cuda_status(e, "in-list lengths")) != MG_OK) return st;
     std::vector<int32_t> heavy;
-    size_t hub = 0;
-    for (size_t v = 0; v < V; ++v) {
+    for (size_t v = 0; v < V; ++v)
       if (off[v + 1] - off[v] > kMsHeavyList) heavy.push_back((int32_t)v);
-      if (off[v + 1] - off[v] > off[hub + 1] - off[hub]) hub = v;
-    }
-    const double mean = std::max(1.0, (double)g->edges / (double)V);
-    g->mss_hub = (double)(off[hub + 1] - off[hub]) > kMssSkew * mean ? (int32_t)hub : -1;
+    g->mss_hub = (double)g->hub_degree > kMssSkew * std::max(1.0, (double)g->edges / (double)V) ? g->hub : -1;
     if ((st = device_alloc(g, (void **)&g->mss_offs, 67 * 4)) != MG_OK) return st;
     std::stable_sort(heavy.begin(), heavy.end(),
                      [&](int32_t x, int32_t y) { return off[x + 1] - off[x] > off[y + 1] - off[y]; });
@@ -129,6 +125,15 @@ int ensure_multi(mg_graph *g) {
 using namespace mg;
 
 namespace {
+
+// The vertex with the longest in-list (the first of them) and its length.
+void find_hub(mg_graph *g, const int32_t *in_off) {
+  for (int64_t v = 0; v < g->nodes; ++v)
+    if (g->hub < 0 || in_off[v + 1] - in_off[v] > g->hub_degree) {
+      g->hub = (int32_t)v;
+      g->hub_degree = in_off[v + 1] - in_off[v];
+    }
+}
 
 // Copy of the in-lists with every list ordered by descending out-degree of the
 // neighbour (ties by id), for the bottom-up kernels only: a high-degree
@@ -234,6 +239,7 @@ int create_common(const int32_t *row_offsets, const int32_t *col, const void *va
   if (directed) {
     std::vector<int32_t> t_off(ro_n, (int32_t)edges), t_rows(E ? E : 1), t_eid(E ? E : 1);
     host_transpose(nodes, edges, row_offsets, col, t_off.data(), t_rows.data(), t_eid.data());
+    find_hub(g, t_off.data());
     if ((st = device_alloc(g, (void **)&c.csc_offsets, ro_n * 4)) != MG_OK ||
         (st = device_alloc(g, (void **)&c.csc_rows, E * 4 + 64)) != MG_OK ||
         (st = device_alloc(g, (void **)&c.csc_eid, E * 4 + 64)) != MG_OK) {
@@ -254,6 +260,7 @@ int create_common(const int32_t *row_offsets, const int32_t *col, const void *va
     c.csc_offsets = c.row_offsets;
     c.csc_rows = c.col;
     c.csc_eid = nullptr;
+    find_hub(g, row_offsets);
     if ((st = upload_pull_rows(g, row_offsets, col, row_offsets)) != MG_OK) {
       mg_graph_destroy(g);
       return st;

@@ -95,6 +95,7 @@ struct mg_graph {
   int64_t nodes = 0;
   int64_t edges = 0;
   mg::DevCsr csr;
+  int32_t hub = -1, hub_degree = 0;    // the vertex with the longest in-list
   std::vector<int64_t> graph_offsets;  // batch of graphs: first vertex of each graph
   mg::Workspace ws;
   float *inv_outdeg = nullptr;          // PageRank 1/outdeg (0 for dangling vertices)
@@ -109,8 +110,8 @@ struct mg_graph {
   uint32_t *multi_stk_bm = nullptr;     // [kMsStackLevels][V/32] valid entries of push-made stack levels
   int32_t *ms_heavy = nullptr;          // vertices with more than kMsHeavyList in-edges, longest first
   int32_t ms_nheavy = -1;               // their number (-1: not built yet)
-  int32_t *mss_offs = nullptr;          // batched SSSP: offsets of the edge bounds (multi.cu)
-  int32_t mss_hub = -1;                 // the vertex they are measured at, -1: the graph is not skewed
+  int32_t *mss_offs = nullptr;          // batched SSSP: per-source words (multi.cu)
+  int32_t mss_hub = -1;                 // the vertex its edge bounds are measured at, -1: the graph is not skewed
   int32_t *multi_stage = nullptr;       // [64][V] transposed results on their way to host memory
   size_t multi_bytes = 0;
   // PageRank plan (built on first mg_pagerank): heavy in-lists split into

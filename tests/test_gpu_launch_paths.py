@@ -204,6 +204,23 @@ def test_sssp_one_launch_equals_level_loop(name, lo, hi):
         assert np.array_equal(host, ref), s
 
 
+@pytest.mark.parametrize("name", list(GRAPHS))
+def test_cc_labels_at_the_edges(name):
+    hg = GRAPHS[name]()
+    if name == "directed":
+        pytest.skip("union-find serves symmetric graphs")
+    g = Graph(hg)
+    ref, _ = g.cc(generic_engine=1)
+    for _ in range(5):
+        assert np.array_equal(g.cc()[0], ref)
+    # lists in any order: the first neighbour need not be the smallest
+    col = hg.column_indices.copy()
+    for v in range(hg.nodes):
+        b, e = hg.row_offsets[v], hg.row_offsets[v + 1]
+        col[b:e] = col[b:e][::-1]
+    assert np.array_equal(Graph(HostGraph(hg.row_offsets, col, None)).cc()[0], ref)
+
+
 def _lists(lengths, n):
     """Directed graph whose vertex i has lengths[i] in-edges from distinct vertices; the rest feed vertex 0 in a ring."""
     edges = set()
