@@ -1,4 +1,6 @@
-// Direction-optimising BFS (push/pull switching): push levels run the bfs Program's
+// Direction-optimising BFS (push/pull switching): the calls, and the
+// level-by-level loop for those that the one-launch loop (bfs_loop.cu) does not
+// take (see bfs_run). Push levels run the bfs Program's
 // expand + contract (Algorithms/BFS/bfs.h:28-298) fused into k_bfs_push over a
 // vertex queue; pull levels run a bottom-up sweep in which every unvisited
 // vertex scans its in-edges (hubs first) for a parent in the frontier bitmap
@@ -481,6 +483,7 @@ static int bfs_one_launch(mg_graph *g, cudaStream_t s, const std::vector<int32_t
   const size_t bytes = (size_t)g->nodes * 4;
   const bool direct = dev && on_device(g, depths);
   int32_t *labels = direct ? depths : g->ws.vbuf[0];
+  std::lock_guard<std::mutex> lock(loop_mutex(g->device));
   int st = bfs_loop_run(g, s, roots, max_iter, o, labels);
   if (st != MG_OK) return st;
   cudaError_t e = cudaSuccess;

@@ -280,7 +280,9 @@ int cc_union_find(mg_graph *g, int32_t *labels, mg_stats *stats, const mg_option
   k_ctl_init<<<1, 32, 0, s>>>(ctl, 1u, 1u, (unsigned long long)o->spin_limit, MODE_QUEUE, ctl_flags(nullptr));
   const bool by_bfs = g->hub >= 0 && o->use_cuda_graph && !prof_on() && o->spin_limit >= kSpinLimitDefault &&
                       (double)g->hub_degree > kCcSkew * std::max(1.0, (double)g->edges / (double)V);
+  std::unique_lock<std::mutex> lock(loop_mutex(g->device), std::defer_lock);
   if (by_bfs) {
+    lock.lock();
     int32_t *depth = g->ws.gather_tmp;
     mg_options bo;
     mg_options_init(&bo);

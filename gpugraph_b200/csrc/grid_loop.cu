@@ -4,6 +4,11 @@
 
 namespace mg {
 
+std::mutex &loop_mutex(int device) {
+  static std::mutex m[16];
+  return m[device & 15];
+}
+
 GridLoop loop_begin(mg_graph *g, const mg_options *o) {
   GridLoop l;
   l.c = g->loop_ctl;

@@ -9,6 +9,8 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <mutex>
+
 #include "common.cuh"
 #include "graph.cuh"
 
@@ -89,6 +91,9 @@ MG_DEVINL bool grid_level_end(const GridLoop &g, LoopShared *sh, uint32_t slot, 
   return !sh->fail;
 }
 
+// Held from before a loop's launch until its stream was synchronised: two loops
+// launched by different threads would each wait for SMs the other one holds.
+std::mutex &loop_mutex(int device);
 // The GridLoop of a run about to be launched.
 GridLoop loop_begin(mg_graph *g, const mg_options *o);
 // After the stream was synchronised: accounts for the barriers the run used and

@@ -566,6 +566,7 @@ static int pr_one_launch(mg_graph *g, cudaStream_t s, const PrArgs &a, float *ra
   p.base0 = base0;
   p.max_iter = max_iter;
   p.by_thread = g->pr_max_list <= kPrThreadList ? 1 : 0;
+  std::lock_guard<std::mutex> lock(loop_mutex(g->device));
   p.loop = loop_begin(g, o);
   void *args[] = {&p};
   cudaError_t e = cudaEventRecord(g->ev0, s);

@@ -1,4 +1,6 @@
-// Single-source SSSP as one fused relaxation kernel per level. The reference's
+// Single-source SSSP. The default is the one-launch loop (sssp_loop.cu); the loop
+// below, one fused relaxation kernel per level, serves the calls that it does
+// not take (see sssp_fused). The reference's
 // sssp program (Algorithms/SSSP/sssp.h:34-393) runs each Bellman-Ford level as
 // expand (candidate src_dist + w, :334-343), contract (atomicMin into a
 // temporary, :383), apply (min with the distance, :240-255) and post_apply
@@ -169,6 +171,7 @@ static int sssp_one_launch(mg_graph *g, cudaStream_t s, int32_t src, int32_t *di
                            const mg_options *o) {
   const bool dev = o->outputs_on_device != 0, direct = dev && on_device(g, dists);
   int32_t *dist = direct ? dists : g->ws.vbuf[0];
+  std::lock_guard<std::mutex> lock(loop_mutex(g->device));
   int st = sssp_loop_run(g, s, src, o, dist);
   if (st != MG_OK) return st;
   cudaError_t e = cudaSuccess;

@@ -256,3 +256,35 @@ def test_pagerank_renumbered_graph_both_loops(scale, ef):
         ref, _, _ = oracle.pagerank_fp64(hg.row_offsets, t.row_offsets, t.column_indices, 0.85, 0.0,
                                          int(st["iterations"]))
         assert np.abs(r - ref).sum() < 1e-6
+
+
+def test_one_launch_calls_from_several_threads():
+    # each thread has its own graph and stream; the calls overlap in time
+    torch = pytest.importorskip("torch")
+    import threading
+
+    hgs = [HostGraph.rmat(13, 8, seed=50 + i).with_weights(1, 20, seed=i) for i in range(4)]
+    refs = [(oracle.bfs(h.row_offsets, h.column_indices, 1), oracle.sssp(h.row_offsets, h.column_indices,
+                                                                        h.edge_values, 1)) for h in hgs]
+    bad = []
+
+    def work(i):
+        try:
+            g, st = Graph(hgs[i]), torch.cuda.Stream()
+            lab = g.cc()[0]
+            for _ in range(25):
+                ok = np.array_equal(g.bfs(1, stream=st.cuda_stream)[0], refs[i][0])
+                ok &= np.array_equal(g.sssp(1, stream=st.cuda_stream)[0], refs[i][1])
+                ok &= np.array_equal(g.cc(stream=st.cuda_stream)[0], lab)
+                g.pagerank(stream=st.cuda_stream, iter_num=5)
+                if not ok:
+                    bad.append(i)
+        except Exception as e:  # reported by the main thread
+            bad.append(repr(e))
+
+    th = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+    for t in th:
+        t.start()
+    for t in th:
+        t.join()
+    assert not bad
