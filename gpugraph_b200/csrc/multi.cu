@@ -1099,7 +1099,8 @@ __global__ void k_ms_mask_stats(const u64 *visit, u64 all, const int32_t *ro, in
 // than it) and no expand warp reserves queue space. A warp takes kMsScanWords
 // words, a lane a vertex of the current word, twice: totals first, then, with
 // the prefixes of the earlier tiles (two look-backs, the vertices by warp 0 and
-// the degrees by warp 1), the entries. With it a batched SSSP took 4.5 instead
+// the degrees by warp 1), the entries. The previous level's masks, read by its
+// expand, are cleared at its queue entries on the way. With it a batched SSSP took 4.5 instead
 // of 4.9 ms at R-MAT 20 (37 sources) and 19.2 instead of 23.8 ms on the
 // 1200x1200 road grid (64 sources).
 constexpr int kMsScanWords = 16;
@@ -1122,6 +1123,10 @@ __global__ void __launch_bounds__(kNT) k_mss_scan(MultiArgs a, uint32_t *scan, i
   const int lane = lane_id(), warp = warp_id();
   unsigned long long my_bytes = 0;
   if (threadIdx.x == 0) s_fail = 0;
+  const uint32_t pn = ctl->prev_size;
+  u64 *Fp = nxt_F(a, L);
+  const int32_t *Qp = nxt_Q(a, L);
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < pn; i += gridDim.x * blockDim.x) Fp[Qp[i]] = 0;
   for (;;) {
     const uint32_t tile = next_tile(&ctl->tile_ctr[0], &s_tile);
     if (tile >= ntiles || s_fail) break;
@@ -1211,18 +1216,15 @@ struct MssBounds {
   int32_t hub;  // < 0: no bounds on this graph
 };
 
-// Clears the previous level's masks (they were read by the previous expand) and
-// brings the bounds up to date. A warp takes four rows at
-// a time, lane l the entries 2l and 2l+1; bound by the row reads (256 bytes per
-// vertex: 50 us for every row of R-MAT 20).
+// Brings the bounds up to date (launched on skewed graphs only). A warp takes
+// four rows at a time, lane l the entries 2l and 2l+1; bound by the row reads
+// (256 bytes per vertex: 50 us for every row of R-MAT 20).
 __global__ void __launch_bounds__(kNT) k_mss_bounds(MultiArgs a, MssBounds m) {
   Ctl *ctl = a.ctl;
   if (!ctl->active) return;
-  const uint32_t L = ctl->level, pn = ctl->prev_size, n = ctl->frontier_size;
-  u64 *Fp = nxt_F(a, L);
-  const int32_t *Qp = nxt_Q(a, L), *Q = cur_Q(a, L);
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < pn; i += gridDim.x * blockDim.x) Fp[Qp[i]] = 0;
-  if (m.hub < 0 || !m.offs[64]) return;
+  const uint32_t L = ctl->level, n = ctl->frontier_size;
+  const int32_t *Q = cur_Q(a, L);
+  if (!m.offs[64]) return;
   const bool full = m.offs[65] != 0;
   const int lane = lane_id();
   const int nsrc = m.offs[66];
@@ -1763,17 +1765,18 @@ int mg_sssp_multi(mg_graph *g, const int32_t *srcs, int32_t nsrc, int32_t *dists
   mb.lo = g->ws.vbuf[0];
   mb.hi = g->ws.vbuf[1];
   mb.offs = g->mss_offs;
-  mb.hub = g->mss_hub;
+  // (rows of up to 8 sources are one sector: a bound would cost as much as it saves)
+  mb.hub = nsrc > 8 ? g->mss_hub : -1;
   LevelBody body = [=](cudaStream_t ss, cudaGraphConditionalHandle h, int use_h) {
     MG_LAUNCH(KID_SCAN, ss, k_mss_scan<kMSVT><<<grid, kNT, 0, ss>>>(a, scan, part, status2));
-    MG_LAUNCH(KID_MS_APPLY, ss, k_mss_bounds<<<grid, kNT, 0, ss>>>(a, mb));
+    if (mb.hub >= 0) MG_LAUNCH(KID_MS_APPLY, ss, k_mss_bounds<<<grid, kNT, 0, ss>>>(a, mb));
     MG_LAUNCH(KID_MSS_EXPAND, ss, k_mss_expand<kMSVT><<<grid, kNT, 0, ss>>>(a, mb, scan, part));
     MG_LAUNCH(KID_OTHER, ss, k_mss_level_end<<<1, 64, 0, ss>>>(a, mb, h, use_h));
   };
   LoopResult res;
   const auto epi = transpose_epilogue(g, nsrc, dists, false, false);
-  st = run_level_loop(g, s, "sssp_multi/" + std::to_string(grid), 4, body, o->use_cuda_graph != 0, &res,
-                      o->outputs_on_device ? &epi : nullptr);
+  st = run_level_loop(g, s, std::string(mb.hub >= 0 ? "sssp_multi_bounds/" : "sssp_multi/") + std::to_string(grid),
+                      mb.hub >= 0 ? 4 : 3, body, o->use_cuda_graph != 0, &res, o->outputs_on_device ? &epi : nullptr);
   if (st != MG_OK) return st;
   return multi_finish(g, s, nsrc, dists, programs::sssp::INIT_VALUE, stats, o, res, false);
 }
