@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(kLoopNT, 1) k_bfs_loop(BfsLoopArgs a) {
   const uint32_t nw = nt / 32, gw = warp_id() * gridDim.x + blockIdx.x;
   LoopCtl *c = a.loop.c;
   if (threadIdx.x == 0) {
-    sh.my_count = sh.my_edges = 0;
+    sh.my_count = sh.my_edges = sh.my_mask = 0;
     sh.fail = 0;
   }
   __syncthreads();

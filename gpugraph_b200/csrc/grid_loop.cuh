@@ -26,6 +26,8 @@ struct LoopCtl {
   unsigned long long count[3];  // vertices found in a level
   unsigned long long edges[3];  // sum of their out-degrees
   uint32_t items[3];            // items appended to the next queue
+  uint32_t ranges[3];           // batched BFS: edge ranges, beside the vertices counted by items
+  unsigned long long mask[3];   // batched BFS: OR of the level's source masks
   int32_t low[3];               // SSSP: smallest pending distance
   double residual[3], dangling[3];  // PageRank: L1 change and dangling mass
   uint32_t arrived;
@@ -42,9 +44,9 @@ struct LoopOut {
 };
 
 struct LoopShared {
-  unsigned long long my_count, my_edges;  // this CTA's totals of the level
-  unsigned long long count, edges;        // the grid's, after the level's barrier
-  uint32_t items;
+  unsigned long long my_count, my_edges, my_mask;  // this CTA's totals of the level
+  unsigned long long count, edges, mask;           // the grid's, after the level's barrier
+  uint32_t items, ranges;
   int32_t low;
   double residual, dangling;
   int fail;
@@ -57,7 +59,7 @@ struct GridLoop {
   LoopOut *out;
 };
 
-// End of a level: adds this CTA's totals (my_count and my_edges, summed by its
+// End of a level: adds this CTA's totals (my_count, my_edges, my_mask, summed by its
 // threads since the last call; cleared here) to slot `slot`, waits for the whole
 // grid and leaves the grid's totals in sh. `n` counts the barriers of the run. False when the wait ran out.
 // Data written before the barrier by any CTA is visible after it to ordinary
@@ -68,7 +70,8 @@ MG_DEVINL bool grid_level_end(const GridLoop &g, LoopShared *sh, uint32_t slot, 
   if (threadIdx.x == 0) {
     if (sh->my_count) atomicAdd(&g.c->count[slot], sh->my_count);
     if (sh->my_edges) atomicAdd(&g.c->edges[slot], sh->my_edges);
-    sh->my_count = sh->my_edges = 0;
+    if (sh->my_mask) atomicOr(&g.c->mask[slot], sh->my_mask);
+    sh->my_count = sh->my_edges = sh->my_mask = 0;
     __threadfence();
     atomicAdd(&g.c->arrived, 1u);
     const uint32_t target = g.base + n * gridDim.x;
@@ -82,7 +85,9 @@ MG_DEVINL bool grid_level_end(const GridLoop &g, LoopShared *sh, uint32_t slot, 
     __threadfence();
     sh->count = *(volatile unsigned long long *)&g.c->count[slot];
     sh->edges = *(volatile unsigned long long *)&g.c->edges[slot];
+    sh->mask = *(volatile unsigned long long *)&g.c->mask[slot];
     sh->items = *(volatile uint32_t *)&g.c->items[slot];
+    sh->ranges = *(volatile uint32_t *)&g.c->ranges[slot];
     sh->low = *(volatile int32_t *)&g.c->low[slot];
     sh->residual = *(volatile double *)&g.c->residual[slot];
     sh->dangling = *(volatile double *)&g.c->dangling[slot];

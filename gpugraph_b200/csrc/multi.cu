@@ -42,6 +42,7 @@
 #include "gas/driver.cuh"
 #include "gas/engine.cuh"
 #include "gas/programs.cuh"
+#include "grid_loop.cuh"
 
 namespace mg {
 
@@ -539,29 +540,19 @@ MG_DEVINL void ms_segment(u64 x, int ck, int b, int e, bool starts, bool take, u
 // and balanced across lanes. The next masks go to the level stack; past it,
 // the new depths of a vertex are written by the whole warp (lane l: sources l
 // and l+32 of its row).
-template <typename DT>
-__global__ void __launch_bounds__(kNT, 6) k_ms_pull(MultiArgs a) {
-  Ctl *ctl = a.ctl;
-  if (!ctl->active || ctl->mode != MODE_BITMAP) return;
-  const uint32_t L = ctl->level;
-  const u64 active_src = ctl->srcmask[L & 1] & a.all;
-  const u64 *Fc = front_masks(a, ctl, L);
-  // next masks: written for every vertex, into the level stack while it has
-  // room (the depths are read from it at the end), else into the parity array
-  // with the new depths written to the rows
-  const bool to_stk = L + 1 < ctl->stk_levels;
-  u64 *Fn = to_stk ? stk_level(a, L + 1) : nxt_F(a, L);
+template <bool RO>
+MG_DEVINL u64 ms_front(const u64 *p) {
+  return RO ? __ldg(p) : *p;  // RO: not written while the kernel runs
+}
+template <typename DT, bool RO>
+MG_DEVINL void ms_pull_sweep(const MultiArgs &a, uint32_t L, const u64 *Fc, u64 *Fn, bool to_stk, u64 active_src,
+                             uint32_t gw, uint32_t nwarps, u64 &act, unsigned long long &my_cnt,
+                             unsigned long long &my_edges, unsigned long long &my_bytes) {
   const int32_t V = a.g.V;
   const int32_t *coff = a.g.csc_offsets, *crow = a.g.pull_rows, *ro = a.g.row_offsets;
   const int lane = lane_id();
   const uint32_t le = 0xffffffffu >> (31 - lane);  // lanes [0, lane]
-  unsigned long long my_cnt = 0, my_edges = 0, my_bytes = 0;
-  u64 act = 0;
   const uint32_t groups = ((uint32_t)V + 31) / 32;
-  __shared__ unsigned long long s_tot[3];
-  if (threadIdx.x < 3) s_tot[threadIdx.x] = 0;
-  __syncthreads();
-  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5, gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   // Long in-lists first, dealt back and forth over the warps in order of length
   // (the groups below skip them). Lane k of a warp takes the warp's k-th list:
   // its visit mask and, when it needs a source, its first kMsProbe in-edges
@@ -587,7 +578,7 @@ __global__ void __launch_bounds__(kNT, 6) k_ms_pull(MultiArgs a) {
 #pragma unroll
       for (int q = 0; q < kMsProbe; ++q) u[q] = __ldcs(crow + hb + q);  // a long list has more than kMsProbe
 #pragma unroll
-      for (int q = 0; q < kMsProbe; ++q) hacc |= __ldg(&Fc[u[q]]);
+      for (int q = 0; q < kMsProbe; ++q) hacc |= ms_front<RO>(&Fc[u[q]]);
       my_bytes += 12ull * kMsProbe;
     }
     bool open = hneed != 0ull && (hacc & hneed) != hneed;
@@ -608,7 +599,7 @@ __global__ void __launch_bounds__(kNT, 6) k_ms_pull(MultiArgs a) {
 #pragma unroll
         for (int q = 0; q < kMsHeavyK; ++q)
           if (uu[q] >= 0) {
-            x |= __ldg(&Fc[uu[q]]);
+            x |= ms_front<RO>(&Fc[uu[q]]);
             ++probes;
           }
         all |= ((u64)__reduce_or_sync(0xffffffffu, (uint32_t)(x >> 32)) << 32) |
@@ -657,7 +648,7 @@ __global__ void __launch_bounds__(kNT, 6) k_ms_pull(MultiArgs a) {
       for (int k = 0; k < kMsProbe; ++k) u[k] = (open && bs + k < lim) ? __ldcs(crow + bs + k) : -1;
 #pragma unroll
       for (int k = 0; k < kMsProbe; ++k)
-        if (u[k] >= 0) acc |= __ldg(&Fc[u[k]]);
+        if (u[k] >= 0) acc |= ms_front<RO>(&Fc[u[k]]);
       if (open) {
         probes += (unsigned long long)(lim - bs);
         bs = lim;
@@ -677,7 +668,7 @@ __global__ void __launch_bounds__(kNT, 6) k_ms_pull(MultiArgs a) {
           const int i = c + 32 * k + lane;
           x[k] = 0;
           if (i < lim) {
-            x[k] = __ldg(&Fc[__ldcs(crow + i)]);
+            x[k] = ms_front<RO>(&Fc[__ldcs(crow + i)]);
             ++probes;
           }
         }
@@ -712,6 +703,26 @@ __global__ void __launch_bounds__(kNT, 6) k_ms_pull(MultiArgs a) {
       if ((m >> (lane + 32)) & 1ull) row[lane + 32] = (DT)(L + 1);
     }
   }
+}
+
+template <typename DT>
+__global__ void __launch_bounds__(kNT, 6) k_ms_pull(MultiArgs a) {
+  Ctl *ctl = a.ctl;
+  if (!ctl->active || ctl->mode != MODE_BITMAP) return;
+  const uint32_t L = ctl->level;
+  // next masks: written for every vertex, into the level stack while it has
+  // room (the depths are read from it at the end), else into the parity array
+  // with the new depths written to the rows
+  const bool to_stk = L + 1 < ctl->stk_levels;
+  const int lane = lane_id();
+  unsigned long long my_cnt = 0, my_edges = 0, my_bytes = 0;
+  u64 act = 0;
+  __shared__ unsigned long long s_tot[3];
+  if (threadIdx.x < 3) s_tot[threadIdx.x] = 0;
+  __syncthreads();
+  ms_pull_sweep<DT, true>(a, L, front_masks(a, ctl, L), to_stk ? stk_level(a, L + 1) : nxt_F(a, L), to_stk,
+                          ctl->srcmask[L & 1] & a.all, (blockIdx.x * blockDim.x + threadIdx.x) >> 5,
+                          (gridDim.x * blockDim.x) >> 5, act, my_cnt, my_edges, my_bytes);
   add_bytes(ctl, KID_MS_PULL, my_bytes);
   // totals per CTA, then one atomic per CTA and counter on the control block
   act = warp_or(act);
@@ -855,6 +866,295 @@ __global__ void k_ms_level_end(Ctl *ctl, int32_t V, int64_t E, cudaGraphConditio
     ctl->active = (n_next > 0 && ctl->level < ctl->max_iter && ctl->error == 0) ? 1u : 0u;
   }
   if (use_handle) cudaGraphSetConditional(h, ctl->active);
+}
+
+// A whole batched BFS in one cooperative launch (grid_loop.cuh), for graphs whose
+// levels are short beside the six launches of a level in the loop above. The
+// rules of the direction and the result layout (level stack, depth rows) are the
+// same, and so are the depths.
+//
+// A push level takes a queue of edge ranges that carry their tail's mask. Heads
+// get the new sources by an atomic OR; the thread that finds the mask empty puts
+// the head on the level's list. After a barrier the list's vertices take their
+// new sources (visit, stack or rows), and, when they are few, their ranges are
+// appended at once; a level that pulls next does not need them. The masks of a
+// push-made level stay in its parity array until the level was expanded, then
+// they are cleared through its list. A pull level writes the next masks for
+// every vertex (stack, or past it the parity array, which is then cleared as a
+// whole before a push writes into it).
+// Vertices + edges up to which a run is one launch (64 sources, level loop / one
+// launch: R-MAT 10 210 / 99 us, 18 766 / 309, 20 559 / 455, 21 686 / 643, 22 no
+// difference past the noise; 1200x1200 road grid 4.4 / 3.4 ms).
+constexpr int64_t kMsLoopWork = 1ll << 26;
+constexpr int kMsLoopU = 4;                  // edges per lane in flight
+constexpr uint32_t kMsLoopList = 1u << 17;   // list length up to which its ranges are appended with the masks
+
+struct MsLoopArgs {
+  MultiArgs a;
+  SrcList src;
+  int4 *q;       // (first edge, length, tail's mask)
+  uint32_t cap;
+  uint32_t max_iter;
+  GridLoop loop;
+};
+
+// Appends the ranges of every lane's vertex (deg 0: none), one reservation per warp.
+MG_DEVINL void ms_append(const MsLoopArgs &p, uint32_t *tail, int beg, int deg, u64 mask) {
+  const uint32_t k = (uint32_t)(deg + kRange - 1) / kRange;
+  if (!__any_sync(0xffffffffu, k != 0u)) return;
+  const uint32_t inc = warp_inclusive_sum(k);
+  uint32_t at = 0;
+  if (lane_id() == 31) at = atomicAdd(tail, inc);
+  at = __shfl_sync(0xffffffffu, at, 31) + inc - k;
+  if (at + k > p.cap) {
+    atomicCAS(&p.loop.c->error, 0, (int)MG_ERR_OVERFLOW);
+    return;
+  }
+  for (int i = 0; i < deg; i += kRange)
+    p.q[at++] = make_int4(beg + i, min(kRange, deg - i), (int)(uint32_t)mask, (int)(uint32_t)(mask >> 32));
+}
+
+MG_DEVINL void ms_loop_push(const MsLoopArgs &p, uint32_t n, u64 *N, int32_t *list, uint32_t *tail, bool probe,
+                            uint32_t gw, uint32_t nw) {
+  const MultiArgs &a = p.a;
+  const int lane = lane_id();
+  const uint32_t V = (uint32_t)a.g.V;
+  const uint32_t per = min(32u, (n + nw - 1) / nw);
+  for (uint32_t base = gw; base < n; base += nw * per) {
+    int4 r = make_int4(0, 0, 0, 0);
+    if (lane < (int)per && base + lane * nw < n) r = __ldcg(&p.q[base + lane * nw]);
+    const int inc = warp_inclusive_sum(r.y);
+    const int total = __shfl_sync(0xffffffffu, inc, 31);
+    const int off = r.x - (inc - r.y);
+    for (int t = 0; t < total; t += 32 * kMsLoopU) {
+      int u[kMsLoopU];
+      u64 m[kMsLoopU];
+#pragma unroll
+      for (int k = 0; k < kMsLoopU; ++k) {
+        const int pos = t + 32 * k + lane;
+        int own = 0;  // the first range that ends past pos
+        if (per > 1) {
+#pragma unroll
+          for (int s = 16; s > 0; s >>= 1)
+            if (__shfl_sync(0xffffffffu, inc, own + s - 1) <= pos) own += s;
+          own = min(own, 31);
+        }
+        const int e = __shfl_sync(0xffffffffu, off, own) + pos;
+        const uint32_t lo = (uint32_t)__shfl_sync(0xffffffffu, r.z, own), hi = (uint32_t)__shfl_sync(0xffffffffu, r.w, own);
+        u[k] = pos < total && (unsigned)e < (unsigned)a.g.E ? __ldcs(a.g.col + e) : -1;
+        m[k] = ((u64)hi << 32) | lo;
+      }
+#pragma unroll
+      for (int k = 0; k < kMsLoopU; ++k) m[k] = (unsigned)u[k] < V ? m[k] & ~a.visit[u[k]] : 0ull;
+      if (probe) {
+#pragma unroll
+        for (int k = 0; k < kMsLoopU; ++k)
+          if (m[k]) m[k] &= ~__ldcg(&N[u[k]]);
+      }
+      uint32_t won = 0;
+#pragma unroll
+      for (int k = 0; k < kMsLoopU; ++k)
+        if (m[k] && atomicOr(&N[u[k]], m[k]) == 0ull) won |= 1u << k;
+      const uint32_t c = (uint32_t)__popc(won);
+      if (!__any_sync(0xffffffffu, c != 0u)) continue;
+      const uint32_t sum = warp_inclusive_sum(c);
+      uint32_t at = 0;
+      if (lane == 31) at = atomicAdd(tail, sum);
+      at = __shfl_sync(0xffffffffu, at, 31) + sum - c;
+#pragma unroll
+      for (int k = 0; k < kMsLoopU; ++k)
+        if ((won >> k) & 1u) {
+          if (at < V) list[at] = u[k];
+          ++at;
+        }
+    }
+  }
+}
+
+__global__ void __launch_bounds__(kLoopNT, 1) k_ms_loop(MsLoopArgs p) {
+  typedef uint16_t DT;
+  __shared__ LoopShared sh;
+  const MultiArgs &a = p.a;
+  const int lane = lane_id();
+  const uint32_t V = (uint32_t)a.g.V, words = (V + 31) / 32;
+  const uint32_t tid = blockIdx.x * kLoopNT + threadIdx.x, nt = gridDim.x * kLoopNT;
+  const uint32_t nw = nt / 32, gw = warp_id() * gridDim.x + blockIdx.x;
+  const int32_t *ro = a.g.row_offsets;
+  LoopCtl *c = p.loop.c;
+  auto clear_slot = [&](uint32_t s) {
+    c->count[s] = c->edges[s] = c->mask[s] = 0;
+    c->items[s] = c->ranges[s] = 0;
+  };
+  if (threadIdx.x == 0) {
+    sh.my_count = sh.my_edges = sh.my_mask = 0;
+    sh.fail = 0;
+  }
+  __syncthreads();
+  for (uint32_t v = tid; v < V; v += nt) a.visit[v] = a.F0[v] = a.F1[v] = 0;
+  for (uint32_t w = tid; w < words * kMsStackLevels; w += nt) a.stk_bm[w] = 0;
+  if (blockIdx.x == 0 && threadIdx.x < 3) {
+    clear_slot(threadIdx.x);
+    if (threadIdx.x == 0) c->error = 0;
+  }
+  uint32_t nbar = 0;
+  bool ok = grid_level_end(p.loop, &sh, 2, nbar);
+  if (ok) {
+    if (blockIdx.x == 0 && threadIdx.x < 64) {  // level 0: the distinct source vertices
+      const int t = threadIdx.x;
+      int b = 0, d = 0;
+      u64 m = 0;
+      if (t < p.src.ndistinct) {
+        const int v = p.src.distinct[t];
+        for (int s = 0; s < p.src.nsrc; ++s)
+          if (p.src.src[s] == v) m |= 1ull << s;
+        a.visit[v] = a.F0[v] = stk_level(a, 0)[v] = m;
+        a.q0[t] = v;
+        atomicOr(&a.stk_bm[v >> 5], 1u << (v & 31));
+        b = ro[v];
+        d = ro[v + 1] - b;
+      }
+      ms_append(p, &c->ranges[2], b, d, m);
+    }
+    ok = grid_level_end(p.loop, &sh, 2, nbar);
+  }
+  uint32_t L = 0, push = 0, pull = 0, stk_pull = 0;
+  uint32_t n = (uint32_t)p.src.ndistinct, ranges = sh.ranges;
+  u64 active = a.all;
+  bool by_pull = p.src.dir == MG_DIR_PULL, ready = true;  // ready: the ranges of this level exist
+  bool made_by_push = true;                               // its masks are in the parity array, through its list
+  bool dirty[2] = {false, false};                         // a pull past the stack wrote the whole parity array
+  int to_clear = -1;                                      // parity whose list's masks wait to be cleared ...
+  uint32_t clear_n = 0;                                   // ... and that list's length
+  while (ok && n > 0 && L < p.max_iter) {
+    const uint32_t slot = L % 3, par = L & 1;
+    if (blockIdx.x == 0 && threadIdx.x == 0) clear_slot((L + 1) % 3);  // last read before the previous level
+    u64 *Np = par ? a.F1 : a.F0, *Nn = par ? a.F0 : a.F1;
+    int32_t *Q = cur_Q(a, L), *Qn = nxt_Q(a, L);
+    const u64 *front = !made_by_push && L < kMsStackLevels ? stk_level(a, L) : Np;
+    const bool to_stk = L + 1 < kMsStackLevels;
+    u64 act = 0;
+    unsigned long long cnt = 0, edges = 0, bytes = 0;
+    uint32_t n_next;
+    if (by_pull) {
+      if (to_clear >= 0) {  // the level before this one was pulled from a push-made frontier
+        u64 *F = to_clear ? a.F1 : a.F0;
+        const int32_t *l = to_clear ? a.q1 : a.q0;
+        if (to_stk || F != Nn)
+          for (uint32_t i = tid; i < clear_n; i += nt) F[l[i]] = 0;
+        to_clear = -1;
+      }
+      ms_pull_sweep<DT, false>(a, L, front, to_stk ? stk_level(a, L + 1) : Nn, to_stk, active & a.all, gw, nw, act, cnt,
+                               edges, bytes);
+      if (made_by_push) {
+        to_clear = (int)par;
+        clear_n = n;
+      }
+      if (to_stk) stk_pull |= 1u << (L + 1);
+      else dirty[par ^ 1] = true;
+      ++pull;
+    } else {
+      if (!ready) {
+        if (made_by_push) {  // a long list, kept without ranges
+          for (uint32_t i0 = gw * 32; i0 < n; i0 += nw * 32) {
+            int b = 0, d = 0;
+            u64 m = 0;
+            if (i0 + lane < n) {
+              const int v = __ldcg(&Q[i0 + lane]);
+              m = Np[v];
+              b = ro[v];
+              d = m ? ro[v + 1] - b : 0;
+            }
+            ms_append(p, &c->ranges[(L + 2) % 3], b, d, m);
+          }
+        } else {  // pull -> push: every vertex with a mask; the parity arrays made clean
+          if (to_clear >= 0) {
+            u64 *F = to_clear ? a.F1 : a.F0;
+            const int32_t *l = to_clear ? a.q1 : a.q0;
+            for (uint32_t i = tid; i < clear_n; i += nt) F[l[i]] = 0;
+            to_clear = -1;
+          }
+          for (uint32_t v0 = gw * 32; v0 < V; v0 += nw * 32) {
+            const uint32_t v = v0 + lane;
+            const u64 m = v < V ? front[v] : 0ull;
+            if (v < V && dirty[par]) Np[v] = 0;
+            if (v < V && dirty[par ^ 1]) Nn[v] = 0;
+            int b = 0, d = 0;
+            if (m) {
+              b = ro[v];
+              d = ro[v + 1] - b;
+            }
+            ms_append(p, &c->ranges[(L + 2) % 3], b, d, m);
+          }
+          dirty[0] = dirty[1] = false;
+        }
+        if (!(ok = grid_level_end(p.loop, &sh, (L + 2) % 3, nbar))) break;
+        ranges = sh.ranges;
+      }
+      ms_loop_push(p, ranges, Nn, Qn, &c->items[slot], ranges > (1u << 13), gw, nw);
+      if (!(ok = grid_level_end(p.loop, &sh, slot, nbar))) break;
+      // the new sources of the list's vertices
+      const uint32_t len = min(sh.items, V);
+      const bool append = len <= kMsLoopList;
+      u64 *Sk = to_stk ? stk_level(a, L + 1) : nullptr;
+      uint32_t *Sb = to_stk ? a.stk_bm + (size_t)(L + 1) * a.stk_words : nullptr;
+      for (uint32_t i0 = gw * 32; i0 < len; i0 += nw * 32) {
+        int v = -1, b = 0, d = 0;
+        u64 m = 0;
+        if (i0 + lane < len) {
+          v = __ldcg(&Qn[i0 + lane]);
+          m = __ldcg(&Nn[v]);
+          a.visit[v] |= m;
+          b = ro[v];
+          d = ro[v + 1] - b;
+          edges += (unsigned long long)d;
+          act |= m;
+          if (to_stk) {
+            Sk[v] = m;
+            atomicOr(&Sb[v >> 5], 1u << (v & 31));
+          }
+        }
+        if (!to_stk) ms_write_rows<DT>(a, v, m, L + 1, lane);
+        if (append) ms_append(p, &c->ranges[slot], b, d, m);
+      }
+      cnt = gw == 0 && lane == 0 ? len : 0;
+      if (made_by_push)  // this level's masks, expanded above
+        for (uint32_t i = tid; i < n; i += nt) Np[Q[i]] = 0;
+      ++push;
+    }
+    act = warp_or(act);
+    cnt = warp_sum(cnt);
+    edges = warp_sum(edges);
+    if (lane == 0 && act) atomicOr(&sh.my_mask, act);
+    if (lane == 0 && cnt) atomicAdd(&sh.my_count, cnt);
+    if (lane == 0 && edges) atomicAdd(&sh.my_edges, edges);
+    if (!(ok = grid_level_end(p.loop, &sh, slot, nbar))) break;
+    n_next = (uint32_t)sh.count;
+    bool next_pull = by_pull;
+    if (p.src.dir == MG_DIR_PUSH) next_pull = false;
+    else if (p.src.dir == MG_DIR_PULL) next_pull = true;
+    else if (!by_pull) next_pull = (double)sh.edges > (double)a.g.E / (double)p.src.alpha;
+    else next_pull = !((double)n_next < (double)V / (double)p.src.beta && n_next < n);
+    active = sh.mask;
+    ranges = sh.ranges;
+    ready = !by_pull && n_next <= kMsLoopList;
+    made_by_push = !by_pull;
+    by_pull = next_pull;
+    n = n_next;
+    ++L;
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    LoopOut *o = p.loop.out;
+    o->level = L;
+    o->push_levels = push;
+    o->pull_levels = pull;
+    o->frontier_size = n;
+    o->barriers = nbar;
+    o->error = ok ? *(volatile int32_t *)&c->error : (int32_t)MG_ERR_TIMEOUT;
+    // what the transpose reads
+    a.ctl->level = L;
+    a.ctl->stk_levels = kMsStackLevels;
+    a.ctl->stk_pull = stk_pull;
+  }
 }
 
 // [V][64] -> [ns][V] for sources s_begin .. s_begin+ns-1, widening uint16
@@ -1544,7 +1844,7 @@ static MultiArgs multi_args(mg_graph *g) {
 }
 
 static int multi_prepare(mg_graph *g, const int32_t *srcs, int32_t nsrc, const mg_options *o, cudaStream_t s,
-                         SrcList *list, int32_t fill, bool stack = false) {
+                         SrcList *list, int32_t fill, bool stack = false, bool clear = true) {
   if (nsrc < 1 || nsrc > 64) return set_error(MG_ERR_ARG, "nsrc must be in [1, 64]");
   std::vector<int32_t> distinct;
   int st = check_sources(g, srcs, nsrc, &distinct);
@@ -1556,6 +1856,7 @@ static int multi_prepare(mg_graph *g, const int32_t *srcs, int32_t nsrc, const m
   list->ndistinct = (int32_t)distinct.size();
   if ((st = ensure_workspace(g)) != MG_OK) return st;
   if ((st = ensure_multi(g)) != MG_OK) return st;
+  if (!clear) return MG_OK;  // the one-launch loop starts its own state
   if ((st = prepare_run(g, s)) != MG_OK) return st;
   const size_t V = (size_t)g->nodes;
   cudaError_t e = cudaMemsetAsync(g->mask[0], 0, V * 8, s);
@@ -1654,13 +1955,60 @@ static int bfs_multi_run(mg_graph *g, const int32_t *srcs, int32_t nsrc, int32_t
   *depth_overflow = false;
   cudaStream_t s = run_stream(g, o);
   SrcList list;
-  int st = multi_prepare(g, srcs, nsrc, o, s, &list, -1, d16);
+  // short levels: one launch (kMsLoopWork); the loop below serves the rest, the
+  // host-driven runs, the ordered frontier, limited levels (whose last push level
+  // it leaves unapplied) and callers that shorten the waits
+  const bool one = d16 && o->use_cuda_graph && !o->ordered_frontier && !prof_on() &&
+                   o->spin_limit >= kSpinLimitDefault && (int64_t)o->iter_num >= g->nodes + 2 &&
+                   g->nodes + g->edges <= kMsLoopWork;
+  int st = multi_prepare(g, srcs, nsrc, o, s, &list, -1, d16, !one);
   if (st != MG_OK) return st;
   MultiArgs a = multi_args(g);
   a.all = (nsrc == 64) ? ~0ull : ((1ull << nsrc) - 1);
   if (d16) {
     a.stk = stack_of(g);
     a.rows = rows16_of(g);
+  }
+  const uint32_t max_iter_asked = (uint32_t)std::min<int64_t>(o->iter_num > 0 ? o->iter_num : 0, g->nodes + 2);
+  const uint32_t max_iter = d16 ? std::min(max_iter_asked, kMsDepth16Levels) : max_iter_asked;
+  // direction policy and switch factors
+  const int dir = o->direction;
+  list.dir = (uint32_t)dir;
+  list.alpha = (float)(o->alpha_multi > 0 ? o->alpha_multi : 5.0);
+  list.beta = (float)o->beta;
+  LoopResult res;
+  const auto epi = transpose_epilogue(g, nsrc, depths, true, d16);
+  if (one) {
+    std::lock_guard<std::mutex> lock(loop_mutex(g->device));
+    MsLoopArgs p;
+    p.a = a;
+    p.src = list;
+    p.q = reinterpret_cast<int4 *>(g->loop_queue);
+    p.cap = (uint32_t)g->loop_cap;
+    p.max_iter = max_iter;
+    p.loop = loop_begin(g, o);
+    void *args[] = {&p};
+    cudaError_t e = cudaEventRecord(g->ev0, s);
+    if (e == cudaSuccess)
+      e = cudaLaunchCooperativeKernel((const void *)k_ms_loop, dim3(g->num_sms), dim3(kLoopNT), args, 0, s);
+    if (e == cudaSuccess) e = cudaEventRecord(g->ev1, s);
+    count_launch();
+    if (e == cudaSuccess && o->outputs_on_device) epi(s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if ((st = cuda_status(e, "batched bfs")) != MG_OK || (st = loop_end(g, s, "batched traversal")) != MG_OK) return st;
+    memset(&res.ctl, 0, sizeof(res.ctl));
+    res.ctl.level = g->loop_out->level;
+    res.ctl.push_levels = g->loop_out->push_levels;
+    res.ctl.pull_levels = g->loop_out->pull_levels;
+    res.ctl.frontier_size = g->loop_out->frontier_size;
+    float ms = 0.f;
+    cudaEventElapsedTime(&ms, g->ev0, g->ev1);
+    res.ms = ms;
+    if (res.ctl.frontier_size > 0 && res.ctl.level >= kMsDepth16Levels && max_iter_asked > kMsDepth16Levels) {
+      *depth_overflow = true;  // deeper than a uint16 depth row holds
+      return MG_OK;
+    }
+    return multi_finish(g, s, nsrc, depths, -1, stats, o, res, d16);
   }
   GasArgs<msbfs_push> ga;
   ga.g = g->csr;
@@ -1682,13 +2030,6 @@ static int bfs_multi_run(mg_graph *g, const int32_t *srcs, int32_t nsrc, int32_t
   ga.ctl = g->ws.ctl;
   ga.expand_in = 0;
   ga.gather_dir = NO_GATHER_EDGES;
-  const uint32_t max_iter_asked = (uint32_t)std::min<int64_t>(o->iter_num > 0 ? o->iter_num : 0, g->nodes + 2);
-  const uint32_t max_iter = d16 ? std::min(max_iter_asked, kMsDepth16Levels) : max_iter_asked;
-  const int dir = o->direction;
-  // direction policy and switch factors go to the control block with the sources
-  list.dir = (uint32_t)dir;
-  list.alpha = (float)(o->alpha_multi > 0 ? o->alpha_multi : 5.0);
-  list.beta = (float)o->beta;
   k_ctl_init<<<1, 32, 0, s>>>(g->ws.ctl, (uint32_t)list.ndistinct, max_iter, (unsigned long long)o->spin_limit,
                               dir == MG_DIR_PULL ? MODE_BITMAP : MODE_QUEUE, ctl_flags(o));
   k_ms_init<<<1, 64, 0, s>>>(a, list, d16 ? 2 : 1);
@@ -1708,8 +2049,6 @@ static int bfs_multi_run(mg_graph *g, const int32_t *srcs, int32_t nsrc, int32_t
     MG_LAUNCH(KID_MS_PULL, ss, k_ms_pull<DT><<<pull_grid, kNT, 0, ss>>>(a));
     MG_LAUNCH(KID_OTHER, ss, k_ms_level_end<<<1, 32, 0, ss>>>(a.ctl, V, E, h, use_h));
   };
-  LoopResult res;
-  const auto epi = transpose_epilogue(g, nsrc, depths, true, d16);
   st = run_level_loop(g, s, std::string(d16 ? "bfs_multi16/" : "bfs_multi/") + std::to_string(grid), 6, body,
                       o->use_cuda_graph != 0, &res, o->outputs_on_device ? &epi : nullptr);
   if (st != MG_OK) return st;

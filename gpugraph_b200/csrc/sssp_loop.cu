@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(kLoopNT, 1) k_sssp_loop(SsspLoopArgs a) {
   const int32_t *ro = a.g.row_offsets, *col = a.g.col, *wgt = a.g.wgt;
   LoopCtl *c = a.loop.c;
   if (threadIdx.x == 0) {
-    sh.my_count = sh.my_edges = 0;
+    sh.my_count = sh.my_edges = sh.my_mask = 0;
     sh.fail = 0;
     s_min = INT_MAX;
   }

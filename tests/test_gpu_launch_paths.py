@@ -288,3 +288,29 @@ def test_one_launch_calls_from_several_threads():
     for t in th:
         t.join()
     assert not bad
+
+
+@pytest.mark.parametrize("name", list(GRAPHS) + ["long_lists"])
+def test_bfs_multi_one_launch_equals_level_loop(name):
+    # levels before and past the 16 of the level stack, both directions and runs that flip between them
+    # (alpha_multi, beta), lists with and without ranges, duplicated sources, limited runs
+    # long_lists: in-lists past 512 edges and more found vertices in a level than get their ranges at once
+    hg = HostGraph.rmat(18, 8, seed=3) if name == "long_lists" else GRAPHS[name]()
+    g = Graph(hg, directed=name == "directed")
+    deg = hg.out_degree()
+    rng = np.random.default_rng(4)
+    for nsrc in (1, 33, 64):
+        srcs = rng.integers(0, hg.nodes, nsrc).astype(np.int32)
+        srcs[0] = hg.max_degree_vertex()
+        some = {int(s): oracle.bfs(hg.row_offsets, hg.column_indices, int(s)) for s in srcs[:6]}
+        host, _ = g.bfs_multi(srcs, use_cuda_graph=0)
+        reached = host >= 0
+        for d in DIRS:
+            for mode in ({}, dict(alpha_multi=1e9, beta=0.5), dict(alpha_multi=1e-9, beta=1e9)):
+                out, st = g.bfs_multi(srcs, direction=d, **mode)
+                assert np.array_equal(out, host), (nsrc, d, mode)
+                assert st["vertices_reached"] == int(reached.sum()) and st["converged"] == 1
+                assert st["edges_traversed"] == int((reached * deg[None, :]).sum())
+        for k, s in enumerate(srcs):
+            if int(s) in some:
+                assert np.array_equal(host[k], some[int(s)])
