@@ -28,7 +28,7 @@ struct LoopCtl {
   uint32_t items[3];            // items appended to the next queue
   uint32_t ranges[3];           // batched BFS: edge ranges, beside the vertices counted by items
   unsigned long long mask[3];   // batched BFS: OR of the level's source masks
-  int32_t low[3];               // SSSP: smallest pending distance
+  int32_t low[3];               // SSSP: smallest waiting distance
   double residual[3], dangling[3];  // PageRank: L1 change and dangling mass
   uint32_t arrived;
   int32_t error;

@@ -1,12 +1,12 @@
 // Single-source SSSP in one cooperative launch (grid_loop.cuh), by distance
-// windows. The vertices whose distance was lowered and not yet relaxed are the
-// bits of a pending bitmap. A step selects those below the window's end (the
-// smallest pending distance plus `delta`), turns them into edge ranges, and
-// relaxes the ranges: an improving candidate lowers the head's distance and
-// sets its pending bit, both without waiting for a result. With non-negative
-// weights the smallest pending distance is final, so every step settles a
-// vertex and V steps suffice; the fixpoint is the one of the level-by-level
-// loop (sssp.cu), the unique shortest distances.
+// windows. done[v] is the distance at which v's edges were last relaxed; v waits
+// while its distance is smaller. A step selects the waiting vertices below the
+// window's end (the smallest waiting distance plus `delta`), turns them into edge
+// ranges, and relaxes the ranges: an improving candidate lowers the head's
+// distance without waiting for the result, and that is all an edge writes. With
+// non-negative weights the smallest waiting distance is final, so every step
+// settles a vertex and V steps suffice; the fixpoint is the one of the
+// level-by-level loop (sssp.cu), the unique shortest distances.
 //
 // Why windows: on a power-law graph relaxing every pending vertex per level
 // expands 3.0 times the edges (R-MAT 17, weights 1..64, simulated), a window of
@@ -27,7 +27,7 @@
 namespace mg {
 
 constexpr int kSpU = 8;        // edges per lane in flight (R-MAT 21: 1.30 ms a run, 1.38 with 4)
-constexpr int kSpWords = 4;    // pending words per warp and step of the selection
+constexpr int kSpVerts = 8;    // vertices per lane and step of the selection
 // Window: this many times the largest weight over the mean degree (with uniform
 // weights a vertex has about that many edges inside it). R-MAT 21, weights
 // 1..64: 1.39 ms a run at 2, 1.38 at 4, 1.44 at 8, 1.52 at 32 (no window in effect).
@@ -36,7 +36,7 @@ constexpr double kSsspWindow = 4.0;
 struct SsspLoopArgs {
   DevCsr g;
   int32_t *dist;
-  uint32_t *pending;
+  int32_t *done;
   int4 *q;       // (first edge, length, distance of the tail, unused)
   uint32_t cap;  // entries of q
   int32_t src, delta;
@@ -49,7 +49,7 @@ __global__ void __launch_bounds__(kLoopNT, 1) k_sssp_loop(SsspLoopArgs a) {
   __shared__ LoopShared sh;
   __shared__ int s_min;
   const int lane = lane_id();
-  const uint32_t V = (uint32_t)a.g.V, words = (V + 31) / 32;
+  const uint32_t V = (uint32_t)a.g.V;
   const uint32_t tid = blockIdx.x * kLoopNT + threadIdx.x, nt = gridDim.x * kLoopNT;
   const uint32_t nw = nt / 32, gw = warp_id() * gridDim.x + blockIdx.x;
   const int32_t *ro = a.g.row_offsets, *col = a.g.col, *wgt = a.g.wgt;
@@ -60,8 +60,10 @@ __global__ void __launch_bounds__(kLoopNT, 1) k_sssp_loop(SsspLoopArgs a) {
     s_min = INT_MAX;
   }
   __syncthreads();
-  for (uint32_t i = tid; i < V; i += nt) a.dist[i] = i == (uint32_t)a.src ? 0 : INF;
-  for (uint32_t i = tid; i < words; i += nt) a.pending[i] = i == (uint32_t)a.src >> 5 ? 1u << (a.src & 31) : 0u;
+  for (uint32_t i = tid; i < V; i += nt) {
+    a.dist[i] = i == (uint32_t)a.src ? 0 : INF;
+    a.done[i] = INF;
+  }
   if (blockIdx.x == 0 && threadIdx.x < 3) {
     c->count[threadIdx.x] = c->edges[threadIdx.x] = 0;
     c->items[threadIdx.x] = 0;
@@ -70,7 +72,7 @@ __global__ void __launch_bounds__(kLoopNT, 1) k_sssp_loop(SsspLoopArgs a) {
   }
   uint32_t nbar = 0, step = 0;
   bool ok = grid_level_end(a.loop, &sh, 2, nbar);
-  int low = 0;  // smallest pending distance
+  int low = 0;  // smallest waiting distance
   while (ok && low != INT_MAX && step < a.max_iter) {
     const uint32_t slot = step % 3;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -78,45 +80,49 @@ __global__ void __launch_bounds__(kLoopNT, 1) k_sssp_loop(SsspLoopArgs a) {
       c->low[(step + 1) % 3] = INT_MAX;
     }
     const int end = (int)min((long long)INT_MAX - 1, (long long)low + a.delta);
-    int rest = INT_MAX;  // smallest pending distance past the window
-    // selection: kSpWords words per warp step, a lane a vertex of each
-    for (uint32_t w0 = gw * kSpWords; w0 < words; w0 += nw * kSpWords) {
-      const uint32_t mine = lane < kSpWords && w0 + lane < words ? __ldcg(&a.pending[w0 + lane]) : 0u;
-      if (!__any_sync(0xffffffffu, mine != 0u)) continue;
-      int d[kSpWords], b[kSpWords], n[kSpWords];
-      bool sel[kSpWords];
-      uint32_t x[kSpWords];
+    int rest = INT_MAX;  // smallest waiting distance past the window
+    // selection: 32 * kSpVerts vertices per warp step (two coalesced streams)
+    for (uint32_t v0 = gw * 32 * kSpVerts; v0 < V; v0 += nw * 32 * kSpVerts) {
+      int d[kSpVerts], n[kSpVerts], b[kSpVerts];
+      uint32_t sel = 0;  // bit k: the lane's k-th vertex is selected
 #pragma unroll
-      for (int k = 0; k < kSpWords; ++k) {
-        x[k] = __shfl_sync(0xffffffffu, mine, k);
-        const uint32_t v = (w0 + k) * 32 + lane;
-        sel[k] = (x[k] >> lane) & 1u;
-        d[k] = sel[k] ? __ldcg(&a.dist[v]) : INT_MAX;
-        b[k] = sel[k] ? ro[v] : 0;
-        n[k] = sel[k] ? ro[v + 1] : 0;
+      for (int k = 0; k < kSpVerts; ++k) {
+        const uint32_t v = v0 + 32 * k + lane;
+        d[k] = v < V ? __ldcg(&a.dist[v]) : INT_MAX;
+        n[k] = v < V ? a.done[v] : 0;
+      }
+#pragma unroll
+      for (int k = 0; k < kSpVerts; ++k)
+        if (d[k] < n[k]) {
+          if (d[k] < end) sel |= 1u << k;
+          else rest = min(rest, d[k]);
+        }
+      if (!__any_sync(0xffffffffu, sel != 0u)) continue;
+#pragma unroll
+      for (int k = 0; k < kSpVerts; ++k) {
+        const uint32_t v = v0 + 32 * k + lane;
+        b[k] = n[k] = 0;
+        if ((sel >> k) & 1u) {
+          a.done[v] = d[k];
+          b[k] = ro[v];
+          n[k] = ro[v + 1];
+        }
       }
       uint32_t need = 0;
 #pragma unroll
-      for (int k = 0; k < kSpWords; ++k) {
-        if (sel[k] && d[k] >= end) {
-          rest = min(rest, d[k]);
-          sel[k] = false;
-        }
-        n[k] = sel[k] ? n[k] - b[k] : 0;
-        const uint32_t bal = __ballot_sync(0xffffffffu, sel[k]);
-        if (lane == 0 && bal) a.pending[w0 + k] = x[k] & ~bal;
+      for (int k = 0; k < kSpVerts; ++k) {
+        n[k] -= b[k];
         need += (uint32_t)(n[k] + kRange - 1) / kRange;
       }
-      if (!__any_sync(0xffffffffu, need != 0u)) continue;
       const uint32_t inc = warp_inclusive_sum(need);
       uint32_t at = 0;
-      if (lane == 31) at = atomicAdd(&c->items[slot], inc);
+      if (lane == 31 && inc) at = atomicAdd(&c->items[slot], inc);
       at = __shfl_sync(0xffffffffu, at, 31) + inc - need;
       if (at + need > a.cap) {
         atomicCAS(&c->error, 0, (int)MG_ERR_OVERFLOW);
       } else {
 #pragma unroll
-        for (int k = 0; k < kSpWords; ++k)
+        for (int k = 0; k < kSpVerts; ++k)
           for (int i = 0; i < n[k]; i += kRange)
             a.q[at++] = make_int4(b[k] + i, min(kRange, n[k] - i), d[k], 0);
       }
@@ -160,7 +166,6 @@ __global__ void __launch_bounds__(kLoopNT, 1) k_sssp_loop(SsspLoopArgs a) {
         for (int k = 0; k < kSpU; ++k)
           if (cand[k] < dv[k]) {
             atomicMin(&a.dist[u[k]], cand[k]);
-            atomicOr(&a.pending[u[k] >> 5], 1u << (u[k] & 31));
             best = min(best, cand[k]);
           }
       }
@@ -192,7 +197,7 @@ int sssp_loop_run(mg_graph *g, cudaStream_t s, int32_t src, const mg_options *o,
   SsspLoopArgs a;
   a.g = g->csr;
   a.dist = dist;
-  a.pending = g->ws.visited;
+  a.done = g->ws.vbuf[1];
   // the room of the two BFS queues: a step selects every vertex at most once
   static_assert(sizeof(int4) == 2 * sizeof(int2), "one queue of the same number of entries");
   a.q = reinterpret_cast<int4 *>(g->loop_queue);
