@@ -29,6 +29,7 @@ namespace mg {
 
 constexpr int kLoopU = 4;     // edges per lane in flight
 constexpr int kLoopWords = 4; // 32-vertex words per warp and step of a pull level
+constexpr int kConvWords = 8; // and of the pull -> push conversion (256 small graphs: one word at a time took 65 us)
 
 struct BfsLoopArgs {
   DevCsr g;
@@ -290,10 +291,18 @@ __global__ void __launch_bounds__(kLoopNT, 1) k_bfs_loop(BfsLoopArgs a) {
     int2 *q = (L & 1) ? a.q1 : a.q0, *qn = (L & 1) ? a.q0 : a.q1;
     if (bitmap) {
       if (!ready) {  // push -> pull: the bitmap of the vertices at depth L
-        for (uint32_t w = gw; w < words; w += nw) {
-          const uint32_t v = w * 32 + lane;
-          const uint32_t bal = __ballot_sync(0xffffffffu, v < (uint32_t)V && a.labels[v] == (int)L);
-          if (lane == 0) cur[w] = bal;
+        for (uint32_t w0 = gw * kConvWords; w0 < words; w0 += nw * kConvWords) {
+          int l[kConvWords];
+#pragma unroll
+          for (int k = 0; k < kConvWords; ++k) {
+            const uint32_t v = (w0 + k) * 32 + lane;
+            l[k] = v < (uint32_t)V ? a.labels[v] : -1;
+          }
+#pragma unroll
+          for (int k = 0; k < kConvWords; ++k) {
+            const uint32_t bal = __ballot_sync(0xffffffffu, l[k] == (int)L);
+            if (lane == 0 && w0 + k < words) cur[w0 + k] = bal;
+          }
         }
         if (!(ok = grid_level_end(a.loop, &sh, slot, nbar))) break;
       }
@@ -301,14 +310,20 @@ __global__ void __launch_bounds__(kLoopNT, 1) k_bfs_loop(BfsLoopArgs a) {
       ++pull;
     } else {
       if (!ready) {  // pull -> push: the ranges of the bitmap's vertices
-        for (uint32_t w = gw; w < words; w += nw) {
-          const uint32_t x = cur[w];
-          if (!x) continue;
-          int b[1] = {0}, d[1] = {0};
-          if ((x >> lane) & 1u) {
-            b[0] = ro[w * 32 + lane];
-            d[0] = ro[w * 32 + lane + 1] - b[0];
+        // kConvWords words per warp step: their row offsets in flight, one reservation
+        for (uint32_t w0 = gw * kConvWords; w0 < words; w0 += nw * kConvWords) {
+          const uint32_t mine = lane < kConvWords && w0 + lane < words ? cur[w0 + lane] : 0u;
+          if (!__any_sync(0xffffffffu, mine != 0u)) continue;
+          int b[kConvWords], d[kConvWords];
+#pragma unroll
+          for (int k = 0; k < kConvWords; ++k) {
+            const uint32_t x = __shfl_sync(0xffffffffu, mine, k), v = (w0 + k) * 32 + lane;
+            const bool in = (x >> lane) & 1u;
+            b[k] = in ? ro[v] : 0;
+            d[k] = in ? ro[v + 1] : 0;
           }
+#pragma unroll
+          for (int k = 0; k < kConvWords; ++k) d[k] -= b[k];
           append_ranges(q, &c->items[(L + 2) % 3], a.cap, &c->error, b, d);
         }
         if (!(ok = grid_level_end(a.loop, &sh, (L + 2) % 3, nbar))) break;
