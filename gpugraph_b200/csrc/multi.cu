@@ -53,14 +53,14 @@ constexpr int kMVT = 8;
 // tiles are the smallest the workspace allows (1024 items): more CTAs share a
 // level's edges.
 constexpr int kMSVT = 4;
-// Edges whose row loads a warp has in flight (R-MAT 20, 37 sources: 4.9 ms with
-// 8, 5.1 with 16, 5.1 with 4 and the tails' rows held in registers).
+// Edges whose row loads a warp has in flight, two side by side (R-MAT 20, 37
+// sources / road 1200, 64 sources: 3.9 / 18.4 ms with 8, 4.6 / 19.4 with 16).
 constexpr int kMssEdges = 8;
 // Active sources per edge up to which a lane relaxes a whole edge alone: below,
-// the row accesses of a warp-wide edge carry mostly inactive entries, above, the
-// lane's scalar loads touch a sector per source (R-MAT 20, 37 sources / road
-// 1200, 64 sources: 5.1 / 26.2 ms at 4, 4.9 / 23.8 at 12, 5.5 / 24.5 at 24).
-constexpr int kMssSparse = 12;
+// the row accesses of a half warp's edge carry mostly inactive entries, above, the
+// lane's scalar loads touch a sector per source (the same two runs: 4.0 / 19.6 ms
+// at 4, 3.9 / 18.4 at 8, 4.1 / 18.3 at 12, 5.0 / 19.3 at 20).
+constexpr int kMssSparse = 8;
 
 // Push step of the batched BFS as a GAS Program: expand_edge emits the
 // sources that reach the neighbour for the first time, contract ORs them into
@@ -160,10 +160,10 @@ struct SrcList {
   float alpha, beta;
 };
 
-// The mask bit of source s in a batched SSSP, and back: the two sources of a
-// row pair are the two bits of one lane (k_mss_expand).
-MG_DEVINL int mss_bit(int s) { return (s >> 1) + 32 * (s & 1); }
-MG_DEVINL int mss_source(int bit) { return 2 * (bit & 31) + (bit >> 5); }
+// The mask bit of source s in a batched SSSP, and back: 16 lanes hold a row, the
+// four sources of a lane are a bit of each 16-bit piece of the mask (k_mss_expand).
+MG_DEVINL int mss_bit(int s) { return (s >> 2) + 16 * (s & 3); }
+MG_DEVINL int mss_source(int bit) { return 4 * (bit & 15) + (bit >> 4); }
 
 // Level-0 state of a batched run (one CTA of 64 threads).
 // bfs: 0 = SSSP (int32 rows), 1 = BFS with int32 depth rows, 2 = BFS with the
@@ -1530,6 +1530,7 @@ __global__ void __launch_bounds__(kNT) k_mss_bounds(MultiArgs a, MssBounds m) {
   const int nsrc = m.offs[66];
   const bool k0 = 2 * lane < nsrc, k1 = 2 * lane + 1 < nsrc;
   const int c0 = m.offs[2 * lane], c1 = m.offs[2 * lane + 1];
+  const int bit0 = mss_bit(2 * lane), bit1 = mss_bit(2 * lane + 1);
   const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
   const u64 *Fc = cur_F(a, L);
   constexpr int R = 4;
@@ -1563,8 +1564,8 @@ __global__ void __launch_bounds__(kNT) k_mss_bounds(MultiArgs a, MssBounds m) {
 #pragma unroll
     for (int q = 0; q < R; ++q) {
       const int x0 = d[q].x - c0, x1 = d[q].y - c1;
-      const int lo = __reduce_min_sync(0xffffffffu, min((am[q] >> lane) & 1ull ? x0 : INT_MAX,
-                                                        (am[q] >> (lane + 32)) & 1ull ? x1 : INT_MAX));
+      const int lo = __reduce_min_sync(0xffffffffu, min((am[q] >> bit0) & 1ull ? x0 : INT_MAX,
+                                                        (am[q] >> bit1) & 1ull ? x1 : INT_MAX));
       const int hi = __reduce_max_sync(0xffffffffu, max(k0 ? x0 : INT_MIN, k1 ? x1 : INT_MIN));
       if (lane == 0 && v[q] >= 0) {
         m.lo[v[q]] = lo;
@@ -1593,18 +1594,18 @@ MG_DEVINL void relax_min(int32_t *p, int32_t c, u64 &imp, int t) {
 // shared memory; then each warp relaxes its own kept edges 32 at a time. If
 // every edge of a batch carries at most kMssSparse active sources, each lane
 // relaxes its own edge source by source (scalar loads from the two 256-byte
-// rows); otherwise the whole warp takes the edges kMssEdges at a time, lane l
-// owning sources 2l and 2l+1: a row is one coalesced load (of the pairs with an
-// active source; relaxing the other source of a pair as well is harmless) and
-// the improved-source mask the two ballots, which is why source s is bit
-// s/2 + 32 (s%2) of an SSSP mask.
+// rows); otherwise the warp takes the edges kMssEdges at a time, two side by side:
+// lane l of a half owns sources 4l to 4l+3, a row is one coalesced load (of the
+// pieces with an active source; relaxing the other sources of a piece as well is
+// harmless) and the improved-source masks are the halves of four ballots, which
+// is why source s is bit s/4 + 16 (s%4) of an SSSP mask.
 //
 // Bound by the latency of the random row reads (the rows are larger than L2):
 // what counts is edges in flight per SM, 32 warps of 8 here; fewer registers
 // and more warps, or more edges and fewer warps, were slower (48 registers and
 // 5 CTAs per SM: 5.8 ms at R-MAT 20; 3 CTAs: 5.2 ms, against 4.3). Before, with
 // a 32-byte row piece per lane, 8 scattered reductions per step and a queue
-// reservation per 4 edges: 7.8 ms a run, now 4.5.
+// reservation per 4 edges: 7.8 ms a run, 4.4 with a whole warp per edge, now 3.9.
 template <int VT>
 __global__ void __launch_bounds__(kNT, 4) k_mss_expand(MultiArgs a, MssBounds mb, const uint32_t *scan,
                                                        const int32_t *part) {
@@ -1631,7 +1632,8 @@ __global__ void __launch_bounds__(kNT, 4) k_mss_expand(MultiArgs a, MssBounds mb
   bool any = false;
   const bool bounds = mb.hub >= 0 && mb.offs[64] != 0;
   const int lane = lane_id(), warp = warp_id();
-  const uint32_t lbit = 1u << lane;
+  const int half = lane >> 4, sub = lane & 15;  // two edges side by side, 16 lanes each
+  const uint32_t sbit = 1u << sub;
   unsigned long long my_bytes = 0;
   // the tile after the current one is reserved ahead (the ticket's round trip
   // is hidden behind the tile's work; a CTA leaves one ticket unused)
@@ -1701,7 +1703,7 @@ __global__ void __launch_bounds__(kNT, 4) k_mss_expand(MultiArgs a, MssBounds mb
         const uint32_t kb = __ballot_sync(0xffffffffu, am != 0ull);
         if (am)
           we[kept + __popc(kb & lanemask_lt())] =
-              make_int4(j[r], v[r], w[r], (int)((uint32_t)am | (uint32_t)(am >> 32)));
+              make_int4(j[r], v[r], w[r], (int)((am | am >> 16 | am >> 32 | am >> 48) & 0xffffull));
         kept += __popc(kb);
       }
     }
@@ -1744,30 +1746,40 @@ __global__ void __launch_bounds__(kNT, 4) k_mss_expand(MultiArgs a, MssBounds mb
           // the heads' rows of all kMssEdges edges in flight; the tails' rows come
           // through L1 as they are needed (the edges of a tail are neighbours in
           // the batch; an entry lowered meanwhile is marked and relaxed again next
-          // level), so an edge in flight holds two registers
-          int2 h[kMssEdges];
+          // level), so two edges in flight hold four registers
+          int4 h[kMssEdges / 2];
 #pragma unroll
-          for (int q = 0; q < kMssEdges; ++q) {
-            h[q] = make_int2(INT_MIN, INT_MIN);  // a pair that is not loaded is never improved
-            const int4 e = we[b0 + j0 + q];
-            if (j0 + q < nb && ((uint32_t)e.w & lbit))
-              h[q] = __ldcg(reinterpret_cast<const int2 *>(a.out + (int64_t)e.y * 64 + 2 * lane));
+          for (int q = 0; q < kMssEdges / 2; ++q) {
+            h[q] = make_int4(INT_MIN, INT_MIN, INT_MIN, INT_MIN);  // a piece that is not loaded is never improved
+            const int i = j0 + 2 * q + half;
+            const int4 e = we[b0 + i];
+            if (i < nb && ((uint32_t)e.w & sbit))
+              h[q] = __ldcg(reinterpret_cast<const int4 *>(a.out + (int64_t)e.y * 64 + 4 * sub));
           }
 #pragma unroll
-          for (int q = 0; q < kMssEdges; ++q) {
-            const int4 e = we[b0 + j0 + q];
-            bool p0 = false, p1 = false;
+          for (int q = 0; q < kMssEdges / 2; ++q) {
+            const int4 e = we[b0 + j0 + 2 * q + half];
+            bool p0 = false, p1 = false, p2 = false, p3 = false;
             if (h[q].x != INT_MIN) {
-              const int2 t = *reinterpret_cast<const int2 *>(a.out + (int64_t)s_v[e.x] * 64 + 2 * lane);
-              const int c0 = t.x + e.z, c1 = t.y + e.z;
-              int32_t *hp = a.out + (int64_t)e.y * 64 + 2 * lane;
-              p0 = c0 < h[q].x;
-              p1 = c1 < h[q].y;
-              if (p0) atomicMin(hp, c0);  // result unused: a reduction (see relax_min)
-              if (p1) atomicMin(hp + 1, c1);
+              const int4 t = *reinterpret_cast<const int4 *>(a.out + (int64_t)s_v[e.x] * 64 + 4 * sub);
+              int32_t *hp = a.out + (int64_t)e.y * 64 + 4 * sub;
+              p0 = t.x + e.z < h[q].x;
+              p1 = t.y + e.z < h[q].y;
+              p2 = t.z + e.z < h[q].z;
+              p3 = t.w + e.z < h[q].w;
+              // results unused: reductions (see relax_min)
+              if (p0) atomicMin(hp, t.x + e.z);
+              if (p1) atomicMin(hp + 1, t.y + e.z);
+              if (p2) atomicMin(hp + 2, t.z + e.z);
+              if (p3) atomicMin(hp + 3, t.w + e.z);
             }
             const uint32_t m0 = __ballot_sync(0xffffffffu, p0), m1 = __ballot_sync(0xffffffffu, p1);
-            if (lane == j0 + q) imp = ((u64)m1 << 32) | m0;
+            const uint32_t m2 = __ballot_sync(0xffffffffu, p2), m3 = __ballot_sync(0xffffffffu, p3);
+            // the low halves are edge j0 + 2q, the high halves the next one
+            if ((lane >> 1) == (j0 >> 1) + q) {
+              const uint32_t pick = (lane & 1) ? 0x7632u : 0x5410u;
+              imp = ((u64)__byte_perm(m2, m3, pick) << 32) | __byte_perm(m0, m1, pick);
+            }
           }
         }
       }
