@@ -38,7 +38,7 @@ struct LoopCtl {
 struct LoopOut {
   uint32_t level, push_levels, pull_levels, frontier_size;
   unsigned long long visited_count, visited_edges;
-  double residual;
+  double residual, norm;
   uint32_t barriers;
   int32_t error;
 };

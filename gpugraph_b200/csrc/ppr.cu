@@ -13,10 +13,10 @@
 // distributions that is tolerance * nvec), or after iter_num iterations.
 //
 // Layout and work split: the solve's rows are padded to nv = nvec rounded up to
-// a multiple of 4, so every row is 16-byte aligned. A group of G lanes (nv/4
-// rounded up to a power of two) owns one chunk of one vertex's adjacency and
-// lane l of the group columns 4l..4l+3: an edge costs one coalesced row read,
-// and a warp works on 32/G chunks at once. The chunks are taken in descending
+// a multiple of 4, so every row is 16-byte aligned and falls into G pieces of 4
+// columns (nv/4 rounded up to a power of two). A group of 8 lanes (16 for more
+// than 32 columns) owns one chunk of one vertex's adjacency (PprGroup): an edge
+// costs one coalesced row read, and a warp works on 4 (2) chunks at once. The chunks are taken in descending
 // order of length (vertex order within a length), so the groups of a warp run
 // the same number of steps. Adjacencies longer than kPprChunk are cut into
 // chunks whose partial rows are added in chunk order by a fix-up pass
@@ -27,14 +27,23 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
+#include <cstring>
 #include <vector>
 
 #include "algo_util.cuh"
 #include "gas/driver.cuh"
 #include "gas/engine.cuh"
+#include "grid_loop.cuh"
 
 namespace mg {
 
+// Longest chunk. On a graph of up to kPprSmall edges the chunks are as long as the
+// square root of the longest list, to a power of two from 64 on: a chunk is summed
+// step by step, a cut list's partial rows one after the other, and the longer of
+// the two chains is the iteration there (R-MAT 12, 32 columns, forward and
+// backward: 3.25 ms with chunks of 256, 1.84 with 64; R-MAT 18, 12 columns: 6.5 /
+// 7.1 ms with 128).
+constexpr int64_t kPprSmall = 1 << 21;
 constexpr int kPprChunk = 256;
 constexpr int kPprMaxVec = 64;
 
@@ -65,98 +74,114 @@ MG_DEVINL void ppr_finalize_row(const PprArgs &a, int v, const float (&acc)[NC],
   }
 }
 
-// The edges [k, k + kPprStep) of a group's chunk, held by its G lanes: lane l
-// has edge k + l (and k + l + G, ... when G < kPprStep). Past the end: u = -1.
+// A group of kPprStep lanes (16 when a row has more than 8 pieces) takes a chunk
+// in steps of kPprStep edges. Its lanes are G column pieces x ES edge slots: the
+// lane of slot e takes the step's edges e, e + ES, ..., and the slots' sums are
+// added at the end of the chunk (one slot from 17 columns on).
 constexpr int kPprStep = 8;
 template <int G>
-struct PprStep {
-  static constexpr int N = G < kPprStep ? kPprStep / G : 1;
-  int u[N];
-  float w[N];
-  MG_DEVINL void load(const int32_t *idx, const float *wgt, int k, int e, int gl) {
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-      const int p = k + (gl & (kPprStep - 1)) + i * G;
-      const bool in = p < e;
-      u[i] = in ? __ldcs(idx + p) : -1;
-      w[i] = in && wgt ? __ldcs(wgt + p) : 0.f;
-    }
+struct PprGroup {
+  static constexpr int kLanes = G < kPprStep ? kPprStep : G;
+  static constexpr int kPer = 32 / kLanes;      // chunks per warp
+  static constexpr int kSlots = kLanes / G;     // edge slots
+  static constexpr int kEdges = kPprStep / kSlots;  // edges of a step per lane
+  int gl, piece, slot;
+  MG_DEVINL PprGroup() : gl(lane_id() & (kLanes - 1)), piece(gl % G), slot(gl / G) {}
+  // the step's edges [k, k + kPprStep): lane l holds edge k + l (-1 past the end)
+  MG_DEVINL void load(const int32_t *idx, const float *wgt, int k, int e, int &u, float &w) const {
+    const int p = k + (gl & (kPprStep - 1));
+    u = p < e ? __ldcs(idx + p) : -1;
+    w = p < e && wgt ? __ldcs(wgt + p) : 0.f;
   }
-  MG_DEVINL int edge(int j) const { return __shfl_sync(0xffffffffu, u[j / G < N ? j / G : 0], j % G, G); }
-  MG_DEVINL float weight(int j) const { return __shfl_sync(0xffffffffu, w[j / G < N ? j / G : 0], j % G, G); }
+  template <typename T>
+  MG_DEVINL T of(T x, int j) const {  // the value of this lane's j-th edge of the step
+    return __shfl_sync(0xffffffffu, x, j * kSlots + slot, kLanes);
+  }
+  MG_DEVINL float sum_slots(float x) const {
+#pragma unroll
+    for (int o = G; o < kLanes; o <<= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    return x;
+  }
 };
 
-// One iteration over the chunks. A step's kPprStep row loads are in flight
+// One iteration's sweep over the chunks. A step's row loads are in flight
 // together, its indices and weights were loaded one step ahead (one coalesced
 // load per group each, passed on by shuffles). Vertices without edges keep
 // alpha*rhs: both iterates hold it after the first two iterations, and from
 // then on their chunks are not visited.
-template <int G>
-__global__ void __launch_bounds__(kNT, 4) k_ppr_iter(PprArgs a) {
-  constexpr int PER = 32 / G;
-  Ctl *ctl = a.ctl;
-  if (!ctl->active) return;
-  const uint32_t L = ctl->level;
+template <int G, bool RO>
+MG_DEVINL void ppr_sweep(const PprArgs &a, uint32_t L, uint32_t gw, uint32_t nw, double &res,
+                         unsigned long long &my_bytes) {
+  using P = PprGroup<G>;
+  const P g;
   const float *xold = (L & 1) ? a.x1 : a.x0;
   float *xnew = (L & 1) ? a.x0 : a.x1;
-  const int lane = lane_id();
-  const int gl = lane & (G - 1);
-  const int col = gl * 4;
+  const int col = g.piece * 4;
   const bool cok = col < a.nv;
-  double res = 0.0;
-  unsigned long long my_bytes = 0;
   const uint32_t n = (uint32_t)(L < 2 ? a.nchunks : a.nfull);
-  const uint32_t nslots = gridDim.x * kNW * PER;
-  for (uint32_t c0 = (blockIdx.x * kNW + warp_id()) * PER; c0 < n; c0 += nslots) {
-    const uint32_t c = c0 + lane / G;
+  for (uint32_t c0 = gw * P::kPer; c0 < n; c0 += nw * P::kPer) {
+    const uint32_t c = c0 + lane_id() / P::kLanes;
     const bool has = c < n;
     const int v = has ? a.cv[c] : 0, b = has ? a.cb[c] : 0, e = has ? a.ce[c] : 0;
     const int slot = has ? a.cslot[c] : 0;
     const int steps = (__reduce_max_sync(0xffffffffu, e - b) + kPprStep - 1) / kPprStep;
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    PprStep<G> cur;
-    cur.load(a.idx, a.w, b, e, gl);
+    int u, un;
+    float w, wn;
+    g.load(a.idx, a.w, b, e, u, w);
     for (int s = 0; s < steps; ++s) {
-      PprStep<G> nxt;
-      nxt.load(a.idx, a.w, b + (s + 1) * kPprStep, e, gl);
-      float4 row[kPprStep];
+      g.load(a.idx, a.w, b + (s + 1) * kPprStep, e, un, wn);
+      float4 row[P::kEdges];
 #pragma unroll
-      for (int j = 0; j < kPprStep; ++j) {
-        const int u = cur.edge(j);
+      for (int j = 0; j < P::kEdges; ++j) {
+        const int t = g.of(u, j);
         row[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (u >= 0 && cok) row[j] = __ldg(reinterpret_cast<const float4 *>(xold + (int64_t)u * a.nv + col));
+        if (t >= 0 && cok) {
+          const float4 *r = reinterpret_cast<const float4 *>(xold + (int64_t)t * a.nv + col);
+          row[j] = RO ? __ldg(r) : *r;
+        }
       }
 #pragma unroll
-      for (int j = 0; j < kPprStep; ++j) {
-        const float wt = cur.weight(j);
+      for (int j = 0; j < P::kEdges; ++j) {
+        const float wt = g.of(w, j);
         acc.x = fmaf(wt, row[j].x, acc.x);
         acc.y = fmaf(wt, row[j].y, acc.y);
         acc.z = fmaf(wt, row[j].z, acc.z);
         acc.w = fmaf(wt, row[j].w, acc.w);
       }
-      cur = nxt;
+      u = un;
+      w = wn;
     }
+    acc = make_float4(g.sum_slots(acc.x), g.sum_slots(acc.y), g.sum_slots(acc.z), g.sum_slots(acc.w));
     if (!has) continue;
-    if (gl == 0) my_bytes += (unsigned long long)(e - b) * (8ull + 4ull * a.nv);
+    if (g.gl == 0) my_bytes += (unsigned long long)(e - b) * (8ull + 4ull * a.nv);
+    if (g.slot != 0 || !cok) continue;
     if (slot < 0) {
-      if (cok) {
-        const int64_t o = (int64_t)v * a.nv + col;
-        const float4 r = *reinterpret_cast<const float4 *>(a.rhs + o);
-        const float4 xo = *reinterpret_cast<const float4 *>(xold + o);
-        float4 xn;
-        xn.x = fmaf(a.d, acc.x, a.alpha * r.x);
-        xn.y = fmaf(a.d, acc.y, a.alpha * r.y);
-        xn.z = fmaf(a.d, acc.z, a.alpha * r.z);
-        xn.w = fmaf(a.d, acc.w, a.alpha * r.w);
-        res += (double)fabsf(xn.x - xo.x) + (double)fabsf(xn.y - xo.y) + (double)fabsf(xn.z - xo.z) +
-               (double)fabsf(xn.w - xo.w);
-        *reinterpret_cast<float4 *>(xnew + o) = xn;
-      }
-      if (gl == 0) my_bytes += 12ull * a.nv;
-    } else if (cok) {
+      const int64_t o = (int64_t)v * a.nv + col;
+      const float4 r = *reinterpret_cast<const float4 *>(a.rhs + o);
+      const float4 xo = *reinterpret_cast<const float4 *>(xold + o);
+      float4 xn;
+      xn.x = fmaf(a.d, acc.x, a.alpha * r.x);
+      xn.y = fmaf(a.d, acc.y, a.alpha * r.y);
+      xn.z = fmaf(a.d, acc.z, a.alpha * r.z);
+      xn.w = fmaf(a.d, acc.w, a.alpha * r.w);
+      res += (double)fabsf(xn.x - xo.x) + (double)fabsf(xn.y - xo.y) + (double)fabsf(xn.z - xo.z) +
+             (double)fabsf(xn.w - xo.w);
+      *reinterpret_cast<float4 *>(xnew + o) = xn;
+      if (g.piece == 0) my_bytes += 12ull * a.nv;
+    } else {
       *reinterpret_cast<float4 *>(a.partial + (int64_t)slot * a.nv + col) = acc;
     }
   }
+}
+
+template <int G>
+__global__ void __launch_bounds__(kNT, 4) k_ppr_iter(PprArgs a) {
+  Ctl *ctl = a.ctl;
+  if (!ctl->active) return;
+  double res = 0.0;
+  unsigned long long my_bytes = 0;
+  ppr_sweep<G, true>(a, ctl->level, blockIdx.x * kNW + warp_id(), gridDim.x * kNW, res, my_bytes);
   add_bytes(ctl, KID_PPR, my_bytes);
   res = cta_sum_f64(res);
   if (threadIdx.x == 0 && res != 0.0) atomicAdd(&ctl->acc[1], res);
@@ -164,16 +189,11 @@ __global__ void __launch_bounds__(kNT, 4) k_ppr_iter(PprArgs a) {
 
 // Split vertices: partial rows added in chunk order.
 template <int NC>
-__global__ void __launch_bounds__(kNT) k_ppr_fixup(PprArgs a) {
-  Ctl *ctl = a.ctl;
-  if (!ctl->active) return;
-  const uint32_t L = ctl->level;
+MG_DEVINL void ppr_fix(const PprArgs &a, uint32_t L, uint32_t gw, uint32_t nw, double &res) {
   const float *xold = (L & 1) ? a.x1 : a.x0;
   float *xnew = (L & 1) ? a.x0 : a.x1;
   const int lane = lane_id();
-  double res = 0.0;
-  const uint32_t nwarps = gridDim.x * kNW;
-  for (uint32_t m = blockIdx.x * kNW + warp_id(); m < (uint32_t)a.nmulti; m += nwarps) {
+  for (uint32_t m = gw; m < (uint32_t)a.nmulti; m += nw) {
     const int v = a.mv[m];
     float acc[NC];
 #pragma unroll
@@ -204,8 +224,75 @@ __global__ void __launch_bounds__(kNT) k_ppr_fixup(PprArgs a) {
       }
     ppr_finalize_row<NC>(a, v, acc, xold, xnew, res);
   }
+}
+
+template <int NC>
+__global__ void __launch_bounds__(kNT) k_ppr_fixup(PprArgs a) {
+  Ctl *ctl = a.ctl;
+  if (!ctl->active) return;
+  double res = 0.0;
+  ppr_fix<NC>(a, ctl->level, blockIdx.x * kNW + warp_id(), gridDim.x * kNW, res);
   res = cta_sum_f64(res);
   if (threadIdx.x == 0 && res != 0.0) atomicAdd(&ctl->acc[1], res);
+}
+
+// A whole solve in one cooperative launch (grid_loop.cuh): one barrier per
+// iteration, two where adjacencies are cut, one more for the norm of the
+// right-hand side. For solves whose iteration is short beside the launches of
+// the level loop.
+template <int G>
+__global__ void __launch_bounds__(kLoopNT, 1) k_ppr_loop(PprArgs a, double tol, uint32_t max_iter, GridLoop loop) {
+  __shared__ LoopShared sh;
+  const uint32_t tid = blockIdx.x * kLoopNT + threadIdx.x, nt = gridDim.x * kLoopNT;
+  const uint32_t nw = nt / 32, gw = warp_id() * gridDim.x + blockIdx.x;
+  LoopCtl *c = loop.c;
+  if (threadIdx.x == 0) {
+    sh.my_count = sh.my_edges = sh.my_mask = 0;
+    sh.fail = 0;
+  }
+  // slot 1 takes the norm, slot 0 the first iteration
+  if (blockIdx.x == 0 && threadIdx.x < 3) {
+    c->residual[threadIdx.x] = 0.0;
+    if (threadIdx.x == 0) c->error = 0;
+  }
+  uint32_t nbar = 0, L = 0;
+  __syncthreads();
+  bool ok = grid_level_end(loop, &sh, 2, nbar);
+  double sum = 0.0;
+  for (int64_t i = tid; i < (int64_t)a.V * a.nv; i += nt) sum += fabs((double)a.rhs[i]);
+  sum = cta_sum_f64(sum);
+  if (threadIdx.x == 0 && sum != 0.0) atomicAdd(&c->residual[1], sum);
+  ok = ok && grid_level_end(loop, &sh, 1, nbar);
+  const double norm = sh.residual;
+  // (the slots below start at 2: iteration L uses slot (L + 2) % 3, cleared two barriers earlier)
+  double last = 0.0;
+  bool more = max_iter > 0;
+  unsigned long long my_bytes = 0;
+  while (ok && more) {
+    const uint32_t slot = (L + 2) % 3;
+    // slot of the next iteration: last read before the previous one
+    if (blockIdx.x == 0 && threadIdx.x == 0) c->residual[(L + 3) % 3] = 0.0;
+    double res = 0.0;
+    ppr_sweep<G, false>(a, L, gw, nw, res, my_bytes);
+    if (a.nmulti) {
+      if (!(ok = grid_level_end(loop, &sh, slot, nbar))) break;
+      ppr_fix<(G > 8 ? 2 : 1)>(a, L, gw, nw, res);
+    }
+    res = cta_sum_f64(res);
+    if (threadIdx.x == 0 && res != 0.0) atomicAdd(&c->residual[slot], res);
+    if (!(ok = grid_level_end(loop, &sh, slot, nbar))) break;
+    last = sh.residual;
+    ++L;
+    more = last > tol * norm && L < max_iter;
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    LoopOut *o = loop.out;
+    o->level = L;
+    o->residual = last;
+    o->norm = norm;
+    o->barriers = nbar;
+    o->error = ok ? *(volatile int32_t *)&c->error : (int32_t)MG_ERR_TIMEOUT;
+  }
 }
 
 // ctl->acc[2] holds the L1 norm of the right-hand side (k_ppr_rhs_norm).
@@ -222,56 +309,53 @@ __global__ void k_ppr_level_end(Ctl *ctl, double tol, cudaGraphConditionalHandle
   if (use_handle) cudaGraphSetConditional(h, ctl->active);
 }
 
-// dL/dw(u,v) = d <lambda[v,:], R[u,:]>: a group of G lanes per out-edge chunk of
+// dL/dw(u,v) = d <lambda[v,:], R[u,:]>: a group of lanes per out-edge chunk of
 // the CSR chunk plan (a row, or at most kPprChunk edges of a long row), laid out
-// as in k_ppr_iter: R[u,:] held in registers, kPprStep lambda rows in flight,
-// the dot products reduced within the group. R has the caller's row stride nvec.
+// as in ppr_sweep: R[u,:] held in registers, a step's lambda rows in flight, the
+// dot products reduced over a slot's pieces. R has the caller's row stride nvec.
 template <int G>
 __global__ void __launch_bounds__(kNT, 4) k_ppr_edge_grad(const int32_t *cv, const int32_t *cb, const int32_t *ce,
                                                           int32_t n, const int32_t *idx, int32_t nvec, int32_t nv,
                                                           const float *lam, const float *R, float d, float *grad_w,
                                                           Ctl *ctl) {
-  constexpr int PER = 32 / G;
-  const int lane = lane_id();
-  const int gl = lane & (G - 1);
-  const int col = gl * 4;
-  const uint32_t nslots = gridDim.x * kNW * PER;
+  using P = PprGroup<G>;
+  const P g;
+  const int col = g.piece * 4;
+  const uint32_t nw = gridDim.x * kNW;
   unsigned long long my_bytes = 0;
-  for (uint32_t c0 = (blockIdx.x * kNW + warp_id()) * PER; c0 < (uint32_t)n; c0 += nslots) {
-    const uint32_t c = c0 + lane / G;
+  for (uint32_t c0 = (blockIdx.x * kNW + warp_id()) * P::kPer; c0 < (uint32_t)n; c0 += nw * P::kPer) {
+    const uint32_t c = c0 + lane_id() / P::kLanes;
     const bool has = c < (uint32_t)n;
     const int u = has ? cv[c] : 0, b = has ? cb[c] : 0, e = has ? ce[c] : 0;
     float ru[4];
 #pragma unroll
     for (int q = 0; q < 4; ++q) ru[q] = has && col + q < nvec ? R[(int64_t)u * nvec + col + q] : 0.f;
     const int steps = (__reduce_max_sync(0xffffffffu, e - b) + kPprStep - 1) / kPprStep;
-    PprStep<G> cur;
-    cur.load(idx, nullptr, b, e, gl);
+    int v, vn;
+    float none;
+    g.load(idx, nullptr, b, e, v, none);
     for (int s = 0; s < steps; ++s) {
       const int k = b + s * kPprStep;
-      PprStep<G> nxt;
-      nxt.load(idx, nullptr, k + kPprStep, e, gl);
-      float dot[kPprStep];
-      float4 row[kPprStep];
+      g.load(idx, nullptr, k + kPprStep, e, vn, none);
+      float4 row[P::kEdges];
 #pragma unroll
-      for (int j = 0; j < kPprStep; ++j) {
-        const int v = cur.edge(j);
+      for (int j = 0; j < P::kEdges; ++j) {
+        const int t = g.of(v, j);
         row[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (v >= 0 && col < nv) row[j] = __ldg(reinterpret_cast<const float4 *>(lam + (int64_t)v * nv + col));
+        if (t >= 0 && col < nv) row[j] = __ldg(reinterpret_cast<const float4 *>(lam + (int64_t)t * nv + col));
       }
 #pragma unroll
-      for (int j = 0; j < kPprStep; ++j) {
-        dot[j] = fmaf(row[j].w, ru[3], fmaf(row[j].z, ru[2], fmaf(row[j].y, ru[1], row[j].x * ru[0])));
+      for (int j = 0; j < P::kEdges; ++j) {
+        float dot = fmaf(row[j].w, ru[3], fmaf(row[j].z, ru[2], fmaf(row[j].y, ru[1], row[j].x * ru[0])));
 #pragma unroll
-        for (int o = G / 2; o > 0; o >>= 1) dot[j] += __shfl_xor_sync(0xffffffffu, dot[j], o);
+        for (int o = G / 2; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+        // the slot's lane j (of its pieces, in turn) writes the edge
+        const int i = k + j * P::kSlots + g.slot;
+        if (g.piece == j % G && i < e) grad_w[i] = d * dot;
       }
-      // lane l of the group writes edge k + l (and k + l + G, ...)
-#pragma unroll
-      for (int j = 0; j < kPprStep; ++j)
-        if (gl == j % G && k + j < e) grad_w[k + j] = d * dot[j];
-      cur = nxt;
+      v = vn;
     }
-    if (has && gl == 0) my_bytes += 4ull * nvec + (unsigned long long)(e - b) * (8ull + 4ull * nv);
+    if (has && g.gl == 0) my_bytes += 4ull * nvec + (unsigned long long)(e - b) * (8ull + 4ull * nv);
   }
   add_bytes(ctl, KID_PPR, my_bytes);
 }
@@ -311,19 +395,23 @@ __global__ void k_gather_f32(const int32_t *idx, const float *src, float *dst, i
 // slots and split vertices stay in vertex order.
 static int build_plan(mg_graph *g, const std::vector<int32_t> &off, mg_graph::PprPlan *p, cudaStream_t s) {
   const int64_t V = g->nodes;
-  std::vector<int64_t> at(kPprChunk + 2, 0);  // at[kPprChunk - len + 1]: chunks of a length, then their first place
+  int64_t longest = 0;
+  for (int64_t v = 0; v < V; ++v) longest = std::max<int64_t>(longest, off[v + 1] - off[v]);
+  int32_t chunk = g->edges <= kPprSmall ? 64 : kPprChunk;
+  while (chunk < kPprChunk && (int64_t)chunk * chunk < longest) chunk *= 2;
+  std::vector<int64_t> at((size_t)chunk + 2, 0);  // at[chunk - len + 1]: chunks of a length, then their first place
   for (int64_t v = 0; v < V; ++v) {
     const int32_t len = off[v + 1] - off[v];
-    if (len > kPprChunk) at[1] += len / kPprChunk;
-    if (len <= kPprChunk || len % kPprChunk) at[kPprChunk - (len <= kPprChunk ? len : len % kPprChunk) + 1] += 1;
+    if (len > chunk) at[1] += len / chunk;
+    if (len <= chunk || len % chunk) at[chunk - (len <= chunk ? len : len % chunk) + 1] += 1;
   }
-  const int64_t n_empty = at[kPprChunk + 1];
-  for (int i = 1; i < kPprChunk + 2; ++i) at[i] += at[i - 1];
-  const size_t n = (size_t)at[kPprChunk + 1];
+  const int64_t n_empty = at[chunk + 1];
+  for (int i = 1; i < chunk + 2; ++i) at[i] += at[i - 1];
+  const size_t n = (size_t)at[chunk + 1];
   std::vector<int32_t> cv(n), cb(n), ce(n), cs(n), mv, mf;
   int32_t slots = 0;
   auto put = [&](int64_t v, int32_t b, int32_t e, int32_t slot) {
-    const int64_t i = at[kPprChunk - (e - b)]++;
+    const int64_t i = at[chunk - (e - b)]++;
     cv[i] = (int32_t)v;
     cb[i] = b;
     ce[i] = e;
@@ -331,12 +419,12 @@ static int build_plan(mg_graph *g, const std::vector<int32_t> &off, mg_graph::Pp
   };
   for (int64_t v = 0; v < V; ++v) {
     const int32_t b = off[v], e = off[v + 1];
-    if (e - b <= kPprChunk) {
+    if (e - b <= chunk) {
       put(v, b, e, -1);
     } else {
       mv.push_back((int32_t)v);
       mf.push_back(slots);
-      for (int32_t x = b; x < e; x += std::min(kPprChunk, e - x)) put(v, x, x + std::min(kPprChunk, e - x), slots++);
+      for (int32_t x = b; x < e; x += std::min(chunk, e - x)) put(v, x, x + std::min(chunk, e - x), slots++);
     }
   }
   mf.push_back(slots);
@@ -411,6 +499,43 @@ static bool is_device_ptr(const void *p) {
   return at.type == cudaMemoryTypeDevice || at.type == cudaMemoryTypeManaged;
 }
 
+// (vertices + edges) times row width up to which a solve is one launch (forward
+// and backward, level loop / one launch: R-MAT 9, 32 columns 2.33 / 1.96 ms,
+// R-MAT 14, 2 columns 2.27 / 2.10, R-MAT 16, 7 columns 3.34 / 2.86, R-MAT 18,
+// 12 columns 6.54 / 6.90).
+constexpr int64_t kPprLoopWork = 1ll << 24;
+
+static int ppr_one_launch(mg_graph *g, cudaStream_t s, PprArgs a, uint32_t max_iter, const mg_options *o,
+                          const char *name, LoopResult *res) {
+  std::lock_guard<std::mutex> lock(loop_mutex(g->device));
+  GridLoop loop = loop_begin(g, o);
+  double tol = o->tolerance;
+  void *args[] = {&a, &tol, &max_iter, &loop};
+  const void *kernel;
+  switch (ppr_group(a.nv)) {
+    case 1: kernel = (const void *)k_ppr_loop<1>; break;
+    case 2: kernel = (const void *)k_ppr_loop<2>; break;
+    case 4: kernel = (const void *)k_ppr_loop<4>; break;
+    case 8: kernel = (const void *)k_ppr_loop<8>; break;
+    default: kernel = (const void *)k_ppr_loop<16>;
+  }
+  cudaError_t e = cudaEventRecord(g->ev0, s);
+  if (e == cudaSuccess) e = cudaLaunchCooperativeKernel(kernel, dim3(g->num_sms), dim3(kLoopNT), args, 0, s);
+  if (e == cudaSuccess) e = cudaEventRecord(g->ev1, s);
+  count_launch();
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  int st;
+  memset(&res->ctl, 0, sizeof(res->ctl));
+  if ((st = cuda_status(e, name)) != MG_OK || (st = loop_end(g, s, name)) != MG_OK) return st;
+  res->ctl.level = g->loop_out->level;
+  res->ctl.residual = g->loop_out->residual;
+  res->ctl.acc[2] = g->loop_out->norm;
+  float ms = 0.f;
+  cudaEventElapsedTime(&ms, g->ev0, g->ev1);
+  res->ms = ms;
+  return MG_OK;
+}
+
 // Runs one power-iteration solve; on return the solution is in *result.
 static int ppr_solve(mg_graph *g, int dir, const float *w, const float *rhs, float alpha, int32_t nvec,
                      const mg_options *o, cudaStream_t s, const char *name, float **result, LoopResult *res) {
@@ -450,10 +575,18 @@ static int ppr_solve(mg_graph *g, int dir, const float *w, const float *rhs, flo
   a.ctl = g->ws.ctl;
   // start from the right-hand side
   k_copy_f32<<<g->num_sms * 4, 256, 0, s>>>(rhs, a.x0, n);
+  count_launch();
   const uint32_t max_iter = (uint32_t)std::max<int32_t>(0, std::min<int32_t>(o->iter_num, 100000));
+  // Short iterations: one launch. The level loop serves the rest, the host-driven
+  // runs and callers that shorten the waits.
+  if (o->use_cuda_graph && !prof_on() && o->spin_limit >= kSpinLimitDefault && (g->nodes + g->edges) * nv <= kPprLoopWork) {
+    const int st = ppr_one_launch(g, s, a, max_iter, o, name, res);
+    *result = (res->ctl.level & 1) ? a.x1 : a.x0;
+    return st;
+  }
   k_ctl_init<<<1, 32, 0, s>>>(a.ctl, 1u, max_iter, (unsigned long long)o->spin_limit, MODE_QUEUE, ctl_flags(nullptr));
   k_ppr_rhs_norm<<<g->num_sms * 4, 256, 0, s>>>(rhs, n, a.ctl);
-  count_launch(3);
+  count_launch(2);
   const int grid = persistent_grid(g, o, 4);
   const double tol = o->tolerance;
   LevelBody body = [=](cudaStream_t ss, cudaGraphConditionalHandle h, int use_h) {
