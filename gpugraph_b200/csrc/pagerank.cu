@@ -270,12 +270,12 @@ __global__ void __launch_bounds__(kNT) k_pr_fixup(PrArgs a) {
 }
 
 // The sweep for graphs whose in-lists are all short (a grid): a thread sums a
-// vertex's list in CSC order, kPrVerts vertices at a time with all their index
-// loads, then all their gathers in flight; a list's entries past kPrSerial one
-// by one. The 1200x1200 road grid: 946 us a solve in the level loop, 728 with
-// the warp sweep in one launch, 565 with this one (three vertices at a time: 679,
-// registers spill).
-constexpr int kPrVerts = 2;
+// vertex's list in CSC order, kPrVerts vertices at a time with the index loads,
+// then the gathers of their first kPrThreadEdges entries in flight, the rest one
+// by one. The 1200x1200 road grid: 946 us a solve in the level loop, 728 with the
+// warp sweep in one launch, 498 with this one (2 vertices of 8 entries 569, 3 of 5
+// 540, 3 of 6 573, 4 of 4 709: registers spill).
+constexpr int kPrVerts = 2, kPrThreadEdges = 5;
 MG_DEVINL void pr_thread_sweep(const PrArgs &a, uint32_t L, float base, uint32_t tid, uint32_t nt, float &rs,
                                float &rc, float &ds, float &dc) {
   const float *cold = (L & 1) ? a.c1 : a.c0;
@@ -283,8 +283,8 @@ MG_DEVINL void pr_thread_sweep(const PrArgs &a, uint32_t L, float base, uint32_t
   float *rnew = (L & 1) ? a.r0 : a.r1;
   float *cnew = (L & 1) ? a.c0 : a.c1;
   for (uint32_t v0 = tid; v0 < (uint32_t)a.V; v0 += nt * kPrVerts) {
-    int b[kPrVerts], e[kPrVerts], u[kPrVerts][kPrSerial];
-    float r_old[kPrVerts], iv[kPrVerts], x[kPrVerts][kPrSerial];
+    int b[kPrVerts], e[kPrVerts], u[kPrVerts][kPrThreadEdges];
+    float r_old[kPrVerts], iv[kPrVerts], x[kPrVerts][kPrThreadEdges];
 #pragma unroll
     for (int q = 0; q < kPrVerts; ++q) {
       const uint32_t v = v0 + q * nt;
@@ -297,19 +297,19 @@ MG_DEVINL void pr_thread_sweep(const PrArgs &a, uint32_t L, float base, uint32_t
 #pragma unroll
     for (int q = 0; q < kPrVerts; ++q)
 #pragma unroll
-      for (int k = 0; k < kPrSerial; ++k) u[q][k] = b[q] + k < e[q] ? a.crow[b[q] + k] : -1;
+      for (int k = 0; k < kPrThreadEdges; ++k) u[q][k] = b[q] + k < e[q] ? a.crow[b[q] + k] : -1;
 #pragma unroll
     for (int q = 0; q < kPrVerts; ++q)
 #pragma unroll
-      for (int k = 0; k < kPrSerial; ++k) x[q][k] = u[q][k] >= 0 ? cold[u[q][k]] : 0.f;
+      for (int k = 0; k < kPrThreadEdges; ++k) x[q][k] = u[q][k] >= 0 ? cold[u[q][k]] : 0.f;
 #pragma unroll
     for (int q = 0; q < kPrVerts; ++q) {
       const uint32_t v = v0 + q * nt;
       if (v >= (uint32_t)a.V) continue;
       float acc = 0.f;
 #pragma unroll
-      for (int k = 0; k < kPrSerial; ++k) acc += x[q][k];
-      for (int k = b[q] + kPrSerial; k < e[q]; ++k) acc += cold[a.crow[k]];
+      for (int k = 0; k < kPrThreadEdges; ++k) acc += x[q][k];
+      for (int k = b[q] + kPrThreadEdges; k < e[q]; ++k) acc += cold[a.crow[k]];
       pr_store(a.damping, (int)v, acc, base, r_old[q], iv[q], rnew, cnew, rs, rc, ds, dc);
     }
   }
