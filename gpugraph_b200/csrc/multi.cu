@@ -1391,30 +1391,26 @@ __global__ void k_ms_mask_stats(const u64 *visit, u64 all, const int32_t *ro, in
 
 // ------------------------------------------------------------ batched SSSP --
 // Start of a level: the frontier's vertices (the bits the previous expand set)
-// in vertex order into the queue, with the exclusive prefix of their degrees and
-// the merge-path tile partitions of k_mss_expand (as k_frontier_scan makes them
-// from a queue); the bitmap words are cleared on the way. In vertex order the
-// rows a level touches follow each other in memory, so on a grid the four
-// edges that meet at a vertex find its row in L2 (the distance rows are larger
-// than it) and no expand warp reserves queue space. A warp takes kMsScanWords
-// words, a lane a vertex of the current word, twice: totals first, then, with
-// the prefixes of the earlier tiles (two look-backs, the vertices by warp 0 and
-// the degrees by warp 1), the entries. The previous level's masks, read by its
-// expand, are cleared at its queue entries on the way. With it a batched SSSP took 4.5 instead
-// of 4.9 ms at R-MAT 20 (37 sources) and 19.2 instead of 23.8 ms on the
-// 1200x1200 road grid (64 sources).
+// into the queue, with the exclusive prefix of their degrees and the merge-path
+// tile partitions of k_mss_expand (as k_frontier_scan makes them from a queue);
+// the bitmap words and the previous level's masks are cleared on the way. The
+// queue is in vertex order but for the order of the 4096-vertex tiles, which
+// reserve their part of it, vertices and degrees together, with one 64-bit
+// atomic: the rows a level touches follow each other in memory, so on a grid the
+// four edges that meet at a vertex find its row in L2 (the distance rows are
+// larger than it), and no expand warp reserves queue space. A warp takes
+// kMsScanWords words, a lane a vertex of each. In vertex order a batched SSSP took
+// 4.5 instead of 4.9 ms at R-MAT 20 (37 sources) and 19.2 instead of 23.8 ms on
+// the 1200x1200 road grid (64 sources); with a look-back over the tiles instead
+// of the atomic a level cost 12 us more.
 constexpr int kMsScanWords = 16;
 template <int VT>
-__global__ void __launch_bounds__(kNT) k_mss_scan(MultiArgs a, uint32_t *scan, int32_t *part,
-                                                  unsigned long long *status2) {
+__global__ void __launch_bounds__(kNT) k_mss_scan(MultiArgs a, uint32_t *scan, int32_t *part) {
   constexpr uint32_t NV = kNT * VT, W = kMsScanWords;
   __shared__ uint32_t s_cnt[kNW], s_deg[kNW];
-  __shared__ uint32_t s_tile;
-  __shared__ int s_fail;
   Ctl *ctl = a.ctl;
   if (!ctl->active) return;
-  const uint32_t L = ctl->level, epoch = ctl->epoch;
-  const unsigned long long spin_limit = ctl->spin_limit;
+  const uint32_t L = ctl->level, pn = ctl->prev_size;
   uint32_t *bm = (L & 1) ? a.bm1 : a.bm0;
   int32_t *Q = cur_Q(a, L);
   const int32_t *ro = a.g.row_offsets;
@@ -1422,14 +1418,10 @@ __global__ void __launch_bounds__(kNT) k_mss_scan(MultiArgs a, uint32_t *scan, i
   const uint32_t ntiles = (words + W * kNW - 1) / (W * kNW);
   const int lane = lane_id(), warp = warp_id();
   unsigned long long my_bytes = 0;
-  if (threadIdx.x == 0) s_fail = 0;
-  const uint32_t pn = ctl->prev_size;
   u64 *Fp = nxt_F(a, L);
   const int32_t *Qp = nxt_Q(a, L);
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < pn; i += gridDim.x * blockDim.x) Fp[Qp[i]] = 0;
-  for (;;) {
-    const uint32_t tile = next_tile(&ctl->tile_ctr[0], &s_tile);
-    if (tile >= ntiles || s_fail) break;
+  for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     const uint32_t w0 = (tile * kNW + warp) * W;
     const uint32_t mine = lane < (int)W && w0 + lane < words ? bm[w0 + lane] : 0u;
     if (mine) bm[w0 + lane] = 0u;
@@ -1444,33 +1436,25 @@ __global__ void __launch_bounds__(kNT) k_mss_scan(MultiArgs a, uint32_t *scan, i
     for (uint32_t q = 0; q < W; ++q) deg += d[q];
     const uint32_t cw = warp_sum((uint32_t)__popc(mine));
     deg = warp_sum(deg);
+    __syncthreads();  // the previous tile's prefixes have been read
     if (lane == 0) {
       s_cnt[warp] = cw;
       s_deg[warp] = deg;
     }
     __syncthreads();
-    if (warp < 2) {
-      uint32_t *p = warp == 0 ? s_cnt : s_deg;
-      const uint32_t x = lane < kNW ? p[lane] : 0u;
-      const uint32_t inc = warp_inclusive_sum(x);
-      const uint32_t tot = __shfl_sync(0xffffffffu, inc, kNW - 1);
-      bool failed = false;
-      const uint32_t pre = lookback(warp == 0 ? a.status : status2, tile, tot, epoch + warp, spin_limit, &failed);
-      if (lane < kNW) p[lane] = pre + inc - x;
-      if (lane == 0 && failed) {
-        s_fail = 1;
-        raise_error(ctl, MG_ERR_TIMEOUT);
-      }
-      if (lane == 0 && !failed && tile == ntiles - 1) {
-        if (warp == 0) ctl->frontier_size = pre + tot;
-        else ctl->edge_total = pre + tot;
+    if (warp == 0) {
+      const uint32_t x = lane < kNW ? s_cnt[lane] : 0u, y = lane < kNW ? s_deg[lane] : 0u;
+      const uint32_t xi = warp_inclusive_sum(x), yi = warp_inclusive_sum(y);
+      u64 base = 0;
+      if (lane == 31 && xi) base = atomicAdd(&ctl->next_edges, ((unsigned long long)xi << 32) | yi);
+      base = __shfl_sync(0xffffffffu, base, 31);
+      if (lane < kNW) {
+        s_cnt[lane] = (uint32_t)(base >> 32) + xi - x;
+        s_deg[lane] = (uint32_t)base + yi - y;
       }
     }
     __syncthreads();
-    if (s_fail) break;
     uint32_t pos = s_cnt[warp], run = s_deg[warp];
-    if (tile == ntiles - 1 && warp == kNW - 1 && lane == 0)
-      ctl->exp_tiles = (uint32_t)(((unsigned long long)(pos + cw) + (run + deg) + NV - 1) / NV);
 #pragma unroll
     for (uint32_t q = 0; q < W; ++q) {
       const uint32_t x = __shfl_sync(0xffffffffu, mine, q);
@@ -1492,6 +1476,9 @@ __global__ void __launch_bounds__(kNT) k_mss_scan(MultiArgs a, uint32_t *scan, i
   }
   add_bytes(ctl, KID_SCAN, my_bytes);
 }
+// The totals of the scan: queued vertices, and their degrees.
+MG_DEVINL uint32_t mss_queued(const Ctl *ctl) { return (uint32_t)(ctl->next_edges >> 32); }
+MG_DEVINL uint32_t mss_edges(const Ctl *ctl) { return (uint32_t)ctl->next_edges; }
 
 // Edge bounds of a batched SSSP on a skewed graph. With any constants c_s per
 // source, an edge (u,v) of weight w can improve no source when
@@ -1522,7 +1509,7 @@ struct MssBounds {
 __global__ void __launch_bounds__(kNT) k_mss_bounds(MultiArgs a, MssBounds m) {
   Ctl *ctl = a.ctl;
   if (!ctl->active) return;
-  const uint32_t L = ctl->level, n = ctl->frontier_size;
+  const uint32_t L = ctl->level, n = mss_queued(ctl);
   const int32_t *Q = cur_Q(a, L);
   if (!m.offs[64]) return;
   const bool full = m.offs[65] != 0;
@@ -1622,8 +1609,9 @@ __global__ void __launch_bounds__(kNT, 4) k_mss_expand(MultiArgs a, MssBounds mb
   __shared__ int s_fail;
   Ctl *ctl = a.ctl;
   if (!ctl->active) return;
-  const uint32_t L = ctl->level, n = ctl->frontier_size, total = ctl->edge_total, ntiles = ctl->exp_tiles;
+  const uint32_t L = ctl->level, n = mss_queued(ctl), total = mss_edges(ctl);
   const unsigned long long items = (unsigned long long)n + total;
+  const uint32_t ntiles = (uint32_t)((items + NV - 1) / NV);
   const int32_t *Q = cur_Q(a, L);
   const u64 *Fc = cur_F(a, L);
   u64 *Fn = nxt_F(a, L);
@@ -1817,13 +1805,12 @@ __global__ void k_mss_level_end(MultiArgs a, MssBounds m, cudaGraphConditionalHa
   }
   if (t != 0) return;
   if (ctl->active) {
-    ctl->prev_size = ctl->frontier_size;
+    ctl->prev_size = mss_queued(ctl);
     ctl->level += 1;
     ctl->push_levels += 1;
-    ctl->frontier_size = ctl->next_size;
+    ctl->frontier_size = ctl->next_size;  // whether there is one: the scan counts it
     ctl->next_size = 0;
-    ctl->edge_total = 0;
-    ctl->exp_tiles = 0;
+    ctl->next_edges = 0;
     ctl->epoch += 4;
     for (int i = 0; i < 4; ++i) ctl->tile_ctr[i] = 0;
     ctl->active = (ctl->frontier_size > 0 && ctl->level < ctl->max_iter && ctl->error == 0) ? 1u : 0u;
@@ -2110,8 +2097,6 @@ int mg_sssp_multi(mg_graph *g, const int32_t *srcs, int32_t nsrc, int32_t *dists
   const int grid = persistent_grid(g, o, 4);
   uint32_t *scan = g->ws.scan;
   int32_t *part = g->ws.part;
-  // the scan's second look-back: it has at most V/4096 + 1 tiles, fewer than half the words
-  unsigned long long *status2 = g->ws.status + g->ws.status_cap / 2;
   MssBounds mb;
   mb.lo = g->ws.vbuf[0];
   mb.hi = g->ws.vbuf[1];
@@ -2119,7 +2104,7 @@ int mg_sssp_multi(mg_graph *g, const int32_t *srcs, int32_t nsrc, int32_t *dists
   // (rows of up to 8 sources are one sector: a bound would cost as much as it saves)
   mb.hub = nsrc > 8 ? g->mss_hub : -1;
   LevelBody body = [=](cudaStream_t ss, cudaGraphConditionalHandle h, int use_h) {
-    MG_LAUNCH(KID_SCAN, ss, k_mss_scan<kMSVT><<<grid, kNT, 0, ss>>>(a, scan, part, status2));
+    MG_LAUNCH(KID_SCAN, ss, k_mss_scan<kMSVT><<<grid, kNT, 0, ss>>>(a, scan, part));
     if (mb.hub >= 0) MG_LAUNCH(KID_MS_APPLY, ss, k_mss_bounds<<<grid, kNT, 0, ss>>>(a, mb));
     MG_LAUNCH(KID_MSS_EXPAND, ss, k_mss_expand<kMSVT><<<grid, kNT, 0, ss>>>(a, mb, scan, part));
     MG_LAUNCH(KID_OTHER, ss, k_mss_level_end<<<1, 64, 0, ss>>>(a, mb, h, use_h));
