@@ -471,7 +471,7 @@ __global__ void k_bfs_start(Ctl *ctl, int32_t *queue0, int32_t root, int32_t *la
 }
 
 int bfs_loop_run(mg_graph *g, cudaStream_t s, const std::vector<int32_t> &roots, uint32_t max_iter,
-                 const mg_options *o, int32_t *labels);  // bfs_loop.cu
+                 const mg_options *o, int32_t *labels, bool timed);  // bfs_loop.cu
 
 // The whole BFS in one launch: the depths go straight to the caller's device
 // buffer, the statistics come with the result block.
@@ -484,7 +484,7 @@ static int bfs_one_launch(mg_graph *g, cudaStream_t s, const std::vector<int32_t
   const bool direct = dev && on_device(g, depths);
   int32_t *labels = direct ? depths : g->ws.vbuf[0];
   std::lock_guard<std::mutex> lock(loop_mutex(g->device));
-  int st = bfs_loop_run(g, s, roots, max_iter, o, labels);
+  int st = bfs_loop_run(g, s, roots, max_iter, o, labels, stats != nullptr);
   if (st != MG_OK) return st;
   cudaError_t e = cudaSuccess;
   if (preds) {

@@ -371,7 +371,7 @@ __global__ void __launch_bounds__(kLoopNT, 1) k_bfs_loop(BfsLoopArgs a) {
 
 // Runs a BFS on stream s in one launch, depths to `labels` (device).
 int bfs_loop_run(mg_graph *g, cudaStream_t s, const std::vector<int32_t> &roots, uint32_t max_iter,
-                 const mg_options *o, int32_t *labels) {
+                 const mg_options *o, int32_t *labels, bool timed) {
   BfsLoopArgs a;
   a.g = g->csr;
   a.labels = labels;
@@ -395,11 +395,7 @@ int bfs_loop_run(mg_graph *g, cudaStream_t s, const std::vector<int32_t> &roots,
   a.beta = (float)o->beta;
   a.loop = loop_begin(g, o);
   void *args[] = {&a};
-  cudaError_t e = cudaEventRecord(g->ev0, s);
-  if (e == cudaSuccess) e = cudaLaunchCooperativeKernel((const void *)k_bfs_loop, dim3(g->num_sms), dim3(kLoopNT), args, 0, s);
-  if (e == cudaSuccess) e = cudaEventRecord(g->ev1, s);
-  count_launch();
-  return cuda_status(e, "bfs loop launch");
+  return cuda_status(loop_launch(g, (const void *)k_bfs_loop, args, timed, s), "bfs loop launch");
 }
 
 }  // namespace mg

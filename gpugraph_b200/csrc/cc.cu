@@ -259,7 +259,7 @@ constexpr double kCcSkew = 8.0;      // longest list over the mean from which th
 constexpr uint32_t kCcLevels = 16;
 
 int bfs_loop_run(mg_graph *g, cudaStream_t s, const std::vector<int32_t> &roots, uint32_t max_iter,
-                 const mg_options *o, int32_t *labels);  // bfs_loop.cu
+                 const mg_options *o, int32_t *labels, bool timed);  // bfs_loop.cu
 
 // Union-find CC on a symmetric graph (called by mg_cc).
 int cc_union_find(mg_graph *g, int32_t *labels, mg_stats *stats, const mg_options *o) {
@@ -286,7 +286,7 @@ int cc_union_find(mg_graph *g, int32_t *labels, mg_stats *stats, const mg_option
     int32_t *depth = g->ws.gather_tmp;
     mg_options bo;
     mg_options_init(&bo);
-    if ((st = bfs_loop_run(g, s, {g->hub}, kCcLevels, &bo, depth)) != MG_OK) return st;
+    if ((st = bfs_loop_run(g, s, {g->hub}, kCcLevels, &bo, depth, false)) != MG_OK) return st;
     k_fill_i32<<<1, 32, 0, s>>>(giant, INT_MAX, 1);
     k_cc_low<<<vgrid, kNT, 0, s>>>(depth, V, giant);
     k_cc_seed<<<vgrid, kNT, 0, s>>>(depth, V, giant, parent, ctl);

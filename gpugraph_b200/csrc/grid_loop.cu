@@ -9,6 +9,14 @@ std::mutex &loop_mutex(int device) {
   return m[device & 15];
 }
 
+cudaError_t loop_launch(mg_graph *g, const void *kernel, void **args, bool timed, cudaStream_t s) {
+  cudaError_t e = timed ? cudaEventRecord(g->ev0, s) : cudaSuccess;
+  if (e == cudaSuccess) e = cudaLaunchCooperativeKernel(kernel, dim3(g->num_sms), dim3(kLoopNT), args, 0, s);
+  if (e == cudaSuccess && timed) e = cudaEventRecord(g->ev1, s);
+  count_launch();
+  return e;
+}
+
 GridLoop loop_begin(mg_graph *g, const mg_options *o) {
   GridLoop l;
   l.c = g->loop_ctl;

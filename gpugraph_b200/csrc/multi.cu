@@ -1987,11 +1987,7 @@ static int bfs_multi_run(mg_graph *g, const int32_t *srcs, int32_t nsrc, int32_t
     p.max_iter = max_iter;
     p.loop = loop_begin(g, o);
     void *args[] = {&p};
-    cudaError_t e = cudaEventRecord(g->ev0, s);
-    if (e == cudaSuccess)
-      e = cudaLaunchCooperativeKernel((const void *)k_ms_loop, dim3(g->num_sms), dim3(kLoopNT), args, 0, s);
-    if (e == cudaSuccess) e = cudaEventRecord(g->ev1, s);
-    count_launch();
+    cudaError_t e = loop_launch(g, (const void *)k_ms_loop, args, stats != nullptr, s);
     if (e == cudaSuccess && o->outputs_on_device) epi(s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if ((st = cuda_status(e, "batched bfs")) != MG_OK || (st = loop_end(g, s, "batched traversal")) != MG_OK) return st;
@@ -2001,7 +1997,7 @@ static int bfs_multi_run(mg_graph *g, const int32_t *srcs, int32_t nsrc, int32_t
     res.ctl.pull_levels = g->loop_out->pull_levels;
     res.ctl.frontier_size = g->loop_out->frontier_size;
     float ms = 0.f;
-    cudaEventElapsedTime(&ms, g->ev0, g->ev1);
+    if (stats) cudaEventElapsedTime(&ms, g->ev0, g->ev1);
     res.ms = ms;
     if (res.ctl.frontier_size > 0 && res.ctl.level >= kMsDepth16Levels && max_iter_asked > kMsDepth16Levels) {
       *depth_overflow = true;  // deeper than a uint16 depth row holds

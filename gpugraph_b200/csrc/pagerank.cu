@@ -569,11 +569,7 @@ static int pr_one_launch(mg_graph *g, cudaStream_t s, const PrArgs &a, float *ra
   std::lock_guard<std::mutex> lock(loop_mutex(g->device));
   p.loop = loop_begin(g, o);
   void *args[] = {&p};
-  cudaError_t e = cudaEventRecord(g->ev0, s);
-  if (e == cudaSuccess)
-    e = cudaLaunchCooperativeKernel((const void *)k_pr_loop, dim3(g->num_sms), dim3(kLoopNT), args, 0, s);
-  if (e == cudaSuccess) e = cudaEventRecord(g->ev1, s);
-  count_launch();
+  cudaError_t e = loop_launch(g, (const void *)k_pr_loop, args, stats != nullptr, s);
   if (e == cudaSuccess && !direct)
     e = cudaMemcpyAsync(ranks, p.out, (size_t)g->nodes * 4, dev ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);

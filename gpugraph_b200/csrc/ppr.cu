@@ -519,10 +519,7 @@ static int ppr_one_launch(mg_graph *g, cudaStream_t s, PprArgs a, uint32_t max_i
     case 8: kernel = (const void *)k_ppr_loop<8>; break;
     default: kernel = (const void *)k_ppr_loop<16>;
   }
-  cudaError_t e = cudaEventRecord(g->ev0, s);
-  if (e == cudaSuccess) e = cudaLaunchCooperativeKernel(kernel, dim3(g->num_sms), dim3(kLoopNT), args, 0, s);
-  if (e == cudaSuccess) e = cudaEventRecord(g->ev1, s);
-  count_launch();
+  cudaError_t e = loop_launch(g, kernel, args, true, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   int st;
   memset(&res->ctl, 0, sizeof(res->ctl));

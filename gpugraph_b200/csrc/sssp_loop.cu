@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(kLoopNT, 1) k_sssp_loop(SsspLoopArgs a) {
 }
 
 // Runs an SSSP on stream s in one launch, distances to `dist` (device).
-int sssp_loop_run(mg_graph *g, cudaStream_t s, int32_t src, const mg_options *o, int32_t *dist) {
+int sssp_loop_run(mg_graph *g, cudaStream_t s, int32_t src, const mg_options *o, int32_t *dist, bool timed) {
   SsspLoopArgs a;
   a.g = g->csr;
   a.dist = dist;
@@ -208,11 +208,7 @@ int sssp_loop_run(mg_graph *g, cudaStream_t s, int32_t src, const mg_options *o,
   a.max_iter = (uint32_t)(g->nodes + 2);
   a.loop = loop_begin(g, o);
   void *args[] = {&a};
-  cudaError_t e = cudaEventRecord(g->ev0, s);
-  if (e == cudaSuccess) e = cudaLaunchCooperativeKernel((const void *)k_sssp_loop, dim3(g->num_sms), dim3(kLoopNT), args, 0, s);
-  if (e == cudaSuccess) e = cudaEventRecord(g->ev1, s);
-  count_launch();
-  return cuda_status(e, "sssp loop launch");
+  return cuda_status(loop_launch(g, (const void *)k_sssp_loop, args, timed, s), "sssp loop launch");
 }
 
 }  // namespace mg
