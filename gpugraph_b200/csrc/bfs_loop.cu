@@ -13,10 +13,10 @@
 // does, so push levels keep no bitmap.
 //
 // Bound by the round trips of a level (ranges, columns, test-and-sets, the
-// reservation, the barrier: about 7 us a level) on small frontiers, by the
+// reservation, the barrier: under 7 us a level) on small frontiers, by the
 // bottom-up sweeps' loads on large ones. Against the level-by-level loop, per
-// run: R-MAT 16 with host output 215 -> 91 us, R-MAT 21 234 -> 121 us,
-// 1200x1200 road grid (67 levels) 1542 -> 498 us, 256 small graphs 309 -> 228 us.
+// run: R-MAT 16 with host output 215 -> 91 us, R-MAT 21 234 -> 97 us,
+// 1200x1200 road grid (67 levels) 1542 -> 458 us, 256 small graphs 309 -> 155 us.
 #include <cuda_runtime.h>
 
 #include <vector>
@@ -29,7 +29,7 @@ namespace mg {
 
 constexpr int kLoopU = 4;     // edges per lane in flight
 constexpr int kLoopWords = 4; // 32-vertex words per warp and step of a pull level
-constexpr int kConvWords = 8; // and of the pull -> push conversion (256 small graphs: one word at a time took 65 us)
+constexpr int kConvWords = 8; // and of a change of direction (256 small graphs: 160 us a run, 228 one word at a time)
 
 struct BfsLoopArgs {
   DevCsr g;

@@ -13,7 +13,8 @@
 // a few weights 1.3 to 1.9 times. It takes two to four times as many steps,
 // which only pays with steps as cheap as here (two grid barriers and no scan;
 // the level loop lost by it: 4.7 against 3.3 ms at R-MAT 22). R-MAT 21: 1.8 ms a
-// run level by level, 1.3 here.
+// run level by level, 1.2 here. 0.8 ms of it are three steps that relax 1.9 times
+// the edges at 150 G/s, bound by the gathers and reductions in L2.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -26,11 +27,12 @@
 
 namespace mg {
 
-constexpr int kSpU = 8;        // edges per lane in flight (R-MAT 21: 1.30 ms a run, 1.38 with 4)
-constexpr int kSpVerts = 8;    // vertices per lane and step of the selection
+constexpr int kSpU = 8;        // edges per lane in flight (R-MAT 21: 1.30 ms a run against 1.38 with 4)
+constexpr int kSpVerts = 8;    // vertices per lane and step of the selection (R-MAT 21: 1.21 ms, 1.40 with 4)
 // Window: this many times the largest weight over the mean degree (with uniform
 // weights a vertex has about that many edges inside it). R-MAT 21, weights
-// 1..64: 1.39 ms a run at 2, 1.38 at 4, 1.44 at 8, 1.52 at 32 (no window in effect).
+// 1..64: 1.21 ms a run at 4, 1.33 at 8; with a pending bitmap, before done[], 1.39
+// at 2, 1.38 at 4, 1.44 at 8, 1.52 at 32 (no window in effect).
 constexpr double kSsspWindow = 4.0;
 
 struct SsspLoopArgs {

@@ -58,14 +58,15 @@ typedef struct mg_options {
   int32_t direction;         /* MG_DIR_* (BFS only) */
   double alpha;              /* push->pull when frontier edges > unvisited edges / alpha */
   double beta;               /* pull->push when frontier vertices < nodes / beta */
-  int32_t use_cuda_graph;    /* 1: capture the level loop in a CUDA graph */
+  int32_t use_cuda_graph;    /* 1: loops driven by the device (one cooperative launch, or
+                                the level loop captured in a CUDA graph); 0: by the host */
   int32_t threshold;         /* reference "threshold": frontier size above which the
                                 grid-cooperative expand is used (0: always) */
   double damping;            /* PageRank damping (0.85) */
   double tolerance;          /* PageRank L1 stop tolerance */
   int64_t spin_limit;        /* iteration cap of every device-side spin wait */
-  int32_t tile_items;        /* items per expand tile (0: autotuned) */
-  int32_t ctas_per_sm;       /* persistent CTAs per SM (0: autotuned) */
+  int32_t tile_items;        /* items per expand tile (0: autotuned); level-by-level loops */
+  int32_t ctas_per_sm;       /* persistent CTAs per SM (0: autotuned); level-by-level loops */
   int32_t compute_stats;     /* 1: fill mg_stats.edges_traversed (one extra pass) */
   int32_t pad0;
   double alpha_multi;        /* batched BFS: push->pull when the next level's frontier
@@ -79,7 +80,7 @@ typedef struct mg_options {
 
 /* Per-run statistics (reference: Statistics::stats_per_iter, GASengine/statistics.h:31-81). */
 typedef struct mg_stats {
-  int32_t iterations;        /* GAS iterations (BFS levels) executed */
+  int32_t iterations;        /* GAS iterations (BFS levels, SSSP steps) executed */
   int32_t push_iterations;   /* iterations run top-down (push) */
   int32_t pull_iterations;   /* iterations run bottom-up (pull) */
   int32_t converged;         /* 1 if the stop criterion was met within iter_num */
