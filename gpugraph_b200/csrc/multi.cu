@@ -61,6 +61,10 @@ constexpr int kMssEdges = 8;
 // lane's scalar loads touch a sector per source (the same two runs: 4.0 / 19.6 ms
 // at 4, 3.9 / 18.4 at 8, 4.1 / 18.3 at 12, 5.0 / 19.3 at 20).
 constexpr int kMssSparse = 8;
+// On graphs without edge bounds, sources up to which every edge is relaxed by its
+// lane, from registers: the row path's shared memory would come out of L1 (600x600
+// road grid, 7 / 30 sources: 2.27 / 3.46 ms, 3.48 / 5.3 with it).
+constexpr int kMssLaneSources = 56;
 
 // Push step of the batched BFS as a GAS Program: expand_edge emits the
 // sources that reach the neighbour for the first time, contract ORs them into
@@ -1593,7 +1597,10 @@ MG_DEVINL void relax_min(int32_t *p, int32_t c, u64 &imp, int t) {
 // 5 CTAs per SM: 5.8 ms at R-MAT 20; 3 CTAs: 5.2 ms, against 4.3). Before, with
 // a 32-byte row piece per lane, 8 scattered reductions per step and a queue
 // reservation per 4 edges: 7.8 ms a run, 4.4 with a whole warp per edge, now 3.9.
-template <int VT>
+//
+// ROWS = false (no edge bounds and up to kMssLaneSources sources): every edge is
+// relaxed by its lane at once.
+template <int VT, bool ROWS>
 __global__ void __launch_bounds__(kNT, 4) k_mss_expand(MultiArgs a, MssBounds mb, const uint32_t *scan,
                                                        const int32_t *part) {
   constexpr int NV = kNT * VT;
@@ -1602,9 +1609,9 @@ __global__ void __launch_bounds__(kNT, 4) k_mss_expand(MultiArgs a, MssBounds mb
   __shared__ int32_t s_base[NV + 1];
   __shared__ int32_t s_rs[NV + 1];
   __shared__ int32_t s_own[NV];
-  __shared__ int32_t s_lo[NV + 1];  // per block: its tail's lower bound
+  __shared__ int32_t s_lo[ROWS ? NV + 1 : 1];  // per block: its tail's lower bound
   __shared__ u64 s_am[NV + 1];      // per block: its tail's active sources
-  __shared__ int4 s_e[NV];          // per warp: its kept edges (block, head, weight, lanes with an active source)
+  __shared__ int4 s_e[ROWS ? NV : 1];  // per warp: its kept edges (block, head, weight, lanes with an active source)
   __shared__ uint32_t s_tile;
   __shared__ int s_fail;
   Ctl *ctl = a.ctl;
@@ -1618,7 +1625,7 @@ __global__ void __launch_bounds__(kNT, 4) k_mss_expand(MultiArgs a, MssBounds mb
   uint32_t *next_bm = (L & 1) ? a.bm0 : a.bm1;
   const int32_t *ro = a.g.row_offsets, *col = a.g.col, *wgt = a.g.wgt;
   bool any = false;
-  const bool bounds = mb.hub >= 0 && mb.offs[64] != 0;
+  const bool bounds = ROWS && mb.hub >= 0 && mb.offs[64] != 0;
   const int lane = lane_id(), warp = warp_id();
   const int half = lane >> 4, sub = lane & 15;  // two edges side by side, 16 lanes each
   const uint32_t sbit = 1u << sub;
@@ -1654,7 +1661,41 @@ __global__ void __launch_bounds__(kNT, 4) k_mss_expand(MultiArgs a, MssBounds mb
     }
     const int k0 = warp * PER_WARP;
     const int k1 = min(cnt, k0 + PER_WARP);
-    int4 *we = s_e + k0;
+    // one edge, source by source: four active sources per step, their row entries
+    // loaded together; returns the improved ones
+    auto relax_edge = [&](int u, int v, int w, u64 am) {
+      u64 imp = 0;
+      const int32_t *du = a.out + (int64_t)u * 64;
+      int32_t *dv = a.out + (int64_t)v * 64;
+      for (u64 m = am; m;) {
+        int t[4], s[4], du4[4], dv4[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          t[q] = m ? __ffsll((long long)m) - 1 : -1;
+          s[q] = mss_source(t[q]);
+          m &= m - 1;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (t[q] >= 0) {
+            du4[q] = __ldcg(du + s[q]);
+            dv4[q] = __ldcg(dv + s[q]);
+          }
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (t[q] >= 0 && du4[q] + w < dv4[q]) relax_min(dv + s[q], du4[q] + w, imp, t[q]);
+      }
+      return imp;
+    };
+    // next-level mask and frontier bit of a head that improved
+    auto mark = [&](int v, u64 imp) {
+      my_bytes += 8 + 4ull * (unsigned long long)__popcll(imp);
+      atomicOr(&Fn[v], imp);
+      const uint32_t bit = 1u << (v & 31);
+      if (!(ld_volatile(&next_bm[v >> 5]) & bit)) atomicOr(&next_bm[v >> 5], bit);
+      any = true;
+    };
+    int4 *we = s_e + (ROWS ? k0 : 0);
     int kept = 0;  // warp-uniform
     {
       constexpr int R = PER_WARP / 32;
@@ -1688,6 +1729,11 @@ __global__ void __launch_bounds__(kNT, 4) k_mss_expand(MultiArgs a, MssBounds mb
           if (bounds && (int)((uint32_t)s_lo[j[r]] + (uint32_t)w[r]) >= hi[r]) am = 0;
           my_bytes += (bounds ? 12 : 8) + 8ull * (unsigned long long)__popcll(am);
         }
+        if (!ROWS) {
+          const u64 imp = am ? relax_edge(s_v[j[r]], v[r], w[r], am) : 0ull;
+          if (imp) mark(v[r], imp);
+          continue;
+        }
         const uint32_t kb = __ballot_sync(0xffffffffu, am != 0ull);
         if (am)
           we[kept + __popc(kb & lanemask_lt())] =
@@ -1705,29 +1751,7 @@ __global__ void __launch_bounds__(kNT, 4) k_mss_expand(MultiArgs a, MssBounds mb
         bam = s_am[be.x];
       }
       if (__all_sync(0xffffffffu, __popcll(bam) <= kMssSparse)) {
-        if (bam) {
-          const int32_t *du = a.out + (int64_t)s_v[be.x] * 64;
-          int32_t *dv = a.out + (int64_t)be.y * 64;
-          // four active sources per step, their row entries loaded together
-          for (u64 m = bam; m;) {
-            int t[4], s[4], du4[4], dv4[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              t[q] = m ? __ffsll((long long)m) - 1 : -1;
-              s[q] = mss_source(t[q]);
-              m &= m - 1;
-            }
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-              if (t[q] >= 0) {
-                du4[q] = __ldcg(du + s[q]);
-                dv4[q] = __ldcg(dv + s[q]);
-              }
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-              if (t[q] >= 0 && du4[q] + be.z < dv4[q]) relax_min(dv + s[q], du4[q] + be.z, imp, t[q]);
-          }
-        }
+        if (bam) imp = relax_edge(s_v[be.x], be.y, be.z, bam);
       } else {
 #pragma unroll 1
         for (int j0 = 0; j0 < nb; j0 += kMssEdges) {
@@ -1771,14 +1795,7 @@ __global__ void __launch_bounds__(kNT, 4) k_mss_expand(MultiArgs a, MssBounds mb
           }
         }
       }
-      // next-level mask and frontier bit of the heads that improved
-      if (imp) {
-        my_bytes += 8 + 4ull * (unsigned long long)__popcll(imp);
-        atomicOr(&Fn[be.y], imp);
-        const uint32_t bit = 1u << (be.y & 31);
-        if (!(ld_volatile(&next_bm[be.y >> 5]) & bit)) atomicOr(&next_bm[be.y >> 5], bit);
-        any = true;
-      }
+      if (imp) mark(be.y, imp);
     }
   }
   if (any) ctl->next_size = 1;  // the next scan counts them
@@ -2099,15 +2116,18 @@ int mg_sssp_multi(mg_graph *g, const int32_t *srcs, int32_t nsrc, int32_t *dists
   mb.offs = g->mss_offs;
   // (rows of up to 8 sources are one sector: a bound would cost as much as it saves)
   mb.hub = nsrc > 8 ? g->mss_hub : -1;
+  const bool rows = mb.hub >= 0 || nsrc > kMssLaneSources;
   LevelBody body = [=](cudaStream_t ss, cudaGraphConditionalHandle h, int use_h) {
     MG_LAUNCH(KID_SCAN, ss, k_mss_scan<kMSVT><<<grid, kNT, 0, ss>>>(a, scan, part));
     if (mb.hub >= 0) MG_LAUNCH(KID_MS_APPLY, ss, k_mss_bounds<<<grid, kNT, 0, ss>>>(a, mb));
-    MG_LAUNCH(KID_MSS_EXPAND, ss, k_mss_expand<kMSVT><<<grid, kNT, 0, ss>>>(a, mb, scan, part));
+    if (rows) MG_LAUNCH(KID_MSS_EXPAND, ss, (k_mss_expand<kMSVT, true><<<grid, kNT, 0, ss>>>(a, mb, scan, part)));
+    else MG_LAUNCH(KID_MSS_EXPAND, ss, (k_mss_expand<kMSVT, false><<<grid, kNT, 0, ss>>>(a, mb, scan, part)));
     MG_LAUNCH(KID_OTHER, ss, k_mss_level_end<<<1, 64, 0, ss>>>(a, mb, h, use_h));
   };
   LoopResult res;
   const auto epi = transpose_epilogue(g, nsrc, dists, false, false);
-  st = run_level_loop(g, s, std::string(mb.hub >= 0 ? "sssp_multi_bounds/" : "sssp_multi/") + std::to_string(grid),
+  st = run_level_loop(g, s, std::string(mb.hub >= 0 ? "sssp_multi_bounds/" : "sssp_multi/") + std::to_string(grid) +
+                             (rows ? "/rows" : "/lanes"),
                       mb.hub >= 0 ? 4 : 3, body, o->use_cuda_graph != 0, &res, o->outputs_on_device ? &epi : nullptr);
   if (st != MG_OK) return st;
   return multi_finish(g, s, nsrc, dists, programs::sssp::INIT_VALUE, stats, o, res, false);
