@@ -65,6 +65,7 @@ constexpr int kMssSparse = 8;
 // lane, from registers: the row path's shared memory would come out of L1 (600x600
 // road grid, 7 / 30 sources: 2.27 / 3.46 ms, 3.48 / 5.3 with it).
 constexpr int kMssLaneSources = 56;
+constexpr int64_t kMssLargeRows = 1 << 19;  // vertices from which the distance rows are larger than L2
 
 // Push step of the batched BFS as a GAS Program: expand_edge emits the
 // sources that reach the neighbour for the first time, contract ORs them into
@@ -2114,8 +2115,11 @@ int mg_sssp_multi(mg_graph *g, const int32_t *srcs, int32_t nsrc, int32_t *dists
   mb.lo = g->ws.vbuf[0];
   mb.hi = g->ws.vbuf[1];
   mb.offs = g->mss_offs;
-  // (rows of up to 8 sources are one sector: a bound would cost as much as it saves)
-  mb.hub = nsrc > 8 ? g->mss_hub : -1;
+  // Bounds: not for up to 8 sources, whose rows are one sector each, and for up to
+  // 14 only where the rows (256 bytes a vertex) are larger than L2. With / without,
+  // weights 1..64: R-MAT 18, 9 sources 1.36 / 1.19 ms, 16 sources 1.35 / 1.61;
+  // R-MAT 16, 14 sources 1.22 / 1.06; R-MAT 20, 12 sources 3.42 / 4.59.
+  mb.hub = nsrc > 14 || (nsrc > 8 && g->nodes >= kMssLargeRows) ? g->mss_hub : -1;
   const bool rows = mb.hub >= 0 || nsrc > kMssLaneSources;
   LevelBody body = [=](cudaStream_t ss, cudaGraphConditionalHandle h, int use_h) {
     MG_LAUNCH(KID_SCAN, ss, k_mss_scan<kMSVT><<<grid, kNT, 0, ss>>>(a, scan, part));
