@@ -314,3 +314,46 @@ def test_bfs_multi_one_launch_equals_level_loop(name):
         for k, s in enumerate(srcs):
             if int(s) in some:
                 assert np.array_equal(host[k], some[int(s)])
+
+
+def _dag(n, deg, hub, lo, hi, seed):
+    """Directed acyclic graph, edges from lower to higher ids, int32 weights in [lo, hi]; vertex `hub` (if any) is
+    a head of every lower one. Distances by one pass over the vertices in order."""
+    rng = np.random.default_rng(seed)
+    src = np.repeat(np.arange(n - 1), deg)
+    dst = src + 1 + (rng.random(src.size) * np.minimum(60, n - 1 - src)).astype(np.int64)
+    if hub:
+        src, dst = np.concatenate([src, np.arange(hub)]), np.concatenate([dst, np.full(hub, hub)])
+    key = np.unique(src * n + dst)
+    src, dst = key // n, key % n
+    ro = np.concatenate([[0], np.cumsum(np.bincount(src, minlength=n))]).astype(np.int32)
+    w = rng.integers(lo, hi, src.size, endpoint=True)
+    hg = HostGraph(ro, dst.astype(np.int32), w.astype(np.int32), directed=True)
+
+    def dists(srcs):
+        d = np.full((n, len(srcs)), 100000000, np.int64)
+        d[srcs, np.arange(len(srcs))] = 0
+        for u in range(n):
+            b, e = ro[u], ro[u + 1]
+            cand = np.where(d[u] < 100000000, d[u] + w[b:e, None], 100000000)
+            d[dst[b:e]] = np.minimum(d[dst[b:e]], cand)
+        return d.T
+
+    return hg, dists
+
+
+@pytest.mark.parametrize("hub,nsrc", [(0, 57), (0, 64), (1500, 9), (1500, 37), (1500, 64)])
+@pytest.mark.parametrize("lo,hi", [(-40, 60), (-40, -1), (0, 7)])
+def test_sssp_multi_sources_that_do_not_reach_each_other(hub, nsrc, lo, hi):
+    # most sources cannot reach the early vertices, many are active on one edge: a source that has not reached a
+    # tail must stay unreached at the head, also where the weight is negative (100000000 + w < 100000000)
+    hg, dists = _dag(2000, 5, hub, lo, hi, seed=nsrc)
+    srcs = np.sort(np.random.default_rng(1).choice(hub or 1900, nsrc, replace=False)).astype(np.int32)
+    ref = dists(srcs)
+    assert (ref == 100000000).mean() > 0.2
+    g = Graph(hg)
+    for mode in ({}, dict(use_cuda_graph=0)):
+        out, st = g.sssp_multi(srcs, **mode)
+        assert np.array_equal(out, ref)
+        assert st["converged"] == 1 and st["vertices_reached"] == int((ref != 100000000).sum())
+    assert np.array_equal(g.sssp(int(srcs[0]))[0], ref[0])
