@@ -1,6 +1,7 @@
 #include <algorithm>
 
 #include "algo_util.cuh"
+#include "gas/programs.cuh"
 
 namespace mg {
 
@@ -19,6 +20,10 @@ bool on_device(const mg_graph *g, const void *p) {
     return false;
   }
   return at.type == cudaMemoryTypeDevice && at.device == g->device;
+}
+
+bool ordinary_weights(const mg_graph *g) {
+  return g->weight_min >= 0 && g->weight_max <= INT32_MAX - programs::sssp::INIT_VALUE;
 }
 
 __global__ void k_reach_stats(const int32_t *vals, int32_t unreached, int nsrc, int stride, const int32_t *ro, int32_t V,

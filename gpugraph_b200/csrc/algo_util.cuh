@@ -19,6 +19,10 @@ int copy_out(cudaStream_t s, void *dst, const void *src, size_t bytes, bool dst_
 // True for memory of the graph's own GPU, which a kernel may use as its working array.
 bool on_device(const mg_graph *g, const void *p);
 
+// True when every weight is in [0, INT_MAX - 100000000]: then no sum of an SSSP distance
+// and a weight leaves the int range, and distances never fall below 0.
+bool ordinary_weights(const mg_graph *g);
+
 // vertices_reached / edges_traversed: vertices whose value differs from
 // `unreached`, and the sum of their out-degrees (MapGraph "visited edges").
 // vals is [V] or, with stride_src > 1, [V][stride_src] interleaved values of

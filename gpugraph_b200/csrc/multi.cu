@@ -1732,7 +1732,7 @@ __global__ void __launch_bounds__(kNT, 4) k_mss_expand(MultiArgs a, MssBounds mb
         u64 am = 0;
         if (v[r] >= 0) {
           am = s_am[j[r]];
-          // (a sum past the int range wraps to a kept edge, as without bounds)
+          // (a sum past the int range wraps to a kept edge)
           if (bounds && (int)((uint32_t)s_lo[j[r]] + (uint32_t)w[r]) >= hi[r]) am = 0;
           my_bytes += (bounds ? 12 : 8) + 8ull * (unsigned long long)__popcll(am);
         }
@@ -1779,7 +1779,8 @@ __global__ void __launch_bounds__(kNT, 4) k_mss_expand(MultiArgs a, MssBounds mb
           for (int q = 0; q < kMssEdges / 2; ++q) {
             const int4 e = we[b0 + j0 + 2 * q + half];
             bool p0 = false, p1 = false, p2 = false, p3 = false;
-            if (h[q].x != INT_MIN) {
+            // (with weights that GUARD is for, INT_MIN is a distance like any other)
+            if (GUARD ? j0 + 2 * q + half < nb && ((uint32_t)e.w & sbit) != 0u : h[q].x != INT_MIN) {
               const int4 t = *reinterpret_cast<const int4 *>(a.out + (int64_t)s_v[e.x] * 64 + 4 * sub);
               int32_t *hp = a.out + (int64_t)e.y * 64 + 4 * sub;
               p0 = (!GUARD || t.x < INF) && t.x + e.z < h[q].x;
@@ -2124,10 +2125,11 @@ int mg_sssp_multi(mg_graph *g, const int32_t *srcs, int32_t nsrc, int32_t *dists
   // Bounds: not for up to 8 sources, whose rows are one sector each, and for up to
   // 14 only where the rows (256 bytes a vertex) are larger than L2. With / without,
   // weights 1..64: R-MAT 18, 9 sources 1.36 / 1.19 ms, 16 sources 1.35 / 1.61;
-  // R-MAT 16, 14 sources 1.22 / 1.06; R-MAT 20, 12 sources 3.42 / 4.59.
-  mb.hub = nsrc > 14 || (nsrc > 8 && g->nodes >= kMssLargeRows) ? g->mss_hub : -1;
+  // R-MAT 16, 14 sources 1.22 / 1.06; R-MAT 20, 12 sources 3.42 / 4.59. Nor where a
+  // distance can leave [0, 100000000]: the differences of two would wrap.
+  mb.hub = !ordinary_weights(g) ? -1 : nsrc > 14 || (nsrc > 8 && g->nodes >= kMssLargeRows) ? g->mss_hub : -1;
   const bool rows = mb.hub >= 0 || nsrc > kMssLaneSources;
-  const bool guard = g->weight_min < 0 || g->weight_max > INT_MAX - programs::sssp::INIT_VALUE;
+  const bool guard = !ordinary_weights(g);
   LevelBody body = [=](cudaStream_t ss, cudaGraphConditionalHandle h, int use_h) {
     MG_LAUNCH(KID_SCAN, ss, k_mss_scan<kMSVT><<<grid, kNT, 0, ss>>>(a, scan, part));
     if (mb.hub >= 0) MG_LAUNCH(KID_MS_APPLY, ss, k_mss_bounds<<<grid, kNT, 0, ss>>>(a, mb));

@@ -203,9 +203,11 @@ int sssp_fused(mg_graph *g, int32_t src, int32_t *dists, mg_stats *stats, const 
   if (st != MG_OK) return st;
   // Default: one launch. The level loop below serves the host-driven runs
   // (use_cuda_graph = 0, profiling), the ordered frontier, a limit on the levels
-  // (a window is not a level), callers that shorten the waits, and negative weights.
+  // (a window is not a level), callers that shorten the waits, and weights that are
+  // negative or so large that a sum wraps to a negative distance (the smallest
+  // waiting distance is final only without them).
   if (o->use_cuda_graph && !o->ordered_frontier && !prof_on() && o->spin_limit >= kSpinLimitDefault &&
-      (int64_t)o->iter_num >= g->nodes + 2 && g->weight_min >= 0)
+      (int64_t)o->iter_num >= g->nodes + 2 && ordinary_weights(g))
     return sssp_one_launch(g, s, src, dists, stats, o);
   using P = sssp_relax;
   GasArgs<P> a = base_args<P>(g);

@@ -357,3 +357,37 @@ def test_sssp_multi_sources_that_do_not_reach_each_other(hub, nsrc, lo, hi):
         assert np.array_equal(out, ref)
         assert st["converged"] == 1 and st["vertices_reached"] == int((ref != 100000000).sum())
     assert np.array_equal(g.sssp(int(srcs[0]))[0], ref[0])
+
+
+@pytest.mark.parametrize("nsrc", [1, 15, 37, 64])
+def test_sssp_weights_whose_sums_wrap(nsrc):
+    # d + w past the int range gives a negative distance. On a tree every vertex has one path, so its distance is
+    # defined all the same; edge bounds (the last vertex is a sink that all others point to, so the graph is skewed)
+    # and windows rely on distances in [0, 100000000] and must not be used
+    n, inf = 3000, 100000000
+    rng = np.random.default_rng(nsrc)
+    v = np.arange(1, n - 1)
+    par = v - 1 - (rng.random(v.size) * np.minimum(6, v)).astype(np.int64)
+    w = rng.integers(1, 50, v.size)
+    w[rng.random(v.size) < 0.05] = 2147483640
+    src, dst, wt = np.concatenate([par, np.arange(n - 1)]), np.concatenate([v, np.full(n - 1, n - 1)]), np.concatenate(
+        [w, np.ones(n - 1, np.int64)])
+    order = np.lexsort((dst, src))
+    ro = np.concatenate([[0], np.cumsum(np.bincount(src, minlength=n))]).astype(np.int32)
+    hg = HostGraph(ro, dst[order].astype(np.int32), wt[order].astype(np.int32), directed=True)
+    chain = [n - 2]  # the sources: its ancestors, top first, so that each of them reaches a long part of the tree
+    while chain[-1]:
+        chain.append(int(par[chain[-1] - 1]))
+    srcs = np.array(chain[::-1][:nsrc], np.int32)
+    ref = np.full((n - 1, nsrc), inf, np.int64)
+    ref[srcs, np.arange(nsrc)] = 0
+    for x in range(1, n - 1):
+        d = ref[par[x - 1]]
+        ref[x] = np.minimum(ref[x], np.where(d < inf, (d + w[x - 1]).astype(np.int32), inf))
+    assert ref.min() < -2000000000
+    g = Graph(hg)
+    out, st = g.sssp_multi(srcs)
+    assert np.array_equal(out[:, :-1], ref.T) and st["converged"] == 1
+    for mode in ({}, dict(use_cuda_graph=0)):
+        one, st = g.sssp(int(srcs[0]), **mode)
+        assert np.array_equal(one[:-1], ref[:, 0]) and st["converged"] == 1
