@@ -61,10 +61,17 @@ constexpr int kMssEdges = 8;
 // lane's scalar loads touch a sector per source (the same two runs: 4.0 / 19.6 ms
 // at 4, 3.9 / 18.4 at 8, 4.1 / 18.3 at 12, 5.0 / 19.3 at 20).
 constexpr int kMssSparse = 8;
-// On graphs without edge bounds, sources up to which every edge is relaxed by its
-// lane, from registers: the row path's shared memory would come out of L1 (600x600
-// road grid, 7 / 30 sources: 2.27 / 3.46 ms, 3.48 / 5.3 with it).
+// Without edge bounds every edge is relaxed by its lane, from registers (the row
+// path's shared memory comes out of L1), unless there are more sources than this and
+// more edges per vertex than kMssLaneDegree: then an edge carries many active
+// sources. Lanes / rows, weights 1..1000: road grids (4 edges a vertex), 64 sources,
+// 200x200 2.10 / 2.18 ms, 400x400 3.37 / 4.38, 800x800 8.13 / 10.5, 1200x1200 16.3 /
+// 18.0; 40 sources, 1200x1200 12.5 / 16.1. Weights 1..64: R-MAT 12 with 7 edges a
+// vertex, 64 sources 0.48 / 0.48, 24 sources 0.45 / 0.44; with 24 edges a vertex, 64
+// sources 0.58 / 0.43, 40 sources 0.46 / 0.43, 24 sources 0.39 / 0.41, 12 sources
+// 0.32 / 0.37.
 constexpr int kMssLaneSources = 56;
+constexpr int64_t kMssLaneDegree = 8;
 constexpr int64_t kMssLargeRows = 1 << 19;  // vertices from which the distance rows are larger than L2
 
 // Push step of the batched BFS as a GAS Program: expand_edge emits the
@@ -1604,8 +1611,7 @@ MG_DEVINL void relax_min(int32_t *p, int32_t c, u64 &imp, int t) {
 // a 32-byte row piece per lane, 8 scattered reductions per step and a queue
 // reservation per 4 edges: 7.8 ms a run, 4.4 with a whole warp per edge, now 3.9.
 //
-// ROWS = false (no edge bounds and up to kMssLaneSources sources): every edge is
-// relaxed by its lane at once.
+// ROWS = false (see kMssLaneSources): every edge is relaxed by its lane at once.
 template <int VT, bool ROWS, bool GUARD>
 __global__ void __launch_bounds__(kNT, 4) k_mss_expand(MultiArgs a, MssBounds mb, const uint32_t *scan,
                                                        const int32_t *part) {
@@ -2128,7 +2134,7 @@ int mg_sssp_multi(mg_graph *g, const int32_t *srcs, int32_t nsrc, int32_t *dists
   // R-MAT 16, 14 sources 1.22 / 1.06; R-MAT 20, 12 sources 3.42 / 4.59. Nor where a
   // distance can leave [0, 100000000]: the differences of two would wrap.
   mb.hub = !ordinary_weights(g) ? -1 : nsrc > 14 || (nsrc > 8 && g->nodes >= kMssLargeRows) ? g->mss_hub : -1;
-  const bool rows = mb.hub >= 0 || nsrc > kMssLaneSources;
+  const bool rows = mb.hub >= 0 || (nsrc > kMssLaneSources && g->edges > kMssLaneDegree * g->nodes);
   const bool guard = !ordinary_weights(g);
   LevelBody body = [=](cudaStream_t ss, cudaGraphConditionalHandle h, int use_h) {
     MG_LAUNCH(KID_SCAN, ss, k_mss_scan<kMSVT><<<grid, kNT, 0, ss>>>(a, scan, part));

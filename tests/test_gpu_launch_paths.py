@@ -342,12 +342,14 @@ def _dag(n, deg, hub, lo, hi, seed):
     return hg, dists
 
 
-@pytest.mark.parametrize("hub,nsrc", [(0, 57), (0, 64), (1500, 9), (1500, 37), (1500, 64)])
+@pytest.mark.parametrize("hub,nsrc,deg", [(0, 56, 12), (0, 57, 12), (0, 64, 12), (0, 57, 5), (0, 64, 5),
+                                          (1500, 9, 5), (1500, 37, 5), (1500, 64, 12)])
 @pytest.mark.parametrize("lo,hi", [(-40, 60), (-40, -1), (0, 7)])
-def test_sssp_multi_sources_that_do_not_reach_each_other(hub, nsrc, lo, hi):
+def test_sssp_multi_sources_that_do_not_reach_each_other(hub, nsrc, deg, lo, hi):
+    # (5 and 12 edges a vertex: edges relaxed by lanes and by rows, also with 57 sources on flat graphs)
     # most sources cannot reach the early vertices, many are active on one edge: a source that has not reached a
     # tail must stay unreached at the head, also where the weight is negative (100000000 + w < 100000000)
-    hg, dists = _dag(2000, 5, hub, lo, hi, seed=nsrc)
+    hg, dists = _dag(2000, deg, hub, lo, hi, seed=nsrc)
     srcs = np.sort(np.random.default_rng(1).choice(hub or 1900, nsrc, replace=False)).astype(np.int32)
     ref = dists(srcs)
     assert (ref == 100000000).mean() > 0.2
