@@ -13,6 +13,7 @@ LIB_PATH = Path(__file__).resolve().parent / "libmapgraph_b200.so"
 MG_OK, MG_ERR_ARG, MG_ERR_OOM, MG_ERR_OVERFLOW, MG_ERR_TIMEOUT, MG_ERR_CUDA, MG_ERR_UNSUPPORTED, MG_ERR_IO = range(8)
 MG_VAL_NONE, MG_VAL_I32, MG_VAL_F32 = 0, 1, 2
 MG_DIR_AUTO, MG_DIR_PUSH, MG_DIR_PULL = 0, 1, 2
+MG_LOOP_TEST_OFF, MG_LOOP_TEST_FAIL = 0, 1
 
 
 class Options(C.Structure):
@@ -86,6 +87,7 @@ SIGNATURES = {
     "mg_profile_read": (C.c_int, [C.c_int32, C.POINTER(C.c_char_p), C.POINTER(C.c_double), C.POINTER(C.c_int64),
                                   C.POINTER(C.c_uint64)]),
     "mg_selftest_wait_timeout": (C.c_int, [C.c_int64, C.POINTER(C.c_double)]),
+    "mg_selftest_loops": (C.c_int, [C.c_int32]),
     "mg_graph_create": (C.c_int, [P, P, P, C.c_int32, C.c_int64, C.c_int64, C.c_int32, OPTP, C.POINTER(P)]),
     "mg_graph_create_batch": (C.c_int, [P, P, C.c_int64, C.c_int64, P, C.c_int32, OPTP, C.POINTER(P)]),
     "mg_graph_destroy": (C.c_int, [P]),

@@ -470,9 +470,6 @@ __global__ void k_bfs_start(Ctl *ctl, int32_t *queue0, int32_t root, int32_t *la
   }
 }
 
-int bfs_loop_run(mg_graph *g, cudaStream_t s, const std::vector<int32_t> &roots, uint32_t max_iter,
-                 const mg_options *o, int32_t *labels, bool timed);  // bfs_loop.cu
-
 // The whole BFS in one launch: the depths go straight to the caller's device
 // buffer, the statistics come with the result block.
 static int bfs_one_launch(mg_graph *g, cudaStream_t s, const std::vector<int32_t> &roots, uint32_t max_iter,
@@ -483,8 +480,8 @@ static int bfs_one_launch(mg_graph *g, cudaStream_t s, const std::vector<int32_t
   const size_t bytes = (size_t)g->nodes * 4;
   const bool direct = dev && on_device(g, depths);
   int32_t *labels = direct ? depths : g->ws.vbuf[0];
-  std::lock_guard<std::mutex> lock(loop_mutex(g->device));
-  int st = bfs_loop_run(g, s, roots, max_iter, o, labels, stats != nullptr);
+  LoopRun run(g, s);
+  int st = bfs_loop_run(run, g, s, roots, max_iter, o, labels, stats != nullptr);
   if (st != MG_OK) return st;
   cudaError_t e = cudaSuccess;
   if (preds) {
@@ -495,8 +492,7 @@ static int bfs_one_launch(mg_graph *g, cudaStream_t s, const std::vector<int32_t
     e = cudaMemcpyAsync(preds, g->ws.vbuf[1], bytes, kind, s);
   }
   if (e == cudaSuccess && !direct) e = cudaMemcpyAsync(depths, labels, bytes, kind, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  if ((st = cuda_status(e, "bfs")) != MG_OK || (st = loop_end(g, s, "bfs")) != MG_OK) return st;
+  if ((st = run.finish(e, "bfs")) != MG_OK) return st;
   if (stats) {
     const LoopOut &r = *g->loop_out;
     float ms = 0.f;

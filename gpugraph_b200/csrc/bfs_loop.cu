@@ -369,8 +369,7 @@ __global__ void __launch_bounds__(kLoopNT, 1) k_bfs_loop(BfsLoopArgs a) {
   }
 }
 
-// Runs a BFS on stream s in one launch, depths to `labels` (device).
-int bfs_loop_run(mg_graph *g, cudaStream_t s, const std::vector<int32_t> &roots, uint32_t max_iter,
+int bfs_loop_run(LoopRun &run, mg_graph *g, cudaStream_t s, const std::vector<int32_t> &roots, uint32_t max_iter,
                  const mg_options *o, int32_t *labels, bool timed) {
   BfsLoopArgs a;
   a.g = g->csr;
@@ -393,9 +392,9 @@ int bfs_loop_run(mg_graph *g, cudaStream_t s, const std::vector<int32_t> &roots,
   a.dir = o->direction;
   a.alpha = (float)o->alpha;
   a.beta = (float)o->beta;
-  a.loop = loop_begin(g, o);
+  a.loop = run.args(o);
   void *args[] = {&a};
-  return cuda_status(loop_launch(g, (const void *)k_bfs_loop, args, timed, s), "bfs loop launch");
+  return cuda_status(run.launch((const void *)k_bfs_loop, args, timed), "bfs loop launch");
 }
 
 }  // namespace mg

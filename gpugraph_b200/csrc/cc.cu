@@ -33,6 +33,7 @@
 
 #include <algorithm>
 #include <climits>
+#include <optional>
 #include <vector>
 
 #include "algo_util.cuh"
@@ -258,9 +259,6 @@ __global__ void __launch_bounds__(kNT) k_cc_seed(const int32_t *depth, int32_t V
 constexpr double kCcSkew = 8.0;      // longest list over the mean from which the BFS finds the large component
 constexpr uint32_t kCcLevels = 16;
 
-int bfs_loop_run(mg_graph *g, cudaStream_t s, const std::vector<int32_t> &roots, uint32_t max_iter,
-                 const mg_options *o, int32_t *labels, bool timed);  // bfs_loop.cu
-
 // Union-find CC on a symmetric graph (called by mg_cc).
 int cc_union_find(mg_graph *g, int32_t *labels, mg_stats *stats, const mg_options *o) {
   cudaStream_t s = run_stream(g, o);
@@ -280,13 +278,13 @@ int cc_union_find(mg_graph *g, int32_t *labels, mg_stats *stats, const mg_option
   k_ctl_init<<<1, 32, 0, s>>>(ctl, 1u, 1u, (unsigned long long)o->spin_limit, MODE_QUEUE, ctl_flags(nullptr));
   const bool by_bfs = g->hub >= 0 && o->use_cuda_graph && !prof_on() && o->spin_limit >= kSpinLimitDefault &&
                       (double)g->hub_degree > kCcSkew * std::max(1.0, (double)g->edges / (double)V);
-  std::unique_lock<std::mutex> lock(loop_mutex(g->device), std::defer_lock);
+  std::optional<LoopRun> run;
   if (by_bfs) {
-    lock.lock();
+    run.emplace(g, s);
     int32_t *depth = g->ws.gather_tmp;
     mg_options bo;
     mg_options_init(&bo);
-    if ((st = bfs_loop_run(g, s, {g->hub}, kCcLevels, &bo, depth, false)) != MG_OK) return st;
+    if ((st = bfs_loop_run(*run, g, s, {g->hub}, kCcLevels, &bo, depth, false)) != MG_OK) return st;
     k_fill_i32<<<1, 32, 0, s>>>(giant, INT_MAX, 1);
     k_cc_low<<<vgrid, kNT, 0, s>>>(depth, V, giant);
     k_cc_seed<<<vgrid, kNT, 0, s>>>(depth, V, giant, parent, ctl);
@@ -308,7 +306,7 @@ int cc_union_find(mg_graph *g, int32_t *labels, mg_stats *stats, const mg_option
   Ctl c;
   if ((st = read_ctl(g, s, &c)) != MG_OK) return st;
   prof_flush(s, c.kbytes);
-  if (by_bfs && (st = loop_end(g, s, "cc")) != MG_OK) return st;
+  if (by_bfs && (st = run->finish(cudaSuccess, "cc")) != MG_OK) return st;
   if (c.error) return set_error(c.error, std::string("cc: device reported ") + mg_status_string(c.error));
   float ms = 0.f;
   cudaEventElapsedTime(&ms, g->ev0, g->ev1);

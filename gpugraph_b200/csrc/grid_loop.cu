@@ -4,41 +4,78 @@
 
 namespace mg {
 
+namespace {
+
 std::mutex &loop_mutex(int device) {
   static std::mutex m[16];
   return m[device & 15];
 }
 
-cudaError_t loop_launch(mg_graph *g, const void *kernel, void **args, bool timed, cudaStream_t s) {
-  cudaError_t e = timed ? cudaEventRecord(g->ev0, s) : cudaSuccess;
-  if (e == cudaSuccess) e = cudaLaunchCooperativeKernel(kernel, dim3(g->num_sms), dim3(kLoopNT), args, 0, s);
-  if (e == cudaSuccess && timed) e = cudaEventRecord(g->ev1, s);
-  count_launch();
-  return e;
-}
+// What mg_selftest_loops asks of this thread's runs.
+struct LoopTest {
+  int32_t mode = MG_LOOP_TEST_OFF;
+};
+thread_local LoopTest loop_test;
 
-GridLoop loop_begin(mg_graph *g, const mg_options *o) {
+}  // namespace
+
+LoopRun::LoopRun(mg_graph *g, cudaStream_t s) : g_(g), s_(s), turn_(loop_mutex(g->device)) {}
+
+LoopRun::~LoopRun() { settle(nullptr); }
+
+GridLoop LoopRun::args(const mg_options *o) {
   GridLoop l;
-  l.c = g->loop_ctl;
-  l.base = g->loop_base;
+  l.c = g_->loop_ctl;
+  l.base = g_->loop_base;
   l.spin_limit = (unsigned long long)o->spin_limit;
-  l.out = g->loop_out;
-  g->loop_out->error = MG_ERR_TIMEOUT;  // what it stays at when no CTA lives to write it
+  l.out = g_->loop_out;
+  g_->loop_out->error = MG_ERR_TIMEOUT;  // what it stays at when no CTA lives to write it
   return l;
 }
 
-int loop_end(mg_graph *g, cudaStream_t s, const char *what) {
-  const int err = g->loop_out->error;
+cudaError_t LoopRun::launch(const void *kernel, void **args, bool timed) {
+  cudaError_t e = timed ? cudaEventRecord(g_->ev0, s_) : cudaSuccess;
+  if (e == cudaSuccess) e = cudaLaunchCooperativeKernel(kernel, dim3(g_->num_sms), dim3(kLoopNT), args, 0, s_);
+  if (e != cudaSuccess) return e;
+  launched_ = true;
+  count_launch();
+  if (timed) e = cudaEventRecord(g_->ev1, s_);
+  return loop_test.mode == MG_LOOP_TEST_FAIL ? cudaErrorUnknown : e;
+}
+
+cudaError_t LoopRun::settle(int *error) {
+  if (error) *error = MG_OK;
+  if (!launched_) return cudaSuccess;
+  launched_ = false;
+  cudaError_t e = cudaStreamSynchronize(s_);
+  const int err = e == cudaSuccess ? g_->loop_out->error : (int)MG_ERR_CUDA;
   if (err == MG_OK) {
-    g->loop_base += g->loop_out->barriers * (uint32_t)g->num_sms;
-    return MG_OK;
+    g_->loop_base += g_->loop_out->barriers * (uint32_t)g_->num_sms;
+  } else {
+    // the arrivals of a run that broke off are not known: start afresh
+    g_->loop_base = 0;
+    if (e == cudaSuccess) e = cudaMemsetAsync(g_->loop_ctl, 0, sizeof(LoopCtl), s_);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s_);
   }
-  // the arrivals of a run that broke off are not known: start afresh
-  g->loop_base = 0;
-  cudaError_t e = cudaMemsetAsync(g->loop_ctl, 0, sizeof(LoopCtl), s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  turn_.unlock();
+  if (error) *error = err;
+  return e;
+}
+
+int LoopRun::finish(cudaError_t e, const char *what) {
+  int err;
+  const cudaError_t es = settle(&err);
   if (e != cudaSuccess) return cuda_status(e, what);
-  return set_error(err, std::string(what) + ": device reported " + mg_status_string(err));
+  if (es != cudaSuccess) return cuda_status(es, what);
+  if (err != MG_OK) return set_error(err, std::string(what) + ": device reported " + mg_status_string(err));
+  return MG_OK;
 }
 
 }  // namespace mg
+
+extern "C" int mg_selftest_loops(int32_t mode) {
+  mg::clear_error();
+  if (mode < MG_LOOP_TEST_OFF || mode > MG_LOOP_TEST_FAIL) return mg::set_error(MG_ERR_ARG, "unknown loop test");
+  mg::loop_test.mode = mode;
+  return MG_OK;
+}

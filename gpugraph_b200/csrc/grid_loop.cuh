@@ -10,6 +10,7 @@
 #include <cuda_runtime.h>
 
 #include <mutex>
+#include <vector>
 
 #include "common.cuh"
 #include "graph.cuh"
@@ -97,16 +98,37 @@ MG_DEVINL bool grid_level_end(const GridLoop &g, LoopShared *sh, uint32_t slot, 
   return !sh->fail;
 }
 
-// Held from before a loop's launch until its stream was synchronised: two loops
-// launched by different threads would each wait for SMs the other one holds.
-std::mutex &loop_mutex(int device);
-// One cooperative launch of `kernel` (one CTA per SM) on stream s, between the
-// graph's events when the caller wants its time.
-cudaError_t loop_launch(mg_graph *g, const void *kernel, void **args, bool timed, cudaStream_t s);
-// The GridLoop of a run about to be launched.
-GridLoop loop_begin(mg_graph *g, const mg_options *o);
-// After the stream was synchronised: accounts for the barriers the run used and
-// returns its status.
-int loop_end(mg_graph *g, cudaStream_t s, const char *what);
+// One run of a loop kernel: the GPU's turn is held from here until the run's stream
+// was synchronised (two loops launched by different threads would each wait for SMs
+// the other one holds), by finish() or, when a call leaves in between with an error,
+// by the destructor: the arrivals of every run are accounted for.
+class LoopRun {
+ public:
+  LoopRun(mg_graph *g, cudaStream_t s);
+  ~LoopRun();
+  LoopRun(const LoopRun &) = delete;
+  LoopRun &operator=(const LoopRun &) = delete;
+  // The kernel's GridLoop.
+  GridLoop args(const mg_options *o);
+  // One cooperative launch of `kernel` (one CTA per SM), between the graph's events
+  // when the caller wants its time.
+  cudaError_t launch(const void *kernel, void **args, bool timed);
+  // Waits for the stream and returns the run's status; `e` is that of the work
+  // queued behind the kernel.
+  int finish(cudaError_t e, const char *what);
+
+ private:
+  cudaError_t settle(int *error);
+  mg_graph *g_;
+  cudaStream_t s_;
+  std::unique_lock<std::mutex> turn_;
+  bool launched_ = false;
+};
+
+// bfs_loop.cu: a BFS in one launch, depths to `labels` (device).
+int bfs_loop_run(LoopRun &run, mg_graph *g, cudaStream_t s, const std::vector<int32_t> &roots, uint32_t max_iter,
+                 const mg_options *o, int32_t *labels, bool timed);
+// sssp_loop.cu: an SSSP in one launch, distances to `dist` (device).
+int sssp_loop_run(LoopRun &run, mg_graph *g, int32_t src, const mg_options *o, int32_t *dist, bool timed);
 
 }  // namespace mg

@@ -2015,19 +2015,21 @@ static int bfs_multi_run(mg_graph *g, const int32_t *srcs, int32_t nsrc, int32_t
   LoopResult res;
   const auto epi = transpose_epilogue(g, nsrc, depths, true, d16);
   if (one) {
-    std::lock_guard<std::mutex> lock(loop_mutex(g->device));
+    LoopRun run(g, s);
     MsLoopArgs p;
     p.a = a;
     p.src = list;
     p.q = reinterpret_cast<int4 *>(g->loop_queue);
     p.cap = (uint32_t)g->loop_cap;
     p.max_iter = max_iter;
-    p.loop = loop_begin(g, o);
+    p.loop = run.args(o);
     void *args[] = {&p};
-    cudaError_t e = loop_launch(g, (const void *)k_ms_loop, args, stats != nullptr, s);
-    if (e == cudaSuccess && o->outputs_on_device) epi(s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if ((st = cuda_status(e, "batched bfs")) != MG_OK || (st = loop_end(g, s, "batched traversal")) != MG_OK) return st;
+    cudaError_t e = run.launch((const void *)k_ms_loop, args, stats != nullptr);
+    if (e == cudaSuccess && o->outputs_on_device) {
+      epi(s);
+      e = cudaGetLastError();
+    }
+    if ((st = run.finish(e, "batched bfs")) != MG_OK) return st;
     memset(&res.ctl, 0, sizeof(res.ctl));
     res.ctl.level = g->loop_out->level;
     res.ctl.push_levels = g->loop_out->push_levels;

@@ -566,14 +566,13 @@ static int pr_one_launch(mg_graph *g, cudaStream_t s, const PrArgs &a, float *ra
   p.base0 = base0;
   p.max_iter = max_iter;
   p.by_thread = g->pr_max_list <= kPrThreadList ? 1 : 0;
-  std::lock_guard<std::mutex> lock(loop_mutex(g->device));
-  p.loop = loop_begin(g, o);
+  LoopRun run(g, s);
+  p.loop = run.args(o);
   void *args[] = {&p};
-  cudaError_t e = loop_launch(g, (const void *)k_pr_loop, args, stats != nullptr, s);
+  cudaError_t e = run.launch((const void *)k_pr_loop, args, stats != nullptr);
   if (e == cudaSuccess && !direct)
     e = cudaMemcpyAsync(ranks, p.out, (size_t)g->nodes * 4, dev ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  if ((st = cuda_status(e, "pagerank")) != MG_OK || (st = loop_end(g, s, "pagerank")) != MG_OK) return st;
+  if ((st = run.finish(e, "pagerank")) != MG_OK) return st;
   if (stats) {
     const LoopOut &r = *g->loop_out;
     float ms = 0.f;

@@ -507,8 +507,8 @@ constexpr int64_t kPprLoopWork = 1ll << 24;
 
 static int ppr_one_launch(mg_graph *g, cudaStream_t s, PprArgs a, uint32_t max_iter, const mg_options *o,
                           const char *name, LoopResult *res) {
-  std::lock_guard<std::mutex> lock(loop_mutex(g->device));
-  GridLoop loop = loop_begin(g, o);
+  LoopRun run(g, s);
+  GridLoop loop = run.args(o);
   double tol = o->tolerance;
   void *args[] = {&a, &tol, &max_iter, &loop};
   const void *kernel;
@@ -519,11 +519,9 @@ static int ppr_one_launch(mg_graph *g, cudaStream_t s, PprArgs a, uint32_t max_i
     case 8: kernel = (const void *)k_ppr_loop<8>; break;
     default: kernel = (const void *)k_ppr_loop<16>;
   }
-  cudaError_t e = loop_launch(g, kernel, args, true, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  int st;
   memset(&res->ctl, 0, sizeof(res->ctl));
-  if ((st = cuda_status(e, name)) != MG_OK || (st = loop_end(g, s, name)) != MG_OK) return st;
+  const int st = run.finish(run.launch(kernel, args, true), name);
+  if (st != MG_OK) return st;
   res->ctl.level = g->loop_out->level;
   res->ctl.residual = g->loop_out->residual;
   res->ctl.acc[2] = g->loop_out->norm;

@@ -165,21 +165,17 @@ __global__ void k_sssp_seed(int32_t *dist, int32_t *queue0, int32_t src) {
 
 }  // namespace
 
-int sssp_loop_run(mg_graph *g, cudaStream_t s, int32_t src, const mg_options *o, int32_t *dist,
-                  bool timed);  // sssp_loop.cu
-
 static int sssp_one_launch(mg_graph *g, cudaStream_t s, int32_t src, int32_t *dists, mg_stats *stats,
                            const mg_options *o) {
   const bool dev = o->outputs_on_device != 0, direct = dev && on_device(g, dists);
   int32_t *dist = direct ? dists : g->ws.vbuf[0];
-  std::lock_guard<std::mutex> lock(loop_mutex(g->device));
-  int st = sssp_loop_run(g, s, src, o, dist, stats != nullptr);
+  LoopRun run(g, s);
+  int st = sssp_loop_run(run, g, src, o, dist, stats != nullptr);
   if (st != MG_OK) return st;
   cudaError_t e = cudaSuccess;
   if (!direct)
     e = cudaMemcpyAsync(dists, dist, (size_t)g->nodes * 4, dev ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-  if ((st = cuda_status(e, "sssp")) != MG_OK || (st = loop_end(g, s, "sssp")) != MG_OK) return st;
+  if ((st = run.finish(e, "sssp")) != MG_OK) return st;
   if (stats) {
     float ms = 0.f;
     cudaEventElapsedTime(&ms, g->ev0, g->ev1);

@@ -194,8 +194,7 @@ __global__ void __launch_bounds__(kLoopNT, 1) k_sssp_loop(SsspLoopArgs a) {
   }
 }
 
-// Runs an SSSP on stream s in one launch, distances to `dist` (device).
-int sssp_loop_run(mg_graph *g, cudaStream_t s, int32_t src, const mg_options *o, int32_t *dist, bool timed) {
+int sssp_loop_run(LoopRun &run, mg_graph *g, int32_t src, const mg_options *o, int32_t *dist, bool timed) {
   SsspLoopArgs a;
   a.g = g->csr;
   a.dist = dist;
@@ -208,9 +207,9 @@ int sssp_loop_run(mg_graph *g, cudaStream_t s, int32_t src, const mg_options *o,
   const double mean = std::max(1.0, (double)g->edges / (double)g->nodes);
   a.delta = (int32_t)std::min(1e9, std::max(1.0, kSsspWindow * (double)std::max(g->weight_max, 0) / mean));
   a.max_iter = (uint32_t)(g->nodes + 2);
-  a.loop = loop_begin(g, o);
+  a.loop = run.args(o);
   void *args[] = {&a};
-  return cuda_status(loop_launch(g, (const void *)k_sssp_loop, args, timed, s), "sssp loop launch");
+  return cuda_status(run.launch((const void *)k_sssp_loop, args, timed), "sssp loop launch");
 }
 
 }  // namespace mg

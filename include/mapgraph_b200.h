@@ -127,6 +127,12 @@ int mg_profile_read(int32_t kind, const char **name, double *total_ms, int64_t *
  * bounded device-side wait against a status word nothing publishes. Returns
  * MG_ERR_TIMEOUT when the wait ended at spin_limit as designed. */
 int mg_selftest_wait_timeout(int64_t spin_limit, double *elapsed_ms);
+/* The same for the traversals and solves that run in one launch: what the host makes
+ * of the next runs of this thread. MG_LOOP_TEST_FAIL: a launch that succeeded is
+ * reported as failed, so the call returns MG_ERR_CUDA with the kernel in flight; the
+ * graph must serve the next call as if nothing had happened. */
+enum { MG_LOOP_TEST_OFF = 0, MG_LOOP_TEST_FAIL = 1 };
+int mg_selftest_loops(int32_t mode);
 
 /* ----------------------------------------------------------------- graphs -- */
 /* Copy a host CSR to the device and build what the hot path needs (out-degrees,
