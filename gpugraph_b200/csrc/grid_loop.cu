@@ -29,7 +29,9 @@ GridLoop LoopRun::args(const mg_options *o) {
   l.base = g_->loop_base;
   l.spin_limit = (unsigned long long)o->spin_limit;
   l.out = g_->loop_out;
+  if (loop_test.mode == MG_LOOP_TEST_WAITS) l.spin_limit = 1;
   g_->loop_out->error = MG_ERR_TIMEOUT;  // what it stays at when no CTA lives to write it
+  g_->loop_out->timed_out = 0;
   return l;
 }
 
@@ -48,7 +50,7 @@ cudaError_t LoopRun::settle(int *error) {
   if (!launched_) return cudaSuccess;
   launched_ = false;
   cudaError_t e = cudaStreamSynchronize(s_);
-  const int err = e == cudaSuccess ? g_->loop_out->error : (int)MG_ERR_CUDA;
+  const int err = e != cudaSuccess ? (int)MG_ERR_CUDA : g_->loop_out->timed_out ? (int)MG_ERR_TIMEOUT : g_->loop_out->error;
   if (err == MG_OK) {
     g_->loop_base += g_->loop_out->barriers * (uint32_t)g_->num_sms;
   } else {
@@ -75,7 +77,7 @@ int LoopRun::finish(cudaError_t e, const char *what) {
 
 extern "C" int mg_selftest_loops(int32_t mode) {
   mg::clear_error();
-  if (mode < MG_LOOP_TEST_OFF || mode > MG_LOOP_TEST_FAIL) return mg::set_error(MG_ERR_ARG, "unknown loop test");
+  if (mode < MG_LOOP_TEST_OFF || mode > MG_LOOP_TEST_WAITS) return mg::set_error(MG_ERR_ARG, "unknown loop test");
   mg::loop_test.mode = mode;
   return MG_OK;
 }

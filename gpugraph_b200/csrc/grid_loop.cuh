@@ -42,6 +42,7 @@ struct LoopOut {
   double residual, norm;
   uint32_t barriers;
   int32_t error;
+  int32_t timed_out;  // set by every CTA whose wait ran out
 };
 
 struct LoopShared {
@@ -79,7 +80,10 @@ MG_DEVINL bool grid_level_end(const GridLoop &g, LoopShared *sh, uint32_t slot, 
     unsigned long long spins = 0;
     while ((int32_t)(ld_acquire(&g.c->arrived) - target) < 0) {
       if (++spins >= g.spin_limit) {
+        // reported by the CTA itself: at the last barrier CTA 0 may still get
+        // through, and `error` say that all is well
         sh->fail = 1;
+        *(volatile int32_t *)&g.out->timed_out = 1;
         break;
       }
     }

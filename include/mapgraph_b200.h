@@ -130,8 +130,10 @@ int mg_selftest_wait_timeout(int64_t spin_limit, double *elapsed_ms);
 /* The same for the traversals and solves that run in one launch: what the host makes
  * of the next runs of this thread. MG_LOOP_TEST_FAIL: a launch that succeeded is
  * reported as failed, so the call returns MG_ERR_CUDA with the kernel in flight; the
- * graph must serve the next call as if nothing had happened. */
-enum { MG_LOOP_TEST_OFF = 0, MG_LOOP_TEST_FAIL = 1 };
+ * graph must serve the next call as if nothing had happened. MG_LOOP_TEST_WAITS: every
+ * grid barrier gives up after one poll (MG_ERR_TIMEOUT); a spin_limit below the default
+ * would choose the level-by-level loop instead. */
+enum { MG_LOOP_TEST_OFF = 0, MG_LOOP_TEST_FAIL = 1, MG_LOOP_TEST_WAITS = 2 };
 int mg_selftest_loops(int32_t mode);
 
 /* ----------------------------------------------------------------- graphs -- */

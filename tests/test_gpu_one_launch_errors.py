@@ -85,3 +85,15 @@ def test_error_behind_the_launch_leaves_the_graph_usable(name, calls):
         assert calls[name]()
         for other in NAMES:
             assert calls[other](), other
+
+
+@pytest.mark.parametrize("name", NAMES)
+def test_barrier_wait_that_runs_out(name, calls):
+    for _ in range(3):
+        _lib.lib.mg_selftest_loops(_lib.MG_LOOP_TEST_WAITS)
+        with pytest.raises(MapGraphError) as e:
+            calls[name]()
+        assert e.value.status == _lib.MG_ERR_TIMEOUT
+        _lib.lib.mg_selftest_loops(_lib.MG_LOOP_TEST_OFF)
+        for other in [name, *NAMES]:
+            assert calls[other](), other
