@@ -13,7 +13,7 @@ LIB_PATH = Path(__file__).resolve().parent / "libmapgraph_b200.so"
 MG_OK, MG_ERR_ARG, MG_ERR_OOM, MG_ERR_OVERFLOW, MG_ERR_TIMEOUT, MG_ERR_CUDA, MG_ERR_UNSUPPORTED, MG_ERR_IO = range(8)
 MG_VAL_NONE, MG_VAL_I32, MG_VAL_F32 = 0, 1, 2
 MG_DIR_AUTO, MG_DIR_PUSH, MG_DIR_PULL = 0, 1, 2
-MG_LOOP_TEST_OFF, MG_LOOP_TEST_FAIL, MG_LOOP_TEST_WAITS = 0, 1, 2
+MG_LOOP_TEST_OFF, MG_LOOP_TEST_FAIL, MG_LOOP_TEST_WAITS, MG_LOOP_TEST_REFUSE = 0, 1, 2, 3
 
 
 class Options(C.Structure):

@@ -529,8 +529,9 @@ int bfs_run(mg_graph *g, const std::vector<int32_t> &roots, int32_t *depths, mg_
   // Default: one launch. The level-by-level loop below serves the host-driven
   // runs (use_cuda_graph = 0, profiling), the ordered frontier and callers that
   // shorten the waits (a grid barrier waits for the slowest CTA of a level).
-  if (o->use_cuda_graph && !o->ordered_frontier && !prof_on() && o->spin_limit >= kSpinLimitDefault)
-    return bfs_one_launch(g, s, roots, max_iter, depths, stats, o, preds);
+  if (o->use_cuda_graph && !o->ordered_frontier && !prof_on() && o->spin_limit >= kSpinLimitDefault &&
+      (st = bfs_one_launch(g, s, roots, max_iter, depths, stats, o, preds)) != kLoopRefused)
+    return st;
   if ((st = prepare_run(g, s)) != MG_OK) return st;
   Workspace &w = g->ws;
   GasArgs<BfsP> a;

@@ -394,7 +394,7 @@ int bfs_loop_run(LoopRun &run, mg_graph *g, cudaStream_t s, const std::vector<in
   a.beta = (float)o->beta;
   a.loop = run.args(o);
   void *args[] = {&a};
-  return cuda_status(run.launch((const void *)k_bfs_loop, args, timed), "bfs loop launch");
+  return run.launch((const void *)k_bfs_loop, args, timed, "bfs loop launch");
 }
 
 }  // namespace mg

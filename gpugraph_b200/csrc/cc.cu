@@ -276,15 +276,19 @@ int cc_union_find(mg_graph *g, int32_t *labels, mg_stats *stats, const mg_option
   const bool direct = o->outputs_on_device != 0 && on_device(g, labels);
   int32_t *out = direct ? labels : g->ws.vbuf[1];
   k_ctl_init<<<1, 32, 0, s>>>(ctl, 1u, 1u, (unsigned long long)o->spin_limit, MODE_QUEUE, ctl_flags(nullptr));
-  const bool by_bfs = g->hub >= 0 && o->use_cuda_graph && !prof_on() && o->spin_limit >= kSpinLimitDefault &&
+  bool by_bfs = g->hub >= 0 && o->use_cuda_graph && !prof_on() && o->spin_limit >= kSpinLimitDefault &&
                       (double)g->hub_degree > kCcSkew * std::max(1.0, (double)g->edges / (double)V);
   std::optional<LoopRun> run;
+  int32_t *depth = g->ws.gather_tmp;
   if (by_bfs) {
     run.emplace(g, s);
-    int32_t *depth = g->ws.gather_tmp;
     mg_options bo;
     mg_options_init(&bo);
-    if ((st = bfs_loop_run(*run, g, s, {g->hub}, kCcLevels, &bo, depth, false)) != MG_OK) return st;
+    st = bfs_loop_run(*run, g, s, {g->hub}, kCcLevels, &bo, depth, false);
+    if (st != MG_OK && st != kLoopRefused) return st;
+    by_bfs = st == MG_OK;
+  }
+  if (by_bfs) {
     k_fill_i32<<<1, 32, 0, s>>>(giant, INT_MAX, 1);
     k_cc_low<<<vgrid, kNT, 0, s>>>(depth, V, giant);
     k_cc_seed<<<vgrid, kNT, 0, s>>>(depth, V, giant, parent, ctl);

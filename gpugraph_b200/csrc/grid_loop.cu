@@ -35,14 +35,22 @@ GridLoop LoopRun::args(const mg_options *o) {
   return l;
 }
 
-cudaError_t LoopRun::launch(const void *kernel, void **args, bool timed) {
+int LoopRun::launch(const void *kernel, void **args, bool timed, const char *what) {
   cudaError_t e = timed ? cudaEventRecord(g_->ev0, s_) : cudaSuccess;
-  if (e == cudaSuccess) e = cudaLaunchCooperativeKernel(kernel, dim3(g_->num_sms), dim3(kLoopNT), args, 0, s_);
-  if (e != cudaSuccess) return e;
+  if (e != cudaSuccess) return cuda_status(e, what);
+  e = loop_test.mode == MG_LOOP_TEST_REFUSE
+          ? cudaErrorCooperativeLaunchTooLarge
+          : cudaLaunchCooperativeKernel(kernel, dim3(g_->num_sms), dim3(kLoopNT), args, 0, s_);
+  if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported) {
+    cudaGetLastError();
+    turn_.unlock();
+    return kLoopRefused;
+  }
+  if (e != cudaSuccess) return cuda_status(e, what);
   launched_ = true;
   count_launch();
   if (timed) e = cudaEventRecord(g_->ev1, s_);
-  return loop_test.mode == MG_LOOP_TEST_FAIL ? cudaErrorUnknown : e;
+  return cuda_status(loop_test.mode == MG_LOOP_TEST_FAIL ? cudaErrorUnknown : e, what);
 }
 
 cudaError_t LoopRun::settle(int *error) {
@@ -77,7 +85,7 @@ int LoopRun::finish(cudaError_t e, const char *what) {
 
 extern "C" int mg_selftest_loops(int32_t mode) {
   mg::clear_error();
-  if (mode < MG_LOOP_TEST_OFF || mode > MG_LOOP_TEST_WAITS) return mg::set_error(MG_ERR_ARG, "unknown loop test");
+  if (mode < MG_LOOP_TEST_OFF || mode > MG_LOOP_TEST_REFUSE) return mg::set_error(MG_ERR_ARG, "unknown loop test");
   mg::loop_test.mode = mode;
   return MG_OK;
 }

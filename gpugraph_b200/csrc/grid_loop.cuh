@@ -102,6 +102,11 @@ MG_DEVINL bool grid_level_end(const GridLoop &g, LoopShared *sh, uint32_t slot, 
   return !sh->fail;
 }
 
+// The launch's status where the process or the stream has fewer SMs than the GPU (an
+// MPS share, a green context): nothing was launched, the caller takes its
+// level-by-level loop, which needs no CTA beside another.
+constexpr int kLoopRefused = -1;
+
 // One run of a loop kernel: the GPU's turn is held from here until the run's stream
 // was synchronised (two loops launched by different threads would each wait for SMs
 // the other one holds), by finish() or, when a call leaves in between with an error,
@@ -115,8 +120,8 @@ class LoopRun {
   // The kernel's GridLoop.
   GridLoop args(const mg_options *o);
   // One cooperative launch of `kernel` (one CTA per SM), between the graph's events
-  // when the caller wants its time.
-  cudaError_t launch(const void *kernel, void **args, bool timed);
+  // when the caller wants its time. MG_OK, an error, or kLoopRefused.
+  int launch(const void *kernel, void **args, bool timed, const char *what);
   // Waits for the stream and returns the run's status; `e` is that of the work
   // queued behind the kernel.
   int finish(cudaError_t e, const char *what);
@@ -129,6 +134,7 @@ class LoopRun {
   bool launched_ = false;
 };
 
+// The runs below return what LoopRun::launch does.
 // bfs_loop.cu: a BFS in one launch, depths to `labels` (device).
 int bfs_loop_run(LoopRun &run, mg_graph *g, cudaStream_t s, const std::vector<int32_t> &roots, uint32_t max_iter,
                  const mg_options *o, int32_t *labels, bool timed);

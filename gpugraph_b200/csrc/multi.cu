@@ -1879,8 +1879,8 @@ static MultiArgs multi_args(mg_graph *g) {
   return a;
 }
 
-static int multi_prepare(mg_graph *g, const int32_t *srcs, int32_t nsrc, const mg_options *o, cudaStream_t s,
-                         SrcList *list, int32_t fill, bool stack = false, bool clear = true) {
+// Arguments and buffers of a batched run.
+static int multi_prepare(mg_graph *g, const int32_t *srcs, int32_t nsrc, SrcList *list) {
   if (nsrc < 1 || nsrc > 64) return set_error(MG_ERR_ARG, "nsrc must be in [1, 64]");
   std::vector<int32_t> distinct;
   int st = check_sources(g, srcs, nsrc, &distinct);
@@ -1891,8 +1891,12 @@ static int multi_prepare(mg_graph *g, const int32_t *srcs, int32_t nsrc, const m
   list->nsrc = nsrc;
   list->ndistinct = (int32_t)distinct.size();
   if ((st = ensure_workspace(g)) != MG_OK) return st;
-  if ((st = ensure_multi(g)) != MG_OK) return st;
-  if (!clear) return MG_OK;  // the one-launch loop starts its own state
+  return ensure_multi(g);
+}
+
+// The state a level loop starts from.
+static int multi_clear(mg_graph *g, cudaStream_t s, int32_t fill, bool stack = false) {
+  int st;
   if ((st = prepare_run(g, s)) != MG_OK) return st;
   const size_t V = (size_t)g->nodes;
   cudaError_t e = cudaMemsetAsync(g->mask[0], 0, V * 8, s);
@@ -1910,7 +1914,6 @@ static int multi_prepare(mg_graph *g, const int32_t *srcs, int32_t nsrc, const m
     k_fill_i32<<<g->num_sms * 8, 256, 0, s>>>(g->multi_out, fill, (int64_t)V * 64);
     count_launch();
   }
-  (void)o;
   return MG_OK;
 }
 
@@ -1980,6 +1983,38 @@ static const mg_options *opts_or_default(const mg_options *o, mg_options *d) {
   return d;
 }
 
+// A batched BFS in one launch (k_ms_loop), which starts its own state.
+static int ms_one_launch(mg_graph *g, cudaStream_t s, const MultiArgs &a, const SrcList &src, uint32_t max_iter,
+                         const mg_options *o, bool timed, const std::function<void(cudaStream_t)> &epilogue,
+                         LoopResult *res) {
+  LoopRun run(g, s);
+  MsLoopArgs p;
+  p.a = a;
+  p.src = src;
+  p.q = reinterpret_cast<int4 *>(g->loop_queue);
+  p.cap = (uint32_t)g->loop_cap;
+  p.max_iter = max_iter;
+  p.loop = run.args(o);
+  void *args[] = {&p};
+  int st = run.launch((const void *)k_ms_loop, args, timed, "batched bfs");
+  if (st != MG_OK) return st;
+  cudaError_t e = cudaSuccess;
+  if (o->outputs_on_device) {
+    epilogue(s);
+    e = cudaGetLastError();
+  }
+  if ((st = run.finish(e, "batched bfs")) != MG_OK) return st;
+  memset(&res->ctl, 0, sizeof(res->ctl));
+  res->ctl.level = g->loop_out->level;
+  res->ctl.push_levels = g->loop_out->push_levels;
+  res->ctl.pull_levels = g->loop_out->pull_levels;
+  res->ctl.frontier_size = g->loop_out->frontier_size;
+  float ms = 0.f;
+  if (timed) cudaEventElapsedTime(&ms, g->ev0, g->ev1);
+  res->ms = ms;
+  return MG_OK;
+}
+
 // One batched BFS: with DT = uint16_t the level stack plus uint16 depth rows
 // past it, with DT = int32_t int32 depth rows only. A uint16 run stops after
 // level kMsDepth16Levels; *depth_overflow then tells the caller to rerun with
@@ -1997,7 +2032,7 @@ static int bfs_multi_run(mg_graph *g, const int32_t *srcs, int32_t nsrc, int32_t
   const bool one = d16 && o->use_cuda_graph && !o->ordered_frontier && !prof_on() &&
                    o->spin_limit >= kSpinLimitDefault && (int64_t)o->iter_num >= g->nodes + 2 &&
                    g->nodes + g->edges <= kMsLoopWork;
-  int st = multi_prepare(g, srcs, nsrc, o, s, &list, -1, d16, !one);
+  int st = multi_prepare(g, srcs, nsrc, &list);
   if (st != MG_OK) return st;
   MultiArgs a = multi_args(g);
   a.all = (nsrc == 64) ? ~0ull : ((1ull << nsrc) - 1);
@@ -2015,35 +2050,17 @@ static int bfs_multi_run(mg_graph *g, const int32_t *srcs, int32_t nsrc, int32_t
   LoopResult res;
   const auto epi = transpose_epilogue(g, nsrc, depths, true, d16);
   if (one) {
-    LoopRun run(g, s);
-    MsLoopArgs p;
-    p.a = a;
-    p.src = list;
-    p.q = reinterpret_cast<int4 *>(g->loop_queue);
-    p.cap = (uint32_t)g->loop_cap;
-    p.max_iter = max_iter;
-    p.loop = run.args(o);
-    void *args[] = {&p};
-    cudaError_t e = run.launch((const void *)k_ms_loop, args, stats != nullptr);
-    if (e == cudaSuccess && o->outputs_on_device) {
-      epi(s);
-      e = cudaGetLastError();
+    st = ms_one_launch(g, s, a, list, max_iter, o, stats != nullptr, epi, &res);
+    if (st == MG_OK) {
+      if (res.ctl.frontier_size > 0 && res.ctl.level >= kMsDepth16Levels && max_iter_asked > kMsDepth16Levels) {
+        *depth_overflow = true;  // deeper than a uint16 depth row holds
+        return MG_OK;
+      }
+      return multi_finish(g, s, nsrc, depths, -1, stats, o, res, d16);
     }
-    if ((st = run.finish(e, "batched bfs")) != MG_OK) return st;
-    memset(&res.ctl, 0, sizeof(res.ctl));
-    res.ctl.level = g->loop_out->level;
-    res.ctl.push_levels = g->loop_out->push_levels;
-    res.ctl.pull_levels = g->loop_out->pull_levels;
-    res.ctl.frontier_size = g->loop_out->frontier_size;
-    float ms = 0.f;
-    if (stats) cudaEventElapsedTime(&ms, g->ev0, g->ev1);
-    res.ms = ms;
-    if (res.ctl.frontier_size > 0 && res.ctl.level >= kMsDepth16Levels && max_iter_asked > kMsDepth16Levels) {
-      *depth_overflow = true;  // deeper than a uint16 depth row holds
-      return MG_OK;
-    }
-    return multi_finish(g, s, nsrc, depths, -1, stats, o, res, d16);
+    if (st != kLoopRefused) return st;
   }
+  if ((st = multi_clear(g, s, -1, d16)) != MG_OK) return st;
   GasArgs<msbfs_push> ga;
   ga.g = g->csr;
   ga.vl.visit = a.visit;
@@ -2119,8 +2136,8 @@ int mg_sssp_multi(mg_graph *g, const int32_t *srcs, int32_t nsrc, int32_t *dists
   const mg_options *o = opts_or_default(opts, &d);
   cudaStream_t s = run_stream(g, o);
   SrcList list;
-  int st = multi_prepare(g, srcs, nsrc, o, s, &list, programs::sssp::INIT_VALUE);
-  if (st != MG_OK) return st;
+  int st = multi_prepare(g, srcs, nsrc, &list);
+  if (st != MG_OK || (st = multi_clear(g, s, programs::sssp::INIT_VALUE)) != MG_OK) return st;
   MultiArgs a = multi_args(g);
   a.all = (nsrc == 64) ? ~0ull : ((1ull << nsrc) - 1);
   const uint32_t max_iter = (uint32_t)std::min<int64_t>(o->iter_num > 0 ? o->iter_num : 0, g->nodes + 2);

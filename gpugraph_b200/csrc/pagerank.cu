@@ -569,8 +569,9 @@ static int pr_one_launch(mg_graph *g, cudaStream_t s, const PrArgs &a, float *ra
   LoopRun run(g, s);
   p.loop = run.args(o);
   void *args[] = {&p};
-  cudaError_t e = run.launch((const void *)k_pr_loop, args, stats != nullptr);
-  if (e == cudaSuccess && !direct)
+  if ((st = run.launch((const void *)k_pr_loop, args, stats != nullptr, "pagerank")) != MG_OK) return st;
+  cudaError_t e = cudaSuccess;
+  if (!direct)
     e = cudaMemcpyAsync(ranks, p.out, (size_t)g->nodes * 4, dev ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, s);
   if ((st = run.finish(e, "pagerank")) != MG_OK) return st;
   if (stats) {
@@ -635,8 +636,9 @@ extern "C" int mg_pagerank(mg_graph *g, float *ranks, mg_stats *stats, const mg_
   const double base0 = (1.0 - d) * inv_n + d * ((double)g->pr_ndangling * inv_n) * inv_n;
   // Short iterations: one launch (kPrLoopWork). The level loop serves the rest,
   // the host-driven runs and callers that shorten the waits.
-  if (o->use_cuda_graph && !prof_on() && o->spin_limit >= kSpinLimitDefault && g->edges + V <= kPrLoopWork)
-    return pr_one_launch(g, s, a, ranks, stats, o, inv_n, base0, max_iter);
+  if (o->use_cuda_graph && !prof_on() && o->spin_limit >= kSpinLimitDefault && g->edges + V <= kPrLoopWork &&
+      (st = pr_one_launch(g, s, a, ranks, stats, o, inv_n, base0, max_iter)) != kLoopRefused)
+    return st;
   k_pr_init<<<g->num_sms * 4, 256, 0, s>>>(a.inv, a.r0, a.c0, V, (float)inv_n);
   k_pr_ctl_init<<<1, 32, 0, s>>>(a.ctl, max_iter, (unsigned long long)o->spin_limit, ctl_flags(nullptr), base0);
   count_launch(2);

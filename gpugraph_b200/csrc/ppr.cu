@@ -520,8 +520,8 @@ static int ppr_one_launch(mg_graph *g, cudaStream_t s, PprArgs a, uint32_t max_i
     default: kernel = (const void *)k_ppr_loop<16>;
   }
   memset(&res->ctl, 0, sizeof(res->ctl));
-  const int st = run.finish(run.launch(kernel, args, true), name);
-  if (st != MG_OK) return st;
+  int st = run.launch(kernel, args, true, name);
+  if (st != MG_OK || (st = run.finish(cudaSuccess, name)) != MG_OK) return st;
   res->ctl.level = g->loop_out->level;
   res->ctl.residual = g->loop_out->residual;
   res->ctl.acc[2] = g->loop_out->norm;
@@ -577,7 +577,7 @@ static int ppr_solve(mg_graph *g, int dir, const float *w, const float *rhs, flo
   if (o->use_cuda_graph && !prof_on() && o->spin_limit >= kSpinLimitDefault && (g->nodes + g->edges) * nv <= kPprLoopWork) {
     const int st = ppr_one_launch(g, s, a, max_iter, o, name, res);
     *result = (res->ctl.level & 1) ? a.x1 : a.x0;
-    return st;
+    if (st != kLoopRefused) return st;
   }
   k_ctl_init<<<1, 32, 0, s>>>(a.ctl, 1u, max_iter, (unsigned long long)o->spin_limit, MODE_QUEUE, ctl_flags(nullptr));
   k_ppr_rhs_norm<<<g->num_sms * 4, 256, 0, s>>>(rhs, n, a.ctl);

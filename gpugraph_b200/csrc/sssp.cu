@@ -203,8 +203,9 @@ int sssp_fused(mg_graph *g, int32_t src, int32_t *dists, mg_stats *stats, const 
   // negative or so large that a sum wraps to a negative distance (the smallest
   // waiting distance is final only without them).
   if (o->use_cuda_graph && !o->ordered_frontier && !prof_on() && o->spin_limit >= kSpinLimitDefault &&
-      (int64_t)o->iter_num >= g->nodes + 2 && ordinary_weights(g))
-    return sssp_one_launch(g, s, src, dists, stats, o);
+      (int64_t)o->iter_num >= g->nodes + 2 && ordinary_weights(g) &&
+      (st = sssp_one_launch(g, s, src, dists, stats, o)) != kLoopRefused)
+    return st;
   using P = sssp_relax;
   GasArgs<P> a = base_args<P>(g);
   a.vl.dist = g->ws.vbuf[0];

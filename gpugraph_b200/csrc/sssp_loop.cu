@@ -209,7 +209,7 @@ int sssp_loop_run(LoopRun &run, mg_graph *g, int32_t src, const mg_options *o, i
   a.max_iter = (uint32_t)(g->nodes + 2);
   a.loop = run.args(o);
   void *args[] = {&a};
-  return cuda_status(run.launch((const void *)k_sssp_loop, args, timed), "sssp loop launch");
+  return run.launch((const void *)k_sssp_loop, args, timed, "sssp loop launch");
 }
 
 }  // namespace mg

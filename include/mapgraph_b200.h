@@ -132,8 +132,9 @@ int mg_selftest_wait_timeout(int64_t spin_limit, double *elapsed_ms);
  * reported as failed, so the call returns MG_ERR_CUDA with the kernel in flight; the
  * graph must serve the next call as if nothing had happened. MG_LOOP_TEST_WAITS: every
  * grid barrier gives up after one poll (MG_ERR_TIMEOUT); a spin_limit below the default
- * would choose the level-by-level loop instead. */
-enum { MG_LOOP_TEST_OFF = 0, MG_LOOP_TEST_FAIL = 1, MG_LOOP_TEST_WAITS = 2 };
+ * would choose the level-by-level loop instead. MG_LOOP_TEST_REFUSE: the launch is
+ * refused as where the process has too few SMs; the call then runs level by level. */
+enum { MG_LOOP_TEST_OFF = 0, MG_LOOP_TEST_FAIL = 1, MG_LOOP_TEST_WAITS = 2, MG_LOOP_TEST_REFUSE = 3 };
 int mg_selftest_loops(int32_t mode);
 
 /* ----------------------------------------------------------------- graphs -- */

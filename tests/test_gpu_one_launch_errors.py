@@ -97,3 +97,18 @@ def test_barrier_wait_that_runs_out(name, calls):
         _lib.lib.mg_selftest_loops(_lib.MG_LOOP_TEST_OFF)
         for other in [name, *NAMES]:
             assert calls[other](), other
+
+
+@pytest.mark.parametrize("name", NAMES)
+def test_refused_launch_runs_level_by_level(name, calls):
+    _lib.lib.mg_kernel_launches(1)
+    assert calls[name]()
+    one = _lib.lib.mg_kernel_launches(1)
+    for _ in range(2):
+        _lib.lib.mg_selftest_loops(_lib.MG_LOOP_TEST_REFUSE)
+        assert calls[name]()
+        # (CC: without its BFS as many launches, sampling rounds instead)
+        assert _lib.lib.mg_kernel_launches(1) > one or name == "cc"
+        _lib.lib.mg_selftest_loops(_lib.MG_LOOP_TEST_OFF)
+        assert calls[name]()
+        _lib.lib.mg_kernel_launches(1)
