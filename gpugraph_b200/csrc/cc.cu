@@ -268,6 +268,10 @@ int cc_union_find(mg_graph *g, int32_t *labels, mg_stats *stats, const mg_option
   if (V < 1) return set_error(MG_ERR_ARG, "cc: empty graph");
   int32_t *parent = g->ws.vbuf[0];
   Ctl *ctl = g->ws.ctl;
+  bool by_bfs = g->hub >= 0 && o->use_cuda_graph && !prof_on() && o->spin_limit >= kSpinLimitDefault &&
+                (double)g->hub_degree > kCcSkew * std::max(1.0, (double)g->edges / (double)V);
+  std::optional<LoopRun> run;
+  if (by_bfs) run.emplace(g, s);
   cudaError_t e = cudaEventRecord(g->ev0, s);
   if (e != cudaSuccess) return cuda_status(e, "event record");
   int32_t *giant = reinterpret_cast<int32_t *>(g->ws.scan);  // scratch word (the scan buffer is free here)
@@ -276,12 +280,8 @@ int cc_union_find(mg_graph *g, int32_t *labels, mg_stats *stats, const mg_option
   const bool direct = o->outputs_on_device != 0 && on_device(g, labels);
   int32_t *out = direct ? labels : g->ws.vbuf[1];
   k_ctl_init<<<1, 32, 0, s>>>(ctl, 1u, 1u, (unsigned long long)o->spin_limit, MODE_QUEUE, ctl_flags(nullptr));
-  bool by_bfs = g->hub >= 0 && o->use_cuda_graph && !prof_on() && o->spin_limit >= kSpinLimitDefault &&
-                      (double)g->hub_degree > kCcSkew * std::max(1.0, (double)g->edges / (double)V);
-  std::optional<LoopRun> run;
   int32_t *depth = g->ws.gather_tmp;
   if (by_bfs) {
-    run.emplace(g, s);
     mg_options bo;
     mg_options_init(&bo);
     st = bfs_loop_run(*run, g, s, {g->hub}, kCcLevels, &bo, depth, false);

@@ -19,7 +19,24 @@ thread_local LoopTest loop_test;
 
 }  // namespace
 
-LoopRun::LoopRun(mg_graph *g, cudaStream_t s) : g_(g), s_(s), turn_(loop_mutex(g->device)) {}
+// Waits for the work in a caller's stream. (An error of that work comes back from the
+// launch.)
+static void drain(mg_graph *g, cudaStream_t s) {
+  unsigned flags = 0;
+  if (cudaStreamGetFlags(s, &flags) == cudaSuccess && (flags & cudaStreamNonBlocking)) {
+    if (cudaStreamQuery(s) != cudaSuccess) {
+      cudaGetLastError();  // not ready
+      cudaStreamSynchronize(s);
+    }
+  } else if (cudaEventRecord(g->ev0, s) == cudaSuccess) {
+    cudaEventSynchronize(g->ev0);  // with the default stream's work, which a launch would wait for
+  }
+}
+
+LoopRun::LoopRun(mg_graph *g, cudaStream_t s) : g_(g), s_(s), turn_(loop_mutex(g->device), std::defer_lock) {
+  if (s != g->stream) drain(g, s);  // the graph's own stream holds nothing that waits for anyone
+  turn_.lock();
+}
 
 LoopRun::~LoopRun() { settle(nullptr); }
 

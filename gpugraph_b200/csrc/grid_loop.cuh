@@ -110,7 +110,9 @@ constexpr int kLoopRefused = -1;
 // One run of a loop kernel: the GPU's turn is held from here until the run's stream
 // was synchronised (two loops launched by different threads would each wait for SMs
 // the other one holds), by finish() or, when a call leaves in between with an error,
-// by the destructor: the arrivals of every run are accounted for.
+// by the destructor: the arrivals of every run are accounted for. What the caller's
+// stream still has to do is waited for first: the turn is held for the run alone, not
+// for work that may take long or depend on another thread's call.
 class LoopRun {
  public:
   LoopRun(mg_graph *g, cudaStream_t s);

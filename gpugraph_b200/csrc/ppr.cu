@@ -28,6 +28,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <optional>
 #include <vector>
 
 #include "algo_util.cuh"
@@ -505,9 +506,8 @@ static bool is_device_ptr(const void *p) {
 // 12 columns 6.54 / 6.90).
 constexpr int64_t kPprLoopWork = 1ll << 24;
 
-static int ppr_one_launch(mg_graph *g, cudaStream_t s, PprArgs a, uint32_t max_iter, const mg_options *o,
-                          const char *name, LoopResult *res) {
-  LoopRun run(g, s);
+static int ppr_one_launch(LoopRun &run, mg_graph *g, PprArgs a, uint32_t max_iter, const mg_options *o, const char *name,
+                          LoopResult *res) {
   GridLoop loop = run.args(o);
   double tol = o->tolerance;
   void *args[] = {&a, &tol, &max_iter, &loop};
@@ -539,6 +539,11 @@ static int ppr_solve(mg_graph *g, int dir, const float *w, const float *rhs, flo
   // from the graph's own buffers, so callers may pass different pointers.
   const int32_t nv = ppr_stride(nvec);
   const int64_t n = (int64_t)g->nodes * nv;
+  // Short iterations: one launch. The level loop serves the rest, the host-driven
+  // runs and callers that shorten the waits.
+  std::optional<LoopRun> run;
+  if (o->use_cuda_graph && !prof_on() && o->spin_limit >= kSpinLimitDefault && (g->nodes + g->edges) * nv <= kPprLoopWork)
+    run.emplace(g, s);
   k_rows_f32<<<g->num_sms * 8, 256, 0, s>>>(rhs, nvec, g->ppr_rhs, nv, 1.0f, g->nodes);
   // the weights in the order the solve reads its adjacency (CSC order for the
   // forward pull, so no edge-id indirection per edge and iteration)
@@ -572,10 +577,8 @@ static int ppr_solve(mg_graph *g, int dir, const float *w, const float *rhs, flo
   k_copy_f32<<<g->num_sms * 4, 256, 0, s>>>(rhs, a.x0, n);
   count_launch();
   const uint32_t max_iter = (uint32_t)std::max<int32_t>(0, std::min<int32_t>(o->iter_num, 100000));
-  // Short iterations: one launch. The level loop serves the rest, the host-driven
-  // runs and callers that shorten the waits.
-  if (o->use_cuda_graph && !prof_on() && o->spin_limit >= kSpinLimitDefault && (g->nodes + g->edges) * nv <= kPprLoopWork) {
-    const int st = ppr_one_launch(g, s, a, max_iter, o, name, res);
+  if (run) {
+    const int st = ppr_one_launch(*run, g, a, max_iter, o, name, res);
     *result = (res->ctl.level & 1) ? a.x1 : a.x0;
     if (st != kLoopRefused) return st;
   }

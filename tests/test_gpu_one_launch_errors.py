@@ -1,5 +1,9 @@
 """The calls that run in one cooperative launch, when something goes wrong on the way: the status they return, and
 that the next call on the same graph is exact. The failures are made on the host; nothing faults or hangs."""
+import ctypes as C
+import threading
+import time
+
 import numpy as np
 import pytest
 
@@ -112,3 +116,29 @@ def test_refused_launch_runs_level_by_level(name, calls):
         _lib.lib.mg_selftest_loops(_lib.MG_LOOP_TEST_OFF)
         assert calls[name]()
         _lib.lib.mg_kernel_launches(1)
+
+
+def test_call_behind_unfinished_work_does_not_hold_up_other_threads(calls):
+    # thread A's call is queued on a stream whose host function waits until this thread's calls have returned
+    torch = pytest.importorskip("torch")
+    hg = HostGraph.rmat(11, 8, seed=3)
+    g, ref = Graph(hg), oracle.bfs(hg.row_offsets, hg.column_indices, 1)
+    assert np.array_equal(g.bfs(1)[0], ref)
+    stream, release, released, out = torch.cuda.Stream(), threading.Event(), [], []
+
+    @C.CFUNCTYPE(None, C.c_void_p)
+    def wait(_):
+        released.append(release.wait(20))
+
+    launch = C.CDLL("libcudart.so.12").cudaLaunchHostFunc
+    launch.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p]
+    assert launch(stream.cuda_stream, C.cast(wait, C.c_void_p), None) == 0
+    t = threading.Thread(target=lambda: out.append(g.bfs(1, stream=stream.cuda_stream)[0]))
+    t.start()
+    time.sleep(0.5)
+    for name in NAMES:
+        assert calls[name](), name
+    assert not out
+    release.set()
+    t.join(30)
+    assert released == [True] and np.array_equal(out[0], ref)
