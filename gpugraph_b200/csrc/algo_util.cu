@@ -15,7 +15,7 @@ int copy_out(cudaStream_t s, void *dst, const void *src, size_t bytes, bool dst_
 
 bool on_device(const mg_graph *g, const void *p) {
   cudaPointerAttributes at;
-  if (!p || cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+  if (!p || (uintptr_t)p % 4 || cudaPointerGetAttributes(&at, p) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }

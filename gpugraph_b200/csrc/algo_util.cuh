@@ -16,7 +16,8 @@ namespace mg {
 // and waits for it.
 int copy_out(cudaStream_t s, void *dst, const void *src, size_t bytes, bool dst_on_device);
 
-// True for memory of the graph's own GPU, which a kernel may use as its working array.
+// True for memory of the graph's own GPU at a 4-byte boundary, which a kernel may use
+// as its working array. (A copy takes any other device pointer: another GPU's, an odd one.)
 bool on_device(const mg_graph *g, const void *p);
 
 // True when every weight is in [0, INT_MAX - 100000000]: then no sum of an SSSP distance

@@ -662,8 +662,13 @@ int mg_ppr_forward(mg_graph *g, const float *edge_weights, const float *teleport
   ppr_stats(stats, res, o->tolerance, g);
   const int32_t nv = ppr_stride(nvec);
   if (nv == nvec) return copy_out(s, ranks, x, (size_t)g->nodes * nvec * 4, true);
-  k_rows_f32<<<g->num_sms * 8, 256, 0, s>>>(x, nv, ranks, nvec, 1.0f, g->nodes);
+  // into the other iterate's buffer when a kernel cannot write `ranks`
+  const bool direct = on_device(g, ranks);
+  float *out = direct ? ranks : x == g->ppr_x[0] ? g->ppr_x[1] : g->ppr_x[0];
+  k_rows_f32<<<g->num_sms * 8, 256, 0, s>>>(x, nv, out, nvec, 1.0f, g->nodes);
   count_launch();
+  if ((st = launch_check("ppr forward")) != MG_OK) return st;
+  if (!direct) return copy_out(s, ranks, out, (size_t)g->nodes * nvec * 4, true);
   return cuda_status(cudaStreamSynchronize(s), "ppr forward");
 }
 

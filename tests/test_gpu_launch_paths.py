@@ -393,3 +393,45 @@ def test_sssp_weights_whose_sums_wrap(nsrc):
     for mode in ({}, dict(use_cuda_graph=0)):
         one, st = g.sssp(int(srcs[0]), **mode)
         assert np.array_equal(one[:-1], ref[:, 0]) and st["converged"] == 1
+
+
+@pytest.mark.parametrize("shift", [0, 1, 2, 4])
+def test_device_results_at_any_address(shift):
+    # a kernel writes a device buffer itself where it is aligned; at an odd address the result is copied there
+    torch = pytest.importorskip("torch")
+    import ctypes as C
+
+    from gpugraph_b200.ppr import ppr
+
+    lib = _lib.lib
+    hg = HostGraph.rmat(10, 8, seed=3).with_weights(1, 64, seed=1)
+    hd = HostGraph.rmat(9, 8, seed=5, symmetrize=False)
+    g, gd = Graph(hg), Graph(hd, directed=True)
+    s, opts = hg.max_degree_vertex(), _lib.default_options(outputs_on_device=1)
+    w = torch.tensor(1.0 / np.repeat(np.maximum(hd.out_degree(), 1), hd.out_degree()), dtype=torch.float32,
+                     device="cuda")
+
+    def result(call, n, dtype):
+        buf = torch.full((4 * n + 8,), 0x55, dtype=torch.uint8, device="cuda")
+        torch.cuda.synchronize()
+        _lib.check(call(buf.data_ptr() + shift), "call")
+        h = buf.cpu().numpy()
+        assert (h[:shift] == 0x55).all() and (h[shift + 4 * n:] == 0x55).all()
+        return h[shift:shift + 4 * n].copy().view(dtype)
+
+    o = C.byref(opts)
+    n, nd = hg.nodes, hd.nodes
+    ref = oracle.bfs(hg.row_offsets, hg.column_indices, s)
+    assert np.array_equal(result(lambda p: lib.mg_bfs(g.handle, s, p, None, o), n, np.int32), ref)
+    assert np.array_equal(result(lambda p: lib.mg_sssp(g.handle, s, p, None, o), n, np.int32), g.sssp(s)[0])
+    assert np.array_equal(result(lambda p: lib.mg_cc(g.handle, p, None, o), n, np.int32), g.cc()[0])
+    rank = result(lambda p: lib.mg_pagerank(gd.handle, p, None, o), nd, np.float32)
+    assert np.abs(rank - gd.pagerank(iter_num=opts.iter_num)[0]).sum() < 1e-6
+    opts.tolerance = 1e-7
+    for nvec in (3, 4):
+        tele = torch.zeros((nd, nvec), device="cuda")
+        tele[::5] = 5.0 / nd
+        torch.cuda.synchronize()
+        r = result(lambda p: lib.mg_ppr_forward(gd.handle, w.data_ptr(), tele.data_ptr(), nvec, p, None, o), nd * nvec,
+                   np.float32).reshape(nd, nvec)
+        assert np.abs(r - ppr(gd, w, tele, max_iter=opts.iter_num).cpu().numpy()).max() < 1e-7
