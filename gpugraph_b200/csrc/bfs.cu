@@ -527,9 +527,11 @@ int bfs_run(mg_graph *g, const std::vector<int32_t> &roots, int32_t *depths, mg_
   // the device loop even if a Program never empties its frontier.
   const uint32_t max_iter = (uint32_t)std::min<int64_t>(o->iter_num > 0 ? o->iter_num : 0, g->nodes + 2);
   // Default: one launch. The level-by-level loop below serves the host-driven
-  // runs (use_cuda_graph = 0, profiling), the ordered frontier and callers that
-  // shorten the waits (a grid barrier waits for the slowest CTA of a level).
+  // runs (use_cuda_graph = 0, profiling), the ordered frontier, graphs with an
+  // in-list too long to pull within a barrier's wait, and callers that shorten the
+  // waits (a grid barrier waits for the slowest CTA of a level).
   if (o->use_cuda_graph && !o->ordered_frontier && !prof_on() && o->spin_limit >= kSpinLimitDefault &&
+      (o->direction == MG_DIR_PUSH || g->hub_degree <= kLoopPullList) &&
       (st = bfs_one_launch(g, s, roots, max_iter, depths, stats, o, preds)) != kLoopRefused)
     return st;
   if ((st = prepare_run(g, s)) != MG_OK) return st;

@@ -269,6 +269,7 @@ int cc_union_find(mg_graph *g, int32_t *labels, mg_stats *stats, const mg_option
   int32_t *parent = g->ws.vbuf[0];
   Ctl *ctl = g->ws.ctl;
   bool by_bfs = g->hub >= 0 && o->use_cuda_graph && !prof_on() && o->spin_limit >= kSpinLimitDefault &&
+                g->hub_degree <= kLoopPullList &&
                 (double)g->hub_degree > kCcSkew * std::max(1.0, (double)g->edges / (double)V);
   std::optional<LoopRun> run;
   if (by_bfs) run.emplace(g, s);

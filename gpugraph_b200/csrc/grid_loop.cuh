@@ -19,6 +19,11 @@ namespace mg {
 
 constexpr int kLoopNT = 1024;  // one CTA per SM: the fewest arrivals a barrier can have
 constexpr int kRange = 256;    // edges per entry of a queue of edge ranges
+// In-edges of a vertex up to which k_bfs_loop may pull it: one lane walks the list, four
+// edges per two dependent loads (about 1.2 us), while every other CTA polls at the
+// barrier, 2^22 times (2 to 3 s) by default. 2^20 edges take 0.3 s. Longer lists are left
+// to the level loop, whose kernels have no time limit.
+constexpr int32_t kLoopPullList = 1 << 20;
 
 // Device state of a loop. `arrived` grows for the life of the graph (a run
 // starts from the value the host passes in); the totals rotate over three
