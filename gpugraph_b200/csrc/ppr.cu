@@ -55,7 +55,9 @@ struct PprArgs {
   float alpha, d;                  // X' = alpha*rhs + d*sum(...)
   float *x0, *x1, *partial;
   const int32_t *cv, *cb, *ce, *cslot, *mv, *mfirst;
-  int32_t nchunks, nfull, nmulti, nv, V;  // nfull: chunks that have edges (they come first)
+  // nfull: chunks that have edges (they come first); columns [nvec, nv) are padding and
+  // stay 0 (their sums may not: 0 times an infinite weight), so they add nothing to a residual
+  int32_t nchunks, nfull, nmulti, nvec, nv, V;
   Ctl *ctl;
 };
 
@@ -68,7 +70,7 @@ MG_DEVINL void ppr_finalize_row(const PprArgs &a, int v, const float (&acc)[NC],
     const int c = lane + 32 * q;
     if (c < a.nv) {
       const int64_t o = (int64_t)v * a.nv + c;
-      const float xn = fmaf(a.d, acc[q], a.alpha * a.rhs[o]);
+      const float xn = c < a.nvec ? fmaf(a.d, acc[q], a.alpha * a.rhs[o]) : 0.f;
       res += (double)fabsf(xn - xold[o]);
       xnew[o] = xn;
     }
@@ -166,6 +168,9 @@ MG_DEVINL void ppr_sweep(const PprArgs &a, uint32_t L, uint32_t gw, uint32_t nw,
       xn.y = fmaf(a.d, acc.y, a.alpha * r.y);
       xn.z = fmaf(a.d, acc.z, a.alpha * r.z);
       xn.w = fmaf(a.d, acc.w, a.alpha * r.w);
+      if (col + 1 >= a.nvec) xn.y = 0.f;
+      if (col + 2 >= a.nvec) xn.z = 0.f;
+      if (col + 3 >= a.nvec) xn.w = 0.f;
       res += (double)fabsf(xn.x - xo.x) + (double)fabsf(xn.y - xo.y) + (double)fabsf(xn.z - xo.z) +
              (double)fabsf(xn.w - xo.w);
       *reinterpret_cast<float4 *>(xnew + o) = xn;
@@ -570,6 +575,7 @@ static int ppr_solve(mg_graph *g, int dir, const float *w, const float *rhs, flo
   a.nchunks = p.nchunks;
   a.nfull = p.nfull;
   a.nmulti = p.nmulti;
+  a.nvec = nvec;
   a.nv = nv;
   a.V = g->csr.V;
   a.ctl = g->ws.ctl;
@@ -601,7 +607,7 @@ static int ppr_solve(mg_graph *g, int dir, const float *w, const float *rhs, flo
   };
   char key[160];
   // (ppr_cap_nvec: a wider solve replaced the buffers the cached graph's arguments point to)
-  snprintf(key, sizeof(key), "%s/%d/%d/%d/%.9g/%.17g/%.17g", name, grid, nv, g->ppr_cap_nvec, (double)alpha, o->damping,
+  snprintf(key, sizeof(key), "%s/%d/%d/%d/%.9g/%.17g/%.17g", name, grid, nvec, g->ppr_cap_nvec, (double)alpha, o->damping,
            tol);
   int st = run_level_loop(g, s, key, 3, body, o->use_cuda_graph != 0, res);
   if (st != MG_OK) return st;

@@ -452,3 +452,37 @@ def test_bfs_in_list_too_long_for_a_barrier_wait(leaves):
         assert (_lib.lib.mg_kernel_launches(1) == 1) == one, d
         assert np.array_equal(out, ref)
     assert not g.cc()[0].any()
+
+
+@pytest.mark.parametrize("mode", [{}, dict(use_cuda_graph=0)])
+@pytest.mark.parametrize("nvec", [1, 2, 3, 7, 33])
+def test_ppr_infinite_weight_in_padded_rows(nvec, mode):
+    # an infinite weight makes its head's ranks infinite, and the solve stops when the change is no longer a number.
+    # The padding columns of a row (0 times that weight) must not stop it earlier: a solve whose last columns repeat
+    # up to a full row runs as many iterations and gives the same columns
+    torch = pytest.importorskip("torch")
+    import ctypes as C
+
+    hd = HostGraph.rmat(9, 8, seed=5, symmetrize=False)
+    g = Graph(hd, directed=True)
+    w = 1.0 / np.repeat(np.maximum(hd.out_degree(), 1), hd.out_degree())
+    w[hd.row_offsets[hd.max_degree_vertex()]] = np.inf
+    w = torch.tensor(w, dtype=torch.float32, device="cuda")
+    full = torch.rand((hd.nodes, nvec), device="cuda", generator=torch.Generator("cuda").manual_seed(1)) + 0.1
+    full = torch.cat([full, full[:, -1:].expand(-1, -nvec % 4)], 1)
+    got = []
+    for k in (nvec, full.shape[1]):
+        t = full[:, :k].contiguous()
+        r, gt, gw = torch.empty_like(t), torch.empty_like(t), torch.empty_like(w)
+        st, o = _lib.Stats(), _lib.default_options(tolerance=1e-7, iter_num=50, **mode)
+        torch.cuda.synchronize()
+        _lib.check(_lib.lib.mg_ppr_forward(g.handle, w.data_ptr(), t.data_ptr(), k, r.data_ptr(), C.byref(st),
+                                           C.byref(o)), "forward")
+        it = st.iterations
+        _lib.check(_lib.lib.mg_ppr_backward(g.handle, w.data_ptr(), r.data_ptr(), t.data_ptr(), k, gw.data_ptr(),
+                                            gt.data_ptr(), C.byref(st), C.byref(o)), "backward")
+        got.append((it, st.iterations, r[:, :nvec].cpu().numpy(), gt[:, :nvec].cpu().numpy()))
+    assert got[0][:2] == got[1][:2] and got[0][0] >= 2
+    assert np.isinf(got[0][2]).any()
+    assert np.array_equal(got[0][2], got[1][2], equal_nan=True)
+    assert np.array_equal(got[0][3], got[1][3], equal_nan=True)
