@@ -21,6 +21,15 @@ from . import _lib
 from ._lib import check, default_options, lib
 
 
+def _stream() -> int:
+    """torch's current stream. The default stream's handle, 0, stands for the graph's own stream, which is not
+    ordered after it: what torch has queued there (the inputs' producers) is waited for."""
+    s = torch.cuda.current_stream()
+    if s.cuda_stream == 0:
+        s.synchronize()
+    return s.cuda_stream
+
+
 class _PPR(torch.autograd.Function):
     @staticmethod
     def forward(ctx, edge_weights, teleport, graph, damping, tol, max_iter, extra):
@@ -33,7 +42,7 @@ class _PPR(torch.autograd.Function):
         nvec = int(t.shape[1])
         out = torch.empty_like(t)
         o = default_options(damping=damping, tolerance=tol, iter_num=max_iter,
-                            stream=torch.cuda.current_stream().cuda_stream, **extra)
+                            stream=_stream(), **extra)
         st = _lib.Stats()
         check(lib.mg_ppr_forward(graph.handle, w.data_ptr(), t.data_ptr(), nvec, out.data_ptr(), C.byref(st),
                                  C.byref(o)), "mg_ppr_forward")
@@ -51,7 +60,7 @@ class _PPR(torch.autograd.Function):
         gw = torch.empty_like(w) if need_w else None
         gt = torch.empty_like(R) if need_t else None
         o = default_options(damping=ctx.damping, tolerance=ctx.tol, iter_num=ctx.max_iter,
-                            stream=torch.cuda.current_stream().cuda_stream, **ctx.extra)
+                            stream=_stream(), **ctx.extra)
         st = _lib.Stats()
         check(lib.mg_ppr_backward(ctx.graph.handle, w.data_ptr(), R.data_ptr(), g.data_ptr(), nvec,
                                   gw.data_ptr() if gw is not None else None,

@@ -136,3 +136,27 @@ def test_ppr_rejects_symmetric_graph_and_host_pointers():
     gd = Graph(HostGraph.rmat(8, 4, seed=1, symmetrize=False), directed=True)
     with pytest.raises(TypeError):
         ppr(gd, torch.ones(gd.edges), torch.ones((gd.nodes, 4)))
+
+
+@pytest.mark.parametrize("side", [False, True])
+def test_ppr_inputs_still_being_produced(side):
+    # the inputs of both passes are written by work that torch has only queued, on its default stream or another one
+    from gpugraph_b200.ppr import ppr
+
+    hg, g, src, w, T, C = _setup(scale=9, nvec=5)
+    wt, tt, ct = (torch.tensor(x, dtype=torch.float32, device="cuda") for x in (w, T, C))
+
+    def step(delay):
+        w0, t0 = torch.zeros_like(wt).requires_grad_(True), torch.zeros_like(tt).requires_grad_(True)
+        torch.cuda.synchronize()
+        torch.cuda._sleep(delay)
+        r = ppr(g, w0 + wt, t0 + tt)
+        torch.cuda._sleep(delay)
+        return (r.detach(), *torch.autograd.grad((r * ct).sum(), (w0, t0)))
+
+    stream = torch.cuda.Stream() if side else torch.cuda.current_stream()
+    with torch.cuda.stream(stream):
+        ready, late = step(0), step(40_000_000)  # nothing in front, and 20 ms
+        torch.cuda.synchronize()
+    for a, b in zip(late, ready):
+        assert a.abs().sum() > 0 and (a - b).norm() <= 1e-5 * b.norm()
