@@ -10,6 +10,11 @@
 // BFS), then the pull->push factor (beta); for PageRank and PPR, the CTAs per
 // SM of their SpMV over a fixed number of iterations. The best options are
 // written back to *inout; a JSON report of every trial goes to report (if given).
+//
+// Only the level-by-level loops read the launch geometry (tile, CTAs per SM), so
+// those trials run there, whatever loop the call takes by itself ("loop":"level" in
+// the report); alpha and beta are tried on the loop that the call takes ("call"),
+// and best_ms is that of the call with the chosen options.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -26,6 +31,7 @@ namespace {
 struct Trial {
   mg_options o;
   double ms;
+  bool level;  // run level by level
 };
 
 // Inputs of the PPR trials: row-normalised uniform weights and one-hot teleport
@@ -128,9 +134,12 @@ extern "C" int mg_autotune(mg_graph *g, int32_t kind, const int32_t *srcs, int32
     base.tolerance = 0.0;
   }
   std::vector<Trial> trials;
-  auto eval = [&](const mg_options &o, double *ms) -> int {
-    int rc = measure(g, kind, srcs, nsrc, o, out, pi, ms);
-    if (rc == MG_OK) trials.push_back({o, *ms});
+  auto eval = [&](const mg_options &o, bool level, double *ms) -> int {
+    mg_options run = o;
+    // a shortened wait chooses the level loop (no wait comes near the limit)
+    if (level) run.spin_limit = std::min<int64_t>(run.spin_limit, kSpinLimitDefault - 1);
+    int rc = measure(g, kind, srcs, nsrc, run, out, pi, ms);
+    if (rc == MG_OK) trials.push_back({o, *ms, level});
     return rc;
   };
   mg_options best = base;
@@ -142,7 +151,7 @@ extern "C" int mg_autotune(mg_graph *g, int32_t kind, const int32_t *srcs, int32
       mg_options o = best;
       o.ctas_per_sm = cps;
       double ms;
-      if ((rc = eval(o, &ms)) != MG_OK) break;
+      if ((rc = eval(o, true, &ms)) != MG_OK) break;
       if (ms < best_ms) best_ms = ms, best = o;
     }
   }
@@ -154,11 +163,13 @@ extern "C" int mg_autotune(mg_graph *g, int32_t kind, const int32_t *srcs, int32
       o.tile_items = tile;
       o.ctas_per_sm = cps;
       double ms;
-      if ((rc = eval(o, &ms)) != MG_OK) break;
+      if ((rc = eval(o, true, &ms)) != MG_OK) break;
       if (ms < best_ms) best_ms = ms, best = o;
     }
     if (rc != MG_OK) break;
   }
+  // the call itself from here on
+  if (rc == MG_OK) rc = measure(g, kind, srcs, nsrc, best, out, pi, &best_ms);
   // 2) push -> pull factor, 3) pull -> push factor (traversals with direction switching)
   if (rc == MG_OK && (kind == MG_TUNE_BFS || kind == MG_TUNE_BFS_MULTI)) {
     const std::vector<double> alphas = kind == MG_TUNE_BFS ? std::vector<double>{5, 10, 15, 25, 40}
@@ -168,7 +179,7 @@ extern "C" int mg_autotune(mg_graph *g, int32_t kind, const int32_t *srcs, int32
       mg_options o = cur;
       (kind == MG_TUNE_BFS ? o.alpha : o.alpha_multi) = a;
       double ms;
-      if ((rc = eval(o, &ms)) != MG_OK) break;
+      if ((rc = eval(o, false, &ms)) != MG_OK) break;
       if (ms < best_ms) best_ms = ms, best = o;
     }
     cur = best;
@@ -177,7 +188,7 @@ extern "C" int mg_autotune(mg_graph *g, int32_t kind, const int32_t *srcs, int32
       mg_options o = cur;
       o.beta = b;
       double ms;
-      if ((rc = eval(o, &ms)) != MG_OK) break;
+      if ((rc = eval(o, false, &ms)) != MG_OK) break;
       if (ms < best_ms) best_ms = ms, best = o;
     }
   }
@@ -195,8 +206,9 @@ extern "C" int mg_autotune(mg_graph *g, int32_t kind, const int32_t *srcs, int32
     for (size_t i = 0; i < trials.size(); ++i) {
       char buf[256];
       snprintf(buf, sizeof(buf),
-               "%s{\"tile_items\":%d,\"ctas_per_sm\":%d,\"alpha\":%g,\"alpha_multi\":%g,\"beta\":%g,\"ms\":%.5f}",
-               i ? "," : "", trials[i].o.tile_items, trials[i].o.ctas_per_sm, trials[i].o.alpha,
+               "%s{\"loop\":\"%s\",\"tile_items\":%d,\"ctas_per_sm\":%d,\"alpha\":%g,\"alpha_multi\":%g,\"beta\":%g,"
+               "\"ms\":%.5f}",
+               i ? "," : "", trials[i].level ? "level" : "call", trials[i].o.tile_items, trials[i].o.ctas_per_sm, trials[i].o.alpha,
                trials[i].o.alpha_multi, trials[i].o.beta, trials[i].ms);
       js += buf;
     }

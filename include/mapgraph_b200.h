@@ -252,7 +252,9 @@ enum { MG_TUNE_BFS = 0, MG_TUNE_BFS_MULTI = 1, MG_TUNE_SSSP = 2, MG_TUNE_CC = 3,
  * MG_TUNE_PAGERANK (mg_pagerank) and MG_TUNE_PPR (mg_ppr_forward) search
  * ctas_per_sm of their SpMV (2..8), timing a fixed number of iterations; PPR
  * solves nsrc teleport columns, one-hot at srcs, over row-normalised uniform
- * weights (the launch shape does not depend on the values).
+ * weights (the launch shape does not depend on the values). tile_items and
+ * ctas_per_sm are read by the level-by-level loops alone and tried there; alpha and
+ * beta are tried on the loop that the call takes.
  * *inout is the starting point and receives the best options; report (may be
  * NULL) receives a JSON record of every trial. srcs: 1..64 sources (unused for
  * MG_TUNE_CC and MG_TUNE_PAGERANK). */

@@ -57,3 +57,22 @@ def test_autotune_pagerank_and_ppr():
     a = ppr(g, wt, Tt)
     b = ppr(g, wt, Tt, ctas_per_sm=best_p["ctas_per_sm"])
     assert torch.allclose(a, b, atol=1e-6)
+
+
+def test_geometry_is_tried_on_the_loop_that_reads_it():
+    # a road grid: many short levels, so the level loop's trials take several times as long as the one-launch call
+    hg = HostGraph.road_grid(200, 0.02, 0.0, seed=3).with_weights(1, 64, seed=2)
+    g = Graph(hg)
+    s = np.array([0, 777], np.int32)
+    for kind, srcs in (("bfs", s), ("sssp", s), ("bfs_multi", s)):
+        best, report = autotune(g, kind, srcs)
+        level = [t for t in report["trials"] if t["loop"] == "level"]
+        call = [t for t in report["trials"] if t["loop"] == "call"]
+        assert len(level) == 8 and len({(t["tile_items"], t["ctas_per_sm"]) for t in level}) == 8
+        assert len(call) == (0 if kind == "sssp" else 9)
+        first = min(level, key=lambda t: t["ms"])
+        assert (best["tile_items"], best["ctas_per_sm"]) == (first["tile_items"], first["ctas_per_sm"])
+        assert report["best_ms"] < 0.7 * first["ms"], kind
+        assert all(report["best_ms"] <= t["ms"] + 1e-5 for t in call)  # (the trials are printed to 1e-5)
+    best, report = autotune(Graph(HostGraph.rmat(10, 8, seed=5, symmetrize=False), directed=True), "pagerank")
+    assert all(t["loop"] == "level" for t in report["trials"])
