@@ -22,7 +22,7 @@
 // linked from its other end, which is not in it; on power-law graphs step 4
 // touches a small share of the edges.
 //
-// On a skewed graph (kCcSkew) the links of steps 1 and 2 queue up on a few roots
+// On a skewed graph (kCcLongShare) the links of steps 1 and 2 queue up on a few roots
 // (sampling alone took 340 us at R-MAT 21). There a one-launch BFS from the hub,
 // of at most kCcLevels levels, finds the large component instead: what it
 // reached starts under its smallest id, every other vertex links all its edges
@@ -31,7 +31,6 @@
 // R-MAT 22: 1.61 -> 0.31 ms.
 #include <cuda_runtime.h>
 
-#include <algorithm>
 #include <climits>
 #include <optional>
 #include <vector>
@@ -256,7 +255,13 @@ __global__ void __launch_bounds__(kNT) k_cc_seed(const int32_t *depth, int32_t V
   add_bytes(ctl, KID_CC, my_bytes);
 }
 
-constexpr double kCcSkew = 8.0;      // longest list over the mean from which the BFS finds the large component
+// Share of the edges in long lists (kLongList) from which the BFS finds the large
+// component: R-MAT graphs have 0.15 (scale 10) to 0.65, and the hub is in their large
+// component. A hub alone says nothing about the rest: from a vertex of 200 leaves beside
+// a 4000x4000 lattice 16 levels reach little, and the rest's hooks without the sampling
+// took 1.64 ms a run, 1.09 with it. (Sparse R-MAT 21 graphs, one or two edges drawn a
+// vertex, with / without the BFS: 175 / 306, 167 / 483 us.)
+constexpr double kCcLongShare = 0.1;
 constexpr uint32_t kCcLevels = 16;
 
 // Union-find CC on a symmetric graph (called by mg_cc).
@@ -270,7 +275,7 @@ int cc_union_find(mg_graph *g, int32_t *labels, mg_stats *stats, const mg_option
   Ctl *ctl = g->ws.ctl;
   bool by_bfs = g->hub >= 0 && o->use_cuda_graph && !prof_on() && o->spin_limit >= kSpinLimitDefault &&
                 g->hub_degree <= kLoopPullList &&
-                (double)g->hub_degree > kCcSkew * std::max(1.0, (double)g->edges / (double)V);
+                (double)g->long_list_edges > kCcLongShare * (double)g->edges;
   std::optional<LoopRun> run;
   if (by_bfs) run.emplace(g, s);
   cudaError_t e = cudaEventRecord(g->ev0, s);

@@ -8,6 +8,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cstring>
+#include <mutex>
 #include <vector>
 
 #include "graph.cuh"
@@ -126,13 +127,26 @@ using namespace mg;
 
 namespace {
 
-// The vertex with the longest in-list (the first of them) and its length.
+// The vertex with the longest in-list (the first of them) and its length, and the
+// edges in lists of more than kLongList times the mean.
 void find_hub(mg_graph *g, const int32_t *in_off) {
-  for (int64_t v = 0; v < g->nodes; ++v)
-    if (g->hub < 0 || in_off[v + 1] - in_off[v] > g->hub_degree) {
-      g->hub = (int32_t)v;
-      g->hub_degree = in_off[v + 1] - in_off[v];
+  const double lim = kLongList * std::max(1.0, (double)g->edges / (double)std::max<int64_t>(g->nodes, 1));
+  std::mutex m;
+  host_parallel_for(g->nodes, [&](int64_t b, int64_t e, unsigned) {
+    int64_t hub = b, in_long = 0;
+    auto len = [&](int64_t v) { return in_off[v + 1] - in_off[v]; };
+    for (int64_t v = b; v < e; ++v) {
+      if (len(v) > len(hub)) hub = v;
+      if ((double)len(v) > lim) in_long += len(v);
     }
+    if (b >= e) return;
+    std::lock_guard<std::mutex> lock(m);
+    g->long_list_edges += in_long;
+    if (g->hub < 0 || len(hub) > g->hub_degree || (len(hub) == g->hub_degree && hub < g->hub)) {
+      g->hub = (int32_t)hub;
+      g->hub_degree = len(hub);
+    }
+  });
 }
 
 // Copy of the in-lists with every list ordered by descending out-degree of the

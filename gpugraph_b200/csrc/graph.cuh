@@ -37,6 +37,9 @@ constexpr int32_t kMsHeavyList = 512;
 // many times the mean.
 constexpr double kMssSkew = 64.0;
 
+// An in-list is long from this many times the mean on (mg_graph::long_list_edges).
+constexpr double kLongList = 8.0;
+
 struct DevCsr {
   int32_t *row_offsets = nullptr;
   int32_t *col = nullptr;
@@ -96,6 +99,7 @@ struct mg_graph {
   int64_t edges = 0;
   mg::DevCsr csr;
   int32_t hub = -1, hub_degree = 0;    // the vertex with the longest in-list
+  int64_t long_list_edges = 0;         // edges in in-lists over kLongList times the mean
   std::vector<int64_t> graph_offsets;  // batch of graphs: first vertex of each graph
   mg::Workspace ws;
   float *inv_outdeg = nullptr;          // PageRank 1/outdeg (0 for dangling vertices)

@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 
 import oracle
-from gpugraph_b200 import Graph, HostGraph, _lib
+from gpugraph_b200 import Graph, HostGraph, MapGraphError, _lib
 
 pytestmark = pytest.mark.gpu
 
@@ -486,3 +486,29 @@ def test_ppr_infinite_weight_in_padded_rows(nvec, mode):
     assert np.isinf(got[0][2]).any()
     assert np.array_equal(got[0][2], got[1][2], equal_nan=True)
     assert np.array_equal(got[0][3], got[1][3], equal_nan=True)
+
+
+@pytest.mark.parametrize("leaves,by_bfs", [(200, False), (40000, True)])
+def test_cc_hub_beside_a_lattice(leaves, by_bfs):
+    # a hub whose edges are few beside the lattice's says nothing about the large component (sampling rounds); one
+    # with a tenth of them is found by the BFS
+    grid = HostGraph.road_grid(150, 0.3, 0.0, seed=5)
+    n = grid.nodes
+    a, b = np.zeros(leaves, np.int64), n + np.arange(leaves)
+    src = np.concatenate([np.repeat(np.arange(n), np.diff(grid.row_offsets)), a, b])
+    dst = np.concatenate([grid.column_indices, b, a])
+    order = np.lexsort((dst, src))
+    ro = np.concatenate([[0], np.cumsum(np.bincount(src, minlength=n + leaves))]).astype(np.int32)
+    g = Graph(HostGraph(ro, dst[order].astype(np.int32)))
+    ref, _ = g.cc(generic_engine=1)
+    assert np.array_equal(g.cc()[0], ref)
+    _lib.lib.mg_selftest_loops(_lib.MG_LOOP_TEST_WAITS)  # the BFS's barriers give up; the sampling has none
+    try:
+        if by_bfs:
+            with pytest.raises(MapGraphError):
+                g.cc()
+        else:
+            assert np.array_equal(g.cc()[0], ref)
+    finally:
+        _lib.lib.mg_selftest_loops(_lib.MG_LOOP_TEST_OFF)
+    assert np.array_equal(g.cc()[0], ref)
