@@ -11,8 +11,8 @@
 // Graph Connectivity Computation via Subgraph Sampling", IPDPS 2018, with its
 // first round done without atomics: hanging every vertex under a smaller
 // neighbour, which only its own thread writes, is a valid forest):
-//   1. every vertex starts under its first neighbour if that is smaller, else
-//      as a root;
+//   1. every vertex starts under its first neighbour if that is smaller (but for
+//      one in eight, kCcBreak), else as a root;
 //   2. every vertex links with its second neighbour, a root of step 1 with its
 //      first as well; the trees are flattened;
 //   3. the most frequent root among kCcProbe fixed sample vertices names the
@@ -80,7 +80,10 @@ MG_DEVINL bool cc_unite(int32_t *parent, int32_t a, int32_t b, unsigned long lon
 // distinct larger root: the lane with the smallest other root hooks it, the
 // lanes that hold the same larger root go on to join their other root with that
 // one. Neighbouring vertices of a grid hang under the same few roots, and their
-// hooks would queue up on one address (1200x1200 road grid: 335 instead of 430 us).
+// hooks would queue up on one address (1200x1200 road grid with a third of its edges
+// missing: 343 us for a run, 477 with a hook per lane). For the first neighbours
+// alone: the lanes wait for one another, and second neighbours of a lattice form a
+// chain through the warp (3000x3000 lattice: 1.24 ms, 1.57 with them by warps too).
 MG_DEVINL bool cc_unite_warp(int32_t *parent, int32_t a, int32_t b, bool pending, unsigned long long limit) {
   const int lane = lane_id();
   for (unsigned long long it = 0; it < limit; ++it) {
@@ -113,13 +116,23 @@ MG_DEVINL bool cc_unite_warp(int32_t *parent, int32_t a, int32_t b, bool pending
 constexpr int kCcSample = 2;    // neighbours linked per vertex before the large component is picked
 constexpr int kCcProbe = 1024;  // sample vertices voting for the large component (one CTA)
 
+// One vertex in 2^kCcBreak, spread by a multiplicative hash, stays a root in step 1 and
+// links its first neighbour in step 2: on a lattice or a path every first neighbour is
+// the one before, and the trees of step 1 were chains as long as it (1200x1200 road grid
+// with 2 % of the edges dropped 523 -> 355 us, 3000x3000 1.88 -> 1.11 ms, a path of 4 M
+// vertices 7.5 -> 0.63 ms; 316 us, 1.13 and 0.67 ms with one vertex in four). A lattice
+// with no edge missing still prefers two rounds of links with a flattening between them
+// (1200x1200 0.21 against 0.43 ms); road grids lose by those (464 and 355 us at 2 %).
+constexpr int kCcBreak = 3;
+MG_DEVINL bool cc_breaks(int32_t v) { return ((uint32_t)v * 0x9E3779B1u) >> (32 - kCcBreak) == 0u; }
+
 // Step 1: parent[v] = min(v, first neighbour).
 __global__ void __launch_bounds__(kNT) k_cc_start(const int32_t *ro, const int32_t *col, int32_t *parent, int32_t V,
                                                   Ctl *ctl) {
   unsigned long long my_bytes = 0;
   for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x) {
     const int b = ro[v], e = ro[v + 1];
-    parent[v] = b < e ? min(v, col[b]) : v;
+    parent[v] = b < e && !cc_breaks(v) ? min(v, col[b]) : v;
     my_bytes += b < e ? 16 : 12;  // two offsets, the neighbour id, the parent
   }
   add_bytes(ctl, KID_CC, my_bytes);
@@ -137,9 +150,10 @@ __global__ void __launch_bounds__(kNT) k_cc_sample(const int32_t *ro, const int3
     const int v = (int)v0 + lane_id();
     const int b = v < V ? ro[v] : 0, e = v < V ? ro[v + 1] : 0;
     const int u0 = b < e ? col[b] : -1, u1 = b + 1 < e ? col[b + 1] : -1;
-    my_bytes += 8 + (u0 > v ? 12 : b < e ? 4 : 0) + (u1 >= 0 ? 12 : 0);  // offsets; neighbour ids, parents read
-    ok &= cc_unite_warp(parent, v, u0, u0 > v, limit);
-    ok &= cc_unite_warp(parent, v, u1, u1 >= 0, limit);
+    const bool own0 = u0 > v || (u0 >= 0 && cc_breaks(v));  // step 1 left v a root
+    my_bytes += 8 + (own0 ? 12 : b < e ? 4 : 0) + (u1 >= 0 ? 12 : 0);  // offsets; neighbour ids, parents read
+    ok &= cc_unite_warp(parent, v, u0, own0, limit);
+    if (u1 >= 0) ok &= cc_unite(parent, v, u1, limit);
   }
   if (!ok) raise_error(ctl, MG_ERR_TIMEOUT);
   add_bytes(ctl, KID_CC, my_bytes);

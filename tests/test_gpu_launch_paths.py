@@ -512,3 +512,29 @@ def test_cc_hub_beside_a_lattice(leaves, by_bfs):
     finally:
         _lib.lib.mg_selftest_loops(_lib.MG_LOOP_TEST_OFF)
     assert np.array_equal(g.cc()[0], ref)
+
+
+@pytest.mark.parametrize("kind", ["path", "reversed path", "lattice", "combs", "two lattices"])
+def test_cc_long_chains(kind):
+    # graphs whose first neighbours chain up; ids in order, reversed and shuffled
+    n = 1 << 15
+    if kind.endswith("path"):
+        a, b = np.arange(n - 1), np.arange(1, n)
+    else:
+        ids = np.arange(n).reshape(256, 128)
+        a, b = ids[:-1].ravel(), ids[1:].ravel()
+        rows = ids if kind == "lattice" else ids[:1] if kind == "combs" else np.concatenate([ids[:100], ids[101:]])
+        a, b = np.concatenate([a, rows[:, :-1].ravel()]), np.concatenate([b, rows[:, 1:].ravel()])
+        if kind == "two lattices":
+            keep = (a // 128 != 100) & (b // 128 != 100)
+            a, b = a[keep], b[keep]
+    if kind == "reversed path":
+        a, b = n - 1 - a, n - 1 - b
+    for perm in (np.arange(n), np.random.default_rng(2).permutation(n)):
+        src, dst = np.concatenate([perm[a], perm[b]]), np.concatenate([perm[b], perm[a]])
+        order = np.lexsort((dst, src))
+        ro = np.concatenate([[0], np.cumsum(np.bincount(src, minlength=n))]).astype(np.int32)
+        g = Graph(HostGraph(ro, dst[order].astype(np.int32)))
+        ref = oracle.cc(ro, dst[order].astype(np.int32))
+        for _ in range(3):
+            assert np.array_equal(g.cc()[0], ref)
