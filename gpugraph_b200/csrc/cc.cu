@@ -28,7 +28,9 @@
 // reached starts under its smallest id, every other vertex links all its edges
 // as in step 4. Any connected set serves, so the cap on the levels keeps long
 // paths out of the BFS without changing a label. R-MAT 21: 0.68 -> 0.20 ms,
-// R-MAT 22: 1.61 -> 0.31 ms.
+// R-MAT 22: 1.61 -> 0.31 ms. Where the first run of a graph finds that the BFS reaches
+// fewer than kCcReach of the edges (several large components: 8 R-MAT graphs of scale 10
+// to 16 in one took 1.06 ms by it, 0.31 without), the graph keeps to the sampling.
 #include <cuda_runtime.h>
 
 #include <climits>
@@ -277,6 +279,10 @@ __global__ void __launch_bounds__(kNT) k_cc_seed(const int32_t *depth, int32_t V
 // vertex, with / without the BFS: 175 / 306, 167 / 483 us.)
 constexpr double kCcLongShare = 0.1;
 constexpr uint32_t kCcLevels = 16;
+// Share of the edges whose tails the BFS must reach: two R-MAT graphs of scales 10 and 11
+// side by side (it reaches two thirds) 250 us, 145 by sampling. In one R-MAT graph it
+// reaches all but a few edges.
+constexpr double kCcReach = 0.8;
 
 // Union-find CC on a symmetric graph (called by mg_cc).
 int cc_union_find(mg_graph *g, int32_t *labels, mg_stats *stats, const mg_options *o) {
@@ -289,7 +295,7 @@ int cc_union_find(mg_graph *g, int32_t *labels, mg_stats *stats, const mg_option
   Ctl *ctl = g->ws.ctl;
   bool by_bfs = g->hub >= 0 && o->use_cuda_graph && !prof_on() && o->spin_limit >= kSpinLimitDefault &&
                 g->hub_degree <= kLoopPullList &&
-                (double)g->long_list_edges > kCcLongShare * (double)g->edges;
+                g->cc_by_bfs != 0 && (double)g->long_list_edges > kCcLongShare * (double)g->edges;
   std::optional<LoopRun> run;
   if (by_bfs) run.emplace(g, s);
   cudaError_t e = cudaEventRecord(g->ev0, s);
@@ -307,6 +313,12 @@ int cc_union_find(mg_graph *g, int32_t *labels, mg_stats *stats, const mg_option
     st = bfs_loop_run(*run, g, s, {g->hub}, kCcLevels, &bo, depth, false);
     if (st != MG_OK && st != kLoopRefused) return st;
     by_bfs = st == MG_OK;
+    if (by_bfs && g->cc_by_bfs < 0) {
+      // the graph's first run: later ones queue the rest without waiting here
+      if ((st = run->finish(cudaSuccess, "cc")) != MG_OK) return st;
+      by_bfs = (double)g->loop_out->visited_edges >= kCcReach * (double)g->edges;
+      g->cc_by_bfs = by_bfs ? 1 : 0;
+    }
   }
   if (by_bfs) {
     k_fill_i32<<<1, 32, 0, s>>>(giant, INT_MAX, 1);

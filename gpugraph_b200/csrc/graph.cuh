@@ -100,6 +100,7 @@ struct mg_graph {
   mg::DevCsr csr;
   int32_t hub = -1, hub_degree = 0;    // the vertex with the longest in-list
   int64_t long_list_edges = 0;         // edges in in-lists over kLongList times the mean
+  int cc_by_bfs = -1;                  // CC's route: whether the BFS from the hub reaches kCcReach of the edges, -1: not tried
   std::vector<int64_t> graph_offsets;  // batch of graphs: first vertex of each graph
   mg::Workspace ws;
   float *inv_outdeg = nullptr;          // PageRank 1/outdeg (0 for dangling vertices)

@@ -488,13 +488,15 @@ def test_ppr_infinite_weight_in_padded_rows(nvec, mode):
     assert np.array_equal(got[0][3], got[1][3], equal_nan=True)
 
 
-@pytest.mark.parametrize("leaves,by_bfs", [(200, False), (40000, True)])
-def test_cc_hub_beside_a_lattice(leaves, by_bfs):
-    # a hub whose edges are few beside the lattice's says nothing about the large component (sampling rounds); one
-    # with a tenth of them is found by the BFS
+@pytest.mark.parametrize("kind,by_bfs", [("200 leaves", False), ("40000 leaves", False), ("wheel", True)])
+def test_cc_hub_beside_a_lattice(kind, by_bfs):
+    # a hub with few of the edges, or with many but not in the large component, says nothing about that (sampling
+    # rounds); one joined to every vertex finds it
     grid = HostGraph.road_grid(150, 0.3, 0.0, seed=5)
     n = grid.nodes
-    a, b = np.zeros(leaves, np.int64), n + np.arange(leaves)
+    leaves = 0 if kind == "wheel" else int(kind.split()[0])
+    b = 1 + np.arange(n - 1) if kind == "wheel" else n + np.arange(leaves)
+    a = np.zeros(b.size, np.int64)
     src = np.concatenate([np.repeat(np.arange(n), np.diff(grid.row_offsets)), a, b])
     dst = np.concatenate([grid.column_indices, b, a])
     order = np.lexsort((dst, src))
@@ -538,3 +540,31 @@ def test_cc_long_chains(kind):
         ref = oracle.cc(ro, dst[order].astype(np.int32))
         for _ in range(3):
             assert np.array_equal(g.cc()[0], ref)
+
+
+@pytest.mark.parametrize("parts", [1, 2, 3, 9])
+def test_cc_route_follows_what_the_bfs_reached(parts):
+    # equal R-MAT graphs side by side: the hub's one holds 1/parts of the edges
+    one = HostGraph.rmat(11, 16, seed=4)
+    n, m = one.nodes, one.edges
+    ro = np.concatenate([[0], (one.row_offsets[1:] + m * np.arange(parts)[:, None]).ravel()]).astype(np.int32)
+    col = (one.column_indices + n * np.arange(parts)[:, None]).ravel().astype(np.int32)
+    sub, reached = oracle.cc(one.row_offsets, one.column_indices), oracle.bfs(
+        one.row_offsets, one.column_indices, one.max_degree_vertex())
+    share = one.out_degree()[reached >= 0].sum() / (parts * m)
+    by_bfs = share >= 0.8
+    assert by_bfs == (parts == 1)
+    ref = (sub + n * np.arange(parts)[:, None]).ravel()
+    g = Graph(HostGraph(ro, col))
+    for _ in range(3):
+        assert np.array_equal(g.cc()[0], ref)
+    _lib.lib.mg_selftest_loops(_lib.MG_LOOP_TEST_WAITS)
+    try:
+        if by_bfs:
+            with pytest.raises(MapGraphError):
+                g.cc()
+        else:
+            assert np.array_equal(g.cc()[0], ref)
+    finally:
+        _lib.lib.mg_selftest_loops(_lib.MG_LOOP_TEST_OFF)
+    assert np.array_equal(g.cc()[0], ref)
