@@ -3,7 +3,8 @@
 // while its distance is smaller. A step selects the waiting vertices below the
 // window's end (the smallest waiting distance plus `delta`), turns them into edge
 // ranges, and relaxes the ranges: an improving candidate lowers the head's
-// distance without waiting for the result, and that is all an edge writes. With
+// distance without waiting for the result, and that is all an edge writes (on large
+// graphs a flag as well, kSpWide). With
 // non-negative weights the smallest waiting distance is final, so every step
 // settles a vertex and V steps suffice; the fixpoint is the one of the
 // level-by-level loop (sssp.cu), the unique shortest distances.
@@ -35,10 +36,21 @@ constexpr int kSpVerts = 8;    // vertices per lane and step of the selection (R
 // at 2, 1.38 at 4, 1.44 at 8, 1.52 at 32 (no window in effect).
 constexpr double kSsspWindow = 4.0;
 
+constexpr uint32_t kSpBlock = 32 * kSpVerts;  // vertices a warp step selects from
+// Vertices from which the selection looks only into blocks in which one may wait, by a
+// flag per block that an improving edge sets (WIDE): the two arrays it reads (8 bytes a
+// vertex) are larger than L2 then, and every step read them whole. With the flags /
+// without / level by level: R-MAT 24 with a path of 2000 vertices attached 20.8 / 58.3 /
+// 35.4 ms, 6000x6000 lattice, weights 1..1000, 162 / 716 / 1131, with shortcuts and
+// weights 1 7.6 / 8.9 / 7.5, R-MAT 24, weights 1..64, 7.1 / 7.3 / 11.7. With 9 M vertices
+// (3000x3000, weights 1) the flags still lose, 2.4 / 2.1 ms.
+constexpr int64_t kSpWide = 3ll << 22;
+
 struct SsspLoopArgs {
   DevCsr g;
   int32_t *dist;
   int32_t *done;
+  uint8_t *open;  // per block of kSpBlock vertices: one of them may wait (WIDE)
   int4 *q;       // (first edge, length, distance of the tail, unused)
   uint32_t cap;  // entries of q
   int32_t src, delta;
@@ -46,6 +58,7 @@ struct SsspLoopArgs {
   GridLoop loop;
 };
 
+template <bool WIDE>
 __global__ void __launch_bounds__(kLoopNT, 1) k_sssp_loop(SsspLoopArgs a) {
   constexpr int32_t INF = programs::sssp::INIT_VALUE;
   __shared__ LoopShared sh;
@@ -66,6 +79,8 @@ __global__ void __launch_bounds__(kLoopNT, 1) k_sssp_loop(SsspLoopArgs a) {
     a.dist[i] = i == (uint32_t)a.src ? 0 : INF;
     a.done[i] = INF;
   }
+  if (WIDE)
+    for (uint32_t i = tid; i < (V + kSpBlock - 1) / kSpBlock; i += nt) a.open[i] = i == (uint32_t)a.src / kSpBlock;
   if (blockIdx.x == 0 && threadIdx.x < 3) {
     c->count[threadIdx.x] = c->edges[threadIdx.x] = 0;
     c->items[threadIdx.x] = 0;
@@ -83,10 +98,12 @@ __global__ void __launch_bounds__(kLoopNT, 1) k_sssp_loop(SsspLoopArgs a) {
     }
     const int end = (int)min((long long)INT_MAX - 1, (long long)low + a.delta);
     int rest = INT_MAX;  // smallest waiting distance past the window
-    // selection: 32 * kSpVerts vertices per warp step (two coalesced streams)
-    for (uint32_t v0 = gw * 32 * kSpVerts; v0 < V; v0 += nw * 32 * kSpVerts) {
+    // selection from the block at v0: 32 * kSpVerts vertices (two coalesced streams);
+    // whether one is left waiting
+    auto select = [&](uint32_t v0) {
       int d[kSpVerts], n[kSpVerts], b[kSpVerts];
       uint32_t sel = 0;  // bit k: the lane's k-th vertex is selected
+      bool left = false;
 #pragma unroll
       for (int k = 0; k < kSpVerts; ++k) {
         const uint32_t v = v0 + 32 * k + lane;
@@ -97,9 +114,9 @@ __global__ void __launch_bounds__(kLoopNT, 1) k_sssp_loop(SsspLoopArgs a) {
       for (int k = 0; k < kSpVerts; ++k)
         if (d[k] < n[k]) {
           if (d[k] < end) sel |= 1u << k;
-          else rest = min(rest, d[k]);
+          else rest = min(rest, d[k]), left = true;
         }
-      if (!__any_sync(0xffffffffu, sel != 0u)) continue;
+      if (!__any_sync(0xffffffffu, sel != 0u)) return left;
 #pragma unroll
       for (int k = 0; k < kSpVerts; ++k) {
         const uint32_t v = v0 + 32 * k + lane;
@@ -127,6 +144,22 @@ __global__ void __launch_bounds__(kLoopNT, 1) k_sssp_loop(SsspLoopArgs a) {
         for (int k = 0; k < kSpVerts; ++k)
           for (int i = 0; i < n[k]; i += kRange)
             a.q[at++] = make_int4(b[k] + i, min(kRange, n[k] - i), d[k], 0);
+      }
+      return left;
+    };
+    if (!WIDE) {
+      for (uint32_t v0 = gw * kSpBlock; v0 < V; v0 += nw * kSpBlock) select(v0);
+    } else {
+      // the flags of 32 of the warp's blocks at a time
+      const uint32_t blocks = (V + kSpBlock - 1) / kSpBlock;
+      for (uint32_t b0 = gw; b0 < blocks; b0 += nw * 32) {
+        const uint32_t mine = b0 + lane * nw;
+        const bool waits = mine < blocks && __ldcg(&a.open[mine]);
+        for (uint32_t todo = __ballot_sync(0xffffffffu, waits); todo; todo &= todo - 1) {
+          const uint32_t blk = b0 + (__ffs(todo) - 1) * nw;
+          const bool left = __any_sync(0xffffffffu, select(blk * kSpBlock));
+          if (lane == 0 && !left) a.open[blk] = 0;
+        }
       }
     }
     rest = __reduce_min_sync(0xffffffffu, rest);
@@ -168,6 +201,7 @@ __global__ void __launch_bounds__(kLoopNT, 1) k_sssp_loop(SsspLoopArgs a) {
         for (int k = 0; k < kSpU; ++k)
           if (cand[k] < dv[k]) {
             atomicMin(&a.dist[u[k]], cand[k]);
+            if (WIDE) a.open[(uint32_t)u[k] / kSpBlock] = 1;
             best = min(best, cand[k]);
           }
       }
@@ -199,6 +233,7 @@ int sssp_loop_run(LoopRun &run, mg_graph *g, int32_t src, const mg_options *o, i
   a.g = g->csr;
   a.dist = dist;
   a.done = g->ws.vbuf[1];
+  a.open = reinterpret_cast<uint8_t *>(g->ws.queue[0]);  // (a level loop's queue, free here)
   // the room of the two BFS queues: a step selects every vertex at most once
   static_assert(sizeof(int4) == 2 * sizeof(int2), "one queue of the same number of entries");
   a.q = reinterpret_cast<int4 *>(g->loop_queue);
@@ -209,7 +244,8 @@ int sssp_loop_run(LoopRun &run, mg_graph *g, int32_t src, const mg_options *o, i
   a.max_iter = (uint32_t)(g->nodes + 2);
   a.loop = run.args(o);
   void *args[] = {&a};
-  return run.launch((const void *)k_sssp_loop, args, timed, "sssp loop launch");
+  const void *kernel = g->nodes >= kSpWide ? (const void *)k_sssp_loop<true> : (const void *)k_sssp_loop<false>;
+  return run.launch(kernel, args, timed, "sssp loop launch");
 }
 
 }  // namespace mg

@@ -568,3 +568,23 @@ def test_cc_route_follows_what_the_bfs_reached(parts):
     finally:
         _lib.lib.mg_selftest_loops(_lib.MG_LOOP_TEST_OFF)
     assert np.array_equal(g.cc()[0], ref)
+
+
+@pytest.mark.parametrize("n", [(3 << 22) - 1, 3 << 22, (3 << 22) + 77])
+@pytest.mark.parametrize("hi,graph", [(1, "rmat"), (1000, "rmat"), (64, "road"), (1000, "road")])
+def test_sssp_sparse_ids_in_a_wide_graph(n, hi, graph):
+    # a graph spread over n ids: from 3 * 2^22 on the selection looks only into the 256-vertex blocks where one may wait
+    small = (HostGraph.rmat(12, 8, seed=7) if graph == "rmat" else HostGraph.road_grid(70, 0.05, 0.0, seed=7))
+    small = small.with_weights(1, hi, seed=3)
+    ids = np.sort(np.random.default_rng(5).choice(n, small.nodes, replace=False))
+    ids[-1] = n - 1
+    deg = np.zeros(n, np.int64)
+    deg[ids] = small.out_degree()
+    ro = np.concatenate([[0], np.cumsum(deg)]).astype(np.int32)
+    g = Graph(HostGraph(ro, ids[small.column_indices].astype(np.int32), small.edge_values))
+    for s in (small.max_degree_vertex(), small.nodes - 1):
+        ref = np.full(n, 100000000, np.int32)
+        ref[ids] = oracle.sssp(small.row_offsets, small.column_indices, small.edge_values, s)
+        for _ in range(2):
+            out, st = g.sssp(int(ids[s]))
+            assert np.array_equal(out, ref) and st["converged"] == 1
