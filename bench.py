@@ -164,11 +164,20 @@ def profiled(fn, peak: float) -> tuple[dict, dict]:
     """One run of fn with per-kernel profiling on: the level loops run host-driven,
     every launch is bracketed by CUDA events on its stream, and the kernels count
     their algorithmic bytes on the device. Returns the run's roofline summary (all
-    kernels, and the kernel kind with the most time) and the raw profile."""
+    kernels, and the kernel kind with the most time) and the raw profile.
+
+    Calls that run in one cooperative launch by themselves ("call_launches" of 1 or 2)
+    go level by level under the profiler: their summary is that of those kernels ("loop"),
+    not of the timed call."""
     import torch
 
     from gpugraph_b200 import _lib
 
+    torch.cuda.synchronize()
+    _lib.lib.mg_kernel_launches(1)
+    fn()
+    torch.cuda.synchronize()
+    launches = int(_lib.lib.mg_kernel_launches(1))
     _lib.lib.mg_profile_enable(1)
     try:
         fn()
@@ -178,7 +187,7 @@ def profiled(fn, peak: float) -> tuple[dict, dict]:
         _lib.lib.mg_profile_enable(0)
     ms = sum(v[0] for v in prof.values())
     byts = sum(v[2] for v in prof.values())
-    out = {"algorithmic_GB": byts / 1e9, "kernel_ms": ms,
+    out = {"loop": "level by level", "call_launches": launches, "algorithmic_GB": byts / 1e9, "kernel_ms": ms,
            "achieved_GBps": byts / (ms * 1e-3) / 1e9 if ms else None,
            "frac": byts / (ms * 1e-3) / 1e9 / peak if ms else None}
     kernels = {k: v for k, v in prof.items() if k != "other"}

@@ -13,10 +13,11 @@
 // does, so push levels keep no bitmap.
 //
 // Bound by the round trips of a level (ranges, columns, test-and-sets, the
-// reservation, the barrier: under 7 us a level) on small frontiers, by the
-// bottom-up sweeps' loads on large ones. Against the level-by-level loop, per
-// run: R-MAT 16 with host output 215 -> 91 us, R-MAT 21 234 -> 97 us,
-// 1200x1200 road grid (67 levels) 1542 -> 458 us, 256 small graphs 309 -> 155 us.
+// reservation, the barrier: 4 us a level on a path, 7 on a road grid) on small
+// frontiers, by the bottom-up sweeps' loads on large ones. Against the
+// level-by-level loop, per call: R-MAT 16 with host output 210 -> 91 us, R-MAT 21
+// 230 -> 103 us, 1200x1200 road grid (67 levels) 1513 -> 460 us, 256 small graphs
+// 295 -> 150 us.
 #include <cuda_runtime.h>
 
 #include <vector>

@@ -162,7 +162,9 @@ __global__ void __launch_bounds__(kNT) k_cc_sample(const int32_t *ro, const int3
 }
 
 // Step 3: the root held by most of kCcProbe fixed sample vertices (ties: the
-// smaller root); parent[] is flat here. Written to *giant.
+// smaller root). Written to *giant. Where parent[] is not quite flat (k_cc_flatten) it
+// may be an inner vertex of the large tree; that serves as well, since all step 4 needs
+// is that the vertices it skips hang under one and the same vertex.
 __global__ void __launch_bounds__(kCcProbe) k_cc_giant(const int32_t *parent, int32_t V, int32_t *giant) {
   __shared__ int32_t s_lab[kCcProbe];
   __shared__ unsigned long long s_best[kCcProbe / 32];

@@ -8,7 +8,6 @@
 #include <algorithm>
 #include <atomic>
 #include <cstring>
-#include <mutex>
 #include <vector>
 
 #include "graph.cuh"
@@ -128,25 +127,26 @@ using namespace mg;
 namespace {
 
 // The vertex with the longest in-list (the first of them) and its length, and the
-// edges in lists of more than kLongList times the mean.
+// edges in lists of more than kLongList times the mean. (By one thread: starting the
+// others took 2 ms of an 11 ms creation at R-MAT 16, the pass takes less than 0.1 there.)
 void find_hub(mg_graph *g, const int32_t *in_off) {
-  const double lim = kLongList * std::max(1.0, (double)g->edges / (double)std::max<int64_t>(g->nodes, 1));
-  std::mutex m;
-  host_parallel_for(g->nodes, [&](int64_t b, int64_t e, unsigned) {
-    int64_t hub = b, in_long = 0;
-    auto len = [&](int64_t v) { return in_off[v + 1] - in_off[v]; };
-    for (int64_t v = b; v < e; ++v) {
-      if (len(v) > len(hub)) hub = v;
-      if ((double)len(v) > lim) in_long += len(v);
+  const int64_t V = g->nodes;
+  const double lim = kLongList * std::max(1.0, (double)g->edges / (double)std::max<int64_t>(V, 1));
+  const int32_t longer = (int32_t)std::min(lim, (double)INT32_MAX);
+  int64_t in_long = 0, hub = -1;
+  int32_t most = -1;
+  for (int64_t v = 0; v < V; ++v) {
+    const int32_t len = in_off[v + 1] - in_off[v];
+    if (len <= longer && len <= most) continue;
+    if (len > longer) in_long += len;
+    if (len > most) {
+      most = len;
+      hub = v;
     }
-    if (b >= e) return;
-    std::lock_guard<std::mutex> lock(m);
-    g->long_list_edges += in_long;
-    if (g->hub < 0 || len(hub) > g->hub_degree || (len(hub) == g->hub_degree && hub < g->hub)) {
-      g->hub = (int32_t)hub;
-      g->hub_degree = len(hub);
-    }
-  });
+  }
+  g->hub = (int32_t)hub;
+  g->hub_degree = std::max(most, 0);
+  g->long_list_edges = in_long;
 }
 
 // Copy of the in-lists with every list ordered by descending out-degree of the

@@ -1,7 +1,8 @@
 // Whole traversals in one cooperative launch: a grid barrier with a bounded
 // wait, the per-level totals that travel with it, and the result block the host
 // reads. Used where a level's work is short beside the launches of a
-// level-by-level loop (12-25 us a level on a B200, against 5-6 us here).
+// level-by-level loop (12-25 us a level on a B200, against 4 us here on a path graph
+// and 7 on a road grid).
 //
 // The launch is cooperative (cudaLaunchCooperativeKernel), so every CTA is
 // resident and a barrier only waits for CTAs that run. A wait still ends after

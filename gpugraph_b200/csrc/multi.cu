@@ -54,12 +54,12 @@ constexpr int kMVT = 8;
 // level's edges.
 constexpr int kMSVT = 4;
 // Edges whose row loads a warp has in flight, two side by side (R-MAT 20, 37
-// sources / road 1200, 64 sources: 3.9 / 18.4 ms with 8, 4.6 / 19.4 with 16).
+// sources: 3.9 ms with 8, 4.6 with 16).
 constexpr int kMssEdges = 8;
 // Active sources per edge up to which a lane relaxes a whole edge alone: below,
 // the row accesses of a half warp's edge carry mostly inactive entries, above, the
-// lane's scalar loads touch a sector per source (the same two runs: 4.0 / 19.6 ms
-// at 4, 3.9 / 18.4 at 8, 4.1 / 18.3 at 12, 5.0 / 19.3 at 20).
+// lane's scalar loads touch a sector per source (the same run: 4.0 ms at 4, 3.9 at
+// 8, 4.1 at 12, 5.0 at 20).
 constexpr int kMssSparse = 8;
 // Without edge bounds every edge is relaxed by its lane, from registers (the row
 // path's shared memory comes out of L1), unless there are more sources than this and
@@ -1512,7 +1512,10 @@ MG_DEVINL uint32_t mss_edges(const Ctl *ctl) { return (uint32_t)ctl->next_edges;
 // kMssSkew times the mean. A stored hi stays valid while distances fall; it is redone
 // for the queued vertices (the improved ones) each level and for every vertex
 // when a c_s changed (3-4 times a run). At R-MAT 20 with 37 sources the bytes of
-// the expand fell from 21 to 6.8 GB and the run from 6.2 to 5.1 ms.
+// the expand fell from 21 to 6.8 GB and the run from 6.2 to 5.1 ms. They start once every
+// source reached the hub: one that never does (in a component of its own) keeps them off
+// for the batch, 6.2 against 3.8 ms at R-MAT 20 with 37 sources (7.6 before there were
+// bounds).
 struct MssBounds {
   int32_t *lo, *hi;   // [V]; lo is set for the queued vertices
   // c_s of every source, then [64] = 1 once all of them reached the hub,
@@ -1615,7 +1618,8 @@ MG_DEVINL void relax_min(int32_t *p, int32_t c, u64 &imp, int t) {
 // and more warps, or more edges and fewer warps, were slower (48 registers and
 // 5 CTAs per SM: 5.8 ms at R-MAT 20; 3 CTAs: 5.2 ms, against 4.3). Before, with
 // a 32-byte row piece per lane, 8 scattered reductions per step and a queue
-// reservation per 4 edges: 7.8 ms a run, 4.4 with a whole warp per edge, now 3.9.
+// reservation per 4 edges: 7.8 ms a run, 4.4 with a whole warp per edge, now 3.8 to
+// 4.2, by the graph drawn.
 //
 // ROWS = false (see kMssLaneSources): every edge is relaxed by its lane at once.
 template <int VT, bool ROWS, bool GUARD>
