@@ -120,11 +120,12 @@ constexpr int kCcProbe = 1024;  // sample vertices voting for the large componen
 
 // One vertex in 2^kCcBreak, spread by a multiplicative hash, stays a root in step 1 and
 // links its first neighbour in step 2: on a lattice or a path every first neighbour is
-// the one before, and the trees of step 1 were chains as long as it (1200x1200 road grid
-// with 2 % of the edges dropped 523 -> 355 us, 3000x3000 1.88 -> 1.11 ms, a path of 4 M
-// vertices 7.5 -> 0.63 ms; 316 us, 1.13 and 0.67 ms with one vertex in four). A lattice
-// with no edge missing still prefers two rounds of links with a flattening between them
-// (1200x1200 0.21 against 0.43 ms); road grids lose by those (464 and 355 us at 2 %).
+// the one before, and the trees of step 1 were chains as long as it (road grids with 2 %
+// of the edges dropped: 1000x1000 386 -> 293 us, 1200x1200 604 -> 480, 3000x3000 1.88 ->
+// 1.11 ms, 1.13 with one vertex in four; a path of 4 M vertices 7.5 -> 0.63 ms). Two
+// rounds of links with a flattening between them take 395 us, 464 us and 1.16 ms on those
+// grids, 0.21 against 0.38 ms on a 1200x1200 lattice with no edge missing, and 450 against
+// 335 us on a 1200x1200 grid with 35 % missing.
 constexpr int kCcBreak = 3;
 MG_DEVINL bool cc_breaks(int32_t v) { return ((uint32_t)v * 0x9E3779B1u) >> (32 - kCcBreak) == 0u; }
 
@@ -276,13 +277,14 @@ __global__ void __launch_bounds__(kNT) k_cc_seed(const int32_t *depth, int32_t V
 // Share of the edges in long lists (kLongList) from which the BFS finds the large
 // component: R-MAT graphs have 0.15 (scale 10) to 0.65, and the hub is in their large
 // component. A hub alone says nothing about the rest: from a vertex of 200 leaves beside
-// a 4000x4000 lattice 16 levels reach little, and the rest's hooks without the sampling
-// took 1.64 ms a run, 1.09 with it. (Sparse R-MAT 21 graphs, one or two edges drawn a
-// vertex, with / without the BFS: 175 / 306, 167 / 483 us.)
+// a road grid with 2 % of the edges dropped 16 levels reach little, and the BFS and the
+// other edges' hooks take 445 us (1200x1200) and 1.32 ms (3000x3000), the sampling 375 us
+// and 1.14 ms. (Sparse R-MAT 21 graphs, one or two edges drawn a vertex, with / without
+// the BFS: 175 / 306, 167 / 483 us.)
 constexpr double kCcLongShare = 0.1;
 constexpr uint32_t kCcLevels = 16;
 // Share of the edges whose tails the BFS must reach: two R-MAT graphs of scales 10 and 11
-// side by side (it reaches two thirds) 250 us, 145 by sampling. In one R-MAT graph it
+// side by side (it reaches two thirds) 250 us, 137 by sampling. In one R-MAT graph it
 // reaches all but a few edges.
 constexpr double kCcReach = 0.8;
 
