@@ -21,10 +21,11 @@ namespace mg {
 constexpr int kLoopNT = 1024;  // one CTA per SM: the fewest arrivals a barrier can have
 constexpr int kRange = 256;    // edges per entry of a queue of edge ranges
 // In-edges of a vertex up to which k_bfs_loop may pull it: one lane walks the list, four
-// edges per two dependent loads (about 1.2 us), while every other CTA polls at the
-// barrier, 2^22 times (2 to 3 s) by default. 2^20 edges take 0.3 s. Longer lists are left
-// to the level loop, whose kernels have no time limit.
-constexpr int32_t kLoopPullList = 1 << 20;
+// edges a step, while every other CTA polls at the barrier, 2^22 times (2 to 3 s) by
+// default. A list of 2^20 edges walked to its end takes 49 ms (58 in the level loop), so
+// one of 2^22 a tenth of the limit. Longer ones are left to the level loop, whose kernels
+// have no time limit.
+constexpr int32_t kLoopPullList = 1 << 22;
 
 // Device state of a loop. `arrived` grows for the life of the graph (a run
 // starts from the value the host passes in); the totals rotate over three

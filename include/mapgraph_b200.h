@@ -58,8 +58,9 @@ typedef struct mg_options {
   int32_t direction;         /* MG_DIR_* (BFS only) */
   double alpha;              /* push->pull when frontier edges > unvisited edges / alpha */
   double beta;               /* pull->push when frontier vertices < nodes / beta */
-  int32_t use_cuda_graph;    /* 1: loops driven by the device (one cooperative launch, or
-                                the level loop captured in a CUDA graph); 0: by the host */
+  int32_t use_cuda_graph;    /* 1: loops driven by the device (one cooperative launch, which
+                                waits until every SM has room, or the level loop captured
+                                in a CUDA graph); 0: by the host, level by level */
   int32_t threshold;         /* reference "threshold": frontier size above which the
                                 grid-cooperative expand is used (0: always) */
   double damping;            /* PageRank damping (0.85) */

@@ -437,15 +437,16 @@ def test_device_results_at_any_address(shift):
         assert np.abs(r - ppr(gd, w, tele, max_iter=opts.iter_num).cpu().numpy()).max() < 1e-7
 
 
-@pytest.mark.parametrize("leaves", [1 << 20, (1 << 20) + 1])
+@pytest.mark.parametrize("leaves", [1 << 22, (1 << 22) + 1])
 def test_bfs_in_list_too_long_for_a_barrier_wait(leaves):
-    # a lane walks a pulled list: past 2^20 edges pulling calls go level by level, pushing ones stay in one launch
+    # a lane walks a pulled list: past 2^22 edges pulling calls go level by level, pushing ones stay in one launch
     n = leaves + 1
     ro = np.concatenate([[0], leaves + np.arange(n)]).astype(np.int32)
     g = Graph(HostGraph(ro, np.concatenate([np.arange(1, n), np.zeros(leaves)]).astype(np.int32)))
     ref = np.full(n, 2, np.int32)
     ref[0], ref[1] = 1, 0
-    for d, one in ((_lib.MG_DIR_PUSH, True), (_lib.MG_DIR_PULL, leaves <= 1 << 20), (_lib.MG_DIR_AUTO, leaves <= 1 << 20)):
+    short = leaves <= 1 << 22
+    for d, one in ((_lib.MG_DIR_PUSH, True), (_lib.MG_DIR_PULL, short), (_lib.MG_DIR_AUTO, short)):
         g.bfs(1, direction=d)
         _lib.lib.mg_kernel_launches(1)
         out, _ = g.bfs(1, direction=d)
