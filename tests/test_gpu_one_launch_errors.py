@@ -68,7 +68,7 @@ def calls():
 
 
 @pytest.fixture(autouse=True)
-def test_mode_off():
+def loop_test_off():
     yield
     _lib.lib.mg_selftest_loops(_lib.MG_LOOP_TEST_OFF)
 
